@@ -37,6 +37,18 @@ class PlanInfo(C.Structure):
                 ("device", C.c_int)]
 
 
+class TrainStepArgs(C.Structure):
+    _fields_ = [("plan", vp), ("n", i64),
+                ("d_model", i32), ("n_heads", i32), ("n_layers", i32), ("d_ff", i32), ("vocab", i32), ("seq_len", i32),
+                ("params", vp), ("grads", vp),
+                ("tokens", vp), ("pos", vp), ("query_to_node", vp), ("query_offsets", vp), ("radix_ids", vp),
+                ("mass_weights", vp), ("trained", vp), ("unit_of_row", vp), ("n_units", i32), ("n_pos", i32),
+                ("edge_first", vp), ("counts_offset", vp), ("counts_tok", vp), ("counts_val", vp), ("cosv", vp), ("sinv", vp),
+                ("entropy_lambda", f32), ("intermediate_weight", f32),
+                ("ce_only", i32), ("bf16_store", i32), ("grad_mode", i32), ("ffn_recompute", i32),
+                ("loss_sum", vp), ("loss_count", vp), ("tail", vp)]
+
+
 # name -> (restype, argtypes); every symbol include/agpt_b200.h declares
 SIGNATURES = {
     "agpt_b200_last_error": (C.c_char_p, []),
@@ -124,6 +136,9 @@ SIGNATURES = {
     "agpt_b200_static_scratch_bytes": (i64, []),
     "agpt_b200_loss_per_query": (C.c_int, [vp] * 11 + [i64, C.c_int, f32, f32, C.c_int, vp]),
     "agpt_b200_loss_per_node": (C.c_int, [vp] * 7 + [i64, C.c_int, vp]),
+    "agpt_b200_train_step_takes": (C.c_int, [C.c_int] * 4),
+    "agpt_b200_train_step_workspace_bytes": (i64, [C.POINTER(TrainStepArgs)]),
+    "agpt_b200_train_step": (C.c_int, [C.POINTER(TrainStepArgs), vp, i64, vp]),
     "agpt_b200_attn_fwd_bwd_host": (C.c_int, [vp] * 10 + [C.c_int, C.c_int, C.c_int, f32]),
 }
 

@@ -13,7 +13,7 @@ import os
 
 import numpy as np
 
-from ._lib import AgptError, GroupInfo, PlanInfo, TrieInfo, check, lib
+from ._lib import AgptError, GroupInfo, PlanInfo, TrainStepArgs, TrieInfo, check, lib  # noqa: F401
 
 KV_F32, KV_BF16 = 0, 1
 

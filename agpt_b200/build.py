@@ -11,7 +11,8 @@ SOURCES = [os.path.join(HERE, "csrc", "kernels.cu"), os.path.join(HERE, "csrc", 
            os.path.join(HERE, "csrc", "rowops.cu"), os.path.join(HERE, "csrc", "optim.cu"),
            os.path.join(HERE, "csrc", "gemm3x.cu"), os.path.join(HERE, "csrc", "gemm_sm100.cu"),
            os.path.join(HERE, "csrc", "host_trie.cpp"), os.path.join(HERE, "csrc", "trie_suffix.cpp"),
-           os.path.join(HERE, "csrc", "trie_gpu.cu")]
+           os.path.join(HERE, "csrc", "trie_gpu.cu"),
+           os.path.join(HERE, "csrc", "step_gemm.cu"), os.path.join(HERE, "csrc", "train_step.cu")]
 
 
 # The two GEMM translation units instantiate CUTLASS templates, and gemm_sm100.cu re-instantiates the SM100 fast-FP32
@@ -52,7 +53,7 @@ def cutlass_include():
     return None
 
 
-HEADERS = [os.path.join(HERE, "csrc", "internal.h"), os.path.join(HERE, "..", "include", "agpt_b200.h")]
+HEADERS = [os.path.join(HERE, "csrc", "internal.h"), os.path.join(HERE, "csrc", "step_gemm.h"), os.path.join(HERE, "csrc", "tc100.cuh"), os.path.join(HERE, "..", "include", "agpt_b200.h")]
 
 
 OBJ_DIR = os.path.join(HERE, "_build")

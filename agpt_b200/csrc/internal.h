@@ -65,6 +65,7 @@ struct agpt_plan {
 };
 
 int agpt_plan_upload(agpt_plan *p, int device);
+int agpt_step_gemm_status(int *out);       // status word of step_gemm.cu's kernels
 
 // tcgen05 float32 GEMM (gemm_sm100.cu): D[l] = act(alpha * op(A[l]) * op(B[l]) + beta * C + bias row), l < L batches
 bool agpt_gemm_sm100_takes(int trans_a, int trans_b, int relu, int has_source);

@@ -2575,7 +2575,9 @@ extern "C" int agpt_b200_device_status(int32_t *status_out) {
     if (!status_out) return agpt_set_error(AGPT_E_ARG, "device_status: null output");
     int v = 0;
     CUDA_TRY(cudaMemcpyFromSymbol(&v, g_device_status, sizeof(int)));      // synchronises with the work issued so far
-    *status_out = v;
+    int w = 0;
+    if (int rc = agpt_step_gemm_status(&w)) return rc;
+    *status_out = v | w;
     return AGPT_OK;
 }
 

@@ -42,7 +42,8 @@ class LaunchGroup:
         t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device)  # noqa: E731
         self.tokens = t(tokens.astype(np.int64))
         self.tokens32 = t(tokens.astype(np.int32))
-        self.pos = t(np.minimum(np.maximum(depth - 1, 0), seq_len - 1).astype(np.int32))
+        pos = np.minimum(np.maximum(depth - 1, 0), seq_len - 1).astype(np.int32)
+        self.pos, self.n_pos = t(pos), int(pos.max()) + 1 if self.n else 0
         starts = np.concatenate([[True], radix_of[1:] != radix_of[:-1]])
         if trained is not None:                      # a context row never shares a loss node with trained rows
             starts |= np.concatenate([[True], trained[1:] != trained[:-1]])
@@ -67,6 +68,14 @@ class LaunchGroup:
         self.trained = None if trained is None else t(trained.astype(np.float32))
         self.mass_w = None if mw is None else t(mw)
         self.n_trained_rows = self.n if trained is None else int(trained.sum())
+
+    def step_args(self):
+        """The group's part of the native step's arguments (the model fills in the rest)."""
+        ptr = lambda x: None if x is None else x.data_ptr()  # noqa: E731
+        a = A.TrainStepArgs(plan=self.plan._h, n=self.n, n_units=self.n_units, n_pos=self.n_pos)
+        a.tokens, a.pos, a.query_to_node, a.query_offsets, a.radix_ids = [ptr(x) for x in (self.tokens32, self.pos, self.q2n, self.qoff, self.rid)]
+        a.mass_weights, a.trained, a.unit_of_row, a.edge_first = [ptr(x) for x in (self.mass_w, self.trained, self.unit_of_row, self.edge_first)]
+        return a
 
 
 def build_groups(trie: A.RadixTrie, rank: int, world: int, group_rows: int, mass_mode: str, seq_len: int, device,
@@ -279,6 +288,7 @@ class TrieWalkModel:
             p.copy_(torch.from_numpy(np.ascontiguousarray(a)))
             self.params[name] = p.requires_grad_(True)
         self._offs = offs
+        self._step_ptrs = None           # pointer arrays of the native step, rebuilt when a gradient buffer is replaced
         self.bind_grads()
         hd = model.d_model // model.n_heads
         cos, sin = A.rope_table(model.seq_len, hd)
@@ -289,7 +299,7 @@ class TrieWalkModel:
         self.linear = _linear_function()
         self.norm_skip = _norm_skip_function()
         self.qkv = _qkv_function()
-        self.dense_impl = "tensor"       # "tensor": the library's 3xTF32 GEMM; "torch": torch.addmm (cuBLAS float32)
+        self.dense_impl = "tensor"       # "tensor": the library's kernels; "torch": torch.addmm (cuBLAS float32)
         self.ffn_recompute = False       # True: recompute the d_ff-wide activations in the backward instead of keeping them
         # which attention pairs feed dK/dV: "full" (persistent accumulators, src/agpt/incremental_backward.cr), "local_depth"
         # (the Crystal walker, src/agpt/trie_walk_trainer.cr:189) or "own_edge" (the CUDA trainer, src/cuda/agpt_train.cu:5016-5020)
@@ -370,6 +380,9 @@ class TrieWalkModel:
         float32 device tensor (loss sum, count // 4096, count % 4096), so that the host does not wait for the device
         between groups."""
         import torch
+        m = self.cfg
+        if self.dense_impl == "tensor" and A.lib().agpt_b200_train_step_takes(m.d_model, m.n_heads, m.d_ff, m.vocab):
+            return self._native_step(group, counts, entropy_lambda, intermediate_weight, ce_only, bf16_store, sync)
         logits = self.logits(group, bf16_store).contiguous()
         c_off, c_tok, c_val = counts
         if logits.shape[1] != self.cfg.vocab:
@@ -397,6 +410,45 @@ class TrieWalkModel:
             return float(loss_sum.item()), int(n_trained.item())
         # the count rides in float32 next to the gradients: split so that sums over groups and ranks stay exact
         return torch.stack([loss_sum.to(torch.float32), (n_trained // 4096).to(torch.float32), (n_trained % 4096).to(torch.float32)])
+
+
+    def _native_step(self, group, counts, entropy_lambda, intermediate_weight, ce_only, bf16_store, sync):
+        """group_step as one call of the library (agpt_b200_train_step): no tape, no host decision between the kernels."""
+        import ctypes as C
+
+        import torch
+        grads = []
+        for p in self.params.values():
+            if p.grad is None:
+                p.grad = torch.zeros_like(p)
+            grads.append(p.grad)
+        if self._step_ptrs is None or any(a is not b for a, b in zip(grads, self._step_ptrs[0])):
+            for g, p in zip(grads, self.params.values()):
+                if g.dtype != torch.float32 or not g.is_contiguous() or g.shape != p.shape or g.device != p.device:
+                    raise A.AgptError("gradients must be contiguous float32 tensors on the device of their parameter")
+            n = len(grads)
+            self._step_ptrs = (grads, (C.c_void_p * n)(*[p.data_ptr() for p in self.params.values()]),
+                               (C.c_void_p * n)(*[g.data_ptr() for g in grads]))
+        for c in counts:
+            if c.dtype != torch.int32 or not c.is_cuda or not c.is_contiguous():
+                raise A.AgptError("counts must be contiguous int32 CUDA tensors")
+        m, out = self.cfg, torch.empty(8, dtype=torch.float32, device=self.device)
+        a = group.step_args()
+        a.d_model, a.n_heads, a.n_layers, a.d_ff, a.vocab, a.seq_len = m.d_model, m.n_heads, m.n_layers, m.d_ff, m.vocab, m.seq_len
+        a.params, a.grads = C.addressof(self._step_ptrs[1]), C.addressof(self._step_ptrs[2])
+        a.counts_offset, a.counts_tok, a.counts_val = [c.data_ptr() for c in counts]
+        a.cosv, a.sinv = self.cos.data_ptr(), self.sin.data_ptr()
+        a.entropy_lambda, a.intermediate_weight, a.ce_only = entropy_lambda, intermediate_weight, int(ce_only)
+        a.bf16_store, a.grad_mode, a.ffn_recompute = int(bf16_store), A.GRAD_MODES[self.grad_mode], int(self.ffn_recompute)
+        a.loss_sum, a.loss_count, a.tail = out.data_ptr(), out.data_ptr() + 8, out.data_ptr() + 16
+        L = A.lib()
+        need = A.check(L.agpt_b200_train_step_workspace_bytes(C.byref(a)), "train_step_workspace_bytes")
+        ws = torch.empty(need, dtype=torch.uint8, device=self.device)
+        A.check(L.agpt_b200_train_step(C.byref(a), ws.data_ptr(), need, torch.cuda.current_stream(self.device).cuda_stream), "train_step")
+        if not sync:
+            return out[4:7]
+        host = out.cpu()
+        return float(host[:2].view(torch.float64)[0]), int(host[2:4].view(torch.int64)[0])
 
 
 class SampleSpace:

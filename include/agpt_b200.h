@@ -463,7 +463,7 @@ int64_t agpt_b200_static_scratch_bytes(void);
 
 /* Device status word of the current GPU (waits for the work issued so far): 0 when every kernel ran to completion.
  * Bit 0: a bounded wait for a bulk asynchronous copy in the loss kernel ran out; the affected rows were not
- * written.  Kernels never trap; this word is how a failure on the device reaches the host. */
+ * written.  Bit 1: the same for a wait in the training step's projections.  Kernels never trap; this word is how a failure on the device reaches the host. */
 int agpt_b200_device_status(int32_t *status_out);
 
 /* Replaces agpt_loss_per_query_kernel (src/cuda/agpt_train.cu:2069-2216).  Same arguments. */
@@ -478,6 +478,39 @@ int agpt_b200_loss_per_query(const float *d_logits, const int32_t *d_query_to_no
 int agpt_b200_loss_per_node(const float *d_logits, const int32_t *d_node_ids, const int32_t *d_counts_offset,
                             const int32_t *d_counts_tok, const int32_t *d_counts_val, float *d_dlogits,
                             float *d_loss, int64_t N, int V, void *stream);
+
+/* One launch group of the trainer in one call: embedding, every layer, the per-query loss and the whole backward
+ * (the chunk step of src/cuda/agpt_train.cu:4560-5100), asynchronous on `stream`.  Gradients are added to what the
+ * gradient buffers hold, each row scaled by 1 / (trained queries of its unit).  params / grads: host arrays of
+ * 1 + 16 * n_layers + 4 device pointers in the order of the model file (token_emb; per layer wq.w, wq.b, wk.w, wk.b,
+ * wv.w, wv.b, wo.w, wo.b, ln1.gamma, ln1.beta, l1.w, l1.b, l2.w, l2.b, ln2.gamma, ln2.beta; final.gamma, final.beta,
+ * out.w, out.b).  Group arrays as in agpt_b200_loss_per_query and agpt_b200_rope; trained (NULL: every row) is 0 for
+ * context rows; edge_first is read in the own-edge gradient mode only; n_pos is 1 + the largest
+ * entry of pos.  The sum and number of the trained queries'
+ * positive losses go to loss_sum and loss_count, and to tail[3] = {sum, count / 4096, count % 4096}.
+ * agpt_b200_train_step_takes: d_model a multiple of 32 up to 1024, head_dim 16, 32 or 64, d_ff a multiple of 32, vocabulary
+ * up to 400. */
+typedef struct {
+    const agpt_plan *plan;
+    int64_t n;
+    int32_t d_model, n_heads, n_layers, d_ff, vocab, seq_len;
+    const float *const *params;
+    float *const *grads;
+    const int32_t *tokens, *pos, *query_to_node, *query_offsets, *radix_ids;
+    const float *mass_weights, *trained;
+    const int64_t *unit_of_row;
+    int32_t n_units, n_pos;
+    const int32_t *edge_first, *counts_offset, *counts_tok, *counts_val;
+    const float *cosv, *sinv;
+    float entropy_lambda, intermediate_weight;
+    int32_t ce_only, bf16_store, grad_mode, ffn_recompute;
+    double *loss_sum;
+    int64_t *loss_count;
+    float *tail;
+} agpt_train_step_args;
+int agpt_b200_train_step_takes(int d_model, int n_heads, int d_ff, int vocab);
+int64_t agpt_b200_train_step_workspace_bytes(const agpt_train_step_args *args);
+int agpt_b200_train_step(const agpt_train_step_args *args, void *workspace, int64_t workspace_bytes, void *stream);
 
 /* Host-buffer convenience of the same step (what gpu_batched_attention /
  * gpu_attention_backward_depth do around the kernels, src/agpt/batched_depth_forward.cr:745-823,
