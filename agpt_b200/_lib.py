@@ -37,6 +37,11 @@ class PlanInfo(C.Structure):
                 ("device", C.c_int)]
 
 
+class RunGroupInfo(C.Structure):
+    _fields_ = [("n", i64), ("n_loss_nodes", i64), ("n_trained", i64), ("bytes", i64), ("n_units", i32), ("n_pos", i32), ("seq_len", i32)] + \
+               [(k, i64) for k in ("tokens", "pos", "q2n", "edge_first", "unit_of_row", "mass_w", "trained", "qoff", "rid", "unit_off")]
+
+
 class TrainStepArgs(C.Structure):
     _fields_ = [("plan", vp), ("n", i64),
                 ("d_model", i32), ("n_heads", i32), ("n_layers", i32), ("d_ff", i32), ("vocab", i32), ("seq_len", i32),
@@ -78,6 +83,15 @@ SIGNATURES = {
     "agpt_b200_trie_char_tree": (C.c_int, [vp, vp, vp, vp, vp]),
     "agpt_b200_plan_create": (C.c_int, [vp, i64, C.c_int, C.c_int, C.POINTER(vp)]),
     "agpt_b200_plan_info": (C.c_int, [vp, C.POINTER(PlanInfo)]),
+    "agpt_b200_plan_array": (C.c_int, [vp, C.c_int, vp]),
+    "agpt_b200_plan_sizes": (C.c_int, [vp, C.POINTER(PlanInfo)]),
+    "agpt_b200_trie_groups_create": (C.c_int, [vp, C.c_int, i64, C.c_int, C.c_int, i64, C.POINTER(vp)]),
+    "agpt_b200_trie_ranks": (C.c_int, [vp, vp]),
+    "agpt_b200_trie_sample_group": (C.c_int, [vp, vp, vp, i64, vp, i64, C.POINTER(vp)]),
+    "agpt_b200_trie_groups_count": (i64, [vp]),
+    "agpt_b200_trie_group_prepare": (C.c_int, [vp, i64, C.c_int, C.c_int, C.c_int, C.POINTER(RunGroupInfo)]),
+    "agpt_b200_trie_group_upload": (C.c_int, [vp, C.c_int, vp, vp, C.POINTER(vp)]),
+    "agpt_b200_trie_groups_free": (None, [vp]),
     "agpt_b200_plan_destroy": (None, [vp]),
     "agpt_b200_attn_bwd_workspace_bytes": (i64, [vp, C.c_int]),
     "agpt_b200_plan_units": (i64, [vp, C.c_int, i64, vp, vp]),

@@ -13,7 +13,7 @@ import os
 
 import numpy as np
 
-from ._lib import AgptError, GroupInfo, PlanInfo, TrainStepArgs, TrieInfo, check, lib  # noqa: F401
+from ._lib import AgptError, GroupInfo, PlanInfo, RunGroupInfo, TrainStepArgs, TrieInfo, check, lib  # noqa: F401
 
 KV_F32, KV_BF16 = 0, 1
 
@@ -186,27 +186,39 @@ def token_hash(tokens) -> int:
 class WalkerPlan:
     """Depth-first layout of a tree plus the tile index the attention kernels walk."""
 
+    _ARRAYS = ("dfs_to_node", "node_to_dfs", "parent_dfs", "depth", "sub_end")
+
     def __init__(self, parent, tile_m: int = 64, device: int = -1):
         par = _np_i32(parent)
         h = C.c_void_p()
         check(lib().agpt_b200_plan_create(_vp(par), par.size, tile_m, device, C.byref(h)), "plan_create")
-        self._h = h
+        self._adopt(h)
+
+    def _adopt(self, h, keep=None):
+        """Take over a plan handle; keep: what its device arrays lie in."""
+        self._h, self._keep = h, keep
         info = PlanInfo()
-        check(lib().agpt_b200_plan_info(h, C.byref(info)), "plan_info")
+        check(lib().agpt_b200_plan_sizes(h, C.byref(info)), "plan_sizes")
         self.info = info
-        n = int(info.n)
-        self.n, self.tile_m, self.n_tiles = n, info.tile_m, int(info.n_tiles)
+        self.n, self.tile_m, self.n_tiles = int(info.n), info.tile_m, int(info.n_tiles)
         self.max_depth, self.sum_depth = info.max_depth, int(info.sum_depth)
         self.sum_group_prefix, self.n_groups = int(info.sum_group_prefix), int(info.n_groups)
         self.chain_rows = int(info.chain_rows)
         # kernels one backward launches: the tile kernel plus the reduction passes that have work
         self.bwd_launches = 1 + int(info.n_reduce_items > 0) + int(info.n_reduce_multi > 0)
-        self.dfs_to_node = _view(info.dfs_to_node, n, np.int32)
-        self.node_to_dfs = _view(info.node_to_dfs, n, np.int32)
-        self.parent_dfs = _view(info.parent_dfs, n, np.int32)
-        self.depth = _view(info.depth, n, np.int32)
-        self.sub_end = _view(info.sub_end, n, np.int32)
         self.device = info.device
+
+    def __getattr__(self, name):
+        # dfs_to_node, node_to_dfs, parent_dfs, depth, sub_end: copied from the library when first asked for (a training run
+        # never looks at most of them)
+        if name not in WalkerPlan._ARRAYS:
+            raise AttributeError(name)
+        if self.__dict__.get("_h") is None:
+            raise AgptError(f"{name}: the plan is closed")
+        a = np.empty(self.n, np.int32)
+        check(lib().agpt_b200_plan_array(self._h, WalkerPlan._ARRAYS.index(name), _vp(a)), "plan_array")
+        setattr(self, name, a)
+        return a
 
     def workspace_bytes(self, d_model: int) -> int:
         return check(lib().agpt_b200_attn_bwd_workspace_bytes(self._h, d_model), "attn_bwd_workspace_bytes")
@@ -261,15 +273,75 @@ class WalkerPlan:
         return fwd, bwd
 
     def close(self):
+        """Give the plan back; its row arrays stay readable."""
         if self._h is not None:
+            for name in WalkerPlan._ARRAYS:
+                getattr(self, name)
+            self._free()
+
+    def _free(self):
+        if self.__dict__.get("_h") is not None:
             lib().agpt_b200_plan_destroy(self._h)
-            self._h = None
+            self._h = self._keep = None
 
     def __del__(self):
         try:
-            self.close()
+            self._free()
         except Exception:
             pass
+
+
+class RunGroups:
+    """Launch groups of a trie made per radix edge (agpt_b200_trie_groups_create / agpt_b200_trie_sample_group): the arrays of
+    char_tree, WalkerPlan and launch_groups without their per-position work on the host."""
+
+    def __init__(self, handle, trie):
+        self._h, self._trie = handle, trie
+
+    @classmethod
+    def of_trie(cls, trie: RadixTrie, level: int, unit_cap, world: int, rank: int, group_rows: int) -> "RunGroups":
+        h = C.c_void_p()
+        check(lib().agpt_b200_trie_groups_create(trie._h, level, int(unit_cap or 0), world, rank, int(group_rows), C.byref(h)), "trie_groups_create")
+        return cls(h, trie)
+
+    @classmethod
+    def of_sample(cls, trie: RadixTrie, rank: np.ndarray, nodes, context) -> "RunGroups":
+        nodes, context = _np_i32(nodes), _np_i32(context)
+        h = C.c_void_p()
+        if lib().agpt_b200_trie_sample_group(trie._h, rank.ctypes.data, nodes.ctypes.data, nodes.size, context.ctypes.data, context.size, C.byref(h)):
+            raise ValueError(lib().agpt_b200_last_error().decode())
+        return cls(h, trie)
+
+    def __len__(self):
+        return int(lib().agpt_b200_trie_groups_count(self._h))
+
+    def upload(self, i: int, tile_m: int, mass_mode: str, seq_len: int, device):
+        """(info, device buffer, plan) of group i."""
+        import torch
+        info = RunGroupInfo()
+        check(lib().agpt_b200_trie_group_prepare(self._h, i, tile_m, MASS_MODES[mass_mode], seq_len, C.byref(info)), "trie_group_prepare")
+        buf = torch.empty(int(info.bytes), dtype=torch.uint8, device=device)
+        h = C.c_void_p()
+        check(lib().agpt_b200_trie_group_upload(self._h, device.index, buf.data_ptr(), torch.cuda.current_stream(device).cuda_stream, C.byref(h)),
+              "trie_group_upload")
+        plan = WalkerPlan.__new__(WalkerPlan)
+        plan._adopt(h, buf)
+        return info, buf, plan
+
+    def __del__(self):
+        try:
+            if self._h is not None:
+                lib().agpt_b200_trie_groups_free(self._h)
+                self._h = None
+        except Exception:
+            pass
+
+
+def trie_ranks(trie: RadixTrie) -> np.ndarray:
+    """Place of every radix node in the depth-first order of the trie's rows."""
+    out = np.zeros(trie.radix_count, np.int32)
+    check(lib().agpt_b200_trie_ranks(trie._h, _vp(out)), "trie_ranks")
+    return out
 
 
 def launch_groups(plan: WalkerPlan, unit_begin, unit_end, unit_rank, rank: int, group_rows: int):

@@ -12,7 +12,8 @@ SOURCES = [os.path.join(HERE, "csrc", "kernels.cu"), os.path.join(HERE, "csrc", 
            os.path.join(HERE, "csrc", "gemm3x.cu"), os.path.join(HERE, "csrc", "gemm_sm100.cu"),
            os.path.join(HERE, "csrc", "host_trie.cpp"), os.path.join(HERE, "csrc", "trie_suffix.cpp"),
            os.path.join(HERE, "csrc", "trie_gpu.cu"),
-           os.path.join(HERE, "csrc", "step_gemm.cu"), os.path.join(HERE, "csrc", "train_step.cu")]
+           os.path.join(HERE, "csrc", "step_gemm.cu"), os.path.join(HERE, "csrc", "train_step.cu"),
+           os.path.join(HERE, "csrc", "groups.cu")]
 
 
 # The two GEMM translation units instantiate CUTLASS templates, and gemm_sm100.cu re-instantiates the SM100 fast-FP32

@@ -659,11 +659,8 @@ extern "C" float agpt_b200_compute_lr(float base_lr, int step, int total_steps, 
 // --------------------------------------------------------------------------------------
 // per-query mass weights of a launch (host loop of src/cuda/agpt_train.cu:4608-4637, with the mean taken per unit)
 // --------------------------------------------------------------------------------------
-extern "C" int agpt_b200_mass_weights(const int32_t *edge_mass, const int32_t *edge_len, const int32_t *unit_of_node,
-                                      const uint8_t *counted, int64_t n_nodes, int64_t n_units, int mode, float *out_per_query) {
-    if (!edge_mass || !edge_len || !out_per_query || n_nodes < 0 || n_units < 1 || mode < 0 || mode > 3)
-        return agpt_set_error(AGPT_E_ARG, "mass_weights: bad argument");
-    std::vector<float> w((size_t)n_nodes);
+int agpt_mass_weights_per_node(const int32_t *edge_mass, const int32_t *edge_len, const int32_t *unit_of_node, const uint8_t *counted,
+                               int64_t n_nodes, int64_t n_units, int mode, float *w) {
     std::vector<double> tot((size_t)n_units, 0.0), tq((size_t)n_units, 0.0);
     for (int64_t i = 0; i < n_nodes; i++) {
         const float c = (float)edge_mass[i];
@@ -673,14 +670,24 @@ extern "C" int agpt_b200_mass_weights(const int32_t *edge_mass, const int32_t *e
         if (edge_len[i] < 0) return agpt_set_error(AGPT_E_ARG, "mass_weights: negative edge length");
         if (!counted || counted[i]) { tot[u] += (double)w[i] * edge_len[i]; tq[u] += (double)edge_len[i]; }
     }
-    int64_t q = 0;
     for (int64_t i = 0; i < n_nodes; i++) {
         const int64_t u = unit_of_node ? unit_of_node[i] : 0;
         float mean = tq[u] > 0 ? (float)(tot[u] / tq[u]) : 1.0f;
         if (mean <= 0.0f) mean = 1.0f;
-        const float v = w[i] / mean;
-        for (int32_t j = 0; j < edge_len[i]; j++) out_per_query[q++] = v;
+        w[i] /= mean;
     }
+    return AGPT_OK;
+}
+
+extern "C" int agpt_b200_mass_weights(const int32_t *edge_mass, const int32_t *edge_len, const int32_t *unit_of_node,
+                                      const uint8_t *counted, int64_t n_nodes, int64_t n_units, int mode, float *out_per_query) {
+    if (!edge_mass || !edge_len || !out_per_query || n_nodes < 0 || n_units < 1 || mode < 0 || mode > 3)
+        return agpt_set_error(AGPT_E_ARG, "mass_weights: bad argument");
+    std::vector<float> w((size_t)n_nodes);
+    if (int rc = agpt_mass_weights_per_node(edge_mass, edge_len, unit_of_node, counted, n_nodes, n_units, mode, w.data())) return rc;
+    int64_t q = 0;
+    for (int64_t i = 0; i < n_nodes; i++)
+        for (int32_t j = 0; j < edge_len[i]; j++) out_per_query[q++] = w[i];
     return AGPT_OK;
 }
 
@@ -772,7 +779,8 @@ extern "C" int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_
     P->n_tiles = (n + tile_m - 1) / tile_m;
     P->chain_off.assign(P->n_tiles + 1, 0);
     for (int64_t t = 0; t < P->n_tiles; t++) P->chain_off[t + 1] = P->chain_off[t] + (P->depth[t * tile_m] - 1);
-    P->chain_ids.resize(P->chain_off[P->n_tiles]);
+    P->chain_rows = P->chain_off[P->n_tiles];
+    P->chain_ids.resize(P->chain_rows);
     for (int64_t t = 0; t < P->n_tiles; t++) {
         int32_t a = P->parent_dfs[t * tile_m];
         for (int64_t j = P->chain_off[t + 1] - 1; j >= P->chain_off[t]; j--) { P->chain_ids[j] = a; a = P->parent_dfs[a]; }
@@ -815,9 +823,48 @@ extern "C" int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_
     return AGPT_OK;
 }
 
+// one row array (0 dfs_to_node, 1 node_to_dfs, 2 parent_dfs, 3 depth, 4 sub_end), written straight into the caller's memory
+extern "C" int agpt_b200_plan_array(const agpt_plan *p, int which, int32_t *out) {
+    if (!p || !out || which < 0 || which > 4) return agpt_set_error(AGPT_E_ARG, "plan_array: bad argument");
+    if (!p->lazy) {
+        const std::vector<int32_t> *v[5] = {&p->dfs_to_node, &p->node_to_dfs, &p->parent_dfs, &p->depth, &p->sub_end};
+        std::copy(v[which]->begin(), v[which]->end(), out);
+        return AGPT_OK;
+    }
+    if (which < 2) std::iota(out, out + p->n, 0);
+    else for (size_t e = 0; e < p->run_parent.size(); e++) {
+        const int32_t a0 = p->run_qoff[e], a1 = p->run_qoff[e + 1], up = p->run_parent[e];
+        if (which == 2) { out[a0] = up < 0 ? -1 : p->run_qoff[up + 1] - 1; std::iota(out + a0 + 1, out + a1, a0); }
+        else if (which == 3) std::iota(out + a0, out + a1, p->run_depth[e]);
+        else std::fill(out + a0, out + a1, p->run_end[e]);
+    }
+    return AGPT_OK;
+}
+
+void agpt_plan::need_host() {
+    if (!lazy) return;
+    std::lock_guard<std::mutex> hold(host_lock);
+    if (!lazy) return;
+    std::vector<int32_t> *v[5] = {&dfs_to_node, &node_to_dfs, &parent_dfs, &depth, &sub_end};
+    for (int i = 0; i < 5; i++) { v[i]->resize(n); agpt_b200_plan_array(this, i, v[i]->data()); }
+    lazy = false;
+}
+
+// sizes only: the row arrays of a plan made from runs are not derived for it
+extern "C" int agpt_b200_plan_sizes(const agpt_plan *p, agpt_plan_info *o) {
+    if (!p || !o) return agpt_set_error(AGPT_E_ARG, "plan_sizes: null");
+    *o = agpt_plan_info();
+    o->n = p->n; o->tile_m = p->tile_m; o->n_tiles = p->n_tiles; o->chain_rows = p->chain_rows;
+    o->max_depth = p->max_depth; o->sum_depth = p->sum_depth; o->sum_group_prefix = p->sum_group_prefix; o->n_groups = p->n_groups;
+    o->n_reduce_items = (int64_t)p->item_node.size(); o->n_reduce_nodes = p->n_reduce_nodes; o->n_reduce_multi = (int64_t)p->multi_node.size();
+    o->device = p->device;
+    return AGPT_OK;
+}
+
 extern "C" int agpt_b200_plan_info(const agpt_plan *p, agpt_plan_info *o) {
     if (!p || !o) return agpt_set_error(AGPT_E_ARG, "plan_info: null");
-    o->n = p->n; o->tile_m = p->tile_m; o->n_tiles = p->n_tiles; o->chain_rows = (int64_t)p->chain_ids.size();
+    const_cast<agpt_plan *>(p)->need_host();
+    o->n = p->n; o->tile_m = p->tile_m; o->n_tiles = p->n_tiles; o->chain_rows = p->chain_rows;
     o->max_depth = p->max_depth; o->sum_depth = p->sum_depth; o->sum_group_prefix = p->sum_group_prefix; o->n_groups = p->n_groups;
     o->n_reduce_items = (int64_t)p->item_node.size(); o->n_reduce_nodes = p->n_reduce_nodes; o->n_reduce_multi = (int64_t)p->multi_node.size();
     o->dfs_to_node = p->dfs_to_node.data(); o->node_to_dfs = p->node_to_dfs.data(); o->parent_dfs = p->parent_dfs.data();
@@ -837,6 +884,7 @@ struct agpt_groups {
 extern "C" int agpt_b200_groups_create(const agpt_plan *p, const int64_t *unit_begin, const int64_t *unit_end, const int32_t *unit_rank,
                                        int64_t n_units, int rank, int64_t group_rows, agpt_groups **out) {
     if (!p || !unit_begin || !unit_end || !out || n_units < 0 || group_rows < 1) return agpt_set_error(AGPT_E_ARG, "groups_create: bad argument");
+    const_cast<agpt_plan *>(p)->need_host();
     agpt_groups *G = new agpt_groups();
     agpt_groups::Group cur;
     auto flush = [&]() {
@@ -889,12 +937,13 @@ extern "C" void agpt_b200_groups_free(agpt_groups *g) { delete g; }
 extern "C" int64_t agpt_b200_attn_bwd_workspace_bytes(const agpt_plan *p, int d_model) {
     if (!p || d_model <= 0) return agpt_set_error(AGPT_E_ARG, "attn_bwd_workspace_bytes: bad argument");
     // partial dK and dV rows of every tile's chain, then the per-segment sums of long reductions
-    int64_t rows = (int64_t)p->chain_ids.size() + p->n_multi_items;
+    int64_t rows = p->chain_rows + p->n_multi_items;
     return std::max<int64_t>(256, rows * 2 * (int64_t)d_model * 4);
 }
 
 extern "C" int64_t agpt_b200_plan_units(const agpt_plan *p, int level, int64_t cap, int64_t *ub, int64_t *ue) {
     if (!p || (level != 1 && level != 2)) return agpt_set_error(AGPT_E_ARG, "plan_units: bad argument");
+    const_cast<agpt_plan *>(p)->need_host();
     int64_t cnt = 0;
     auto emit = [&](int64_t b, int64_t e) { if (cnt < cap && ub && ue) { ub[cnt] = b; ue[cnt] = e; } cnt++; };
     for (int64_t a = 0; a < p->n; a = p->sub_end[a]) {       // depth-1 nodes

@@ -1,6 +1,8 @@
 // Shared between the host walker code and the CUDA translation unit of libagpt_b200.
 #pragma once
+#include <atomic>
 #include <cstdint>
+#include <mutex>
 #include <vector>
 
 #define AGPT_REDUCE_SEG 128   // tiles summed by one warp of the dK/dV reduction before a second pass
@@ -39,16 +41,23 @@ struct agpt_plan {
     int64_t n_tiles = 0;
     int32_t max_depth = 0;
     int64_t sum_depth = 0, sum_group_prefix = 0, n_groups = 0, n_reduce_nodes = 0, n_multi_items = 0;
-    std::vector<int32_t> dfs_to_node, node_to_dfs, parent_dfs, depth, sub_end;
+    std::vector<int32_t> dfs_to_node, node_to_dfs, parent_dfs, depth, sub_end;      // filled on demand if lazy: need_host()
     std::vector<int64_t> chain_off;
+    int64_t chain_rows = 0;                      // chain_off[n_tiles]
     std::vector<int32_t> chain_ids, chain_end;   // chain_end[j] = sub_end[chain_ids[j]]
     // dK/dV reduction work list: item = (node, inclusive tile range); slot >= 0 when the node's range
     // is cut into several items whose sums meet in a second pass
     std::vector<int32_t> item_node, item_t0, item_t1, item_slot;
     std::vector<int32_t> multi_node, multi_count;
     std::vector<int64_t> multi_first;          // first segment slot of each multi-segment node (its slots are consecutive)
-    // device copies (owned)
+    // a plan made from runs of rows (groups.cu): row arrays are derived from these when the host asks for them
+    std::atomic<bool> lazy{false};
+    std::vector<int32_t> run_qoff, run_parent, run_depth, run_end;
+    std::mutex host_lock;
+    void need_host();
+    // device copies (owned, or in a buffer of the caller)
     int device = -1;
+    bool external = false;
     int32_t *d_depth = nullptr, *d_sub_end = nullptr, *d_chain_ids = nullptr, *d_chain_end = nullptr;
     int64_t *d_chain_off = nullptr, *d_multi_first = nullptr;
     int32_t *d_item_node = nullptr, *d_item_t0 = nullptr, *d_item_t1 = nullptr, *d_item_slot = nullptr;
@@ -65,6 +74,9 @@ struct agpt_plan {
 };
 
 int agpt_plan_upload(agpt_plan *p, int device);
+// mass weight of each loss node (agpt_b200_mass_weights without the expansion to queries)
+int agpt_mass_weights_per_node(const int32_t *edge_mass, const int32_t *edge_len, const int32_t *unit_of_node, const uint8_t *counted,
+                               int64_t n_nodes, int64_t n_units, int mode, float *out_per_node);
 int agpt_step_gemm_status(int *out);       // status word of step_gemm.cu's kernels
 
 // tcgen05 float32 GEMM (gemm_sm100.cu): D[l] = act(alpha * op(A[l]) * op(B[l]) + beta * C + bias row), l < L batches

@@ -82,9 +82,11 @@ agpt_plan::~agpt_plan() {
         int cur = -1;
         cudaGetDevice(&cur);
         cudaSetDevice(device);
+        if (!external) {
         cudaFree(d_depth); cudaFree(d_sub_end); cudaFree(d_chain_ids); cudaFree(d_chain_end); cudaFree(d_chain_off);
         cudaFree(d_item_node); cudaFree(d_item_t0); cudaFree(d_item_t1); cudaFree(d_item_slot);
         cudaFree(d_multi_node); cudaFree(d_multi_count); cudaFree(d_multi_first);
+        }
         cudaFree(host_arena);
         if (host_fix) cudaFreeHost(host_fix);
         for (void *e : host_events) cudaEventDestroy((cudaEvent_t)e);
@@ -1998,7 +2000,7 @@ extern "C" int agpt_b200_attn_bwd_mode(const agpt_plan *p, const float *d_q, con
     int64_t need = agpt_b200_attn_bwd_workspace_bytes(p, D);
     if (workspace_bytes < need)
         return agpt_set_error(AGPT_E_ARG, "attn_bwd: workspace %lld bytes < required %lld", (long long)workspace_bytes, (long long)need);
-    const int64_t rows = (int64_t)p->chain_ids.size();
+    const int64_t rows = p->chain_rows;
     float *pk = (float *)d_workspace, *pv = pk + rows * D, *segk = pv + rows * D, *segv = segk + p->n_multi_items * D;
     rc = bwd_dispatch(p, d_q, d_k, d_v, kv_dtype, d_out, d_lse, d_dout, d_dq, d_dk, d_dv, pk, pv, n_heads, head_dim, scale,
                       (cudaStream_t)stream, 0, (int)p->n_tiles, BwdMask{grad_mode, d_edge_first});
@@ -2883,6 +2885,7 @@ static int attn_fwd_bwd_host_impl(const agpt_plan *cp, const float *h_q, const f
     if (kv_dtype != AGPT_KV_F32 && kv_dtype != AGPT_KV_BF16) return agpt_set_error(AGPT_E_ARG, "attn_fwd_bwd_host: bad kv_dtype");
     agpt_plan *p = const_cast<agpt_plan *>(cp);        // the cached arena is the only state a call changes
     CUDA_TRY(cudaSetDevice(p->device));
+    p->need_host();
     const int D = n_heads * head_dim, M = p->tile_m;
     const int64_t n = p->n;
     const size_t rowb = (size_t)D * sizeof(float);
@@ -2912,7 +2915,7 @@ static int attn_fwd_bwd_host_impl(const agpt_plan *cp, const float *h_q, const f
     __nv_bfloat16 *vb = bf ? kb + (size_t)n * D : nullptr;
     char *fix_dev = base + 8 * tens + lseb + wsb + (bf ? tens : 0);
     const void *kk = bf ? (const void *)kb : (const void *)dk_in, *vv = bf ? (const void *)vb : (const void *)dv_in;
-    const int64_t rows = (int64_t)p->chain_ids.size();
+    const int64_t rows = p->chain_rows;
     float *pk = (float *)ws, *pv = pk + rows * D, *segk = pv + rows * D, *segv = segk + p->n_multi_items * D;
 
     while ((int64_t)p->host_events.size() < 3 * n_ch + 1) {
@@ -3041,7 +3044,7 @@ extern "C" int agpt_b200_attn_bwd_static(const agpt_plan *p, const float *d_q, c
     }
     // Every partial row and every segment sum the reduction reads is written earlier in this same call, so nothing
     // left in the array by a previous call is ever read and nothing needs clearing.
-    const int64_t rows = (int64_t)p->chain_ids.size();
+    const int64_t rows = p->chain_rows;
     float *pk = (float *)g_static_scratch_addr[cur], *pv = pk + rows * D, *segk = pv + rows * D, *segv = segk + p->n_multi_items * D;
     rc = bwd_dispatch(p, d_q, d_k, d_v, kv_dtype, d_out, d_lse, d_dout, d_dq, d_dk, d_dv, pk, pv, n_heads, head_dim, scale,
                       (cudaStream_t)stream, 0, (int)p->n_tiles);

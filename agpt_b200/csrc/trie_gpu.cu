@@ -24,12 +24,15 @@ namespace {
         if (e_ != cudaSuccess) { rc = agpt_set_error(AGPT_E_CUDA, "%s: %s", #x, cudaGetErrorString(e_)); goto done; } \
     } while (0)
 
+// digit of count tokens, the first in the highest bits
 template <typename DT>
 __global__ void __launch_bounds__(256) digit_kernel(const int32_t *__restrict__ corpus, const int32_t *__restrict__ sa, int64_t n, int32_t m,
-                                                     int d, DT *__restrict__ digit) {
+                                                     int d, int count, int bits, DT *__restrict__ digit) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t p = (int64_t)sa[i] + d;
-        digit[i] = p < n ? (DT)(corpus[p] + 1) : (DT)0;
+        DT v = 0;
+        for (int k = 0; k < count; k++) v = (DT)(v << (k ? bits : 0)) | (p + k < n ? (DT)(corpus[p + k] + 1) : (DT)0);
+        digit[i] = v;
     }
 }
 
@@ -51,31 +54,43 @@ __global__ void __launch_bounds__(256) lcp_kernel(const int32_t *__restrict__ co
     }
 }
 
+int64_t up256(int64_t x) { return (x + 255) & ~(int64_t)255; }
+
+// One device allocation holds everything (a handful of cudaMalloc and cudaFree calls took longer than the sort of a short
+// corpus); layout: corpus, two position arrays, common prefixes, two digit arrays, cub's scratch.
 template <typename DT>
-int sort_suffixes(const int32_t *d_corpus, int64_t n, int32_t m, int key_len, int bits, int32_t *d_sa0, int32_t *d_sa1, int32_t **d_sorted,
-                  cudaStream_t st) {
+int sort_suffixes(const int32_t *corpus, int64_t n, int32_t m, int key_len, int bits, int per_digit, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1,
+                  int32_t *sa_out, int32_t *lcp_out) {
     int rc = AGPT_OK;
-    DT *d_dig0 = nullptr, *d_dig1 = nullptr;
-    void *d_tmp = nullptr;
+    uint8_t *arena = nullptr;
     size_t tmp_bytes = 0;
+    const int64_t am = up256((int64_t)m * 4), ad = up256((int64_t)m * sizeof(DT)), an = up256(n * 4);
     const unsigned grid = (unsigned)(((int64_t)m + 255) / 256 < 148 * 16 ? ((int64_t)m + 255) / 256 : 148 * 16);
-    int32_t *in = d_sa0, *outp = d_sa1;
-    CUDA_TRY(cudaMalloc(&d_dig0, (size_t)m * sizeof(DT)));
-    CUDA_TRY(cudaMalloc(&d_dig1, (size_t)m * sizeof(DT)));
-    CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, d_dig0, d_dig1, in, outp, m, 0, bits, st));
-    CUDA_TRY(cudaMalloc(&d_tmp, tmp_bytes ? tmp_bytes : 16));
+    int32_t *d_corpus, *in, *outp, *d_lcp;
+    DT *dig0, *dig1;
+    void *tmp;
+    CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (DT *)nullptr, (DT *)nullptr, (int32_t *)nullptr, (int32_t *)nullptr, m, 0,
+                                             bits * per_digit, st));
+    CUDA_TRY(cudaMalloc(&arena, (size_t)(an + 3 * am + 2 * ad) + tmp_bytes + 16));
+    d_corpus = (int32_t *)arena; in = (int32_t *)(arena + an); outp = (int32_t *)(arena + an + am); d_lcp = (int32_t *)(arena + an + 2 * am);
+    dig0 = (DT *)(arena + an + 3 * am); dig1 = (DT *)(arena + an + 3 * am + ad); tmp = arena + an + 3 * am + 2 * ad;
+    CUDA_TRY(cudaMemcpyAsync(d_corpus, corpus, (size_t)n * 4, cudaMemcpyHostToDevice, st));
+    if (e0) CUDA_TRY(cudaEventRecord(e0, st));
     iota_kernel<<<grid, 256, 0, st>>>(in, m);
-    for (int d = key_len - 1; d >= 0; d--) {
-        digit_kernel<DT><<<grid, 256, 0, st>>>(d_corpus, in, n, m, d, d_dig0);
-        CUDA_TRY(cub::DeviceRadixSort::SortPairs(d_tmp, tmp_bytes, d_dig0, d_dig1, in, outp, m, 0, bits, st));
+    for (int end = key_len; end > 0; end -= per_digit) {
+        const int first = end > per_digit ? end - per_digit : 0, count = end - first;
+        digit_kernel<DT><<<grid, 256, 0, st>>>(d_corpus, in, n, m, first, count, bits, dig0);
+        CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, dig0, dig1, in, outp, m, 0, bits * count, st));
         int32_t *t = in; in = outp; outp = t;
     }
+    lcp_kernel<<<grid, 256, 0, st>>>(d_corpus, in, n, m, key_len, d_lcp);
     CUDA_TRY(cudaGetLastError());
-    *d_sorted = in;
+    if (e1) CUDA_TRY(cudaEventRecord(e1, st));
+    CUDA_TRY(cudaMemcpyAsync(sa_out, in, (size_t)m * 4, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaMemcpyAsync(lcp_out, d_lcp, (size_t)m * 4, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
 done:
-    cudaFree(d_dig0);
-    cudaFree(d_dig1);
-    cudaFree(d_tmp);
+    cudaFree(arena);
     return rc;
 }
 
@@ -93,38 +108,24 @@ extern "C" int agpt_b200_suffix_order_gpu(const int32_t *corpus, int64_t n, int 
     if (vocab > 65534) return agpt_set_error(AGPT_E_LIMIT, "suffix_order_gpu: vocabulary beyond 65534");
     int rc = AGPT_OK;
     const int32_t m = (int32_t)(n - 1);
-    int32_t *d_corpus = nullptr, *d_sa0 = nullptr, *d_sa1 = nullptr, *d_lcp = nullptr, *d_sorted = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaStream_t st = nullptr;
     int bits = 1;
     while ((1 << bits) < vocab + 1) bits++;
     CUDA_TRY(cudaSetDevice(device));
     CUDA_TRY(cudaStreamCreate(&st));
-    CUDA_TRY(cudaEventCreate(&e0));
-    CUDA_TRY(cudaEventCreate(&e1));
-    CUDA_TRY(cudaMalloc(&d_corpus, (size_t)n * 4));
-    CUDA_TRY(cudaMalloc(&d_sa0, (size_t)m * 4));
-    CUDA_TRY(cudaMalloc(&d_sa1, (size_t)m * 4));
-    CUDA_TRY(cudaMalloc(&d_lcp, (size_t)m * 4));
-    CUDA_TRY(cudaMemcpyAsync(d_corpus, corpus, (size_t)n * 4, cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaEventRecord(e0, st));
-    rc = vocab + 1 <= 256 ? sort_suffixes<uint8_t>(d_corpus, n, m, key_len, bits, d_sa0, d_sa1, &d_sorted, st)
-                          : sort_suffixes<uint16_t>(d_corpus, n, m, key_len, bits, d_sa0, d_sa1, &d_sorted, st);
-    if (rc) goto done;
-    {
-        const int64_t blocks = ((int64_t)m + 255) / 256;
-        lcp_kernel<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, st>>>(d_corpus, d_sorted, n, m, key_len, d_lcp);
+    if (device_ms_out) {
+        CUDA_TRY(cudaEventCreate(&e0));
+        CUDA_TRY(cudaEventCreate(&e1));
     }
-    CUDA_TRY(cudaEventRecord(e1, st));
-    CUDA_TRY(cudaMemcpyAsync(sa_out, d_sorted, (size_t)m * 4, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(lcp_out, d_lcp, (size_t)m * 4, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    // Below a few million positions a pass is launch latency, so as many tokens as fit 64 bits go into one digit (33 tokens
+    // of 7 bits: 44 launches instead of 165); above, one token per pass moves the fewest bytes.
+    if (m < (4 << 20)) rc = sort_suffixes<uint64_t>(corpus, n, m, key_len, bits, 64 / bits, st, e0, e1, sa_out, lcp_out);
+    else if (vocab + 1 <= 256) rc = sort_suffixes<uint8_t>(corpus, n, m, key_len, bits, 1, st, e0, e1, sa_out, lcp_out);
+    else rc = sort_suffixes<uint16_t>(corpus, n, m, key_len, bits, 1, st, e0, e1, sa_out, lcp_out);
+    if (rc) goto done;
     if (device_ms_out) CUDA_TRY(cudaEventElapsedTime(device_ms_out, e0, e1));
 done:
-    cudaFree(d_corpus);
-    cudaFree(d_sa0);
-    cudaFree(d_sa1);
-    cudaFree(d_lcp);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (st) cudaStreamDestroy(st);

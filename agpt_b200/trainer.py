@@ -69,10 +69,48 @@ class LaunchGroup:
         self.mass_w = None if mw is None else t(mw)
         self.n_trained_rows = self.n if trained is None else int(trained.sum())
 
+    # where the arrays of a group made by the library lie in its device buffer: (dtype, length in terms of the sizes)
+    _LAYOUT = {"tokens32": ("tokens", "int32", lambda i: i.n), "pos": ("pos", "int32", lambda i: i.n), "q2n": ("q2n", "int32", lambda i: i.n),
+               "edge_first": ("edge_first", "int32", lambda i: i.n), "unit_of_row": ("unit_of_row", "int64", lambda i: i.n),
+               "mass_w": ("mass_w", "float32", lambda i: i.n), "trained": ("trained", "float32", lambda i: i.n),
+               "qoff": ("qoff", "int32", lambda i: i.n_loss_nodes + 1), "rid": ("rid", "int32", lambda i: i.n_loss_nodes),
+               "unit_off": ("unit_off", "int64", lambda i: i.n_units + 1)}
+
+    @classmethod
+    def from_runs(cls, runs, i, mass_mode, seq_len, device, tile=64) -> "LaunchGroup":
+        """Group i of an A.RunGroups: one device buffer, written by the library."""
+        self = cls.__new__(cls)
+        self._info, self._buf, self.plan = runs.upload(i, tile, mass_mode, seq_len, device)
+        o = self._info
+        self.n, self.n_units, self.n_pos, self.n_trained_rows = int(o.n), int(o.n_units), int(o.n_pos), int(o.n_trained)
+        return self
+
+    def __getattr__(self, name):
+        # tensors of a group made by the library are views of its buffer, made when first asked for
+        import torch
+        info = self.__dict__.get("_info")
+        if info is None or (name != "tokens" and name not in LaunchGroup._LAYOUT):
+            raise AttributeError(name)
+        if name == "tokens":
+            v = self.tokens32.to(torch.int64)
+        else:
+            field, kind, length = LaunchGroup._LAYOUT[name]
+            at, kind = getattr(info, field), getattr(torch, kind)
+            v = None if at < 0 else self._buf[at:at + int(length(info)) * kind.itemsize].view(kind)
+        setattr(self, name, v)
+        return v
+
     def step_args(self):
         """The group's part of the native step's arguments (the model fills in the rest)."""
-        ptr = lambda x: None if x is None else x.data_ptr()  # noqa: E731
         a = A.TrainStepArgs(plan=self.plan._h, n=self.n, n_units=self.n_units, n_pos=self.n_pos)
+        o = self.__dict__.get("_info")
+        if o is not None:
+            at = self._buf.data_ptr()
+            ptr = lambda off: None if off < 0 else at + off  # noqa: E731
+            a.tokens, a.pos, a.query_to_node, a.query_offsets, a.radix_ids = at + o.tokens, at + o.pos, at + o.q2n, at + o.qoff, at + o.rid
+            a.mass_weights, a.trained, a.unit_of_row, a.edge_first = ptr(o.mass_w), ptr(o.trained), at + o.unit_of_row, at + o.edge_first
+            return a
+        ptr = lambda x: None if x is None else x.data_ptr()  # noqa: E731
         a.tokens, a.pos, a.query_to_node, a.query_offsets, a.radix_ids = [ptr(x) for x in (self.tokens32, self.pos, self.q2n, self.qoff, self.rid)]
         a.mass_weights, a.trained, a.unit_of_row, a.edge_first = [ptr(x) for x in (self.mass_w, self.trained, self.unit_of_row, self.edge_first)]
         return a
@@ -85,10 +123,13 @@ def build_groups(trie: A.RadixTrie, rank: int, world: int, group_rows: int, mass
     (WalkerPlan.units_capped), which bounds the activation memory of a launch.  A unit that does not start at depth 1
     carries its ancestors as context rows (attended, and differentiated through, but not trained), so every chain is
     complete and the summed gradient does not depend on the partition."""
-    parent, token, depth, radix_of = trie.char_tree()
-    gplan = A.WalkerPlan(parent, 64, -1)
     if level is None:
         level = 1 if world == 1 else 2
+    if device.type == "cuda" and bool((trie.parent[1:] < np.arange(1, trie.radix_count)).all()):
+        runs = A.RunGroups.of_trie(trie, level, unit_cap, world, rank, group_rows)
+        return [LaunchGroup.from_runs(runs, i, mass_mode, seq_len, device, tile) for i in range(len(runs))], trie.total_edge_chars
+    parent, token, depth, radix_of = trie.char_tree()
+    gplan = A.WalkerPlan(parent, 64, -1)
     ub, ue = gplan.units(level) if unit_cap is None else gplan.units_capped(level, unit_cap)
     owner = A.partition_lpt(ue - ub, world)
     d2n = gplan.dfs_to_node
@@ -373,6 +414,10 @@ class TrieWalkModel:
             b = torch.cat([b, torch.full((pad,), -1e30, dtype=b.dtype, device=b.device)])
         return lin(xf, w, b)
 
+    def native_step_available(self) -> bool:
+        m = self.cfg
+        return self.dense_impl == "tensor" and bool(A.lib().agpt_b200_train_step_takes(m.d_model, m.n_heads, m.d_ff, m.vocab))
+
     def group_step(self, group: LaunchGroup, counts, entropy_lambda=0.0, intermediate_weight=1.0, ce_only=False,
                    bf16_store=False, sync=True):
         """Forward, loss and backward of one launch group; gradients accumulate into .grad.
@@ -380,8 +425,7 @@ class TrieWalkModel:
         float32 device tensor (loss sum, count // 4096, count % 4096), so that the host does not wait for the device
         between groups."""
         import torch
-        m = self.cfg
-        if self.dense_impl == "tensor" and A.lib().agpt_b200_train_step_takes(m.d_model, m.n_heads, m.d_ff, m.vocab):
+        if self.native_step_available():
             return self._native_step(group, counts, entropy_lambda, intermediate_weight, ce_only, bf16_store, sync)
         logits = self.logits(group, bf16_store).contiguous()
         c_off, c_tok, c_val = counts
@@ -445,10 +489,18 @@ class TrieWalkModel:
         need = A.check(L.agpt_b200_train_step_workspace_bytes(C.byref(a)), "train_step_workspace_bytes")
         ws = torch.empty(need, dtype=torch.uint8, device=self.device)
         A.check(L.agpt_b200_train_step(C.byref(a), ws.data_ptr(), need, torch.cuda.current_stream(self.device).cuda_stream), "train_step")
+        if sync is None:
+            return out
         if not sync:
             return out[4:7]
-        host = out.cpu()
-        return float(host[:2].view(torch.float64)[0]), int(host[2:4].view(torch.int64)[0])
+        return _step_stats(out.cpu())[0]
+
+
+def _step_stats(host):
+    """[(loss sum, queries)] from native steps' result buffers on the host (eight floats each: float64 sum, int64 count, ...)."""
+    import torch
+    host = host.reshape(-1, 8)
+    return list(zip(host[:, :2].contiguous().view(torch.float64).flatten().tolist(), host[:, 2:4].contiguous().view(torch.int64).flatten().tolist()))
 
 
 class SampleSpace:
@@ -456,8 +508,16 @@ class SampleSpace:
 
     def __init__(self, trie: A.RadixTrie):
         self.trie = trie
-        self.parent, self.token, self.depth, self.radix_of = trie.char_tree()
+        ordered = bool((trie.parent[1:] < np.arange(1, trie.radix_count)).all())
+        self.rank = A.trie_ranks(trie) if ordered else None      # depth-first place of every radix node
+
+    def __getattr__(self, name):
+        # the char-level arrays, for groups on a CPU device and tries whose nodes do not follow their parents
+        if name not in ("parent", "token", "depth", "radix_of", "plan"):
+            raise AttributeError(name)
+        self.parent, self.token, self.depth, self.radix_of = self.trie.char_tree()
         self.plan = A.WalkerPlan(self.parent, 64, -1)
+        return self.__dict__[name]
 
     def group(self, node_ids, context_ids, mass_mode, seq_len, device, tile=64) -> LaunchGroup:
         """Launch group of the chars of the radix nodes node_ids (closed under "parent"); chars of context_ids are
@@ -466,6 +526,8 @@ class SampleSpace:
         in the chunk's mass mean (src/cuda/agpt_train.cu:4601-4637; the ancestor count recorded at :4194 is never read,
         and the comment at :4160-4180 that announces a masking describes a variant that was taken out again)."""
         t = self.trie
+        if device.type == "cuda" and self.rank is not None:
+            return LaunchGroup.from_runs(A.RunGroups.of_sample(t, self.rank, node_ids, context_ids), 0, mass_mode, seq_len, device, tile)
         node_ids = np.asarray(node_ids, np.int64)
         lens = t.edge_len[node_ids].astype(np.int64)
         starts = t.edge_start[node_ids].astype(np.int64)
@@ -502,18 +564,29 @@ def train_lightning_epoch(model: TrieWalkModel, space: SampleSpace, counts, opt,
     lr_w = lightning_lr_weights(masses, mass_lr)
     model.bind_grads()
     loss_sum, n_q, n_nodes = 0.0, 0, 0
+    pending = []                         # statistics of native steps, read once at the end so that the host never waits between steps
+    native = model.native_step_available()
     for s in range(steps):
         ids = nodes[off[s]:off[s + 1]]
         # every sampled row is trained, the ancestors the sampler prepends included (src/cuda/agpt_train.cu:4601-4607)
         g = space.group(ids, [], mass_mode, model.cfg.seq_len, model.device)
         opt.zero_grad(set_to_none=False)
-        ls, nq = model.group_step(g, counts, **loss_kw)
+        ls, nq = 0.0, 0
+        if native:
+            pending.append(model.group_step(g, counts, sync=None, **loss_kw))
+        else:
+            ls, nq = model.group_step(g, counts, **loss_kw)
         if hasattr(opt, "lr_scale"):
             opt.lr_scale = float(lr_w[s])
         opt.step()
         loss_sum += ls
         n_q += nq
         n_nodes += int(ids.size)
+    if pending:
+        import torch
+        for ls, nq in _step_stats(torch.stack(pending).cpu()):
+            loss_sum += ls
+            n_q += nq
     return loss_sum, n_q, n_nodes, rng_state
 
 

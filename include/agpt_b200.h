@@ -225,6 +225,10 @@ typedef struct {
  * With device >= 0 the index arrays are also allocated on that device (freed by plan_destroy). */
 int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_m, int device, agpt_plan **out);
 int agpt_b200_plan_info(const agpt_plan *p, agpt_plan_info *out);
+/* The sizes alone (array pointers NULL): the row arrays of a plan that came from runs of rows are derived when asked for. */
+int agpt_b200_plan_sizes(const agpt_plan *p, agpt_plan_info *out);
+/* One of the row arrays copied to out [n]: 0 dfs_to_node, 1 node_to_dfs, 2 parent_dfs, 3 depth, 4 sub_end. */
+int agpt_b200_plan_array(const agpt_plan *p, int which, int32_t *out);
 void agpt_b200_plan_destroy(agpt_plan *p);
 /* Bytes of scratch attn_bwd needs for `d_model` columns. */
 int64_t agpt_b200_attn_bwd_workspace_bytes(const agpt_plan *p, int d_model);
@@ -261,6 +265,30 @@ int64_t agpt_b200_groups_count(const agpt_groups *g);
 int agpt_b200_groups_get(const agpt_groups *g, int64_t i, agpt_group_info *out);
 void agpt_b200_groups_free(agpt_groups *g);
 
+/* The same groups straight from a radix trie, for the training step: units of `level` (1 or 2), cut deeper above unit_cap
+ * rows (0: not), balanced over n_ranks, packed into groups of at most group_rows rows -- the arrays of
+ * agpt_b200_trie_char_tree + agpt_b200_plan_create + agpt_b200_groups_create, but decided per radix edge and expanded to
+ * rows on the device.  trie_sample_group: one group of a set of radix nodes closed under "parent" (context: the nodes that
+ * carry no loss; rank: agpt_b200_trie_ranks).  The trie must outlive the handle.
+ * prepare computes group i and says where its arrays will lie in a device buffer of info.bytes (16-byte aligned; -1: not
+ * there): tokens, pos, q2n, edge_first [n] int32, unit_of_row [n] int64, mass_w, trained [n] float, qoff [n_loss_nodes + 1]
+ * and rid [n_loss_nodes] int32, unit_off [n_units + 1] int64.  upload fills the buffer of the group prepared last
+ * (asynchronous on stream) and returns its plan, whose device arrays lie in the same buffer: it must outlive the plan. */
+typedef struct agpt_run_groups agpt_run_groups;
+typedef struct {
+    int64_t n, n_loss_nodes, n_trained, bytes;
+    int32_t n_units, n_pos, seq_len;
+    int64_t tokens, pos, q2n, edge_first, unit_of_row, mass_w, trained, qoff, rid, unit_off;
+} agpt_run_group_info;
+int agpt_b200_trie_groups_create(const agpt_trie *t, int level, int64_t unit_cap, int n_ranks, int rank, int64_t group_rows,
+                                 agpt_run_groups **out);
+int agpt_b200_trie_ranks(const agpt_trie *t, int32_t *rank_out /* [radix_count] */);
+int agpt_b200_trie_sample_group(const agpt_trie *t, const int32_t *rank, const int32_t *nodes, int64_t n_nodes,
+                                const int32_t *context, int64_t n_context, agpt_run_groups **out);
+int64_t agpt_b200_trie_groups_count(const agpt_run_groups *g);
+int agpt_b200_trie_group_prepare(agpt_run_groups *g, int64_t i, int tile_m, int mass_mode, int seq_len, agpt_run_group_info *out);
+int agpt_b200_trie_group_upload(agpt_run_groups *g, int device, void *d_buffer, void *stream, agpt_plan **plan_out);
+void agpt_b200_trie_groups_free(agpt_run_groups *g);
 
 /* ---- device kernels (all asynchronous on `stream`, a cudaStream_t passed as void*) ---- */
 
