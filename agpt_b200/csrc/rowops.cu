@@ -204,38 +204,86 @@ __global__ void __launch_bounds__(256) embedding_scatter_atomic_kernel(const flo
     }
 }
 
-// Native form: block b sums its rows [b*chunk, ...) into a [vocab][DT] table in shared memory for the column tile
-// blockIdx.y (thread = column, rows visited in order: no atomics), and writes it to partial[b]; the finish kernel
-// adds the blocks in order.
-__global__ void __launch_bounds__(128) embedding_grad_kernel(const float *__restrict__ grad, const int *__restrict__ ids, int64_t n, int d,
-                                                              int vocab, int64_t chunk, float *__restrict__ partial) {
-    extern __shared__ float s_tab[];                  // [vocab][128]
-    const int c = blockIdx.y * 128 + threadIdx.x;
-    for (int v = 0; v < vocab; v++) s_tab[v * 128 + threadIdx.x] = 0.f;
+// Native form: a block is ONE warp.  It sums its rows [b*chunk, ...) into a [vocab][32 W] table of its own in shared memory
+// (lane = W neighbouring columns, rows visited in order: no atomics, no barriers) and writes it to partial[b]; the finish
+// kernel adds the blocks in order.  The ids and gradients of eight rows are in flight while the tables of the rows before are
+// updated, and about six such warps share an SM: bound by memory.  Measured with 65 symbols: 66k x 64 331 -> 27 us, 560k x 128
+// 675 -> 109 us (a block of four warps on one table, one row at a time: every row waited for its load).
+template <int W>
+__global__ void __launch_bounds__(32) embedding_grad_kernel(const float *__restrict__ grad, const int *__restrict__ ids, int64_t n, int d,
+                                                             int vocab, int64_t chunk, float *__restrict__ partial) {
+    extern __shared__ float s_tab[];                  // [vocab][32 W]
+    constexpr int U = 8;
+    const int lane = threadIdx.x, c = blockIdx.y * 32 * W + lane * W;
+    for (int i = lane; i < vocab * 32 * W; i += 32) s_tab[i] = 0.f;
+    __syncwarp();
     const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = (r0 + chunk < n) ? r0 + chunk : n;
+    auto load = [&](int64_t r, float (&v)[W]) {
+        if (W == 4) {
+            const float4 x = __ldcs(reinterpret_cast<const float4 *>(grad + r * d + c));
+            v[0] = x.x; v[1 % W] = x.y; v[2 % W] = x.z; v[3 % W] = x.w;
+        } else if (W == 2) {
+            const float2 x = __ldcs(reinterpret_cast<const float2 *>(grad + r * d + c));
+            v[0] = x.x; v[1 % W] = x.y;
+        } else v[0] = __ldcs(grad + r * d + c);
+    };
+    auto add = [&](int id, const float (&v)[W]) {
+        if (id < 0 || id >= vocab) return;
+        float *t = s_tab + id * 32 * W + lane * W;
+#pragma unroll
+        for (int w = 0; w < W; w++) t[w] += v[w];
+    };
     if (c < d) {
-        for (int64_t r = r0; r < r1; r++) {
-            int id = __ldg(ids + r);
-            if (id >= 0 && id < vocab) s_tab[id * 128 + threadIdx.x] += grad[r * d + c];
+        int64_t r = r0;
+        for (; r + U <= r1; r += U) {
+            int id[U];
+            float v[U][W];
+#pragma unroll
+            for (int u = 0; u < U; u++) { id[u] = __ldg(ids + r + u); load(r + u, v[u]); }
+#pragma unroll
+            for (int u = 0; u < U; u++) add(id[u], v[u]);
         }
-        float *dst = partial + (int64_t)blockIdx.x * vocab * d;
-        for (int v = 0; v < vocab; v++) dst[(int64_t)v * d + c] = s_tab[v * 128 + threadIdx.x];
+        for (; r < r1; r++) { float v[W]; load(r, v); add(__ldg(ids + r), v); }
+        float *dst = partial + (int64_t)blockIdx.x * vocab * d + c;
+        for (int k = 0; k < vocab; k++)
+#pragma unroll
+            for (int w = 0; w < W; w++) dst[(int64_t)k * d + w] = s_tab[k * 32 * W + lane * W + w];
     }
 }
 
 __global__ void __launch_bounds__(256) embedding_grad_finish_kernel(const float *__restrict__ partial, int blocks, int64_t vd, int accumulate,
                                                                      float *__restrict__ demb) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= vd) return;
+    __shared__ float s[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t i = (int64_t)blockIdx.x * 32 + lane;
     float t = 0.f;
-    for (int b = 0; b < blocks; b++) t += partial[(int64_t)b * vd + i];
+    if (i < vd)
+#pragma unroll 4
+        for (int b = w; b < blocks; b += 8) t += __ldcs(partial + (int64_t)b * vd + i);
+    s[w][lane] = t;
+    __syncthreads();
+    if (w || i >= vd) return;
+    t = 0.f;
+    for (int k = 0; k < 8; k++) t += s[k][lane];
     demb[i] = (accumulate ? demb[i] : 0.f) + t;
 }
 
 int embedding_blocks(int64_t n) {
-    int64_t b = (n + 2047) / 2048;
-    int64_t cap = (int64_t)sm_count() * 2;
+    int64_t b = (n + 255) / 256;
+    int64_t cap = (int64_t)sm_count() * 6;
     return (int)(b < 1 ? 1 : (b < cap ? b : cap));
+}
+
+template <int W>
+void launch_embedding_grad(const float *grad, const int *ids, int64_t n, int d, int vocab, int blocks, float *partial, cudaStream_t st) {
+    static bool attr_set[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+        cudaFuncSetAttribute(embedding_grad_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        attr_set[dev] = true;
+    }
+    embedding_grad_kernel<W><<<dim3(blocks, (d + 32 * W - 1) / (32 * W)), 32, (size_t)vocab * 32 * W * 4, st>>>(grad, ids, n, d, vocab, (n + blocks - 1) / blocks, partial);
 }
 
 }  // namespace
@@ -338,18 +386,13 @@ extern "C" int agpt_b200_embedding_grad(const float *d_grad, const int32_t *d_id
     if (!d_workspace || workspace_bytes < (int64_t)blocks * vocab * d_model * 4)
         return agpt_set_error(AGPT_E_ARG, "embedding_grad: workspace too small (agpt_b200_embedding_grad_workspace_bytes)");
     cudaStream_t st = (cudaStream_t)stream;
-    static bool attr_set[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        cudaFuncSetAttribute(embedding_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        attr_set[dev] = true;
-    }
-    const int64_t chunk = (n + blocks - 1) / blocks;
-    dim3 grid(blocks, (d_model + 127) / 128);
-    embedding_grad_kernel<<<grid, 128, smem, st>>>(d_grad, d_ids, n, d_model, vocab, chunk, (float *)d_workspace);
+    // as wide a piece per lane as the row's alignment and width allow
+    if (d_model % 4 == 0 && d_model > 64 && aligned16(d_grad)) launch_embedding_grad<4>(d_grad, d_ids, n, d_model, vocab, blocks, (float *)d_workspace, st);
+    else if (d_model % 2 == 0 && d_model > 32 && (reinterpret_cast<uintptr_t>(d_grad) & 7) == 0)
+        launch_embedding_grad<2>(d_grad, d_ids, n, d_model, vocab, blocks, (float *)d_workspace, st);
+    else launch_embedding_grad<1>(d_grad, d_ids, n, d_model, vocab, blocks, (float *)d_workspace, st);
     const int64_t vd = (int64_t)vocab * d_model;
-    embedding_grad_finish_kernel<<<(unsigned)((vd + 255) / 256), 256, 0, st>>>((const float *)d_workspace, blocks, vd, accumulate, d_emb_grad);
+    embedding_grad_finish_kernel<<<(unsigned)((vd + 31) / 32), 256, 0, st>>>((const float *)d_workspace, blocks, vd, accumulate, d_emb_grad);
     return launch_status("embedding_grad");
 }
 
