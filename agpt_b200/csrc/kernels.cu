@@ -2893,8 +2893,12 @@ static int attn_fwd_bwd_host_impl(const agpt_plan *cp, const float *h_q, const f
     const size_t lseb = (((size_t)n * n_heads * sizeof(float)) + 255) & ~(size_t)255;
     const size_t wsb = (((size_t)agpt_b200_attn_bwd_workspace_bytes(p, D)) + 255) & ~(size_t)255;
     const bool bf = kv_dtype == AGPT_KV_BF16;
-    // chunks of about 64 MB per tensor, whole tiles
-    const int64_t ch_rows = std::max<int64_t>(M, ((64ll << 20) / (int64_t)rowb) / M * M);
+    // Chunks of whole tiles.  What the two directions of the link cannot share is the first chunk's way up and the last one's
+    // way down, so the tensor is cut into about ten chunks (64 MB at most); more, or below 2 MB per tensor, cost more in copies
+    // (nine per chunk) than they save.  174k rows of 128: 11.6 ms in two chunks of 64 MB, 8.8 in ten, 9.4 in 24 (8.0 ms would
+    // be both directions at the 44.7 GB/s each that they reach together).
+    const int64_t ch_bytes = std::min<int64_t>(64ll << 20, std::max<int64_t>(2ll << 20, n * (int64_t)rowb / 10));
+    const int64_t ch_rows = std::max<int64_t>(M, (ch_bytes / (int64_t)rowb) / M * M);
     const int64_t n_ch = (n + ch_rows - 1) / ch_rows;
     const size_t fix_dev_cap = (((size_t)n_ch * (size_t)p->max_depth + p->multi_node.size()) * (2 * rowb + sizeof(int32_t)) + 511) & ~(size_t)255;
     const size_t need = 8 * tens + lseb + wsb + (bf ? tens : 0) + fix_dev_cap;
