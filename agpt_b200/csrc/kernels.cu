@@ -1653,6 +1653,173 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     }
 }
 
+// --------------------------------------------------------------------------------------
+// forward for a bfloat16 store: attn_fwd_bf16_kernel.  K and V rows go to the tensor cores as they are stored: one cp.async per
+// 16 bytes, no conversion, fragments by ldmatrix (16-byte chunks XOR-swizzled with the row).  What is computed in float32 --
+// Q scaled, and P -- is split into two bfloat16 parts (16 significant bits), so a product is two m16n8k16 MMAs, the cost of
+// the one TF32 product of 11 bits per factor that the chunked kernel issues.  Q fragments come straight from global memory.
+// One warp per 16 query rows, online softmax over blocks of 16 keys, 16 x 8 blocks without a valid pair skipped.
+// Bound by issue slots and, on shallow tries, by memory.  Measured (against the chunked TF32 kernel): 8 x 32, 577k rows
+// 636 -> 568 us; 6 x 64, 719k rows of depth up to 128, 1797 -> 1303 us.
+// --------------------------------------------------------------------------------------
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// (x, y) = hi + lo as packed bfloat16 pairs (x in the low half): 16 significant bits, the exponent range of float32
+__device__ __forceinline__ void bf16_split2(float x, float y, uint32_t &hi, uint32_t &lo) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(x - __uint_as_float(hi << 16), y - __uint_as_float(hi & 0xffff0000u));
+    lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+// byte offset of 16-byte chunk c of row r of bfloat16 rows of HD: eight neighbouring rows' same chunk falls into eight
+// different bank groups
+template <int HD>
+__device__ __forceinline__ uint32_t bf16_chunk(int r, int c) {
+    constexpr int SH = HD == 64 ? 0 : HD == 32 ? 1 : 2;
+    return (uint32_t)(r * (HD * 2) + ((c ^ ((r >> SH) & (HD / 8 - 1))) << 4));
+}
+constexpr size_t fwd_bf16_smem_bytes(int hd, int maxk) { return (size_t)maxk * (hd * 4 + 8); }
+
+template <int HD, int MINB>
+__global__ void __launch_bounds__(128, MINB)
+attn_fwd_bf16_kernel(const float *__restrict__ Q, const __nv_bfloat16 *__restrict__ K, const __nv_bfloat16 *__restrict__ V,
+                     float *__restrict__ O, float *__restrict__ LSE, const int32_t *__restrict__ sub_end,
+                     const int64_t *__restrict__ chain_off, const int32_t *__restrict__ chain_ids,
+                     const int32_t *__restrict__ chain_end_all, int n, int H, float scale, int tile0, int maxk) {
+    constexpr int M = 64, NT = 128, KS = HD / 16, NDB = HD / 8, NCH = HD / 8;
+    extern __shared__ __align__(128) unsigned char tile_smem_raw[];
+    unsigned char *sK = tile_smem_raw, *sV = sK + (size_t)maxk * (HD * 2);
+    int2 *s_meta = reinterpret_cast<int2 *>(sV + (size_t)maxk * (HD * 2));           // [maxk] {key id, key subtree end}
+    const int t = blockIdx.x + tile0, h = blockIdx.y, tid = threadIdx.x;
+    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
+    const int D = H * HD, hoff = h * HD;
+    const int i0 = t * M, nt = min(M, n - i0);
+    const int64_t coff = chain_off[t];
+    const int p = (int)(chain_off[t + 1] - coff);
+    const int nkeys = p + nt, nkp = (nkeys + 15) & ~15;
+    const int32_t *chain = chain_ids + coff, *chain_end = chain_end_all + coff;
+
+    for (int idx = tid; idx < nkp * NCH; idx += NT) {
+        const int r = idx / NCH, c = idx % NCH;
+        const uint32_t o = bf16_chunk<HD>(r, c);
+        if (r < nkeys) {
+            const int kid = r < p ? __ldg(chain + r) : i0 + (r - p);
+            const int64_t off = (int64_t)kid * D + hoff + c * 8;
+            cp_async16(sK + o, K + off); cp_async16(sV + o, V + off);
+        } else {
+            *reinterpret_cast<uint4 *>(sK + o) = make_uint4(0u, 0u, 0u, 0u);
+            *reinterpret_cast<uint4 *>(sV + o) = make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+    cp_async_commit();
+    for (int j = tid; j < nkp; j += NT) {
+        int kid = 0x7fffffff, kend = 0;
+        if (j < p) { kid = __ldg(chain + j); kend = __ldg(chain_end + j); }
+        else if (j < nkeys) { kid = i0 + (j - p); kend = __ldg(sub_end + kid); }
+        s_meta[j] = make_int2(kid, kend);
+    }
+    const int rg = warp, q0 = rg * 16 + g;
+    const int r0 = i0 + q0, r1 = r0 + 8;
+    uint32_t qh[KS][4], ql[KS][4];
+    {
+        const float qs = scale * LOG2E;
+        const float *p0 = Q + (int64_t)r0 * D + hoff + 2 * tig, *p1 = p0 + (int64_t)8 * D;
+#pragma unroll
+        for (int ks = 0; ks < KS; ks++) {
+            float2 x[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)        // rows r0, r1 of columns 2 tig; then of columns 2 tig + 8
+                x[j] = ((j & 1) ? r1 : r0) < n ? __ldg(reinterpret_cast<const float2 *>(((j & 1) ? p1 : p0) + ks * 16 + (j >> 1) * 8)) : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < 4; j++) bf16_split2(x[j].x * qs, x[j].y * qs, qh[ks][j], ql[ks][j]);
+        }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    if (rg * 16 >= nt) return;                                   // rows beyond the end of the plan (no barrier follows)
+
+    const int l8 = lane & 7, mi = lane >> 3;
+    const uint32_t uK = smem_u32_of(sK), uV = smem_u32_of(sV);
+    float o_[NDB][4];
+#pragma unroll
+    for (int db = 0; db < NDB; db++) o_[db][0] = o_[db][1] = o_[db][2] = o_[db][3] = 0.f;
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+    const int kp_lim = min(nkp >> 4, (p + rg * 16 + 16 + 15) >> 4);
+    for (int kp = 0; kp < kp_lim; kp++) {
+        bool vld[2][4];
+        bool on[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int4 mk = *reinterpret_cast<const int4 *>(&s_meta[kp * 16 + u * 8 + 2 * tig]);
+            vld[u][0] = mk.x <= r0 && r0 < mk.y; vld[u][1] = mk.z <= r0 && r0 < mk.w;
+            vld[u][2] = mk.x <= r1 && r1 < mk.y; vld[u][3] = mk.z <= r1 && r1 < mk.w;
+            on[u] = __any_sync(0xffffffffu, vld[u][0] | vld[u][1] | vld[u][2] | vld[u][3]);
+        }
+        if (!(on[0] || on[1])) continue;
+        float s2[2][4];
+        // B fragments of the block's 16 keys for k-step ks: matrices {keys 0-7 chunk 2ks, keys 0-7 chunk 2ks+1, keys 8-15 ..}
+        float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, cx[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int ks = 0; ks < KS; ks++) {
+            uint32_t kf[4];
+            ldmatrix_x4(kf, uK + bf16_chunk<HD>(kp * 16 + (mi >> 1) * 8 + l8, 2 * ks + (mi & 1)));
+#pragma unroll
+            for (int u = 0; u < 2; u++) { mma_bf16(c[u], qh[ks], kf[2 * u], kf[2 * u + 1]); mma_bf16(cx[u], ql[ks], kf[2 * u], kf[2 * u + 1]); }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) s2[u][j] = vld[u][j] ? c[u][j] + cx[u][j] : -INFINITY;
+        float mx0 = fmaxf(fmaxf(s2[0][0], s2[0][1]), fmaxf(s2[1][0], s2[1][1]));
+        float mx1 = fmaxf(fmaxf(s2[0][2], s2[0][3]), fmaxf(s2[1][2], s2[1][3]));
+        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+        const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
+        const float mu0 = mn0 == -INFINITY ? 0.f : mn0, mu1 = mn1 == -INFINITY ? 0.f : mn1;
+        if (__any_sync(0xffffffffu, mn0 != m0 || mn1 != m1)) {   // a maximum moved: rescale
+            const float corr0 = ex2_ftz(m0 - mu0), corr1 = ex2_ftz(m1 - mu1);
+            l0 *= corr0; l1 *= corr1;
+#pragma unroll
+            for (int db = 0; db < NDB; db++) { o_[db][0] *= corr0; o_[db][1] *= corr0; o_[db][2] *= corr1; o_[db][3] *= corr1; }
+        }
+        m0 = mn0; m1 = mn1;
+        uint32_t ph[4], pl[4];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const float p0 = ex2_ftz(s2[u][0] - mu0), p1 = ex2_ftz(s2[u][1] - mu0), p2 = ex2_ftz(s2[u][2] - mu1), p3 = ex2_ftz(s2[u][3] - mu1);
+            l0 += p0 + p1; l1 += p2 + p3;
+            bf16_split2(p0, p1, ph[2 * u], pl[2 * u]); bf16_split2(p2, p3, ph[2 * u + 1], pl[2 * u + 1]);
+        }
+        // matrices {keys 0-7 dims 16 dp.., keys 8-15 the same, keys 0-7 dims 16 dp + 8.., keys 8-15}
+#pragma unroll
+        for (int dp = 0; dp < NDB / 2; dp++) {
+            uint32_t vt[4];
+            ldmatrix_x4_trans(vt, uV + bf16_chunk<HD>(kp * 16 + (mi & 1) * 8 + l8, 2 * dp + (mi >> 1)));
+#pragma unroll
+            for (int u = 0; u < 2; u++) { mma_bf16(o_[2 * dp + u], ph, vt[2 * u], vt[2 * u + 1]); mma_bf16(o_[2 * dp + u], pl, vt[2 * u], vt[2 * u + 1]); }
+        }
+    }
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+    if (r0 < n) {
+        const float inv = 1.0f / l0;
+#pragma unroll
+        for (int db = 0; db < NDB; db++)
+            *reinterpret_cast<float2 *>(O + (int64_t)r0 * D + hoff + db * 8 + 2 * tig) = make_float2(o_[db][0] * inv, o_[db][1] * inv);
+        if (tig == 0) LSE[(int64_t)r0 * H + h] = (m0 + log2f(l0)) * LN2;
+    }
+    if (r1 < n) {
+        const float inv = 1.0f / l1;
+#pragma unroll
+        for (int db = 0; db < NDB; db++)
+            *reinterpret_cast<float2 *>(O + (int64_t)r1 * D + hoff + db * 8 + 2 * tig) = make_float2(o_[db][2] * inv, o_[db][3] * inv);
+        if (tig == 0) LSE[(int64_t)r1 * H + h] = (m1 + log2f(l1)) * LN2;
+    }
+}
+
 // dK/dV reduction, pass 1: one warp per work item = (node, tile range).  The node's row in tile t's
 // partial block is chain_off[t] + depth - 1.  Tiles are summed in increasing order.
 __global__ void reduce_items_kernel(const float *__restrict__ Pk, const float *__restrict__ Pv, float *__restrict__ dK,
@@ -1838,6 +2005,19 @@ static int launch_fwd_tile(const agpt_plan *p, const float *q, const void *k, co
     return launch_status("attn_fwd_tile");
 }
 
+template <int HD, int MINB>
+static int launch_fwd_bf16(const agpt_plan *p, const float *q, const void *k, const void *v, float *out, float *lse, int H,
+                           float scale, cudaStream_t st, int tile0, int ntiles) {
+    static size_t granted[AGPT_MAX_DEVICES];
+    const int maxk = bwd_tile_maxk(p);
+    const size_t smem = fwd_bf16_smem_bytes(HD, maxk);
+    if (int rc = allow_dynamic_smem(attn_fwd_bf16_kernel<HD, MINB>, smem, granted)) return rc;
+    attn_fwd_bf16_kernel<HD, MINB><<<dim3((unsigned)ntiles, (unsigned)H), 128, smem, st>>>(
+        q, (const __nv_bfloat16 *)k, (const __nv_bfloat16 *)v, out, lse, p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_chain_end, (int)p->n, H,
+        scale, tile0, maxk);
+    return launch_status("attn_fwd_bf16");
+}
+
 template <int HD, typename KVT>
 static int launch_fwd_mma(const agpt_plan *p, const float *q, const void *k, const void *v, float *out, float *lse, int H,
                           float scale, cudaStream_t st, int tile0, int ntiles) {
@@ -1864,11 +2044,20 @@ static int fwd_dispatch(const agpt_plan *p, const float *q, const void *k, const
         if (blocks == 6) return launch_fwd_tile<32, 6, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
         return launch_fwd_tile<32, 5, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
     }
-    if (attn_impl() == 1 && p->tile_m == 64 && p->max_depth + 64 <= MAXKEYS) {
-        const bool bf = kv_dtype == AGPT_KV_BF16;
+    // bfloat16 store: whole tiles while two blocks of them fit one SM (head_dim 64: up to 438 keys), deeper plans in chunks
+    if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_BF16 &&
+        fwd_bf16_smem_bytes(head_dim, bwd_tile_maxk(p)) <= (size_t)113 * 1024) {
         switch (head_dim) {
-            case 16: return bf ? launch_fwd_mma<16, __nv_bfloat16>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles) : launch_fwd_mma<16, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
-            case 32: return bf ? launch_fwd_mma<32, __nv_bfloat16>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles) : launch_fwd_mma<32, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            case 16: return launch_fwd_bf16<16, 8>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            case 32: return launch_fwd_bf16<32, 6>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            case 64: return launch_fwd_bf16<64, 4>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+        }
+    }
+    if (attn_impl() == 1 && p->tile_m == 64 && p->max_depth + 64 <= MAXKEYS) {
+        const bool bf = kv_dtype == AGPT_KV_BF16;        // (head_dim 16 and 32: MAXKEYS keys fit the whole-tile kernel)
+        switch (head_dim) {
+            case 16: return launch_fwd_mma<16, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            case 32: return launch_fwd_mma<32, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
             case 64: return bf ? launch_fwd_mma<64, __nv_bfloat16>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles) : launch_fwd_mma<64, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
         }
     }
