@@ -85,11 +85,11 @@ __global__ void __launch_bounds__(256) expand_runs_kernel(const int32_t *__restr
 
 // ancestor chain of the first row of every tile, root side first: up its own run, then run by run
 __global__ void __launch_bounds__(128) tile_chain_kernel(const int32_t *__restrict__ qoff, const int32_t *__restrict__ prun, const int32_t *__restrict__ send,
-                                                          const int64_t *__restrict__ chain_off, int runs, int64_t tiles, int tile_m,
+                                                          const int64_t *__restrict__ chain_off, const int32_t *__restrict__ tile_start, int runs, int64_t tiles,
                                                           int32_t *__restrict__ ids, int32_t *__restrict__ ends) {
     const int64_t t = (int64_t)blockIdx.x * 128 + threadIdx.x;
     if (t >= tiles) return;
-    int row = (int)(t * tile_m), lo = 0, hi = runs - 1;
+    int row = tile_start[t], lo = 0, hi = runs - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (qoff[mid] <= row) lo = mid; else hi = mid - 1;
@@ -116,7 +116,7 @@ struct agpt_run_groups {
     agpt_plan *plan = nullptr;
     agpt_run_group_info info;
     int64_t at_prun = 0, at_fd = 0, at_ld = 0, at_send = 0, at_unit = 0, at_first = 0, at_mw = 0, at_tr = 0, at_choff = 0, at_items[4] = {0, 0, 0, 0},
-            at_multi = 0, at_mcount = 0, at_mfirst = 0, at_depth = 0, at_subend = 0, at_cid = 0, at_cend = 0;
+            at_multi = 0, at_mcount = 0, at_mfirst = 0, at_ts = 0, at_depth = 0, at_subend = 0, at_cid = 0, at_cend = 0;
     ~agpt_run_groups() { delete plan; }
 };
 
@@ -242,7 +242,7 @@ extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int t
     const int64_t n = g.rows(), M = tile_m;
     delete G->plan;
     agpt_plan *P = G->plan = new agpt_plan();
-    P->n = n; P->tile_m = tile_m; P->n_tiles = (n + M - 1) / M;
+    P->n = n; P->tile_m = tile_m;
     P->lazy = true;
     P->run_qoff.assign(g.qoff.begin(), g.qoff.end()); P->run_parent = g.prun;
     std::vector<int32_t> &ld = P->run_depth, &send = P->run_end;
@@ -263,25 +263,55 @@ extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int t
         const int64_t inner = len - (send[e] > g.qoff[e + 1] ? 0 : 1);
         P->n_groups += inner; P->sum_group_prefix += inner * d0 + inner * (inner - 1) / 2;
     }
-    P->chain_off.resize(P->n_tiles + 1);
-    P->chain_off[0] = 0;
-    for (int64_t tl = 0, e = 0; tl < P->n_tiles; tl++) {
-        while (g.qoff[e + 1] <= tl * M) e++;
-        P->chain_off[tl + 1] = P->chain_off[tl] + (ld[e] + (tl * M - g.qoff[e]) - 1);
+    // tiles, as agpt_b200_plan_create cuts them: depths grow along a run, so only its first row in reach can be a better end
+    std::vector<int32_t> &ts = P->tile_start;
+    ts.reserve(n / 32 + 2);
+    P->chain_off.reserve(n / 32 + 2);
+    P->chain_off.push_back(0);
+    int64_t e0 = 0;                             // the run of the tile's first row
+    for (int64_t i = 0; i < n;) {
+        ts.push_back((int32_t)i);
+        int64_t k = std::min(M, n - i), e1 = e0;
+        if (tile_m == 64 && i + M < n) {
+            while (g.qoff[e1 + 1] <= i + 32) e1++;
+            int64_t best = INT64_MAX;
+            for (int64_t e = e1; e < E && g.qoff[e] <= i + M; e++) {
+                const int64_t c = std::max<int64_t>(g.qoff[e] - i, 32), v = agpt_tile_cost((int32_t)(ld[e] + (i + c - g.qoff[e])), c);
+                if (v <= best) { best = v; k = c; e1 = e; }
+            }
+        } else while (e1 < E && g.qoff[e1 + 1] <= i + k) e1++;
+        const int64_t chain = ld[e0] + (i - g.qoff[e0]) - 1;
+        P->chain_off.push_back(P->chain_off.back() + chain);
+        P->max_keys = std::max(P->max_keys, (int32_t)(chain + k));
+        i += k; e0 = e1;
     }
+    P->n_tiles = (int64_t)ts.size();
+    ts.push_back((int32_t)n);
     P->chain_rows = P->chain_off[P->n_tiles];
     // reduction work list: the rows whose subtree reaches into later tiles, ordered by their last tile (a counting sort)
     {
         constexpr int32_t SEG = AGPT_REDUCE_SEG;
-        const int shift = tile_m == 32 ? 5 : tile_m == 64 ? 6 : 7;
         std::vector<int64_t> start(P->n_tiles + 1, 0);
+        std::vector<int32_t> last_tile(E);      // tile of the last row of a run's subtree
+        {   // of every run's last row first; a run's subtree ends with a run's last row
+            std::vector<int32_t> run_end_tile(E);
+            for (int32_t e = 0, t = 0; e < E; e++) {
+                while (ts[t + 1] < g.qoff[e + 1]) t++;
+                run_end_tile[e] = t;
+            }
+            for (int32_t e = E - 1; e >= 0; e--) last_tile[e] = run_end_tile[e];
+            for (int32_t e = E - 1; e >= 0; e--)
+                if (g.prun[e] >= 0) last_tile[g.prun[e]] = std::max(last_tile[g.prun[e]], last_tile[e]);
+        }
         // f(first row, one past the last row, first tile, last tile): the rows of a run that lie in one tile
         auto each = [&](auto &&f) {
+            int32_t t = 0;
             for (int32_t e = 0; e < E; e++) {
-                const int32_t t1 = (send[e] - 1) >> shift, last = std::min(g.qoff[e + 1], t1 << shift);
-                for (int32_t a = g.qoff[e]; a < last;) {
-                    const int32_t t0 = (a >> shift) + 1, b = std::min(last, t0 << shift);
-                    f(a, b, t0, t1);
+                const int32_t t1 = last_tile[e], last = std::min(g.qoff[e + 1], ts[t1]);
+                while (ts[t + 1] <= g.qoff[e]) t++;
+                for (int32_t a = g.qoff[e], u = t; a < last; u++) {
+                    const int32_t b = std::min(last, ts[u + 1]);
+                    f(a, b, u + 1, t1);
                     a = b;
                 }
             }
@@ -321,7 +351,7 @@ extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int t
     o.qoff = take((int64_t)(E + 1) * 4); o.rid = take((int64_t)E * 4);
     G->at_prun = take((int64_t)E * 4); G->at_fd = take((int64_t)E * 4); G->at_ld = take((int64_t)E * 4); G->at_send = take((int64_t)E * 4);
     G->at_unit = take((int64_t)E * 4); G->at_first = take((int64_t)E * 4); G->at_mw = take((int64_t)E * 4); G->at_tr = take(E);
-    G->at_choff = take((P->n_tiles + 1) * 8);
+    G->at_choff = take((P->n_tiles + 1) * 8); G->at_ts = take((P->n_tiles + 1) * 4);
     const std::vector<int32_t> *items[4] = {&P->item_node, &P->item_t0, &P->item_t1, &P->item_slot};
     for (int k = 0; k < 4; k++) G->at_items[k] = take((int64_t)items[k]->size() * 4);
     const int64_t nm = (int64_t)P->multi_node.size();
@@ -351,7 +381,7 @@ extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int t
     put(o.qoff, g.qoff.data(), (int64_t)(E + 1) * 4); put(o.rid, g.rid.data(), (int64_t)E * 4);
     put(G->at_prun, g.prun.data(), (int64_t)E * 4); put(G->at_ld, ld.data(), (int64_t)E * 4); put(G->at_send, send.data(), (int64_t)E * 4);
     put(G->at_unit, g.unit.data(), (int64_t)E * 4); put(G->at_tr, g.trained.data(), E);
-    put(G->at_choff, P->chain_off.data(), (P->n_tiles + 1) * 8);
+    put(G->at_choff, P->chain_off.data(), (P->n_tiles + 1) * 8); put(G->at_ts, P->tile_start.data(), (P->n_tiles + 1) * 4);
     for (int k = 0; k < 4; k++) put(G->at_items[k], items[k]->data(), (int64_t)items[k]->size() * 4);
     put(G->at_multi, P->multi_node.data(), nm * 4); put(G->at_mcount, P->multi_count.data(), nm * 4); put(G->at_mfirst, P->multi_first.data(), nm * 8);
     int32_t *fd = (int32_t *)(s + G->at_fd), *first = (int32_t *)(s + G->at_first), *tok = (int32_t *)(s + o.tokens);
@@ -389,15 +419,15 @@ extern "C" int agpt_b200_trie_group_upload(agpt_run_groups *G, int device, void 
     const int E = (int)o.n_loss_nodes;
     P->device = device; P->external = true;
     P->d_depth = i32(G->at_depth); P->d_sub_end = i32(G->at_subend); P->d_chain_ids = i32(G->at_cid); P->d_chain_end = i32(G->at_cend);
-    P->d_chain_off = (int64_t *)(d + G->at_choff);
+    P->d_chain_off = (int64_t *)(d + G->at_choff); P->d_tile_start = i32(G->at_ts);
     P->d_item_node = i32(G->at_items[0]); P->d_item_t0 = i32(G->at_items[1]); P->d_item_t1 = i32(G->at_items[2]); P->d_item_slot = i32(G->at_items[3]);
     P->d_multi_node = i32(G->at_multi); P->d_multi_count = i32(G->at_mcount); P->d_multi_first = (int64_t *)(d + G->at_mfirst);
     expand_runs_kernel<<<(E + 7) / 8, 256, 0, st>>>(i32(o.qoff), i32(G->at_fd), i32(G->at_ld), i32(G->at_send), i32(G->at_unit), i32(G->at_first),
                                                     (const float *)(d + G->at_mw), d + G->at_tr, E, o.seq_len, i32(o.pos), i32(o.q2n), i32(o.edge_first),
                                                     (int64_t *)(d + o.unit_of_row), o.mass_w < 0 ? nullptr : (float *)(d + o.mass_w),
                                                     o.trained < 0 ? nullptr : (float *)(d + o.trained), P->d_depth, P->d_sub_end);
-    tile_chain_kernel<<<(unsigned)((P->n_tiles + 127) / 128), 128, 0, st>>>(i32(o.qoff), i32(G->at_prun), i32(G->at_send), P->d_chain_off, E, P->n_tiles,
-                                                                            P->tile_m, P->d_chain_ids, P->d_chain_end);
+    tile_chain_kernel<<<(unsigned)((P->n_tiles + 127) / 128), 128, 0, st>>>(i32(o.qoff), i32(G->at_prun), i32(G->at_send), P->d_chain_off, P->d_tile_start, E, P->n_tiles,
+                                                                            P->d_chain_ids, P->d_chain_end);
     err = cudaGetLastError();
     if (err != cudaSuccess) return agpt_set_error(AGPT_E_CUDA, "trie_group_upload: %s", cudaGetErrorString(err));
     *plan_out = P;

@@ -775,24 +775,44 @@ extern "C" int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_
     }
     P->max_depth = 0; P->sum_depth = 0;
     for (int64_t i = 0; i < n; i++) { P->max_depth = std::max(P->max_depth, P->depth[i]); P->sum_depth += P->depth[i]; }
-    // tiles: chain of the first query of each tile, root side first
-    P->n_tiles = (n + tile_m - 1) / tile_m;
+    // tiles; the chain of the first query of each, root side first
+    const bool early = device >= 0 && tile_m == 64;
+    std::vector<int32_t> &ts = P->tile_start;
+    ts.reserve(n / 32 + 2);
+    for (int64_t i = 0; i < n;) {
+        ts.push_back((int32_t)i);
+        int64_t k = tile_m;
+        if (early && i + tile_m < n) {
+            int64_t best = agpt_tile_cost(P->depth[i + k], k);
+            for (int64_t c = k - 1; c >= 32; c--) {
+                const int64_t v = agpt_tile_cost(P->depth[i + c], c);
+                if (v < best) { best = v; k = c; }
+            }
+        }
+        i += k;
+    }
+    P->n_tiles = (int64_t)ts.size();
+    ts.push_back((int32_t)n);
     P->chain_off.assign(P->n_tiles + 1, 0);
-    for (int64_t t = 0; t < P->n_tiles; t++) P->chain_off[t + 1] = P->chain_off[t] + (P->depth[t * tile_m] - 1);
+    for (int64_t t = 0; t < P->n_tiles; t++) {
+        P->chain_off[t + 1] = P->chain_off[t] + (P->depth[ts[t]] - 1);
+        P->max_keys = std::max(P->max_keys, P->depth[ts[t]] - 1 + ts[t + 1] - ts[t]);
+    }
     P->chain_rows = P->chain_off[P->n_tiles];
     P->chain_ids.resize(P->chain_rows);
     for (int64_t t = 0; t < P->n_tiles; t++) {
-        int32_t a = P->parent_dfs[t * tile_m];
+        int32_t a = P->parent_dfs[ts[t]];
         for (int64_t j = P->chain_off[t + 1] - 1; j >= P->chain_off[t]; j--) { P->chain_ids[j] = a; a = P->parent_dfs[a]; }
     }
     P->chain_end.resize(P->chain_ids.size());
     for (size_t j = 0; j < P->chain_ids.size(); j++) P->chain_end[j] = P->sub_end[P->chain_ids[j]];
     // reduction work list: node a receives one partial row from every tile that starts strictly inside
-    // its subtree, i.e. tiles (a / M, (sub_end[a] - 1) / M]; long ranges are cut into segments
+    // its subtree, i.e. tiles (tile of a, tile of sub_end[a] - 1]; long ranges are cut into segments
     const int64_t SEG = AGPT_REDUCE_SEG;
-    for (int64_t a = 0; a < n; a++) {
-        int64_t t0 = a / tile_m + 1, t1 = (P->sub_end[a] - 1) / tile_m;   // inclusive range [t0, t1]
-        if (t1 < t0) continue;
+    for (int64_t a = 0, t0 = 1; a < n; a++) {          // t0: one past the tile of a
+        while (ts[t0] <= a) t0++;
+        if (P->sub_end[a] <= ts[t0]) continue;
+        const int64_t t1 = std::lower_bound(ts.begin() + t0 + 1, ts.end(), P->sub_end[a]) - ts.begin() - 1;   // inclusive range [t0, t1]
         int64_t nseg = (t1 - t0 + 1 + SEG - 1) / SEG;
         if (nseg > 1) { P->multi_node.push_back((int32_t)a); P->multi_first.push_back((int64_t)P->n_multi_items); P->multi_count.push_back((int32_t)nseg); }
         for (int64_t s = 0; s < nseg; s++) {

@@ -32,13 +32,22 @@ struct agpt_trie {
 
 // Walker plan: a tree laid out in depth-first pre-order.  Position i's subtree is the
 // interval [i, sub_end[i]); a is an ancestor-or-self of i iff a <= i < sub_end[a].  Queries
-// are processed in tiles of tile_m consecutive positions; a tile's keys are the ancestor
-// chain of its first position (chain_ids, root side first, chain_off per tile) plus the
-// tile's own rows.
+// are processed in tiles of up to tile_m consecutive positions (tile t: [tile_start[t], tile_start[t + 1])); a tile's keys are
+// the ancestor chain of its first position (chain_ids, root side first, chain_off per tile) plus the tile's own rows.
+//
+// A plan for a GPU with tiles of 64 lets a tile end early, where the next one starts at a shallow position: the chain that the
+// next tile loads again, and gives partial dK/dV rows for, is as long as its first position is deep, and a trie's depth-first
+// order comes back to shallow rows all the time.  The next start is the row k in [32, 64] after this one that makes
+// depth + 0.9 (64 - k) least, the later one of equals: a chain row costs about as much as a row left unfilled, and below a factor of 1
+// a run without branches, one deeper per row, is not worth walking along.  (On tries 0.25 to 0.9 choose the same starts; on bushy
+// trees smaller factors leave more tiles for little.  Tiles below 32 rows leave warps without rows.)  Keys per row on the depth-32 trie
+// of 1.4M rows 1.27 -> 1.07, partial rows 0.27 -> 0.07 per row and their reduction 274 -> 81 us; forward 945 -> 901 us.
 struct agpt_plan {
     int64_t n = 0;
     int32_t tile_m = 64;
     int64_t n_tiles = 0;
+    std::vector<int32_t> tile_start;             // [n_tiles + 1]
+    int32_t max_keys = 0;                        // chain + rows of the tile that has most
     int32_t max_depth = 0;
     int64_t sum_depth = 0, sum_group_prefix = 0, n_groups = 0, n_reduce_nodes = 0, n_multi_items = 0;
     std::vector<int32_t> dfs_to_node, node_to_dfs, parent_dfs, depth, sub_end;      // filled on demand if lazy: need_host()
@@ -58,7 +67,7 @@ struct agpt_plan {
     // device copies (owned, or in a buffer of the caller)
     int device = -1;
     bool external = false;
-    int32_t *d_depth = nullptr, *d_sub_end = nullptr, *d_chain_ids = nullptr, *d_chain_end = nullptr;
+    int32_t *d_depth = nullptr, *d_sub_end = nullptr, *d_chain_ids = nullptr, *d_chain_end = nullptr, *d_tile_start = nullptr;
     int64_t *d_chain_off = nullptr, *d_multi_first = nullptr;
     int32_t *d_item_node = nullptr, *d_item_t0 = nullptr, *d_item_t1 = nullptr, *d_item_slot = nullptr;
     int32_t *d_multi_node = nullptr, *d_multi_count = nullptr;
@@ -74,6 +83,8 @@ struct agpt_plan {
 };
 
 int agpt_plan_upload(agpt_plan *p, int device);
+// cost of a tile that starts k rows after the last one's start, at depth d (in tenths of a row)
+inline int64_t agpt_tile_cost(int32_t d, int64_t k) { return 10 * (int64_t)d + 9 * (64 - k); }
 // mass weight of each loss node (agpt_b200_mass_weights without the expansion to queries)
 int agpt_mass_weights_per_node(const int32_t *edge_mass, const int32_t *edge_len, const int32_t *unit_of_node, const uint8_t *counted,
                                int64_t n_nodes, int64_t n_units, int mode, float *out_per_node);

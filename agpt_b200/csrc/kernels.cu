@@ -67,6 +67,7 @@ int agpt_plan_upload(agpt_plan *p, int device) {
     if ((rc = upload(&p->d_chain_ids, p->chain_ids))) return rc;
     if ((rc = upload(&p->d_chain_end, p->chain_end))) return rc;
     if ((rc = upload(&p->d_chain_off, p->chain_off))) return rc;
+    if ((rc = upload(&p->d_tile_start, p->tile_start))) return rc;
     if ((rc = upload(&p->d_item_node, p->item_node))) return rc;
     if ((rc = upload(&p->d_item_t0, p->item_t0))) return rc;
     if ((rc = upload(&p->d_item_t1, p->item_t1))) return rc;
@@ -83,9 +84,9 @@ agpt_plan::~agpt_plan() {
         cudaGetDevice(&cur);
         cudaSetDevice(device);
         if (!external) {
-        cudaFree(d_depth); cudaFree(d_sub_end); cudaFree(d_chain_ids); cudaFree(d_chain_end); cudaFree(d_chain_off);
-        cudaFree(d_item_node); cudaFree(d_item_t0); cudaFree(d_item_t1); cudaFree(d_item_slot);
-        cudaFree(d_multi_node); cudaFree(d_multi_count); cudaFree(d_multi_first);
+            cudaFree(d_depth); cudaFree(d_sub_end); cudaFree(d_chain_ids); cudaFree(d_chain_end); cudaFree(d_chain_off); cudaFree(d_tile_start);
+            cudaFree(d_item_node); cudaFree(d_item_t0); cudaFree(d_item_t1); cudaFree(d_item_slot);
+            cudaFree(d_multi_node); cudaFree(d_multi_count); cudaFree(d_multi_first);
         }
         cudaFree(host_arena);
         if (host_fix) cudaFreeHost(host_fix);
@@ -157,17 +158,17 @@ __global__ void __launch_bounds__(M) attn_fwd_kernel(const float *__restrict__ Q
                                                      const KVT *__restrict__ V, float *__restrict__ O,
                                                      float *__restrict__ LSE, const int32_t *__restrict__ sub_end,
                                                      const int64_t *__restrict__ chain_off,
-                                                     const int32_t *__restrict__ chain_ids, int n, int H, float scale, int tile0) {
+                                                     const int32_t *__restrict__ chain_ids, const int32_t *__restrict__ tile_start, int H, float scale, int tile0) {
     __shared__ __align__(16) float sK[KC][HD + 4];
     __shared__ __align__(16) float sV[KC][HD + 4];
     __shared__ int s_kid[KC], s_kend[KC];
     const int t = blockIdx.x + tile0, h = blockIdx.y, tid = threadIdx.x;
     const int D = H * HD, hoff = h * HD;
-    const int i0 = t * M, i = i0 + tid;
+    const int i0 = tile_start[t], n = tile_start[t + 1], i = i0 + tid;      // n: one past the tile's last row
     const bool active = i < n;
     const int64_t coff = chain_off[t];
     const int p = (int)(chain_off[t + 1] - coff);
-    const int nkeys = p + min(M, n - i0);
+    const int nkeys = p + n - i0;
     const int32_t *chain = chain_ids + coff;
 
     float q[HD], acc[HD];
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(128) attn_fwd_mma_kernel(const float *__restri
                                                            float *__restrict__ LSE, const int32_t *__restrict__ sub_end,
                                                            const int64_t *__restrict__ chain_off,
                                                            const int32_t *__restrict__ chain_ids,
-                                                           const int32_t *__restrict__ chain_end_all, int n, int H,
+                                                           const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H,
                                                            float scale, int tile0) {
     constexpr int M = 64, KS = HD / 8;
     constexpr bool SPLIT_KV = sizeof(KVT) == 4;
@@ -357,12 +358,12 @@ __global__ void __launch_bounds__(128) attn_fwd_mma_kernel(const float *__restri
     const int t = blockIdx.x + tile0, h = blockIdx.y, tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
     const int D = H * HD, hoff = h * HD;
-    const int i0 = t * M;
+    const int i0 = tile_start[t], n = tile_start[t + 1];
     const int r0 = i0 + warp * 16 + g, r1 = r0 + 8;
     const bool act0 = r0 < n, act1 = r1 < n;
     const int64_t coff = chain_off[t];
     const int p = (int)(chain_off[t + 1] - coff);
-    const int nkeys = p + min(M, n - i0);
+    const int nkeys = p + n - i0;
     const int32_t *chain = chain_ids + coff;
     const float qs = scale * LOG2E;
     load_key_meta(sub_end, chain, chain_end_all + coff, p, i0, nkeys, s_kid, s_kend);
@@ -524,15 +525,15 @@ __global__ void __launch_bounds__(M) attn_bwd_kernel(const float *__restrict__ Q
                                                      float *__restrict__ dV, float *__restrict__ Pk,
                                                      float *__restrict__ Pv, const int32_t *__restrict__ sub_end,
                                                      const int64_t *__restrict__ chain_off,
-                                                     const int32_t *__restrict__ chain_ids, int n, int H, float scale, int tile0,
+                                                     const int32_t *__restrict__ chain_ids, const int32_t *__restrict__ tile_start, int H, float scale, int tile0,
                                                      BwdMask gmask) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BwdSmem<HD, M> &S = *reinterpret_cast<BwdSmem<HD, M> *>(smem_raw);
     const int t = blockIdx.x + tile0, h = blockIdx.y, tid = threadIdx.x;
     const int D = H * HD, hoff = h * HD;
-    const int i0 = t * M, i = i0 + tid;
+    const int i0 = tile_start[t], n = tile_start[t + 1], i = i0 + tid;      // n: one past the tile's last row
     const bool active = i < n;
-    const int nt = min(M, n - i0);
+    const int nt = n - i0;
     const int64_t coff = chain_off[t];
     const int p = (int)(chain_off[t + 1] - coff);
     const int nkeys = p + nt;
@@ -671,7 +672,7 @@ __global__ void __launch_bounds__(128, HD <= 32 ? 4 : (sizeof(KVT) == 2 ? 3 : 1)
                                                            float *__restrict__ Pv, const int32_t *__restrict__ sub_end,
                                                            const int64_t *__restrict__ chain_off,
                                                            const int32_t *__restrict__ chain_ids,
-                                                           const int32_t *__restrict__ chain_end_all, int n, int H,
+                                                           const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H,
                                                            float scale, int tile0, BwdMask gmask) {
     constexpr int M = 64, KS = HD / 8;
     constexpr bool SPLIT_KV = sizeof(KVT) == 4;
@@ -683,8 +684,8 @@ __global__ void __launch_bounds__(128, HD <= 32 ? 4 : (sizeof(KVT) == 2 ? 3 : 1)
     const int t = blockIdx.x + tile0, h = blockIdx.y, tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
     const int D = H * HD, hoff = h * HD;
-    const int i0 = t * M;
-    const int nt = min(M, n - i0);
+    const int i0 = tile_start[t], n = tile_start[t + 1];
+    const int nt = n - i0;
     // tile-local query rows of this thread (pairing an early with a late group of 8 rows per warp, to even out the
     // triangular work between the warps, was measured slower: more 16 x 8 blocks become live)
     const int q0 = warp * 16 + g, q1 = q0 + 8;
@@ -1065,7 +1066,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                      const float *__restrict__ O, const float *__restrict__ LSE, const float *__restrict__ dO,
                      float *__restrict__ dQ, float *__restrict__ dK, float *__restrict__ dV, float *__restrict__ Pk,
                      float *__restrict__ Pv, const int32_t *__restrict__ sub_end, const int64_t *__restrict__ chain_off,
-                     const int32_t *__restrict__ chain_ids, const int32_t *__restrict__ chain_end_all, int n, int H,
+                     const int32_t *__restrict__ chain_ids, const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H,
                      float scale, int tile0, int maxk, int dbg, BwdMask gmask) {
     constexpr int M = 64, NT = NW * 32, TILE_ROW_BYTES = HD * 4, KS = HD / 16, NDB = HD / 8, NCH = HD / 4;
     constexpr bool LP = sizeof(KVT) == 2;              // bfloat16 store: single fp16 products, no lo parts
@@ -1082,8 +1083,8 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     const int t = blockIdx.x + tile0, h = blockIdx.y, tid = threadIdx.x;
     const int lane = tid & 31, g = lane >> 2, tig = lane & 3;
     const int D = H * HD, hoff = h * HD;
-    const int i0 = t * M;
-    const int nt = min(M, n - i0);
+    const int i0 = tile_start[t], n = tile_start[t + 1];
+    const int nt = n - i0;
     const int64_t coff = chain_off[t];
     const int p = (int)(chain_off[t + 1] - coff);
     const int nkeys = p + nt;
@@ -1440,7 +1441,7 @@ __global__ void __launch_bounds__(128, MINB)
 attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, const KVT *__restrict__ V,
                      float *__restrict__ O, float *__restrict__ LSE, const int32_t *__restrict__ sub_end,
                      const int64_t *__restrict__ chain_off, const int32_t *__restrict__ chain_ids,
-                     const int32_t *__restrict__ chain_end_all, int n, int H, float scale, int tile0, int maxk) {
+                     const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H, float scale, int tile0, int maxk) {
     constexpr int M = 64, NT = 128, TILE_ROW_BYTES = HD * 4, KS = HD / 16, NDB = HD / 8, NCH = HD / 4;
     constexpr bool LP = sizeof(KVT) == 2;              // bfloat16 store: single fp16 products, no lo parts
     extern __shared__ __align__(128) unsigned char tile_smem_raw[];
@@ -1451,8 +1452,8 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     const int t = blockIdx.x + tile0, h = blockIdx.y, tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
     const int D = H * HD, hoff = h * HD;
-    const int i0 = t * M;
-    const int nt = min(M, n - i0);
+    const int i0 = tile_start[t], n = tile_start[t + 1];
+    const int nt = n - i0;
     const int64_t coff = chain_off[t];
     const int p = (int)(chain_off[t + 1] - coff);
     const int nkeys = p + nt;
@@ -1688,7 +1689,7 @@ __global__ void __launch_bounds__(128, MINB)
 attn_fwd_bf16_kernel(const float *__restrict__ Q, const __nv_bfloat16 *__restrict__ K, const __nv_bfloat16 *__restrict__ V,
                      float *__restrict__ O, float *__restrict__ LSE, const int32_t *__restrict__ sub_end,
                      const int64_t *__restrict__ chain_off, const int32_t *__restrict__ chain_ids,
-                     const int32_t *__restrict__ chain_end_all, int n, int H, float scale, int tile0, int maxk) {
+                     const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H, float scale, int tile0, int maxk) {
     constexpr int M = 64, NT = 128, KS = HD / 16, NDB = HD / 8, NCH = HD / 8;
     extern __shared__ __align__(128) unsigned char tile_smem_raw[];
     unsigned char *sK = tile_smem_raw, *sV = sK + (size_t)maxk * (HD * 2);
@@ -1696,7 +1697,7 @@ attn_fwd_bf16_kernel(const float *__restrict__ Q, const __nv_bfloat16 *__restric
     const int t = blockIdx.x + tile0, h = blockIdx.y, tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
     const int D = H * HD, hoff = h * HD;
-    const int i0 = t * M, nt = min(M, n - i0);
+    const int i0 = tile_start[t], n = tile_start[t + 1], nt = n - i0;
     const int64_t coff = chain_off[t];
     const int p = (int)(chain_off[t + 1] - coff);
     const int nkeys = p + nt, nkp = (nkeys + 15) & ~15;
@@ -1899,7 +1900,7 @@ static int launch_fwd(const agpt_plan *p, const float *q, const void *k, const v
                       float scale, cudaStream_t st, int tile0, int ntiles) {
     dim3 grid((unsigned)ntiles, (unsigned)H);
     attn_fwd_kernel<HD, M, KVT><<<grid, M, 0, st>>>(q, (const KVT *)k, (const KVT *)v, out, lse, p->d_sub_end,
-                                                    p->d_chain_off, p->d_chain_ids, (int)p->n, H, scale, tile0);
+                                                    p->d_chain_off, p->d_chain_ids, p->d_tile_start, H, scale, tile0);
     return launch_status("attn_fwd");
 }
 
@@ -1912,7 +1913,7 @@ static int launch_bwd(const agpt_plan *p, const float *q, const void *k, const v
     static size_t granted[AGPT_MAX_DEVICES];
     if (int rc = allow_dynamic_smem(attn_bwd_kernel<HD, M, KVT>, smem, granted)) return rc;
     attn_bwd_kernel<HD, M, KVT><<<grid, M, smem, st>>>(q, (const KVT *)k, (const KVT *)v, o, lse, dout, dq, dk, dv, pk, pv,
-                                                       p->d_sub_end, p->d_chain_off, p->d_chain_ids, (int)p->n, H, scale, tile0, gmask);
+                                                       p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_tile_start, H, scale, tile0, gmask);
     return launch_status("attn_bwd");
 }
 
@@ -1974,7 +1975,7 @@ extern "C" int agpt_b200_set_attn_variant(int whole_tile, int warps) {
     g_bwd_tile = whole_tile; g_bwd_warps = warps;
     return AGPT_OK;
 }
-static inline int bwd_tile_maxk(const agpt_plan *p) { return ((p->max_depth - 1 + 64) + 15) & ~15; }
+static inline int bwd_tile_maxk(const agpt_plan *p) { return (p->max_keys + 15) & ~15; }
 static inline bool tile_kernels_fit(const agpt_plan *p, int head_dim) {
     if (head_dim != 32 && head_dim != 64) return false;
     return bwd_tile_smem_bytes(head_dim, bwd_tile_maxk(p)) <= (head_dim == 32 ? (size_t)56 * 1024 : (size_t)113 * 1024);
@@ -2001,7 +2002,7 @@ static int launch_fwd_tile(const agpt_plan *p, const float *q, const void *k, co
     if (rc) return rc;
     dim3 grid((unsigned)ntiles, (unsigned)H);
     attn_fwd_tile_kernel<HD, MINB, KVT><<<grid, 128, smem, st>>>(q, (const KVT *)k, (const KVT *)v, out, lse, p->d_sub_end,
-                                                                 p->d_chain_off, p->d_chain_ids, p->d_chain_end, (int)p->n, H, scale, tile0, maxk);
+                                                                 p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H, scale, tile0, maxk);
     return launch_status("attn_fwd_tile");
 }
 
@@ -2013,7 +2014,7 @@ static int launch_fwd_bf16(const agpt_plan *p, const float *q, const void *k, co
     const size_t smem = fwd_bf16_smem_bytes(HD, maxk);
     if (int rc = allow_dynamic_smem(attn_fwd_bf16_kernel<HD, MINB>, smem, granted)) return rc;
     attn_fwd_bf16_kernel<HD, MINB><<<dim3((unsigned)ntiles, (unsigned)H), 128, smem, st>>>(
-        q, (const __nv_bfloat16 *)k, (const __nv_bfloat16 *)v, out, lse, p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_chain_end, (int)p->n, H,
+        q, (const __nv_bfloat16 *)k, (const __nv_bfloat16 *)v, out, lse, p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H,
         scale, tile0, maxk);
     return launch_status("attn_fwd_bf16");
 }
@@ -2026,7 +2027,7 @@ static int launch_fwd_mma(const agpt_plan *p, const float *q, const void *k, con
     static size_t granted[AGPT_MAX_DEVICES];
     if (int rc = allow_dynamic_smem(attn_fwd_mma_kernel<HD, KVT>, smem, granted)) return rc;
     attn_fwd_mma_kernel<HD, KVT><<<grid, 128, smem, st>>>(q, (const KVT *)k, (const KVT *)v, out, lse, p->d_sub_end,
-                                                       p->d_chain_off, p->d_chain_ids, p->d_chain_end, (int)p->n, H, scale, tile0);
+                                                       p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H, scale, tile0);
     return launch_status("attn_fwd_mma");
 }
 
@@ -2053,7 +2054,7 @@ static int fwd_dispatch(const agpt_plan *p, const float *q, const void *k, const
             case 64: return launch_fwd_bf16<64, 4>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
         }
     }
-    if (attn_impl() == 1 && p->tile_m == 64 && p->max_depth + 64 <= MAXKEYS) {
+    if (attn_impl() == 1 && p->tile_m == 64 && p->max_keys <= MAXKEYS) {
         const bool bf = kv_dtype == AGPT_KV_BF16;        // (head_dim 16 and 32: MAXKEYS keys fit the whole-tile kernel)
         switch (head_dim) {
             case 16: return launch_fwd_mma<16, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
@@ -2073,7 +2074,7 @@ static int launch_bwd_mma(const agpt_plan *p, const float *q, const void *k, con
     static size_t granted[AGPT_MAX_DEVICES];
     if (int rc = allow_dynamic_smem(attn_bwd_mma_kernel<HD, KVT>, smem, granted)) return rc;
     attn_bwd_mma_kernel<HD, KVT><<<grid, 128, smem, st>>>(q, (const KVT *)k, (const KVT *)v, o, lse, dout, dq, dk, dv, pk, pv,
-                                                          p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_chain_end, (int)p->n, H,
+                                                          p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H,
                                                           scale, tile0, gmask);
     return launch_status("attn_bwd_mma");
 }
@@ -2090,7 +2091,7 @@ static int launch_bwd_tile(const agpt_plan *p, const float *q, const void *k, co
     dim3 grid((unsigned)ntiles, (unsigned)H);
     attn_bwd_tile_kernel<HD, NW, MINB, KVT><<<grid, NW * 32, smem, st>>>(q, (const KVT *)k, (const KVT *)v, o, lse, dout, dq, dk, dv, pk, pv,
                                                                          p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_chain_end,
-                                                                         (int)p->n, H, scale, tile0, maxk, g_bwd_dbg, gmask);
+                                                                         p->d_tile_start, H, scale, tile0, maxk, g_bwd_dbg, gmask);
     return launch_status("attn_bwd_tile");
 }
 
@@ -2122,7 +2123,7 @@ static int bwd_dispatch(const agpt_plan *p, const float *q, const void *k, const
         if (tile_kernels_fit(p, head_dim))
             return launch_bwd_tile_w(p, q, k, v, kv_dtype, o, lse, dout, dq, dk, dv, pk, pv, H, head_dim, scale, st, tile0, ntiles, gmask);
     }
-    if (attn_impl() == 1 && p->tile_m == 64 && p->max_depth + 64 <= MAXKEYS) {
+    if (attn_impl() == 1 && p->tile_m == 64 && p->max_keys <= MAXKEYS) {
         const bool bf = kv_dtype == AGPT_KV_BF16;
 #define BWD_MMA_ARGS p, q, k, v, o, lse, dout, dq, dk, dv, pk, pv, H, scale, st, tile0, ntiles, gmask
         switch (head_dim) {
@@ -3075,7 +3076,7 @@ static int attn_fwd_bwd_host_impl(const agpt_plan *cp, const float *h_q, const f
     agpt_plan *p = const_cast<agpt_plan *>(cp);        // the cached arena is the only state a call changes
     CUDA_TRY(cudaSetDevice(p->device));
     p->need_host();
-    const int D = n_heads * head_dim, M = p->tile_m;
+    const int D = n_heads * head_dim;
     const int64_t n = p->n;
     const size_t rowb = (size_t)D * sizeof(float);
     const size_t tens = (((size_t)n * rowb) + 255) & ~(size_t)255;
@@ -3087,8 +3088,13 @@ static int attn_fwd_bwd_host_impl(const agpt_plan *cp, const float *h_q, const f
     // (nine per chunk) than they save.  174k rows of 128: 11.6 ms in two chunks of 64 MB, 8.8 in ten, 9.4 in 24 (8.0 ms would
     // be both directions at the 44.7 GB/s each that they reach together).
     const int64_t ch_bytes = std::min<int64_t>(64ll << 20, std::max<int64_t>(2ll << 20, n * (int64_t)rowb / 10));
-    const int64_t ch_rows = std::max<int64_t>(M, (ch_bytes / (int64_t)rowb) / M * M);
-    const int64_t n_ch = (n + ch_rows - 1) / ch_rows;
+    const int64_t ch_rows = std::max<int64_t>(p->tile_m, ch_bytes / (int64_t)rowb);
+    std::vector<int64_t> cut{0};                       // first tile of every chunk: as many whole tiles as ch_rows rows hold
+    while (cut.back() < p->n_tiles) {
+        const int64_t t0 = cut.back();
+        cut.push_back(std::upper_bound(p->tile_start.begin() + t0 + 1, p->tile_start.end(), p->tile_start[t0] + ch_rows) - p->tile_start.begin() - 1);
+    }
+    const int64_t n_ch = (int64_t)cut.size() - 1;
     const size_t fix_dev_cap = (((size_t)n_ch * (size_t)p->max_depth + p->multi_node.size()) * (2 * rowb + sizeof(int32_t)) + 511) & ~(size_t)255;
     const size_t need = 8 * tens + lseb + wsb + (bf ? tens : 0) + fix_dev_cap;
     if (p->host_arena_bytes < need) {
@@ -3123,7 +3129,7 @@ static int attn_fwd_bwd_host_impl(const agpt_plan *cp, const float *h_q, const f
     // rows ("fix rows": at most depth per chunk boundary) are downloaded again at the end.
     std::vector<int32_t> fix(p->multi_node.begin(), p->multi_node.end());
     for (int64_t c = 0; c + 1 < n_ch; c++)
-        for (int32_t a = p->parent_dfs[(c + 1) * ch_rows]; a >= 0; a = p->parent_dfs[a]) fix.push_back(a);
+        for (int32_t a = p->parent_dfs[p->tile_start[cut[c + 1]]]; a >= 0; a = p->parent_dfs[a]) fix.push_back(a);
     std::sort(fix.begin(), fix.end());
     fix.erase(std::unique(fix.begin(), fix.end()), fix.end());
     const size_t nfix = fix.size();
@@ -3137,7 +3143,8 @@ static int attn_fwd_bwd_host_impl(const agpt_plan *cp, const float *h_q, const f
     int64_t item_done = 0;
     const int64_t n_items = (int64_t)p->item_node.size();
     for (int64_t c = 0; c < n_ch; c++) {
-        const int64_t r0 = c * ch_rows, r1 = std::min(n, r0 + ch_rows), nr = r1 - r0;
+        const int t0 = (int)cut[c], nt = (int)(cut[c + 1] - cut[c]);
+        const int64_t r0 = p->tile_start[t0], r1 = p->tile_start[t0 + nt], nr = r1 - r0;
         const size_t off = (size_t)r0 * D, bytes = (size_t)nr * rowb;
         CUDA_TRY(cudaMemcpyAsync(dq_in + off, h_q + off, bytes, cudaMemcpyHostToDevice, s_up));
         CUDA_TRY(cudaMemcpyAsync(dk_in + off, h_k + off, bytes, cudaMemcpyHostToDevice, s_up));
@@ -3149,7 +3156,6 @@ static int attn_fwd_bwd_host_impl(const agpt_plan *cp, const float *h_q, const f
             if ((rc = agpt_b200_kv_store_write_bf16(dk_in + off, kb + off, nr, D, s_run))) return rc;
             if ((rc = agpt_b200_kv_store_write_bf16(dv_in + off, vb + off, nr, D, s_run))) return rc;
         }
-        const int t0 = (int)(r0 / M), nt = (int)((r1 + M - 1) / M) - t0;
         if ((rc = fwd_dispatch(p, dq_in, kk, vv, kv_dtype, dout, dlse, n_heads, head_dim, scale, s_run, t0, nt))) return rc;
         CUDA_TRY(cudaEventRecord(ev(c, 1), s_run));
         if ((rc = bwd_dispatch(p, dq_in, kk, vv, kv_dtype, dout, dlse, dg, ddq, ddk, ddv, pk, pv, n_heads, head_dim, scale, s_run, t0, nt))) return rc;

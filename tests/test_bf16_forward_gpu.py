@@ -30,8 +30,8 @@ def _want(parent, q, k, v, H):
 @pytest.mark.parametrize("parent,H,hd,tol", [
     (chain_tree(1), 1, 16, 5e-5), (chain_tree(15), 2, 32, 5e-5), (chain_tree(65), 1, 64, 5e-5),
     (random_tree(64, 9, 1), 3, 16, 5e-5), (random_tree(333, 32, 2), 2, 32, 5e-5), (random_tree(400, 100, 3, 0.1), 2, 64, 5e-5),
-    (chain_tree(440), 1, 16, 5e-5), (chain_tree(448), 1, 32, 5e-5), (chain_tree(368), 1, 64, 5e-5),
-    (chain_tree(400), 1, 64, 2e-3),                      # chunked: one TF32 product
+    (chain_tree(440), 1, 16, 5e-5), (chain_tree(448), 1, 32, 5e-5), (chain_tree(432), 1, 64, 5e-5),
+    (chain_tree(440), 1, 64, 2e-3),                      # chunked: one TF32 product
 ])
 def test_bf16_store_forward(parent, H, hd, tol):
     import torch
