@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(128) attn_fwd_mma_kernel(const float *__restri
                                                            const int32_t *__restrict__ chain_ids,
                                                            const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H,
                                                            float scale, int tile0) {
-    constexpr int M = 64, KS = HD / 8;
+    constexpr int KS = HD / 8;
     constexpr bool SPLIT_KV = sizeof(KVT) == 4;
     // NS key chunks are staged per round and consumed without any barrier in between, so the four warps (whose
     // live key blocks differ a lot: later rows attend more of the tile) do not wait for each other per chunk
@@ -914,14 +914,12 @@ __global__ void __launch_bounds__(128, HD <= 32 ? 4 : (sizeof(KVT) == 2 ? 3 : 1)
 // halves, its 16-byte chunks XOR-swizzled with the row (chunk ^ row % 8), so that every fragment is one
 // conflict-free ldmatrix.x4: "along the row" fragments plain, "across rows" fragments with .trans.
 //
-// Work.  After the staging barriers the warps never meet again.  A warp takes items from a shared counter and runs
-// each from start to end with registers and read-only shared memory:
-//   * row item (16 queries):  S = Q K^T and dP = dO V^T for the 16 rows against every block of 16 keys, P, dS,
-//     dQ += dS K (the score fragments of two 8-key blocks are the A fragment of the next product); writes 16 dQ rows.
-//   * key item (16 keys):     S^T = K Q^T and dP^T = V dO^T for the 16 keys against every block of 16 queries, P^T,
-//     dS^T, dK += dS^T Q, dV += P^T dO;  writes 16 dK/dV rows (tile rows) or partial rows (chain keys).
-// Scores are computed twice (once per orientation) instead of crossing shared memory between two phases: that
-// costs two extra small products per block and removes every barrier, every P/dS store and reload from the loops.
+// Work.  A warp takes key items (16 keys) from a shared counter: S^T = K Q^T and dP^T = V dO^T for the 16 keys against every
+// block of 16 queries, P^T, dS^T, dK += dS^T Q, dV += P^T dO; it writes 16 dK/dV rows (tile rows) or partial rows (chain keys) and
+// leaves dS^T, as the halves that its own products take, in shared memory: the V rows of the block, which only this item reads, hold
+// it.  After one barrier each warp takes 16 queries and sums dQ = dS K from those blocks.  Bound by issue slots: scores are computed
+// once, where computing them again with the queries as rows took 84 products per 16 x 16 block of head_dim 32 instead of 60 and the
+// exponentials twice.  Measured: 4 x 32, 1.4M rows 2134 -> 1916 us; 8 x 64, 600k rows 4090 -> 3708 us.
 // Each output element is produced by exactly one warp in a fixed order, so results do not depend on which warp
 // took which item.
 // --------------------------------------------------------------------------------------
@@ -938,6 +936,9 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t smem_addr
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t smem_addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr));
+}
+__device__ __forceinline__ void stmatrix_x4(uint32_t smem_addr, const uint32_t (&r)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(smem_addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -1056,8 +1057,10 @@ __device__ __forceinline__ void kv_convert_bf16(unsigned char *pa, const KvLane 
     *reinterpret_cast<uint4 *>(pa + L.hi + o) = make_uint4(h[0], h[1], h[2], h[3]);
 }
 
-constexpr size_t bwd_tile_smem_bytes(int hd, int maxk) {
-    return (size_t)(2 * 64 + 2 * maxk) * (size_t)(hd * 4) + (size_t)maxk * 8 + 3 * 64 * 4 + 32;
+// bytes of one key block's dS^T (16 keys x 64 queries) that do not fit the block's own V rows: float32 stores hold hi and lo parts
+template <typename KVT> constexpr int bwd_tile_ds_extra(int hd) { return sizeof(KVT) == 2 || hd >= 64 ? 0 : 16 * 64 * 4 - 16 * hd * 4; }
+constexpr size_t bwd_tile_smem_bytes(int hd, int maxk, int ds_extra) {
+    return (size_t)(2 * 64 + 2 * maxk) * (size_t)(hd * 4) + (size_t)(maxk / 16) * (size_t)ds_extra + (size_t)maxk * 8 + 3 * 64 * 4 + 32 + (size_t)(maxk / 16) * 4;
 }
 
 template <int HD, int NW, int MINB, typename KVT>
@@ -1067,18 +1070,21 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                      float *__restrict__ dQ, float *__restrict__ dK, float *__restrict__ dV, float *__restrict__ Pk,
                      float *__restrict__ Pv, const int32_t *__restrict__ sub_end, const int64_t *__restrict__ chain_off,
                      const int32_t *__restrict__ chain_ids, const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H,
-                     float scale, int tile0, int maxk, int dbg, BwdMask gmask) {
+                     float scale, int tile0, int maxk, BwdMask gmask) {
     constexpr int M = 64, NT = NW * 32, TILE_ROW_BYTES = HD * 4, KS = HD / 16, NDB = HD / 8, NCH = HD / 4;
     constexpr bool LP = sizeof(KVT) == 2;              // bfloat16 store: single fp16 products, no lo parts
     extern __shared__ __align__(128) unsigned char tile_smem_raw[];
     unsigned char *sQ = tile_smem_raw, *sG = sQ + M * TILE_ROW_BYTES, *sK = sG + M * TILE_ROW_BYTES;
     unsigned char *sV = sK + (size_t)maxk * TILE_ROW_BYTES;
-    int2 *s_meta = reinterpret_cast<int2 *>(sV + (size_t)maxk * TILE_ROW_BYTES);   // [maxk] {key id, key subtree end}
+    constexpr int DSX = bwd_tile_ds_extra<KVT>(HD);
+    unsigned char *sDX = sV + (size_t)maxk * TILE_ROW_BYTES;                        // [maxk / 16][DSX] the rest of dS^T
+    int2 *s_meta = reinterpret_cast<int2 *>(sDX + (size_t)(maxk / 16) * DSX);       // [maxk] {key id, key subtree end}
     float *sLse = reinterpret_cast<float *>(s_meta + maxk);                          // [64]  lse * log2(e)
     float *sDelta = sLse + M;                                                        // [64]  dO . O
     int *sFirst = reinterpret_cast<int *>(sDelta + M);                               // [64]  first key id each query feeds in dK/dV
     uint32_t *s_max = reinterpret_cast<uint32_t *>(sFirst + M);                      // [4]   max |x| of Q, K, V, dO (float bits)
     int *s_ctr = reinterpret_cast<int *>(s_max + 4);
+    unsigned *s_on = reinterpret_cast<unsigned *>(s_ctr + 4);                        // [maxk / 16] query blocks for which a key block has dS^T
 
     const int t = blockIdx.x + tile0, h = blockIdx.y, tid = threadIdx.x;
     const int lane = tid & 31, g = lane >> 2, tig = lane & 3;
@@ -1146,7 +1152,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
         int kid = 0x7fffffff, kend = 0;
         if (j < p) { kid = __ldg(chain + j); kend = __ldg(chain_end + j); }
         else if (j < nkeys) { kid = i0 + (j - p); kend = __ldg(sub_end + kid); }
-        s_meta[j] = make_int2(kid, kend);
+        s_meta[j] = make_int2(kid, min(kend, n));        // rows past the tile's end attend nothing
     }
     if (tid < M) {
         sLse[tid] = tid < nt ? __ldg(LSE + (int64_t)(i0 + tid) * H + h) * LOG2E : 0.f;
@@ -1225,107 +1231,21 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     const int tC = (mi >> 1) * NDB;                     // + db
     const uint32_t uQ = smem_u32_of(sQ), uG = smem_u32_of(sG), uK = smem_u32_of(sK), uV = smem_u32_of(sV);
 
-    const int nkb = nkp >> 4;                    // key items
-    const int npc = (p + 15) >> 4;               // key items that hold chain keys (the heaviest: attended by most rows)
-    const int n_items = nkb + 4;
+    // dS^T of (key block kb, query block qp): 16 x 16 halves as four 8 x 8 matrices of 128 bytes {keys 0-7 queries 0-7, keys 8-15
+    // queries 0-7, keys 0-7 queries 8-15, keys 8-15 queries 8-15}.  hi parts and, where they fit, lo parts lie in the key block's own V rows, which
+    // nothing reads any more once the block's item holds its V fragments.
+    const uint32_t uDX = smem_u32_of(sDX);
+    auto ds_hi = [&](int kb, int qp) { return uV + (uint32_t)(kb * 16 * TILE_ROW_BYTES + qp * 512); };
+    auto ds_lo = [&](int kb, int qp) { return DSX ? uDX + (uint32_t)(kb * DSX + qp * 512) : uV + (uint32_t)(kb * 16 * TILE_ROW_BYTES + 2048 + qp * 512); };
 
+    const int nkb = nkp >> 4;                    // key items: chain keys first (attended by most rows), then the tile's own
     for (;;) {
-        int it = 0;
-        if (lane == 0) it = atomicAdd(s_ctr, 1);
-        it = __shfl_sync(0xffffffffu, it, 0);
-        if (it >= n_items) break;
-        // order: chain key items, row items (last rows first), the tile's own key items
-        int kind, which;
-        if (it < npc) { kind = 1; which = it; }
-        else if (it < npc + 4) { kind = 0; which = 3 - (it - npc); }
-        else { kind = 1; which = it - 4; }
-        if ((dbg >> kind) & 1) continue;
-
-        if (kind == 0) {
-            // ================= row item: 16 queries, every block of 16 keys =================
-            const int rg = which;
-            if (rg * 16 >= nt) continue;                                   // rows beyond the end of the plan
-            const int q0 = rg * 16 + g, q1 = q0 + 8;
-            const int r0 = i0 + q0, r1 = i0 + q1;
-            uint32_t qh[KS][4], ql[KS][4], gh[KS][4], gl[KS][4];
-#pragma unroll
-            for (int ks = 0; ks < KS; ks++) {
-                const uint32_t o = (uint32_t)(rg * 16 * TILE_ROW_BYTES) + aRow;
-                const uint32_t ch = (uint32_t)(((2 * ks + aC) ^ l8) << 4), cl = (uint32_t)(((2 * ks + aC + NDB) ^ l8) << 4);
-                ldmatrix_x4(qh[ks], uQ + o + ch); ldmatrix_x4(gh[ks], uG + o + ch);
-                if constexpr (!LP) { ldmatrix_x4(ql[ks], uQ + o + cl); ldmatrix_x4(gl[ks], uG + o + cl); }
-            }
-            const float lse0 = sLse[q0], lse1 = sLse[q1], dl0 = sDelta[q0] * sclG * sclV, dl1 = sDelta[q1] * sclG * sclV;
-            float dq[NDB][4];
-#pragma unroll
-            for (int db = 0; db < NDB; db++) dq[db][0] = dq[db][1] = dq[db][2] = dq[db][3] = 0.f;
-            // the rows of this group attend the chain and the tile's keys up to their own position
-            const int kp_lim = min((nkeys + 15) >> 4, (p + rg * 16 + 16 + 15) >> 4);
-            for (int kp = 0; kp < kp_lim; kp++) {
-                bool vld[2][4];
-                bool on[2];
-#pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    const int4 mk = *reinterpret_cast<const int4 *>(&s_meta[kp * 16 + u * 8 + 2 * tig]);   // keys 2*tig, 2*tig+1 of the block
-                    vld[u][0] = mk.x <= r0 && r0 < mk.y; vld[u][1] = mk.z <= r0 && r0 < mk.w;
-                    vld[u][2] = mk.x <= r1 && r1 < mk.y; vld[u][3] = mk.z <= r1 && r1 < mk.w;
-                    on[u] = __any_sync(0xffffffffu, vld[u][0] | vld[u][1] | vld[u][2] | vld[u][3]);
-                }
-                if (!(on[0] || on[1])) continue;
-                float ds[2][4];
-#pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    ds[u][0] = ds[u][1] = ds[u][2] = ds[u][3] = 0.f;
-                    if (!on[u] && !TileBothHalves<HD>::bwd) continue;                  // warp-uniform
-                    float c[4] = {0.f, 0.f, 0.f, 0.f}, cx[4] = {0.f, 0.f, 0.f, 0.f};
-                    float e[4] = {0.f, 0.f, 0.f, 0.f}, ex[4] = {0.f, 0.f, 0.f, 0.f};
-                    const uint32_t rowb = (uint32_t)((kp * 16 + u * 8) * TILE_ROW_BYTES) + bRow;
-#pragma unroll
-                    for (int ks = 0; ks < KS; ks++) {
-                        const uint32_t o = rowb + (uint32_t)(((2 * ks + bC) ^ l8) << 4);
-                        uint32_t kf[4], vf[4];                 // {b0 hi, b1 hi, b0 lo, b1 lo}
-                        ldmatrix_x4(kf, uK + o); ldmatrix_x4(vf, uV + o);
-                        mma_f16(c, qh[ks], kf[0], kf[1]); mma_f16(e, gh[ks], vf[0], vf[1]);
-                        if constexpr (!LP) {
-                            mma_f16(cx, ql[ks], kf[0], kf[1]); mma_f16(ex, gl[ks], vf[0], vf[1]);
-                            mma_f16(cx, qh[ks], kf[2], kf[3]); mma_f16(ex, gh[ks], vf[2], vf[3]);
-                        }
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const float sc = fmaf(cx[j], LO_DOWN, c[j]), dp = fmaf(ex[j], LO_DOWN, e[j]);
-                        const float pw = vld[u][j] ? ex2_ftz(fmaf(sc, fS, j < 2 ? -lse0 : -lse1)) : 0.f;
-                        ds[u][j] = pw * (dp - (j < 2 ? dl0 : dl1)) * (scale * AUP);
-                    }
-                }
-                // dQ += dS K over the 16 keys: the score fragments of the two 8-key blocks are the A fragment
-                uint32_t ah[4], al[4], as[4];
-                f16_split2<false>(ds[0][0], ds[0][1], ah[0], al[0]); f16_split2<false>(ds[0][2], ds[0][3], ah[1], al[1]);
-                f16_split2<false>(ds[1][0], ds[1][1], ah[2], al[2]); f16_split2<false>(ds[1][2], ds[1][3], ah[3], al[3]);
-#pragma unroll
-                for (int j = 0; j < 4; j++) as[j] = f16_down11(ah[j]);
-                const uint32_t rowt = uK + (uint32_t)(kp * 16 * TILE_ROW_BYTES) + aRow;
-#pragma unroll
-                for (int db = 0; db < NDB; db++) {
-                    uint32_t kt[4];                            // {b0 hi, b1 hi, b0 lo, b1 lo}: keys 0-7 / 8-15 of the block, dims 8 db..
-                    ldmatrix_x4_trans(kt, rowt + (uint32_t)(((db + tC) ^ l8) << 4));
-                    mma_f16(dq[db], ah, kt[0], kt[1]);
-                    if constexpr (!LP) { mma_f16(dq[db], al, kt[0], kt[1]); mma_f16(dq[db], as, kt[2], kt[3]); }
-                }
-            }
-            if (r0 < n) {
-#pragma unroll
-                for (int db = 0; db < NDB; db++)
-                    *reinterpret_cast<float2 *>(dQ + (int64_t)r0 * D + hoff + db * 8 + 2 * tig) = make_float2(dq[db][0] * ADOWN * invG * invV * invK, dq[db][1] * ADOWN * invG * invV * invK);
-            }
-            if (r1 < n) {
-#pragma unroll
-                for (int db = 0; db < NDB; db++)
-                    *reinterpret_cast<float2 *>(dQ + (int64_t)r1 * D + hoff + db * 8 + 2 * tig) = make_float2(dq[db][2] * ADOWN * invG * invV * invK, dq[db][3] * ADOWN * invG * invV * invK);
-            }
-        } else {
+        int kb = 0;
+        if (lane == 0) kb = atomicAdd(s_ctr, 1);
+        kb = __shfl_sync(0xffffffffu, kb, 0);
+        if (kb >= nkb) break;
+        {
             // ================= key item: 16 keys, every block of 16 queries =================
-            const int kb = which;
             const int kA = kb * 16 + g, kB = kA + 8;
             const int2 mA = s_meta[kA], mB = s_meta[kB];
             uint32_t kh[KS][4], kl[KS][4], vh[KS][4], vl[KS][4];
@@ -1342,6 +1262,8 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                 dk[db][0] = dk[db][1] = dk[db][2] = dk[db][3] = 0.f;
                 dv[db][0] = dv[db][1] = dv[db][2] = dv[db][3] = 0.f;
             }
+            __syncwarp();                                                  // every lane holds its V fragments: dS^T may replace the rows
+            unsigned qon = 0u;
             // a key of the tile itself is attended only by queries at or after it
             const int qp_first = max(0, kb * 16 - p) >> 4;
             const int qp_end = (nt + 15) >> 4;
@@ -1351,12 +1273,12 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
                     const int rq0 = i0 + qp * 16 + u * 8 + 2 * tig, rq1 = rq0 + 1;
-                    const int2 fk = *reinterpret_cast<const int2 *>(&sFirst[qp * 16 + u * 8 + 2 * tig]);
-                    vld[u][0] = mA.x <= rq0 && rq0 < mA.y && mA.x >= fk.x; vld[u][1] = mA.x <= rq1 && rq1 < mA.y && mA.x >= fk.y;
-                    vld[u][2] = mB.x <= rq0 && rq0 < mB.y && mB.x >= fk.x; vld[u][3] = mB.x <= rq1 && rq1 < mB.y && mB.x >= fk.y;
+                    vld[u][0] = mA.x <= rq0 && rq0 < mA.y; vld[u][1] = mA.x <= rq1 && rq1 < mA.y;
+                    vld[u][2] = mB.x <= rq0 && rq0 < mB.y; vld[u][3] = mB.x <= rq1 && rq1 < mB.y;
                     on[u] = __any_sync(0xffffffffu, vld[u][0] | vld[u][1] | vld[u][2] | vld[u][3]);
                 }
                 if (!(on[0] || on[1])) continue;
+                qon |= 1u << qp;
                 float ds[2][4], pw[2][4];
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
@@ -1388,11 +1310,31 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                         ds[u][j] = pw[u][j] * (dp - ((j & 1) ? dl.y : dl.x) * sclG * sclV) * scale;
                     }
                 }
-                // dK += dS^T Q, dV += P^T dO over the 16 queries
                 uint32_t sh[4], sl[4], ss[4], ph[4], pl[4], ps[4];
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
                     f16_split2<false>(ds[u][0], ds[u][1], sh[2 * u], sl[2 * u]); f16_split2<false>(ds[u][2], ds[u][3], sh[2 * u + 1], sl[2 * u + 1]);
+                }
+                stmatrix_x4(ds_hi(kb, qp) + lane * 16, sh);
+                if constexpr (!LP) stmatrix_x4(ds_lo(kb, qp) + lane * 16, sl);
+                if (gmask.mode != AGPT_GRAD_FULL) {          // dK and dV take the unmasked pairs only (dQ takes all)
+                    bool any = false;
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        const int2 fk = *reinterpret_cast<const int2 *>(&sFirst[qp * 16 + u * 8 + 2 * tig]);
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const bool keep = vld[u][j] && (j < 2 ? mA.x : mB.x) >= ((j & 1) ? fk.y : fk.x);
+                            any |= keep;
+                            if (!keep) ds[u][j] = pw[u][j] = 0.f;
+                        }
+                        f16_split2<false>(ds[u][0], ds[u][1], sh[2 * u], sl[2 * u]); f16_split2<false>(ds[u][2], ds[u][3], sh[2 * u + 1], sl[2 * u + 1]);
+                    }
+                    if (!__any_sync(0xffffffffu, any)) continue;
+                }
+                // dK += dS^T Q, dV += P^T dO over the 16 queries
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
                     f16_split2<false>(pw[u][0], pw[u][1], ph[2 * u], pl[2 * u]); f16_split2<false>(pw[u][2], pw[u][3], ph[2 * u + 1], pl[2 * u + 1]);
                     ss[2 * u] = f16_down11(sh[2 * u]); ss[2 * u + 1] = f16_down11(sh[2 * u + 1]);
                     ps[2 * u] = f16_down11(ph[2 * u]); ps[2 * u + 1] = f16_down11(ph[2 * u + 1]);
@@ -1410,6 +1352,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                     }
                 }
             }
+            if (lane == 0) s_on[kb] = qon;
 #pragma unroll
             for (int half = 0; half < 2; half++) {
                 const int kk = kb * 16 + g + half * 8;
@@ -1423,6 +1366,43 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                     *reinterpret_cast<float2 *>(ov + db * 8 + 2 * tig) = make_float2(dv[db][2 * half] * ADOWN * invG, dv[db][2 * half + 1] * ADOWN * invG);
                 }
             }
+        }
+    }
+    __syncthreads();
+    // dQ = dS K, 16 queries a warp: A fragments are the stored blocks read across (ldmatrix.trans)
+    for (int rg = tid >> 5; rg * 16 < nt; rg += NW) {
+        float dq[NDB][4];
+#pragma unroll
+        for (int db = 0; db < NDB; db++) dq[db][0] = dq[db][1] = dq[db][2] = dq[db][3] = 0.f;
+        const uint32_t la = (uint32_t)(((mi & 1) * 2 + (mi >> 1)) * 128 + l8 * 16);
+        const int kp_lim = min(nkb, (p + rg * 16 + 16 + 15) >> 4);       // the chain and the tile's keys up to the rows' own position
+        for (int kp = 0; kp < kp_lim; kp++) {
+            if (!((s_on[kp] >> rg) & 1u)) continue;
+            uint32_t ah[4], al[4], as[4];
+            ldmatrix_x4_trans(ah, ds_hi(kp, rg) + la);
+            if constexpr (!LP) ldmatrix_x4_trans(al, ds_lo(kp, rg) + la);
+#pragma unroll
+            for (int j = 0; j < 4; j++) as[j] = f16_down11(ah[j]);
+            const uint32_t rowt = uK + (uint32_t)(kp * 16 * TILE_ROW_BYTES) + aRow;
+#pragma unroll
+            for (int db = 0; db < NDB; db++) {
+                uint32_t kt[4];                            // {b0 hi, b1 hi, b0 lo, b1 lo}: keys 0-7 / 8-15 of the block, dims 8 db..
+                ldmatrix_x4_trans(kt, rowt + (uint32_t)(((db + tC) ^ l8) << 4));
+                mma_f16(dq[db], ah, kt[0], kt[1]);
+                if constexpr (!LP) { mma_f16(dq[db], al, kt[0], kt[1]); mma_f16(dq[db], as, kt[2], kt[3]); }
+            }
+        }
+        const int r0 = i0 + rg * 16 + g, r1 = r0 + 8;
+        const float f = ADOWN * invG;
+        if (r0 < n) {
+#pragma unroll
+            for (int db = 0; db < NDB; db++)
+                *reinterpret_cast<float2 *>(dQ + (int64_t)r0 * D + hoff + db * 8 + 2 * tig) = make_float2(dq[db][0] * f * invV * invK, dq[db][1] * f * invV * invK);
+        }
+        if (r1 < n) {
+#pragma unroll
+            for (int db = 0; db < NDB; db++)
+                *reinterpret_cast<float2 *>(dQ + (int64_t)r1 * D + hoff + db * 8 + 2 * tig) = make_float2(dq[db][2] * f * invV * invK, dq[db][3] * f * invV * invK);
         }
     }
 }
@@ -1502,7 +1482,7 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
         int kid = 0x7fffffff, kend = 0;
         if (j < p) { kid = __ldg(chain + j); kend = __ldg(chain_end + j); }
         else if (j < nkeys) { kid = i0 + (j - p); kend = __ldg(sub_end + kid); }
-        s_meta[j] = make_int2(kid, kend);
+        s_meta[j] = make_int2(kid, min(kend, n));        // rows past the tile's end attend nothing
     }
     cp_async_wait_all();                 // this thread's own chunks have landed (pass A reads only those)
 
@@ -1690,7 +1670,7 @@ attn_fwd_bf16_kernel(const float *__restrict__ Q, const __nv_bfloat16 *__restric
                      float *__restrict__ O, float *__restrict__ LSE, const int32_t *__restrict__ sub_end,
                      const int64_t *__restrict__ chain_off, const int32_t *__restrict__ chain_ids,
                      const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H, float scale, int tile0, int maxk) {
-    constexpr int M = 64, NT = 128, KS = HD / 16, NDB = HD / 8, NCH = HD / 8;
+    constexpr int NT = 128, KS = HD / 16, NDB = HD / 8, NCH = HD / 8;
     extern __shared__ __align__(128) unsigned char tile_smem_raw[];
     unsigned char *sK = tile_smem_raw, *sV = sK + (size_t)maxk * (HD * 2);
     int2 *s_meta = reinterpret_cast<int2 *>(sV + (size_t)maxk * (HD * 2));           // [maxk] {key id, key subtree end}
@@ -1720,7 +1700,7 @@ attn_fwd_bf16_kernel(const float *__restrict__ Q, const __nv_bfloat16 *__restric
         int kid = 0x7fffffff, kend = 0;
         if (j < p) { kid = __ldg(chain + j); kend = __ldg(chain_end + j); }
         else if (j < nkeys) { kid = i0 + (j - p); kend = __ldg(sub_end + kid); }
-        s_meta[j] = make_int2(kid, kend);
+        s_meta[j] = make_int2(kid, min(kend, n));        // rows past the tile's end attend nothing
     }
     const int rg = warp, q0 = rg * 16 + g;
     const int r0 = i0 + q0, r1 = r0 + 8;
@@ -1955,15 +1935,13 @@ extern "C" int agpt_b200_set_attn_impl(int impl) {
 // warps per block of the backward.
 // head_dim 32: four blocks of the backward per SM; head_dim 64 (rows twice as long, twice the registers): two
 static inline bool tile_kernels_fit(const agpt_plan *p, int head_dim);
-static int g_bwd_tile = -1, g_bwd_warps = 0, g_bwd_dbg = 0;
+static int g_bwd_tile = -1, g_bwd_warps = 0;
 static int bwd_tile_enabled() {
     if (g_bwd_tile < 0) {
         const char *e = getenv("AGPT_B200_ATTN_TILE");
         g_bwd_tile = (e && e[0] == '0') ? 0 : 1;
         const char *w = getenv("AGPT_B200_BWD_WARPS");
         g_bwd_warps = w ? atoi(w) : 4;
-        const char *d = getenv("AGPT_B200_BWD_DEBUG");
-        g_bwd_dbg = d ? atoi(d) : 0;
         if (g_bwd_warps != 3 && g_bwd_warps != 6 && g_bwd_warps != 8) g_bwd_warps = 4;
     }
     return g_bwd_tile;
@@ -1978,7 +1956,8 @@ extern "C" int agpt_b200_set_attn_variant(int whole_tile, int warps) {
 static inline int bwd_tile_maxk(const agpt_plan *p) { return (p->max_keys + 15) & ~15; }
 static inline bool tile_kernels_fit(const agpt_plan *p, int head_dim) {
     if (head_dim != 32 && head_dim != 64) return false;
-    return bwd_tile_smem_bytes(head_dim, bwd_tile_maxk(p)) <= (head_dim == 32 ? (size_t)56 * 1024 : (size_t)113 * 1024);
+    // head_dim 32: four blocks of the backward per SM up to 96 keys, three up to 147; head_dim 64: two
+    return bwd_tile_smem_bytes(head_dim, bwd_tile_maxk(p), bwd_tile_ds_extra<float>(head_dim)) <= (head_dim == 32 ? (size_t)75 * 1024 : (size_t)113 * 1024);
 }
 // Whole-tile backward for a bfloat16 store (AGPT_B200_ATTN_TILE_BF16=0: the chunked kernel, which keeps float32-level
 // products).  Measured: head_dim 32 (depth-32 trie, 28.3M positions) 42.3 ms against 45.5 ms chunked; head_dim 64 (4M-node
@@ -2085,13 +2064,13 @@ static int launch_bwd_tile(const agpt_plan *p, const float *q, const void *k, co
                            cudaStream_t st, int tile0, int ntiles, BwdMask gmask) {
     static size_t granted[AGPT_MAX_DEVICES];
     const int maxk = bwd_tile_maxk(p);
-    const size_t smem = bwd_tile_smem_bytes(HD, maxk);
+    const size_t smem = bwd_tile_smem_bytes(HD, maxk, bwd_tile_ds_extra<KVT>(HD));
     int rc = allow_dynamic_smem(attn_bwd_tile_kernel<HD, NW, MINB, KVT>, smem, granted);
     if (rc) return rc;
     dim3 grid((unsigned)ntiles, (unsigned)H);
     attn_bwd_tile_kernel<HD, NW, MINB, KVT><<<grid, NW * 32, smem, st>>>(q, (const KVT *)k, (const KVT *)v, o, lse, dout, dq, dk, dv, pk, pv,
                                                                          p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_chain_end,
-                                                                         p->d_tile_start, H, scale, tile0, maxk, g_bwd_dbg, gmask);
+                                                                         p->d_tile_start, H, scale, tile0, maxk, gmask);
     return launch_status("attn_bwd_tile");
 }
 
