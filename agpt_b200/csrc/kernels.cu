@@ -989,76 +989,94 @@ __device__ __forceinline__ void pow2_scale(uint32_t max_bits, int lift, float &s
     inv = __uint_as_float((uint32_t)(e - lift) << 23);
 }
 
-// One staged row holds head_dim floats raw, then head_dim hi halves followed by head_dim lo halves: 4 * head_dim bytes,
-// head_dim / 4 chunks of 16 bytes, the low three bits of the chunk index XOR-ed with row % 8.
-
-// Staging geometry of one thread: it owns chunk c of rows r0, r0 + s, r0 + 2 s, ... of every plane, s = threads /
-// chunks per row.  s is a multiple of 8, so the swizzle term (row % 8) and with it the three byte offsets below are
-// the same for all its rows up to a multiple of the row step: raw = where the raw float4 sits, hi / lo = where its
-// four hi and four lo halves go after the conversion.
-struct TileLane { int r0, c, raw, hi, lo; };
-template <int HD>
-__device__ __forceinline__ TileLane tile_lane(int tid) {
-    constexpr int NCH = HD / 4;
-    TileLane L;
-    L.r0 = tid / NCH; L.c = tid % NCH;
-    const int x = L.r0 & 7, row = L.r0 * (HD * 4), half = (L.c & 1) << 3;
-    L.raw = row + ((L.c ^ x) << 4);
-    L.hi = row + (((L.c >> 1) ^ x) << 4) + half;
-    L.lo = row + (((HD / 8 + (L.c >> 1)) ^ x) << 4) + half;
-    return L;
-}
-__device__ __forceinline__ float abs_max4(float m, float4 a) {
-    return fmaxf(m, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))));
-}
-// In-place conversion of the thread's chunk (row offset o) of two planes: the eight lanes that own the chunks of one
-// row read them, the warp synchronises, and each lane writes its four hi and four lo halves into the row's hi and lo
-// part.  Called by whole warps.
-__device__ __forceinline__ void tile_convert2(unsigned char *pa, unsigned char *pb, const TileLane &L, int o, float sa, float sb) {
-    const float4 a = *reinterpret_cast<const float4 *>(pa + L.raw + o), b = *reinterpret_cast<const float4 *>(pb + L.raw + o);
-    uint2 ah, al, bh, bl;
-    f16_split2<true>(a.x * sa, a.y * sa, ah.x, al.x); f16_split2<true>(a.z * sa, a.w * sa, ah.y, al.y);
-    f16_split2<true>(b.x * sb, b.y * sb, bh.x, bl.x); f16_split2<true>(b.z * sb, b.w * sb, bh.y, bl.y);
-    __syncwarp();
-    *reinterpret_cast<uint2 *>(pa + L.hi + o) = ah; *reinterpret_cast<uint2 *>(pa + L.lo + o) = al;
-    *reinterpret_cast<uint2 *>(pb + L.hi + o) = bh; *reinterpret_cast<uint2 *>(pb + L.lo + o) = bl;
-    __syncwarp();
+// A staged row holds head_dim hi halves followed by head_dim lo halves: 4 * head_dim bytes, head_dim / 4 chunks of 16 bytes, the
+// chunk index XOR-ed with tile_swz(row).  The swizzle is a bijection of row % 8 onto the chunks that share banks, so that the same chunk of eight
+// rows (one ldmatrix) falls into eight bank groups; and its bits are ordered so that the hi chunks of as many rows as eight lanes hold
+// do too (the stores of the conversion).
+template <int HD> __device__ __forceinline__ int tile_swz(int r) {
+    return HD == 16 ? (r & 2) | ((r >> 2) & 1) : ((r & 1) << 2) | ((r >> 1) & 3);
 }
 
-// bfloat16 store: a key row arrives as head_dim bf16 (head_dim / 8 chunks of 16 bytes).  The raw chunk c is parked in the
-// row's lo part (chunk head_dim / 8 + c, swizzled like every chunk) and converted to the hi chunk c of the same row: a
-// bf16 value has 8 significant bits, so its scaled fp16 image is exact and the row has no lo part.  With such a store
-// every product is a single fp16 product (Q, dO, P and dS are rounded to their 11-bit hi halves): about 1e-3 relative,
-// below the store's own rounding (2^-9).  The thread that copied a chunk is the one that converts it.
-struct KvLane { int r0, raw, hi; };
-template <int HD>
-__device__ __forceinline__ KvLane kv_lane(int tid) {
-    constexpr int NCHK = HD / 8;
-    KvLane L;
-    L.r0 = tid / NCHK;
-    const int c = tid % NCHK, x = L.r0 & 7, row = L.r0 * (HD * 4);
-    L.raw = row + (((NCHK + c) ^ x) << 4);
-    L.hi = row + ((c ^ x) << 4);
-    return L;
-}
-__device__ __forceinline__ float abs_max_bf16x8(float m, uint4 a) {
-    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+// Staging geometry of one thread: it owns the eight elements c8 of rows r0, r0 + step, r0 + 2 step, ... of every plane.  step is a
+// multiple of 8, so the swizzle term and with it the two byte offsets are the same for all its rows up to a multiple of the row step.
+// A raw element passes through registers only: loaded once (32 bytes at a time where the buffers allow), its magnitude taken
+// for the scale, held across the barrier that makes the scale known, and stored as hi and lo halves.  Through shared memory (cp.async of raw
+// rows, a read for the maxima, a read and a write for the conversion, its 8-byte stores four to a bank) the staging was two thirds of all shared-memory
+// wavefronts of the forward and the shared-memory pipe 78 % busy.
+template <int HD, int NT> struct TileStage {
+    static constexpr int NL = HD / 8, STEP = NT / NL, ROWB = HD * 4, OSTEP = STEP * ROWB;
+    static_assert(NT % NL == 0 && STEP % 8 == 0, "a thread's rows must share their swizzle term");
+    int r0, c8, hi, lo;
+    __device__ __forceinline__ explicit TileStage(int tid) {
+        r0 = tid / NL; c8 = tid % NL;
+        const int x = tile_swz<HD>(r0), row = r0 * ROWB;
+        hi = row + ((c8 ^ x) << 4);
+        lo = row + (((NL + c8) ^ x) << 4);
+    }
+};
+// eight consecutive elements of a row as they are stored
+template <typename T> struct Raw8;
+template <> struct Raw8<float> {
+    float v[8];
+    __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int j = 0; j < 4; j++)
-        m = fmaxf(m, fmaxf(fabsf(__uint_as_float(w[j] << 16)), fabsf(__uint_as_float(w[j] & 0xffff0000u))));
+        for (int j = 0; j < 8; j++) v[j] = 0.f;
+    }
+    __device__ __forceinline__ void load(const float *p, bool wide) {      // wide: every row starts on a 32-byte boundary
+        if (wide) asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
+        else {
+            const float4 a = ld4(p), b = ld4(p + 4);
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        }
+    }
+    __device__ __forceinline__ float abs_max(float m) const {
+#pragma unroll
+        for (int j = 0; j < 8; j++) m = fmaxf(m, fabsf(v[j]));
+        return m;
+    }
+    // hi and lo halves of the scaled elements into a plane
+    __device__ __forceinline__ void put(unsigned char *hi, unsigned char *lo, float s) const {
+        uint32_t h[4], l[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) f16_split2<true>(v[2 * j] * s, v[2 * j + 1] * s, h[j], l[j]);
+        *reinterpret_cast<uint4 *>(hi) = make_uint4(h[0], h[1], h[2], h[3]);
+        *reinterpret_cast<uint4 *>(lo) = make_uint4(l[0], l[1], l[2], l[3]);
+    }
+};
+// bfloat16 store: 8 significant bits, so an element's scaled fp16 image is exact and there is no lo part.  With such a store every
+// product is a single fp16 product (Q, dO, P and dS are rounded to their 11-bit hi halves): about 1e-3 relative, below the store's own rounding (2^-9).
+template <> struct Raw8<__nv_bfloat16> {
+    uint32_t w[4];
+    __device__ __forceinline__ void zero() { w[0] = w[1] = w[2] = w[3] = 0u; }
+    __device__ __forceinline__ void load(const __nv_bfloat16 *p, bool) {
+        const uint4 a = __ldg(reinterpret_cast<const uint4 *>(p));
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+    }
+    __device__ __forceinline__ float abs_max(float m) const {
+#pragma unroll
+        for (int j = 0; j < 4; j++) m = fmaxf(m, fmaxf(fabsf(__uint_as_float(w[j] << 16)), fabsf(__uint_as_float(w[j] & 0xffff0000u))));
+        return m;
+    }
+    __device__ __forceinline__ void put(unsigned char *hi, unsigned char *, float s) const {
+        uint32_t h[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) h[j] = f16_pack2(__uint_as_float(w[j] << 16) * s, __uint_as_float(w[j] & 0xffff0000u) * s);
+        *reinterpret_cast<uint4 *>(hi) = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+};
+// passes of key rows that a thread holds in registers: 96 keys.  The rows of a longer tile are loaded once for the maxima and again
+// for the conversion.
+template <int HD, int NT> struct KeyPasses { static constexpr int value = (96 + TileStage<HD, NT>::STEP - 1) / TileStage<HD, NT>::STEP; };
+__device__ __forceinline__ float warp_max(float m) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     return m;
 }
-__device__ __forceinline__ void kv_convert_bf16(unsigned char *pa, const KvLane &L, int o, float sa) {
-    const uint4 a = *reinterpret_cast<const uint4 *>(pa + L.raw + o);
-    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
-    uint32_t h[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) h[j] = f16_pack2(__uint_as_float(w[j] << 16) * sa, __uint_as_float(w[j] & 0xffff0000u) * sa);
-    *reinterpret_cast<uint4 *>(pa + L.hi + o) = make_uint4(h[0], h[1], h[2], h[3]);
-}
 
-// bytes of one key block's dS^T (16 keys x 64 queries) that do not fit the block's own V rows: float32 stores hold hi and lo parts
-template <typename KVT> constexpr int bwd_tile_ds_extra(int hd) { return sizeof(KVT) == 2 || hd >= 64 ? 0 : 16 * 64 * 4 - 16 * hd * 4; }
+// bytes of one key block's dS^T (16 keys x 64 queries, hi and for a float32 store lo halves) that lie outside the block's own V rows: its
+// lo part for head_dim 32, all of it for 16
+template <typename KVT> constexpr int bwd_tile_ds_extra(int hd) { return sizeof(KVT) == 2 || hd >= 64 ? 0 : hd == 32 ? 2048 : 4096; }
 constexpr size_t bwd_tile_smem_bytes(int hd, int maxk, int ds_extra) {
     return (size_t)(2 * 64 + 2 * maxk) * (size_t)(hd * 4) + (size_t)(maxk / 16) * (size_t)ds_extra + (size_t)maxk * 8 + 3 * 64 * 4 + 32 + (size_t)(maxk / 16) * 4;
 }
@@ -1070,8 +1088,8 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                      float *__restrict__ dQ, float *__restrict__ dK, float *__restrict__ dV, float *__restrict__ Pk,
                      float *__restrict__ Pv, const int32_t *__restrict__ sub_end, const int64_t *__restrict__ chain_off,
                      const int32_t *__restrict__ chain_ids, const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H,
-                     float scale, int tile0, int maxk, BwdMask gmask) {
-    constexpr int M = 64, NT = NW * 32, TILE_ROW_BYTES = HD * 4, KS = HD / 16, NDB = HD / 8, NCH = HD / 4;
+                     float scale, int tile0, int maxk, bool wide, BwdMask gmask) {
+    constexpr int M = 64, NT = NW * 32, TILE_ROW_BYTES = HD * 4, KS = HD / 16, NDB = HD / 8;
     constexpr bool LP = sizeof(KVT) == 2;              // bfloat16 store: single fp16 products, no lo parts
     extern __shared__ __align__(128) unsigned char tile_smem_raw[];
     unsigned char *sQ = tile_smem_raw, *sG = sQ + M * TILE_ROW_BYTES, *sK = sG + M * TILE_ROW_BYTES;
@@ -1098,100 +1116,79 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     const int32_t *chain = chain_ids + coff;
     const int32_t *chain_end = chain_end_all + coff;
 
-    // ---- stage 1: raw rows by cp.async (chunk c of row r goes to chunk c ^ r % 8), O rows to registers ----
+    // ---- rows to registers, delta = dO . O ----
     if (tid < 4) s_max[tid] = 0u;
     if (tid == 0) *s_ctr = 0;
-    constexpr int RSTEP = NT / NCH, OSTEP = RSTEP * TILE_ROW_BYTES;
-    static_assert(NT % NCH == 0 && RSTEP % 8 == 0, "a thread's rows must share their swizzle term");
-    constexpr int UQ = (M + RSTEP - 1) / RSTEP;
-    const TileLane L = tile_lane<HD>(tid);
-    float4 ox[UQ];
+    typedef TileStage<HD, NT> Stage;
+    constexpr int UQ = (M + Stage::STEP - 1) / Stage::STEP, UK = KeyPasses<HD, NT>::value;
+    const Stage T(tid);
+    Raw8<float> q8[UQ], g8[UQ];
+    {
+        Raw8<float> o8[UQ];
 #pragma unroll
-    for (int u = 0; u < UQ; u++) {
-        const int r = L.r0 + u * RSTEP, o = L.raw + u * OSTEP;
-        ox[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < M) {
+        for (int u = 0; u < UQ; u++) {
+            const int r = T.r0 + u * T.STEP;
+            q8[u].zero(); g8[u].zero(); o8[u].zero();
             if (r < nt) {
-                const int64_t off = (int64_t)(i0 + r) * D + hoff + L.c * 4;
-                cp_async16(sQ + o, Q + off); cp_async16(sG + o, dO + off);
-                ox[u] = ld4(O + off);
-            } else {
-                *reinterpret_cast<float4 *>(sQ + o) = make_float4(0.f, 0.f, 0.f, 0.f);
-                *reinterpret_cast<float4 *>(sG + o) = make_float4(0.f, 0.f, 0.f, 0.f);
+                const int64_t off = (int64_t)(i0 + r) * D + hoff + T.c8 * 8;
+                q8[u].load(Q + off, wide); g8[u].load(dO + off, wide); o8[u].load(O + off, wide);
             }
+        }
+        if (tid < M) {
+            sLse[tid] = tid < nt ? __ldg(LSE + (int64_t)(i0 + tid) * H + h) * LOG2E : 0.f;
+            sFirst[tid] = bwd_first_key(gmask, i0 + tid, n);
+        }
+#pragma unroll
+        for (int u = 0; u < UQ; u++) {
+            const int r = T.r0 + u * T.STEP;
+            float d = 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; j++) d = fmaf(g8[u].v[j], o8[u].v[j], d);
+#pragma unroll
+            for (int o = 1; o < T.NL; o <<= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+            if (T.c8 == 0 && r < M) sDelta[r] = d;
         }
     }
-    constexpr int RSTEPK = NT / (HD / 8), OSTEPK = RSTEPK * TILE_ROW_BYTES;
-    static_assert(NT % (HD / 8) == 0 && RSTEPK % 8 == 0, "a thread's key rows must share their swizzle term");
-    const KvLane LK = kv_lane<HD>(tid);
-    if constexpr (LP) {
-        for (int r = LK.r0, o = LK.raw; r < nkp; r += RSTEPK, o += OSTEPK) {
-            if (r < nkeys) {
-                const int kid = r < p ? __ldg(chain + r) : i0 + (r - p);
-                const int64_t off = (int64_t)kid * D + hoff + (tid % (HD / 8)) * 8;
-                cp_async16(sK + o, K + off); cp_async16(sV + o, V + off);
-            } else {
-                *reinterpret_cast<uint4 *>(sK + o) = make_uint4(0u, 0u, 0u, 0u);
-                *reinterpret_cast<uint4 *>(sV + o) = make_uint4(0u, 0u, 0u, 0u);
-            }
-        }
-    } else {
-        for (int r = L.r0, o = L.raw; r < nkp; r += RSTEP, o += OSTEP) {
-            if (r < nkeys) {
-                const int kid = r < p ? __ldg(chain + r) : i0 + (r - p);
-                const int64_t off = (int64_t)kid * D + hoff + L.c * 4;
-                cp_async16(sK + o, K + off); cp_async16(sV + o, V + off);
-            } else {
-                *reinterpret_cast<float4 *>(sK + o) = make_float4(0.f, 0.f, 0.f, 0.f);
-                *reinterpret_cast<float4 *>(sV + o) = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+    Raw8<KVT> k8[UK], v8[UK];
+#pragma unroll
+    for (int u = 0; u < UK; u++) {
+        const int r = T.r0 + u * T.STEP;
+        k8[u].zero(); v8[u].zero();
+        if (r < nkeys) {
+            const int kid = r < p ? __ldg(chain + r) : i0 + (r - p);
+            const int64_t off = (int64_t)kid * D + hoff + T.c8 * 8;
+            k8[u].load(K + off, wide); v8[u].load(V + off, wide);
         }
     }
-    cp_async_commit();
+    // key rows beyond the passes held in registers
+    auto far_keys = [&](auto &&f) {
+        for (int r = T.r0 + UK * T.STEP; r < nkp; r += T.STEP) {
+            Raw8<KVT> kx, vx;
+            kx.zero(); vx.zero();
+            if (r < nkeys) {
+                const int kid = r < p ? __ldg(chain + r) : i0 + (r - p);
+                const int64_t off = (int64_t)kid * D + hoff + T.c8 * 8;
+                kx.load(K + off, wide); vx.load(V + off, wide);
+            }
+            f(kx, vx, (r - T.r0) * T.ROWB);
+        }
+    };
     for (int j = tid; j < nkp; j += NT) {
         int kid = 0x7fffffff, kend = 0;
         if (j < p) { kid = __ldg(chain + j); kend = __ldg(chain_end + j); }
         else if (j < nkeys) { kid = i0 + (j - p); kend = __ldg(sub_end + kid); }
         s_meta[j] = make_int2(kid, min(kend, n));        // rows past the tile's end attend nothing
     }
-    if (tid < M) {
-        sLse[tid] = tid < nt ? __ldg(LSE + (int64_t)(i0 + tid) * H + h) * LOG2E : 0.f;
-        sFirst[tid] = bwd_first_key(gmask, i0 + tid, n);
-    }
-    cp_async_wait_all();                 // this thread's own chunks have landed (pass A reads only those)
-
-    // ---- stage 2 (pass A): maxima of |x| per tensor, delta = dO . O per row ----
+    // ---- maxima of |x| per tensor ----
     {
         float mq = 0.f, mg = 0.f, mk = 0.f, mv = 0.f;
 #pragma unroll
-        for (int u = 0; u < UQ; u++) {       // whole warps enter or skip an iteration (a warp holds four whole rows)
-            const int r = L.r0 + u * RSTEP, o = L.raw + u * OSTEP;
-            if (r < M) {
-                const float4 a = *reinterpret_cast<const float4 *>(sQ + o), b = *reinterpret_cast<const float4 *>(sG + o);
-                mq = abs_max4(mq, a); mg = abs_max4(mg, b);
-                float d = b.x * ox[u].x;
-                d = fmaf(b.y, ox[u].y, d); d = fmaf(b.z, ox[u].z, d); d = fmaf(b.w, ox[u].w, d);
+        for (int u = 0; u < UQ; u++) { mq = q8[u].abs_max(mq); mg = g8[u].abs_max(mg); }
 #pragma unroll
-                for (int o = 1; o < NCH; o <<= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-                if (L.c == 0) sDelta[r] = d;
-            }
-        }
-        if constexpr (LP) {
-            for (int r = LK.r0, o = LK.raw; r < nkp; r += RSTEPK, o += OSTEPK) {
-                mk = abs_max_bf16x8(mk, *reinterpret_cast<const uint4 *>(sK + o));
-                mv = abs_max_bf16x8(mv, *reinterpret_cast<const uint4 *>(sV + o));
-            }
-        } else {
-            for (int r = L.r0, o = L.raw; r < nkp; r += RSTEP, o += OSTEP) {
-                mk = abs_max4(mk, *reinterpret_cast<const float4 *>(sK + o));
-                mv = abs_max4(mv, *reinterpret_cast<const float4 *>(sV + o));
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mq = fmaxf(mq, __shfl_xor_sync(0xffffffffu, mq, o)); mg = fmaxf(mg, __shfl_xor_sync(0xffffffffu, mg, o));
-            mk = fmaxf(mk, __shfl_xor_sync(0xffffffffu, mk, o)); mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-        }
+        for (int u = 0; u < UK; u++) { mk = k8[u].abs_max(mk); mv = v8[u].abs_max(mv); }
+        far_keys([&](const Raw8<KVT> &kx, const Raw8<KVT> &vx, int) { mk = kx.abs_max(mk); mv = vx.abs_max(mv); });
+        mq = warp_max(mq); mg = warp_max(mg); mk = warp_max(mk); mv = warp_max(mv);
+        __syncthreads();                     // s_max is zero
         if (lane == 0) {                     // non-negative floats order like their bit patterns
             atomicMax(&s_max[0], __float_as_uint(mq)); atomicMax(&s_max[1], __float_as_uint(mk));
             atomicMax(&s_max[2], __float_as_uint(mv)); atomicMax(&s_max[3], __float_as_uint(mg));
@@ -1202,15 +1199,22 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     pow2_scale(s_max[0], 0, sclQ, invQ); pow2_scale(s_max[1], 0, sclK, invK);
     pow2_scale(s_max[2], 0, sclV, invV); pow2_scale(s_max[3], -2, sclG, invG);
 
-    // ---- stage 3 (pass B): convert in place ----
+    // ---- halves to shared memory ----
 #pragma unroll
     for (int u = 0; u < UQ; u++)
-        if (L.r0 + u * RSTEP < M) tile_convert2(sQ, sG, L, u * OSTEP, sclQ, sclG);
-    if constexpr (LP) {
-        for (int r = LK.r0, o = 0; r < nkp; r += RSTEPK, o += OSTEPK) { kv_convert_bf16(sK, LK, o, sclK); kv_convert_bf16(sV, LK, o, sclV); }
-    } else {
-        for (int r = L.r0, o = 0; r < nkp; r += RSTEP, o += OSTEP) tile_convert2(sK, sV, L, o, sclK, sclV);
-    }
+        if (T.r0 + u * T.STEP < M) {
+            q8[u].put(sQ + T.hi + u * T.OSTEP, sQ + T.lo + u * T.OSTEP, sclQ);
+            g8[u].put(sG + T.hi + u * T.OSTEP, sG + T.lo + u * T.OSTEP, sclG);
+        }
+#pragma unroll
+    for (int u = 0; u < UK; u++)
+        if (T.r0 + u * T.STEP < nkp) {
+            k8[u].put(sK + T.hi + u * T.OSTEP, sK + T.lo + u * T.OSTEP, sclK);
+            v8[u].put(sV + T.hi + u * T.OSTEP, sV + T.lo + u * T.OSTEP, sclV);
+        }
+    far_keys([&](const Raw8<KVT> &kx, const Raw8<KVT> &vx, int o) {
+        kx.put(sK + T.hi + o, sK + T.lo + o, sclK); vx.put(sV + T.hi + o, sV + T.lo + o, sclV);
+    });
     __syncthreads();
 
     // units: S' = (Q sQ)(K sK)^T, dP' = (dO sG)(V sV)^T, P' = 2^11 P, dS' = P' (dP' - delta sG sV) scale = 2^11 dS sG sV
@@ -1219,7 +1223,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     // The powers of two are applied one after the other, never as one product that could leave the float range.
 
     // ldmatrix lane addressing: lane l names row l % 8 of matrix l / 8 (rows of 16 bytes).
-    const int l8 = lane & 7, mi = lane >> 3;
+    const int l8 = lane & 7, mi = lane >> 3, sw = tile_swz<HD>(l8);
     // B fragments of an 8-row block for k-step ks (16 dims): matrices {hi chunk 2ks, hi 2ks+1, lo 2ks, lo 2ks+1}
     const uint32_t bRow = (uint32_t)(l8 * TILE_ROW_BYTES);
     const int bC = (mi & 1) + (mi >> 1) * NDB;          // + 2 ks
@@ -1235,8 +1239,8 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     // queries 0-7, keys 0-7 queries 8-15, keys 8-15 queries 8-15}.  hi parts and, where they fit, lo parts lie in the key block's own V rows, which
     // nothing reads any more once the block's item holds its V fragments.
     const uint32_t uDX = smem_u32_of(sDX);
-    auto ds_hi = [&](int kb, int qp) { return uV + (uint32_t)(kb * 16 * TILE_ROW_BYTES + qp * 512); };
-    auto ds_lo = [&](int kb, int qp) { return DSX ? uDX + (uint32_t)(kb * DSX + qp * 512) : uV + (uint32_t)(kb * 16 * TILE_ROW_BYTES + 2048 + qp * 512); };
+    auto ds_hi = [&](int kb, int qp) { return (DSX == 4096 ? uDX + (uint32_t)(kb * DSX) : uV + (uint32_t)(kb * 16 * TILE_ROW_BYTES)) + (uint32_t)(qp * 512); };
+    auto ds_lo = [&](int kb, int qp) { return DSX == 2048 ? uDX + (uint32_t)(kb * DSX + qp * 512) : ds_hi(kb, qp) + 2048u; };
 
     const int nkb = nkp >> 4;                    // key items: chain keys first (attended by most rows), then the tile's own
     for (;;) {
@@ -1252,7 +1256,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
 #pragma unroll
             for (int ks = 0; ks < KS; ks++) {
                 const uint32_t o = (uint32_t)(kb * 16 * TILE_ROW_BYTES) + aRow;
-                const uint32_t ch = (uint32_t)(((2 * ks + aC) ^ l8) << 4), cl = (uint32_t)(((2 * ks + aC + NDB) ^ l8) << 4);
+                const uint32_t ch = (uint32_t)(((2 * ks + aC) ^ sw) << 4), cl = (uint32_t)(((2 * ks + aC + NDB) ^ sw) << 4);
                 ldmatrix_x4(kh[ks], uK + o + ch); ldmatrix_x4(vh[ks], uV + o + ch);
                 if constexpr (!LP) { ldmatrix_x4(kl[ks], uK + o + cl); ldmatrix_x4(vl[ks], uV + o + cl); }
             }
@@ -1291,7 +1295,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                     const uint32_t rowb = (uint32_t)(qr * TILE_ROW_BYTES) + bRow;
 #pragma unroll
                     for (int ks = 0; ks < KS; ks++) {
-                        const uint32_t o = rowb + (uint32_t)(((2 * ks + bC) ^ l8) << 4);
+                        const uint32_t o = rowb + (uint32_t)(((2 * ks + bC) ^ sw) << 4);
                         uint32_t qf[4], gf[4];                 // {b0 hi, b1 hi, b0 lo, b1 lo}
                         ldmatrix_x4(qf, uQ + o); ldmatrix_x4(gf, uG + o);
                         mma_f16(c, kh[ks], qf[0], qf[1]); mma_f16(e, vh[ks], gf[0], gf[1]);
@@ -1343,7 +1347,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
 #pragma unroll
                 for (int db = 0; db < NDB; db++) {
                     uint32_t qt[4], gt[4];                     // {b0 hi, b1 hi, b0 lo, b1 lo}: queries 0-7 / 8-15 of the block, dims 8 db..
-                    const uint32_t co = (uint32_t)(((db + tC) ^ l8) << 4);
+                    const uint32_t co = (uint32_t)(((db + tC) ^ sw) << 4);
                     ldmatrix_x4_trans(qt, uQ + ro + co); ldmatrix_x4_trans(gt, uG + ro + co);
                     mma_f16(dk[db], sh, qt[0], qt[1]); mma_f16(dv[db], ph, gt[0], gt[1]);
                     if constexpr (!LP) {
@@ -1387,7 +1391,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
 #pragma unroll
             for (int db = 0; db < NDB; db++) {
                 uint32_t kt[4];                            // {b0 hi, b1 hi, b0 lo, b1 lo}: keys 0-7 / 8-15 of the block, dims 8 db..
-                ldmatrix_x4_trans(kt, rowt + (uint32_t)(((db + tC) ^ l8) << 4));
+                ldmatrix_x4_trans(kt, rowt + (uint32_t)(((db + tC) ^ sw) << 4));
                 mma_f16(dq[db], ah, kt[0], kt[1]);
                 if constexpr (!LP) { mma_f16(dq[db], al, kt[0], kt[1]); mma_f16(dq[db], as, kt[2], kt[3]); }
             }
@@ -1421,8 +1425,8 @@ __global__ void __launch_bounds__(128, MINB)
 attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, const KVT *__restrict__ V,
                      float *__restrict__ O, float *__restrict__ LSE, const int32_t *__restrict__ sub_end,
                      const int64_t *__restrict__ chain_off, const int32_t *__restrict__ chain_ids,
-                     const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H, float scale, int tile0, int maxk) {
-    constexpr int M = 64, NT = 128, TILE_ROW_BYTES = HD * 4, KS = HD / 16, NDB = HD / 8, NCH = HD / 4;
+                     const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H, float scale, int tile0, int maxk, bool wide) {
+    constexpr int M = 64, NT = 128, TILE_ROW_BYTES = HD * 4, KS = HD / 16, NDB = HD / 8;
     constexpr bool LP = sizeof(KVT) == 2;              // bfloat16 store: single fp16 products, no lo parts
     extern __shared__ __align__(128) unsigned char tile_smem_raw[];
     unsigned char *sQ = tile_smem_raw, *sK = sQ + M * TILE_ROW_BYTES, *sV = sK + (size_t)maxk * TILE_ROW_BYTES;
@@ -1441,72 +1445,58 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     const int32_t *chain = chain_ids + coff;
     const int32_t *chain_end = chain_end_all + coff;
 
-    // ---- stage 1: raw rows by cp.async ----
+    // ---- rows to registers ----
     if (tid < 3) s_max[tid] = 0u;
-    constexpr int RSTEP = NT / NCH, OSTEP = RSTEP * TILE_ROW_BYTES;
-    const TileLane L = tile_lane<HD>(tid);
+    typedef TileStage<HD, NT> Stage;
+    constexpr int UQ = M / Stage::STEP, UK = KeyPasses<HD, NT>::value;
+    const Stage T(tid);
+    Raw8<float> q8[UQ];
 #pragma unroll
-    for (int u = 0; u < M / RSTEP; u++) {
-        const int r = L.r0 + u * RSTEP, o = L.raw + u * OSTEP;
-        if (r < nt) cp_async16(sQ + o, Q + (int64_t)(i0 + r) * D + hoff + L.c * 4);
-        else *reinterpret_cast<float4 *>(sQ + o) = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = 0; u < UQ; u++) {
+        const int r = T.r0 + u * T.STEP;
+        q8[u].zero();
+        if (r < nt) q8[u].load(Q + (int64_t)(i0 + r) * D + hoff + T.c8 * 8, wide);
     }
-    constexpr int RSTEPK = NT / (HD / 8), OSTEPK = RSTEPK * TILE_ROW_BYTES;
-    static_assert(NT % (HD / 8) == 0 && RSTEPK % 8 == 0, "a thread's key rows must share their swizzle term");
-    const KvLane LK = kv_lane<HD>(tid);
-    if constexpr (LP) {
-        for (int r = LK.r0, o = LK.raw; r < nkp; r += RSTEPK, o += OSTEPK) {
-            if (r < nkeys) {
-                const int kid = r < p ? __ldg(chain + r) : i0 + (r - p);
-                const int64_t off = (int64_t)kid * D + hoff + (tid % (HD / 8)) * 8;
-                cp_async16(sK + o, K + off); cp_async16(sV + o, V + off);
-            } else {
-                *reinterpret_cast<uint4 *>(sK + o) = make_uint4(0u, 0u, 0u, 0u);
-                *reinterpret_cast<uint4 *>(sV + o) = make_uint4(0u, 0u, 0u, 0u);
-            }
-        }
-    } else {
-        for (int r = L.r0, o = L.raw; r < nkp; r += RSTEP, o += OSTEP) {
-            if (r < nkeys) {
-                const int kid = r < p ? __ldg(chain + r) : i0 + (r - p);
-                const int64_t off = (int64_t)kid * D + hoff + L.c * 4;
-                cp_async16(sK + o, K + off); cp_async16(sV + o, V + off);
-            } else {
-                *reinterpret_cast<float4 *>(sK + o) = make_float4(0.f, 0.f, 0.f, 0.f);
-                *reinterpret_cast<float4 *>(sV + o) = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+    Raw8<KVT> k8[UK], v8[UK];
+#pragma unroll
+    for (int u = 0; u < UK; u++) {
+        const int r = T.r0 + u * T.STEP;
+        k8[u].zero(); v8[u].zero();
+        if (r < nkeys) {
+            const int kid = r < p ? __ldg(chain + r) : i0 + (r - p);
+            const int64_t off = (int64_t)kid * D + hoff + T.c8 * 8;
+            k8[u].load(K + off, wide); v8[u].load(V + off, wide);
         }
     }
-    cp_async_commit();
+    // key rows beyond the passes held in registers
+    auto far_keys = [&](auto &&f) {
+        for (int r = T.r0 + UK * T.STEP; r < nkp; r += T.STEP) {
+            Raw8<KVT> kx, vx;
+            kx.zero(); vx.zero();
+            if (r < nkeys) {
+                const int kid = r < p ? __ldg(chain + r) : i0 + (r - p);
+                const int64_t off = (int64_t)kid * D + hoff + T.c8 * 8;
+                kx.load(K + off, wide); vx.load(V + off, wide);
+            }
+            f(kx, vx, (r - T.r0) * T.ROWB);
+        }
+    };
     for (int j = tid; j < nkp; j += NT) {
         int kid = 0x7fffffff, kend = 0;
         if (j < p) { kid = __ldg(chain + j); kend = __ldg(chain_end + j); }
         else if (j < nkeys) { kid = i0 + (j - p); kend = __ldg(sub_end + kid); }
         s_meta[j] = make_int2(kid, min(kend, n));        // rows past the tile's end attend nothing
     }
-    cp_async_wait_all();                 // this thread's own chunks have landed (pass A reads only those)
-
-    // ---- stage 2 (pass A): maxima of |x| per tensor ----
+    // ---- maxima of |x| per tensor ----
     {
         float mq = 0.f, mk = 0.f, mv = 0.f;
 #pragma unroll
-        for (int u = 0; u < M / RSTEP; u++) mq = abs_max4(mq, *reinterpret_cast<const float4 *>(sQ + L.raw + u * OSTEP));
-        if constexpr (LP) {
-            for (int r = LK.r0, o = LK.raw; r < nkp; r += RSTEPK, o += OSTEPK) {
-                mk = abs_max_bf16x8(mk, *reinterpret_cast<const uint4 *>(sK + o));
-                mv = abs_max_bf16x8(mv, *reinterpret_cast<const uint4 *>(sV + o));
-            }
-        } else {
-            for (int r = L.r0, o = L.raw; r < nkp; r += RSTEP, o += OSTEP) {
-                mk = abs_max4(mk, *reinterpret_cast<const float4 *>(sK + o));
-                mv = abs_max4(mv, *reinterpret_cast<const float4 *>(sV + o));
-            }
-        }
+        for (int u = 0; u < UQ; u++) mq = q8[u].abs_max(mq);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mq = fmaxf(mq, __shfl_xor_sync(0xffffffffu, mq, o)); mk = fmaxf(mk, __shfl_xor_sync(0xffffffffu, mk, o));
-            mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-        }
+        for (int u = 0; u < UK; u++) { mk = k8[u].abs_max(mk); mv = v8[u].abs_max(mv); }
+        far_keys([&](const Raw8<KVT> &kx, const Raw8<KVT> &vx, int) { mk = kx.abs_max(mk); mv = vx.abs_max(mv); });
+        mq = warp_max(mq); mk = warp_max(mk); mv = warp_max(mv);
+        __syncthreads();                     // s_max is zero
         if (lane == 0) {
             atomicMax(&s_max[0], __float_as_uint(mq)); atomicMax(&s_max[1], __float_as_uint(mk)); atomicMax(&s_max[2], __float_as_uint(mv));
         }
@@ -1515,20 +1505,24 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     float sclQ, invQ, sclK, invK, sclV, invV;
     pow2_scale(s_max[0], 0, sclQ, invQ); pow2_scale(s_max[1], 0, sclK, invK); pow2_scale(s_max[2], 0, sclV, invV);
 
-    // ---- stage 3 (pass B): convert in place (Q rows two at a time through the two-plane helper) ----
+    // ---- halves to shared memory ----
 #pragma unroll
-    for (int u = 0; u < M / RSTEP; u += 2) tile_convert2(sQ, sQ + OSTEP, L, u * OSTEP, sclQ, sclQ);
-    if constexpr (LP) {
-        for (int r = LK.r0, o = 0; r < nkp; r += RSTEPK, o += OSTEPK) { kv_convert_bf16(sK, LK, o, sclK); kv_convert_bf16(sV, LK, o, sclV); }
-    } else {
-        for (int r = L.r0, o = 0; r < nkp; r += RSTEP, o += OSTEP) tile_convert2(sK, sV, L, o, sclK, sclV);
-    }
+    for (int u = 0; u < UQ; u++) q8[u].put(sQ + T.hi + u * T.OSTEP, sQ + T.lo + u * T.OSTEP, sclQ);
+#pragma unroll
+    for (int u = 0; u < UK; u++)
+        if (T.r0 + u * T.STEP < nkp) {
+            k8[u].put(sK + T.hi + u * T.OSTEP, sK + T.lo + u * T.OSTEP, sclK);
+            v8[u].put(sV + T.hi + u * T.OSTEP, sV + T.lo + u * T.OSTEP, sclV);
+        }
+    far_keys([&](const Raw8<KVT> &kx, const Raw8<KVT> &vx, int o) {
+        kx.put(sK + T.hi + o, sK + T.lo + o, sclK); vx.put(sV + T.hi + o, sV + T.lo + o, sclV);
+    });
     __syncthreads();
 
     const int rg = warp;
     if (rg * 16 >= nt) return;                                   // rows beyond the end of the plan (no barrier follows)
     const float fS = scale * LOG2E * invQ * invK;               // log2-domain score = S' * fS
-    const int l8 = lane & 7, mi = lane >> 3;
+    const int l8 = lane & 7, mi = lane >> 3, sw = tile_swz<HD>(l8);
     const uint32_t bRow = (uint32_t)(l8 * TILE_ROW_BYTES);
     const int bC = (mi & 1) + (mi >> 1) * NDB;
     const uint32_t aRow = (uint32_t)((l8 + (mi & 1) * 8) * TILE_ROW_BYTES);
@@ -1541,8 +1535,8 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
 #pragma unroll
     for (int ks = 0; ks < KS; ks++) {
         const uint32_t o = (uint32_t)(rg * 16 * TILE_ROW_BYTES) + aRow;
-        ldmatrix_x4(qh[ks], uQ + o + (uint32_t)(((2 * ks + aC) ^ l8) << 4));
-        if constexpr (!LP) ldmatrix_x4(ql[ks], uQ + o + (uint32_t)(((2 * ks + aC + NDB) ^ l8) << 4));
+        ldmatrix_x4(qh[ks], uQ + o + (uint32_t)(((2 * ks + aC) ^ sw) << 4));
+        if constexpr (!LP) ldmatrix_x4(ql[ks], uQ + o + (uint32_t)(((2 * ks + aC + NDB) ^ sw) << 4));
     }
     float o_[NDB][4];
 #pragma unroll
@@ -1570,7 +1564,7 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
 #pragma unroll
             for (int ks = 0; ks < KS; ks++) {
                 uint32_t kf[4];
-                ldmatrix_x4(kf, uK + rowb + (uint32_t)(((2 * ks + bC) ^ l8) << 4));
+                ldmatrix_x4(kf, uK + rowb + (uint32_t)(((2 * ks + bC) ^ sw) << 4));
                 mma_f16(c, qh[ks], kf[0], kf[1]);
                 if constexpr (!LP) { mma_f16(cx, ql[ks], kf[0], kf[1]); mma_f16(cx, qh[ks], kf[2], kf[3]); }
             }
@@ -1611,7 +1605,7 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
 #pragma unroll
         for (int db = 0; db < NDB; db++) {
             uint32_t vt[4];                            // {b0 hi, b1 hi, b0 lo, b1 lo}: keys 0-7 / 8-15 of the block, dims 8 db..
-            ldmatrix_x4_trans(vt, rowt + (uint32_t)(((db + tC) ^ l8) << 4));
+            ldmatrix_x4_trans(vt, rowt + (uint32_t)(((db + tC) ^ sw) << 4));
             mma_f16(o_[db], ph, vt[0], vt[1]);
             if constexpr (!LP) { mma_f16(o_[db], pl, vt[0], vt[1]); mma_f16(o_[db], ps, vt[2], vt[3]); }
         }
@@ -1934,7 +1928,6 @@ extern "C" int agpt_b200_set_attn_impl(int impl) {
 // the chunked kernels.  AGPT_B200_ATTN_TILE=0 keeps the chunked kernels (A/B runs); AGPT_B200_BWD_WARPS = 4, 6 or 8
 // warps per block of the backward.
 // head_dim 32: four blocks of the backward per SM; head_dim 64 (rows twice as long, twice the registers): two
-static inline bool tile_kernels_fit(const agpt_plan *p, int head_dim);
 static int g_bwd_tile = -1, g_bwd_warps = 0;
 static int bwd_tile_enabled() {
     if (g_bwd_tile < 0) {
@@ -1953,11 +1946,19 @@ extern "C" int agpt_b200_set_attn_variant(int whole_tile, int warps) {
     g_bwd_tile = whole_tile; g_bwd_warps = warps;
     return AGPT_OK;
 }
+// every head of every row of these buffers starts on a 32-byte boundary
+static bool rows_wide(int D, const void *a, const void *b, const void *c, const void *d, const void *e) {
+    return D % 8 == 0 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)e) & 31) == 0;
+}
 static inline int bwd_tile_maxk(const agpt_plan *p) { return (p->max_keys + 15) & ~15; }
-static inline bool tile_kernels_fit(const agpt_plan *p, int head_dim) {
-    if (head_dim != 32 && head_dim != 64) return false;
-    // head_dim 32: four blocks of the backward per SM up to 96 keys, three up to 147; head_dim 64: two
-    return bwd_tile_smem_bytes(head_dim, bwd_tile_maxk(p), bwd_tile_ds_extra<float>(head_dim)) <= (head_dim == 32 ? (size_t)75 * 1024 : (size_t)113 * 1024);
+// head_dim 16 and 32: three blocks of the backward per SM at least (32: four up to 96 keys, three up to 147); head_dim 64: two
+static inline bool bwd_tile_fits(const agpt_plan *p, int head_dim) {
+    if (head_dim != 16 && head_dim != 32 && head_dim != 64) return false;
+    return bwd_tile_smem_bytes(head_dim, bwd_tile_maxk(p), bwd_tile_ds_extra<float>(head_dim)) <= (head_dim == 64 ? (size_t)113 * 1024 : (size_t)75 * 1024);
+}
+static inline bool fwd_tile_fits(const agpt_plan *p, int head_dim) {
+    if (head_dim != 16 && head_dim != 32 && head_dim != 64) return false;
+    return fwd_tile_smem_bytes(head_dim, bwd_tile_maxk(p)) <= (head_dim == 64 ? (size_t)75 * 1024 : (size_t)56 * 1024);
 }
 // Whole-tile backward for a bfloat16 store (AGPT_B200_ATTN_TILE_BF16=0: the chunked kernel, which keeps float32-level
 // products).  Measured: head_dim 32 (depth-32 trie, 28.3M positions) 42.3 ms against 45.5 ms chunked; head_dim 64 (4M-node
@@ -1981,7 +1982,7 @@ static int launch_fwd_tile(const agpt_plan *p, const float *q, const void *k, co
     if (rc) return rc;
     dim3 grid((unsigned)ntiles, (unsigned)H);
     attn_fwd_tile_kernel<HD, MINB, KVT><<<grid, 128, smem, st>>>(q, (const KVT *)k, (const KVT *)v, out, lse, p->d_sub_end,
-                                                                 p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H, scale, tile0, maxk);
+                                                                 p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H, scale, tile0, maxk, rows_wide(H * HD, q, k, v, q, q));
     return launch_status("attn_fwd_tile");
 }
 
@@ -2012,17 +2013,12 @@ static int launch_fwd_mma(const agpt_plan *p, const float *q, const void *k, con
 
 static int fwd_dispatch(const agpt_plan *p, const float *q, const void *k, const void *v, int kv_dtype, float *out,
                         float *lse, int H, int head_dim, float scale, cudaStream_t st, int tile0, int ntiles) {
-    // head_dim 64: the whole-tile forward (two blocks per SM) measured slower than the chunked one (17.5 vs 15.0 ms on the
-    // 4M-node microbenchmark), the whole-tile backward faster (37.7 vs 50.3 ms): the forward stays chunked there
-    if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_F32 && head_dim == 32 && bwd_tile_enabled() && tile_kernels_fit(p, head_dim))
-    {
-        // six blocks of four warps per SM (80 registers, no spills; the 33.6 KB of a depth-32 tile fit six times): 19.0 ms on
-        // the depth-32 trie against 20.1 ms with five (95 registers; AGPT_B200_FWD_BLOCKS=5).  The backward does not gain
-        // from a fifth block (96 registers with spills: 52.5 against 49.9 ms).
-        static int blocks = 0;
-        if (!blocks) { const char *e = getenv("AGPT_B200_FWD_BLOCKS"); blocks = (e && atoi(e) == 5) ? 5 : 6; }
-        if (blocks == 6) return launch_fwd_tile<32, 6, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
-        return launch_fwd_tile<32, 5, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+    if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_F32 && bwd_tile_enabled() && fwd_tile_fits(p, head_dim)) {
+        switch (head_dim) {
+            case 16: return launch_fwd_tile<16, 8, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            case 32: return launch_fwd_tile<32, 6, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            case 64: return launch_fwd_tile<64, 3, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+        }
     }
     // bfloat16 store: whole tiles while two blocks of them fit one SM (head_dim 64: up to 438 keys), deeper plans in chunks
     if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_BF16 &&
@@ -2070,7 +2066,7 @@ static int launch_bwd_tile(const agpt_plan *p, const float *q, const void *k, co
     dim3 grid((unsigned)ntiles, (unsigned)H);
     attn_bwd_tile_kernel<HD, NW, MINB, KVT><<<grid, NW * 32, smem, st>>>(q, (const KVT *)k, (const KVT *)v, o, lse, dout, dq, dk, dv, pk, pv,
                                                                          p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_chain_end,
-                                                                         p->d_tile_start, H, scale, tile0, maxk, gmask);
+                                                                         p->d_tile_start, H, scale, tile0, maxk, rows_wide(H * HD, q, k, v, o, dout), gmask);
     return launch_status("attn_bwd_tile");
 }
 
@@ -2079,6 +2075,7 @@ static int launch_bwd_tile_w(const agpt_plan *p, const float *q, const void *k, 
                              int head_dim, float scale, cudaStream_t st, int tile0, int ntiles, BwdMask gmask) {
 #define TILE_ARGS p, q, k, v, o, lse, dout, dq, dk, dv, pk, pv, H, scale, st, tile0, ntiles, gmask
     if (kv_dtype == AGPT_KV_BF16) return launch_bwd_tile<32, 4, 4, __nv_bfloat16>(TILE_ARGS);    // head_dim 32 only (bwd_dispatch)
+    if (head_dim == 16) return launch_bwd_tile<16, 4, 5>(TILE_ARGS);
     if (head_dim == 64) {        // twice the fragment and accumulator registers: two blocks per SM
         switch (g_bwd_warps) {
             case 6: case 8: return launch_bwd_tile<64, 8, 1>(TILE_ARGS);
@@ -2099,7 +2096,7 @@ static int bwd_dispatch(const agpt_plan *p, const float *q, const void *k, const
                         int head_dim, float scale, cudaStream_t st, int tile0, int ntiles, BwdMask gmask = BwdMask{AGPT_GRAD_FULL, nullptr}) {
     if (attn_impl() == 1 && p->tile_m == 64 && bwd_tile_enabled() &&
         (kv_dtype == AGPT_KV_F32 || (head_dim == 32 && tile_bf16_enabled()))) {
-        if (tile_kernels_fit(p, head_dim))
+        if (bwd_tile_fits(p, head_dim))
             return launch_bwd_tile_w(p, q, k, v, kv_dtype, o, lse, dout, dq, dk, dv, pk, pv, H, head_dim, scale, st, tile0, ntiles, gmask);
     }
     if (attn_impl() == 1 && p->tile_m == 64 && p->max_keys <= MAXKEYS) {
@@ -2301,11 +2298,6 @@ extern "C" int agpt_b200_kv_store_write_bf16(const float *d_src, void *d_store, 
 // --------------------------------------------------------------------------------------
 // loss: one warp per query row
 // --------------------------------------------------------------------------------------
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
