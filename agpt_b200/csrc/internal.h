@@ -5,7 +5,7 @@
 #include <mutex>
 #include <vector>
 
-#define AGPT_REDUCE_SEG 128   // tiles summed by one warp of the dK/dV reduction before a second pass
+#define AGPT_REDUCE_SEG 16    // tiles summed by one warp of the dK/dV reduction before a second pass (at most 32: one offset per lane)
 
 int agpt_set_error(int code, const char *fmt, ...);
 

@@ -999,10 +999,10 @@ template <int HD> __device__ __forceinline__ int tile_swz(int r) {
 
 // Staging geometry of one thread: it owns the eight elements c8 of rows r0, r0 + step, r0 + 2 step, ... of every plane.  step is a
 // multiple of 8, so the swizzle term and with it the two byte offsets are the same for all its rows up to a multiple of the row step.
-// A raw element passes through registers only: loaded once (32 bytes at a time where the buffers allow), its magnitude taken
-// for the scale, held across the barrier that makes the scale known, and stored as hi and lo halves.  Through shared memory (cp.async of raw
-// rows, a read for the maxima, a read and a write for the conversion, its 8-byte stores four to a bank) the staging was two thirds of all shared-memory
-// wavefronts of the forward and the shared-memory pipe 78 % busy.
+// In the backward a raw element passes through registers only: loaded once (32 bytes at a time where the buffers allow), its magnitude
+// taken for the scale, held across the barrier that makes the scale known, and stored as hi and lo halves.  (Raw rows through shared memory, in the
+// forward's way: 4 x 32, 1.4M rows 1866 against 1731 us, 8 x 64, 600k rows 3474 against 3189.  Not keeping
+// the rows in the L1 gives another 1 to 2 %: 1695, 3151.)
 template <int HD, int NT> struct TileStage {
     static constexpr int NL = HD / 8, STEP = NT / NL, ROWB = HD * 4, OSTEP = STEP * ROWB;
     static_assert(NT % NL == 0 && STEP % 8 == 0, "a thread's rows must share their swizzle term");
@@ -1023,7 +1023,7 @@ template <> struct Raw8<float> {
         for (int j = 0; j < 8; j++) v[j] = 0.f;
     }
     __device__ __forceinline__ void load(const float *p, bool wide) {      // wide: every row starts on a 32-byte boundary
-        if (wide) asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        if (wide) asm("ld.global.nc.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                       : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
         else {
             const float4 a = ld4(p), b = ld4(p + 4);
@@ -1035,7 +1035,7 @@ template <> struct Raw8<float> {
         for (int j = 0; j < 8; j++) m = fmaxf(m, fabsf(v[j]));
         return m;
     }
-    // hi and lo halves of the scaled elements into a plane
+    // hi and lo halves of the scaled elements
     __device__ __forceinline__ void put(unsigned char *hi, unsigned char *lo, float s) const {
         uint32_t h[4], l[4];
 #pragma unroll
@@ -1068,17 +1068,29 @@ template <> struct Raw8<__nv_bfloat16> {
 // passes of key rows that a thread holds in registers: 96 keys.  The rows of a longer tile are loaded once for the maxima and again
 // for the conversion.
 template <int HD, int NT> struct KeyPasses { static constexpr int value = (96 + TileStage<HD, NT>::STEP - 1) / TileStage<HD, NT>::STEP; };
-__device__ __forceinline__ float warp_max(float m) {
+// maxima of four magnitudes over the block, through a slot per warp (no atomics and no reset before them); contains a barrier
+template <int NW> __device__ __forceinline__ float4 block_max4(float4 *s_w, float a, float b, float c, float d, int tid) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    for (int o = 16; o > 0; o >>= 1) {
+        a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o)); b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
+        c = fmaxf(c, __shfl_xor_sync(0xffffffffu, c, o)); d = fmaxf(d, __shfl_xor_sync(0xffffffffu, d, o));
+    }
+    if ((tid & 31) == 0) s_w[tid >> 5] = make_float4(a, b, c, d);
+    __syncthreads();
+    float4 m = s_w[0];
+#pragma unroll
+    for (int w = 1; w < NW; w++) {
+        const float4 x = s_w[w];
+        m.x = fmaxf(m.x, x.x); m.y = fmaxf(m.y, x.y); m.z = fmaxf(m.z, x.z); m.w = fmaxf(m.w, x.w);
+    }
     return m;
 }
 
 // bytes of one key block's dS^T (16 keys x 64 queries, hi and for a float32 store lo halves) that lie outside the block's own V rows: its
 // lo part for head_dim 32, all of it for 16
-template <typename KVT> constexpr int bwd_tile_ds_extra(int hd) { return sizeof(KVT) == 2 || hd >= 64 ? 0 : hd == 32 ? 2048 : 4096; }
+template <typename KVT> __host__ __device__ constexpr int bwd_tile_ds_extra(int hd) { return sizeof(KVT) == 2 || hd >= 64 ? 0 : hd == 32 ? 2048 : 4096; }
 constexpr size_t bwd_tile_smem_bytes(int hd, int maxk, int ds_extra) {
-    return (size_t)(2 * 64 + 2 * maxk) * (size_t)(hd * 4) + (size_t)(maxk / 16) * (size_t)ds_extra + (size_t)maxk * 8 + 3 * 64 * 4 + 32 + (size_t)(maxk / 16) * 4;
+    return (size_t)(2 * 64 + 2 * maxk) * (size_t)(hd * 4) + (size_t)(maxk / 16) * (size_t)ds_extra + (size_t)maxk * 8 + 3 * 64 * 4 + 144 + (size_t)(maxk / 16) * 4;
 }
 
 template <int HD, int NW, int MINB, typename KVT>
@@ -1100,8 +1112,8 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     float *sLse = reinterpret_cast<float *>(s_meta + maxk);                          // [64]  lse * log2(e)
     float *sDelta = sLse + M;                                                        // [64]  dO . O
     int *sFirst = reinterpret_cast<int *>(sDelta + M);                               // [64]  first key id each query feeds in dK/dV
-    uint32_t *s_max = reinterpret_cast<uint32_t *>(sFirst + M);                      // [4]   max |x| of Q, K, V, dO (float bits)
-    int *s_ctr = reinterpret_cast<int *>(s_max + 4);
+    float4 *s_max = reinterpret_cast<float4 *>(sFirst + M);                          // [8] max |x| of Q, K, V, dO per warp
+    int *s_ctr = reinterpret_cast<int *>(s_max + 8);
     unsigned *s_on = reinterpret_cast<unsigned *>(s_ctr + 4);                        // [maxk / 16] query blocks for which a key block has dS^T
 
     const int t = blockIdx.x + tile0, h = blockIdx.y, tid = threadIdx.x;
@@ -1117,7 +1129,6 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     const int32_t *chain_end = chain_end_all + coff;
 
     // ---- rows to registers, delta = dO . O ----
-    if (tid < 4) s_max[tid] = 0u;
     if (tid == 0) *s_ctr = 0;
     typedef TileStage<HD, NT> Stage;
     constexpr int UQ = (M + Stage::STEP - 1) / Stage::STEP, UK = KeyPasses<HD, NT>::value;
@@ -1180,6 +1191,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
         s_meta[j] = make_int2(kid, min(kend, n));        // rows past the tile's end attend nothing
     }
     // ---- maxima of |x| per tensor ----
+    float sclQ, invQ, sclK, invK, sclV, invV, sclG, invG;
     {
         float mq = 0.f, mg = 0.f, mk = 0.f, mv = 0.f;
 #pragma unroll
@@ -1187,17 +1199,10 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
 #pragma unroll
         for (int u = 0; u < UK; u++) { mk = k8[u].abs_max(mk); mv = v8[u].abs_max(mv); }
         far_keys([&](const Raw8<KVT> &kx, const Raw8<KVT> &vx, int) { mk = kx.abs_max(mk); mv = vx.abs_max(mv); });
-        mq = warp_max(mq); mg = warp_max(mg); mk = warp_max(mk); mv = warp_max(mv);
-        __syncthreads();                     // s_max is zero
-        if (lane == 0) {                     // non-negative floats order like their bit patterns
-            atomicMax(&s_max[0], __float_as_uint(mq)); atomicMax(&s_max[1], __float_as_uint(mk));
-            atomicMax(&s_max[2], __float_as_uint(mv)); atomicMax(&s_max[3], __float_as_uint(mg));
-        }
+        const float4 m = block_max4<NW>(s_max, mq, mk, mv, mg, tid);
+        pow2_scale(__float_as_uint(m.x), 0, sclQ, invQ); pow2_scale(__float_as_uint(m.y), 0, sclK, invK);
+        pow2_scale(__float_as_uint(m.z), 0, sclV, invV); pow2_scale(__float_as_uint(m.w), -2, sclG, invG);
     }
-    __syncthreads();
-    float sclQ, invQ, sclK, invK, sclV, invV, sclG, invG;
-    pow2_scale(s_max[0], 0, sclQ, invQ); pow2_scale(s_max[1], 0, sclK, invK);
-    pow2_scale(s_max[2], 0, sclV, invV); pow2_scale(s_max[3], -2, sclG, invG);
 
     // ---- halves to shared memory ----
 #pragma unroll
@@ -1416,22 +1421,69 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
 // fragment addressing as attn_bwd_tile_kernel; one warp per 16 query rows (4 warps), online softmax over blocks of
 // 16 keys, O += P V with V read through ldmatrix.trans.
 // --------------------------------------------------------------------------------------
+// Staging: cp.async brings raw rows to shared memory 16 bytes at a time, whole rows per instruction, piece c of row r to place c ^ raw_swz(r) (the two
+// pieces of a 32-byte sector stay side by side: with a row's even pieces in one half of it and the odd ones in the other the forward took 25 % longer).
+// The ids of the first rows' keys are fetched before any copy, as the copy of a chain row waits for its id (883 against 912 us without).  The owner of eight
+// elements (TileStage) reads them for the maxima and again for the conversion, and a row's owners, lanes of one warp, replace its raw pieces by the
+// halves, 16 bytes a store.  (Eight-byte stores, four to a bank, were a third of all shared-memory wavefronts, that pipe 78 % busy.
+// Rows through registers as in the backward: the loads in flight cost registers, and with them blocks; 1002 us.)  Measured: 4 x 32, 1.4M rows
+// 901 -> 883 us; 8 x 64, 600k rows 1719 (in chunks) -> 1600 us.
+template <int HD> __device__ __forceinline__ int raw_swz(int r) { return HD == 16 ? (r >> 1) & 3 : r & 7; }
+template <int HD> struct FwdStage : TileStage<HD, 128> {
+    typedef TileStage<HD, 128> Base;
+    // head_dim 64: of two neighbouring pieces of a row the upper four of eight lanes read the second one first (bank conflicts)
+    static constexpr bool TURN = HD == 64;
+    int raw[2];                            // where the owner's raw pieces lie, in the order of reading
+    bool turned;
+    int row[2], col[2], dst[2];            // the two pieces that the thread copies per pass: row, first element, byte offset
+    __device__ __forceinline__ explicit FwdStage(int tid) : Base(tid) {
+        const int y = raw_swz<HD>(Base::r0);
+        turned = TURN && (Base::c8 & 4);
+        raw[0] = Base::r0 * Base::ROWB + (((2 * Base::c8 + (turned ? 1 : 0)) ^ y) << 4);
+        raw[1] = Base::r0 * Base::ROWB + (((2 * Base::c8 + (turned ? 0 : 1)) ^ y) << 4);
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int f = j * 32 + (tid & 31), c = f % (2 * Base::NL);
+            row[j] = (tid >> 5) * (32 / Base::NL) + f / (2 * Base::NL);
+            col[j] = c * 4;
+            dst[j] = row[j] * Base::ROWB + ((c ^ raw_swz<HD>(row[j])) << 4);
+        }
+    }
+    static __device__ __forceinline__ void copy_or_zero(unsigned char *dst, const float *src, bool copy) {
+        if (copy) cp_async16(dst, src);
+        else *reinterpret_cast<float4 *>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __device__ __forceinline__ Raw8<float> read(const unsigned char *plane) const {
+        const float4 a = *reinterpret_cast<const float4 *>(plane + raw[0]), b = *reinterpret_cast<const float4 *>(plane + raw[1]);
+        Raw8<float> x;
+        x.v[0] = a.x; x.v[1] = a.y; x.v[2] = a.z; x.v[3] = a.w; x.v[4] = b.x; x.v[5] = b.y; x.v[6] = b.z; x.v[7] = b.w;
+        return x;
+    }
+    // halves of what read() gave, once all lanes of the warp have read
+    __device__ __forceinline__ void put(unsigned char *plane, const Raw8<float> &x, float s) const {
+        uint32_t h[4], l[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) f16_split2<true>(x.v[2 * j] * s, x.v[2 * j + 1] * s, h[j], l[j]);
+        const bool t = TURN && turned;
+        *reinterpret_cast<uint4 *>(plane + Base::hi) = make_uint4(t ? h[2] : h[0], t ? h[3] : h[1], t ? h[0] : h[2], t ? h[1] : h[3]);
+        *reinterpret_cast<uint4 *>(plane + Base::lo) = make_uint4(t ? l[2] : l[0], t ? l[3] : l[1], t ? l[0] : l[2], t ? l[1] : l[3]);
+    }
+};
 constexpr size_t fwd_tile_smem_bytes(int hd, int maxk) {
-    return (size_t)(64 + 2 * maxk) * (size_t)(hd * 4) + (size_t)maxk * 8 + 32;
+    return (size_t)(64 + 2 * maxk) * (size_t)(hd * 4) + (size_t)maxk * 8 + 64;
 }
 
-template <int HD, int MINB, typename KVT>
+template <int HD, int MINB>
 __global__ void __launch_bounds__(128, MINB)
-attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, const KVT *__restrict__ V,
+attn_fwd_tile_kernel(const float *__restrict__ Q, const float *__restrict__ K, const float *__restrict__ V,
                      float *__restrict__ O, float *__restrict__ LSE, const int32_t *__restrict__ sub_end,
                      const int64_t *__restrict__ chain_off, const int32_t *__restrict__ chain_ids,
-                     const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H, float scale, int tile0, int maxk, bool wide) {
+                     const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H, float scale, int tile0, int maxk) {
     constexpr int M = 64, NT = 128, TILE_ROW_BYTES = HD * 4, KS = HD / 16, NDB = HD / 8;
-    constexpr bool LP = sizeof(KVT) == 2;              // bfloat16 store: single fp16 products, no lo parts
     extern __shared__ __align__(128) unsigned char tile_smem_raw[];
     unsigned char *sQ = tile_smem_raw, *sK = sQ + M * TILE_ROW_BYTES, *sV = sK + (size_t)maxk * TILE_ROW_BYTES;
     int2 *s_meta = reinterpret_cast<int2 *>(sV + (size_t)maxk * TILE_ROW_BYTES);   // [maxk] {key id, key subtree end}
-    uint32_t *s_max = reinterpret_cast<uint32_t *>(s_meta + maxk);                  // [3] max |x| of Q, K, V (float bits)
+    float4 *s_max = reinterpret_cast<float4 *>(s_meta + maxk);                      // [4] max |x| of Q, K, V per warp
 
     const int t = blockIdx.x + tile0, h = blockIdx.y, tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
@@ -1445,78 +1497,66 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     const int32_t *chain = chain_ids + coff;
     const int32_t *chain_end = chain_end_all + coff;
 
-    // ---- rows to registers ----
-    if (tid < 3) s_max[tid] = 0u;
-    typedef TileStage<HD, NT> Stage;
-    constexpr int UQ = M / Stage::STEP, UK = KeyPasses<HD, NT>::value;
-    const Stage T(tid);
-    Raw8<float> q8[UQ];
+    // ---- raw rows ----
+    const FwdStage<HD> T(tid);
+    constexpr int UQ = M / T.STEP;
+    auto key_id = [&](int r) { return r < p ? __ldg(chain + r) : i0 + (r - p); };
+    const int kid0[2] = {key_id(T.row[0]), key_id(T.row[1])};
 #pragma unroll
-    for (int u = 0; u < UQ; u++) {
-        const int r = T.r0 + u * T.STEP;
-        q8[u].zero();
-        if (r < nt) q8[u].load(Q + (int64_t)(i0 + r) * D + hoff + T.c8 * 8, wide);
-    }
-    Raw8<KVT> k8[UK], v8[UK];
+    for (int u = 0; u < UQ; u++)
 #pragma unroll
-    for (int u = 0; u < UK; u++) {
-        const int r = T.r0 + u * T.STEP;
-        k8[u].zero(); v8[u].zero();
-        if (r < nkeys) {
-            const int kid = r < p ? __ldg(chain + r) : i0 + (r - p);
-            const int64_t off = (int64_t)kid * D + hoff + T.c8 * 8;
-            k8[u].load(K + off, wide); v8[u].load(V + off, wide);
+        for (int j = 0; j < 2; j++) {
+            const int r = T.row[j] + u * T.STEP;
+            T.copy_or_zero(sQ + T.dst[j] + u * T.OSTEP, Q + (int64_t)(i0 + r) * D + hoff + T.col[j], r < nt);
         }
-    }
-    // key rows beyond the passes held in registers
-    auto far_keys = [&](auto &&f) {
-        for (int r = T.r0 + UK * T.STEP; r < nkp; r += T.STEP) {
-            Raw8<KVT> kx, vx;
-            kx.zero(); vx.zero();
-            if (r < nkeys) {
-                const int kid = r < p ? __ldg(chain + r) : i0 + (r - p);
-                const int64_t off = (int64_t)kid * D + hoff + T.c8 * 8;
-                kx.load(K + off, wide); vx.load(V + off, wide);
-            }
-            f(kx, vx, (r - T.r0) * T.ROWB);
-        }
+    auto copy_keys = [&](int u, int j, int key) {
+        const int r = T.row[j] + u * T.STEP, o = T.dst[j] + u * T.OSTEP;
+        if (r >= nkp) return;
+        const int64_t off = (int64_t)key * D + hoff + T.col[j];
+        T.copy_or_zero(sK + o, K + off, r < nkeys);
+        T.copy_or_zero(sV + o, V + off, r < nkeys);
     };
+#pragma unroll
+    for (int j = 0; j < 2; j++) copy_keys(0, j, kid0[j]);
+    for (int u = 1; u * T.STEP < nkp; u++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) copy_keys(u, j, key_id(min(T.row[j] + u * T.STEP, nkeys - 1)));
+    cp_async_commit();
     for (int j = tid; j < nkp; j += NT) {
         int kid = 0x7fffffff, kend = 0;
         if (j < p) { kid = __ldg(chain + j); kend = __ldg(chain_end + j); }
         else if (j < nkeys) { kid = i0 + (j - p); kend = __ldg(sub_end + kid); }
         s_meta[j] = make_int2(kid, min(kend, n));        // rows past the tile's end attend nothing
     }
+    cp_async_wait_all();
+    __syncwarp();                        // the warp's rows have landed
+
     // ---- maxima of |x| per tensor ----
+    float sclQ, invQ, sclK, invK, sclV, invV;
     {
         float mq = 0.f, mk = 0.f, mv = 0.f;
 #pragma unroll
-        for (int u = 0; u < UQ; u++) mq = q8[u].abs_max(mq);
-#pragma unroll
-        for (int u = 0; u < UK; u++) { mk = k8[u].abs_max(mk); mv = v8[u].abs_max(mv); }
-        far_keys([&](const Raw8<KVT> &kx, const Raw8<KVT> &vx, int) { mk = kx.abs_max(mk); mv = vx.abs_max(mv); });
-        mq = warp_max(mq); mk = warp_max(mk); mv = warp_max(mv);
-        __syncthreads();                     // s_max is zero
-        if (lane == 0) {
-            atomicMax(&s_max[0], __float_as_uint(mq)); atomicMax(&s_max[1], __float_as_uint(mk)); atomicMax(&s_max[2], __float_as_uint(mv));
+        for (int u = 0; u < UQ; u++) mq = T.read(sQ + u * T.OSTEP).abs_max(mq);
+        for (int r = T.r0, o = 0; r < nkp; r += T.STEP, o += T.OSTEP) {
+            mk = T.read(sK + o).abs_max(mk);
+            mv = T.read(sV + o).abs_max(mv);
         }
+        const float4 m = block_max4<4>(s_max, mq, mk, mv, 0.f, tid);
+        pow2_scale(__float_as_uint(m.x), 0, sclQ, invQ); pow2_scale(__float_as_uint(m.y), 0, sclK, invK); pow2_scale(__float_as_uint(m.z), 0, sclV, invV);
     }
-    __syncthreads();
-    float sclQ, invQ, sclK, invK, sclV, invV;
-    pow2_scale(s_max[0], 0, sclQ, invQ); pow2_scale(s_max[1], 0, sclK, invK); pow2_scale(s_max[2], 0, sclV, invV);
 
-    // ---- halves to shared memory ----
+    // ---- halves, in place (whole warps enter or skip an iteration: a warp owns 4, 8 or 16 consecutive rows and nkp is a multiple of 16) ----
 #pragma unroll
-    for (int u = 0; u < UQ; u++) q8[u].put(sQ + T.hi + u * T.OSTEP, sQ + T.lo + u * T.OSTEP, sclQ);
-#pragma unroll
-    for (int u = 0; u < UK; u++)
-        if (T.r0 + u * T.STEP < nkp) {
-            k8[u].put(sK + T.hi + u * T.OSTEP, sK + T.lo + u * T.OSTEP, sclK);
-            v8[u].put(sV + T.hi + u * T.OSTEP, sV + T.lo + u * T.OSTEP, sclV);
-        }
-    far_keys([&](const Raw8<KVT> &kx, const Raw8<KVT> &vx, int o) {
-        kx.put(sK + T.hi + o, sK + T.lo + o, sclK); vx.put(sV + T.hi + o, sV + T.lo + o, sclV);
-    });
+    for (int u = 0; u < UQ; u++) {
+        const Raw8<float> x = T.read(sQ + u * T.OSTEP);
+        __syncwarp();
+        T.put(sQ + u * T.OSTEP, x, sclQ);
+    }
+    for (int r = T.r0, o = 0; r < nkp; r += T.STEP, o += T.OSTEP) {
+        const Raw8<float> x = T.read(sK + o), y = T.read(sV + o);
+        __syncwarp();
+        T.put(sK + o, x, sclK); T.put(sV + o, y, sclV);
+    }
     __syncthreads();
 
     const int rg = warp;
@@ -1536,7 +1576,7 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     for (int ks = 0; ks < KS; ks++) {
         const uint32_t o = (uint32_t)(rg * 16 * TILE_ROW_BYTES) + aRow;
         ldmatrix_x4(qh[ks], uQ + o + (uint32_t)(((2 * ks + aC) ^ sw) << 4));
-        if constexpr (!LP) ldmatrix_x4(ql[ks], uQ + o + (uint32_t)(((2 * ks + aC + NDB) ^ sw) << 4));
+        ldmatrix_x4(ql[ks], uQ + o + (uint32_t)(((2 * ks + aC + NDB) ^ sw) << 4));
     }
     float o_[NDB][4];
 #pragma unroll
@@ -1566,7 +1606,7 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                 uint32_t kf[4];
                 ldmatrix_x4(kf, uK + rowb + (uint32_t)(((2 * ks + bC) ^ sw) << 4));
                 mma_f16(c, qh[ks], kf[0], kf[1]);
-                if constexpr (!LP) { mma_f16(cx, ql[ks], kf[0], kf[1]); mma_f16(cx, qh[ks], kf[2], kf[3]); }
+                { mma_f16(cx, ql[ks], kf[0], kf[1]); mma_f16(cx, qh[ks], kf[2], kf[3]); }
             }
 #pragma unroll
             for (int j = 0; j < 4; j++)
@@ -1607,7 +1647,7 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
             uint32_t vt[4];                            // {b0 hi, b1 hi, b0 lo, b1 lo}: keys 0-7 / 8-15 of the block, dims 8 db..
             ldmatrix_x4_trans(vt, rowt + (uint32_t)(((db + tC) ^ sw) << 4));
             mma_f16(o_[db], ph, vt[0], vt[1]);
-            if constexpr (!LP) { mma_f16(o_[db], pl, vt[0], vt[1]); mma_f16(o_[db], ps, vt[2], vt[3]); }
+            { mma_f16(o_[db], pl, vt[0], vt[1]); mma_f16(o_[db], ps, vt[2], vt[3]); }
         }
     }
     l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
@@ -1795,66 +1835,96 @@ attn_fwd_bf16_kernel(const float *__restrict__ Q, const __nv_bfloat16 *__restric
     }
 }
 
-// dK/dV reduction, pass 1: one warp per work item = (node, tile range).  The node's row in tile t's
-// partial block is chain_off[t] + depth - 1.  Tiles are summed in increasing order.
-__global__ void reduce_items_kernel(const float *__restrict__ Pk, const float *__restrict__ Pv, float *__restrict__ dK,
-                                    float *__restrict__ dV, float *__restrict__ segk, float *__restrict__ segv,
-                                    const int64_t *__restrict__ chain_off, const int32_t *__restrict__ depth,
-                                    const int32_t *__restrict__ item_node, const int32_t *__restrict__ item_t0,
-                                    const int32_t *__restrict__ item_t1, const int32_t *__restrict__ item_slot,
-                                    int64_t item0, int64_t n_items, int D) {
-    int64_t it = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+// dK/dV reduction, pass 1: one warp per work item = (node, up to AGPT_REDUCE_SEG tiles) and 128 columns.  The node's row in tile
+// t's partial block is chain_off[t] + depth - 1.  Tiles are summed in increasing order.
+// Most items are one or two tiles, three dependent accesses (item, offset, partial row) and the sum onto dK/dV; a few near the roots
+// span thousands.  So an item is 16 tiles at most, its offsets are fetched by as many lanes at once, the rows it adds to are on their way before
+// the partial rows', and rows of up to 64 columns take the lower half of a warp for K and the upper for V.  Bound by memory on deep tries
+// and by latency on small ones.  Measured, with pass 2 (against items of 128 tiles, a column loop and a chain of loads per warp): REDFIG.
+template <bool HALF>
+__global__ void __launch_bounds__(256)
+reduce_items_kernel(const float *__restrict__ Pk, const float *__restrict__ Pv, float *__restrict__ dK, float *__restrict__ dV,
+                    float *__restrict__ segk, float *__restrict__ segv, const int64_t *__restrict__ chain_off, const int32_t *__restrict__ depth,
+                    const int32_t *__restrict__ item_node, const int32_t *__restrict__ item_t0, const int32_t *__restrict__ item_t1,
+                    const int32_t *__restrict__ item_slot, int64_t item0, int64_t n_items, int D) {
+    int64_t it = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (it >= n_items) return;
     it += item0;
+    constexpr int NV = HALF ? 1 : 2;
     const int lane = threadIdx.x & 31;
-    const int a = item_node[it], t0 = item_t0[it], t1 = item_t1[it], slot = item_slot[it];
-    const int row = depth[a] - 1;
-    for (int c = lane * 4; c < D; c += 128) {
-        float4 sk = make_float4(0.f, 0.f, 0.f, 0.f), sv = sk;
-#pragma unroll 4
-        for (int t = t0; t <= t1; t++) {
-            int64_t r = (chain_off[t] + row) * D + c;
-            float4 a4 = __ldcs(reinterpret_cast<const float4 *>(Pk + r));
-            float4 b4 = __ldcs(reinterpret_cast<const float4 *>(Pv + r));
-            sk.x += a4.x; sk.y += a4.y; sk.z += a4.z; sk.w += a4.w;
-            sv.x += b4.x; sv.y += b4.y; sv.z += b4.z; sv.w += b4.w;
-        }
-        if (slot < 0) {
-            float4 *pk = reinterpret_cast<float4 *>(dK + (int64_t)a * D + c), *pv = reinterpret_cast<float4 *>(dV + (int64_t)a * D + c);
-            float4 x = *pk, y = *pv;
-            *pk = make_float4(x.x + sk.x, x.y + sk.y, x.z + sk.z, x.w + sk.w);
-            *pv = make_float4(y.x + sv.x, y.y + sv.y, y.z + sv.z, y.w + sv.w);
-        } else {
-            *reinterpret_cast<float4 *>(segk + (int64_t)slot * D + c) = sk;
-            *reinterpret_cast<float4 *>(segv + (int64_t)slot * D + c) = sv;
-        }
+    const int a = __ldg(item_node + it), t0 = __ldg(item_t0 + it), cnt = __ldg(item_t1 + it) - t0 + 1, slot = __ldg(item_slot + it);
+    const int64_t off = lane < cnt ? __ldg(chain_off + t0 + lane) : 0;
+    const int row = __ldg(depth + a) - 1;
+    const int c = HALF ? (lane & 15) * 4 : blockIdx.y * 128 + lane * 4;
+    const bool in = c < D, upper = HALF && lane >= 16;
+    const float *src[NV] = {upper ? Pv : Pk};
+    float *dst[NV] = {slot < 0 ? (upper ? dV : dK) : (upper ? segv : segk)};
+    if constexpr (!HALF) { src[1] = Pv; dst[1] = slot < 0 ? dV : segv; }
+    const int64_t at = (int64_t)(slot < 0 ? a : slot) * D + c;
+    float4 old[NV], sum[NV];
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        old[i] = sum[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (in && slot < 0) old[i] = *reinterpret_cast<const float4 *>(dst[i] + at);
     }
+    auto load = [&](float4 (&x)[NV], int j) {
+        const int64_t r = (__shfl_sync(0xffffffffu, off, j) + row) * D + c;
+#pragma unroll
+        for (int i = 0; i < NV; i++) x[i] = in ? __ldcs(reinterpret_cast<const float4 *>(src[i] + r)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto add = [&](const float4 (&x)[NV]) {
+#pragma unroll
+        for (int i = 0; i < NV; i++) { sum[i].x += x[i].x; sum[i].y += x[i].y; sum[i].z += x[i].z; sum[i].w += x[i].w; }
+    };
+    int j = 0;
+    for (; j + 4 <= cnt; j += 4) {
+        float4 x[4][NV];
+#pragma unroll
+        for (int u = 0; u < 4; u++) load(x[u], j + u);
+#pragma unroll
+        for (int u = 0; u < 4; u++) add(x[u]);
+    }
+    for (; j < cnt; j++) {
+        float4 x[NV];
+        load(x, j);
+        add(x);
+    }
+    if (!in) return;
+#pragma unroll
+    for (int i = 0; i < NV; i++)
+        *reinterpret_cast<float4 *>(dst[i] + at) = make_float4(old[i].x + sum[i].x, old[i].y + sum[i].y, old[i].z + sum[i].z, old[i].w + sum[i].w);
 }
 
-// pass 2: nodes whose range was cut into several items; their segment sums are added in item order.
-__global__ void reduce_multi_kernel(const float *__restrict__ segk, const float *__restrict__ segv, float *__restrict__ dK,
-                                    float *__restrict__ dV, const int32_t *__restrict__ multi_node,
-                                    const int32_t *__restrict__ multi_count, const int64_t *__restrict__ multi_first,
-                                    const int32_t *__restrict__ item_slot, int64_t n_multi, int D) {
-    int64_t mi = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (mi >= n_multi) return;
-    const int lane = threadIdx.x & 31;
-    const int a = multi_node[mi], cnt = multi_count[mi];
-    const int slot0 = (int)multi_first[mi];           // slots of one node are consecutive
-    (void)item_slot;
-    for (int c = lane * 4; c < D; c += 128) {
-        float4 sk = make_float4(0.f, 0.f, 0.f, 0.f), sv = sk;
-        for (int s = 0; s < cnt; s++) {
-            float4 a4 = *reinterpret_cast<const float4 *>(segk + (int64_t)(slot0 + s) * D + c);
-            float4 b4 = *reinterpret_cast<const float4 *>(segv + (int64_t)(slot0 + s) * D + c);
+// pass 2: nodes whose range was cut into several items; their segment sums are added by the eight warps of a block, a range
+// each, and the warps' sums in warp order.
+__global__ void __launch_bounds__(256)
+reduce_multi_kernel(const float *__restrict__ segk, const float *__restrict__ segv, float *__restrict__ dK, float *__restrict__ dV,
+                    const int32_t *__restrict__ multi_node, const int32_t *__restrict__ multi_count, const int64_t *__restrict__ multi_first, int D) {
+    __shared__ float4 s_k[8][32], s_v[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.y * 128 + lane * 4;
+    const int a = multi_node[blockIdx.x], cnt = multi_count[blockIdx.x];
+    const int64_t slot0 = multi_first[blockIdx.x];             // slots of one node are consecutive
+    float4 sk = make_float4(0.f, 0.f, 0.f, 0.f), sv = sk;
+    if (c < D) {
+#pragma unroll 4
+        for (int s = (int)((int64_t)cnt * w / 8); s < (int)((int64_t)cnt * (w + 1) / 8); s++) {
+            const float4 a4 = *reinterpret_cast<const float4 *>(segk + (slot0 + s) * D + c);
+            const float4 b4 = *reinterpret_cast<const float4 *>(segv + (slot0 + s) * D + c);
             sk.x += a4.x; sk.y += a4.y; sk.z += a4.z; sk.w += a4.w;
             sv.x += b4.x; sv.y += b4.y; sv.z += b4.z; sv.w += b4.w;
         }
-        float4 *pk = reinterpret_cast<float4 *>(dK + (int64_t)a * D + c), *pv = reinterpret_cast<float4 *>(dV + (int64_t)a * D + c);
-        float4 x = *pk, y = *pv;
-        *pk = make_float4(x.x + sk.x, x.y + sk.y, x.z + sk.z, x.w + sk.w);
-        *pv = make_float4(y.x + sv.x, y.y + sv.y, y.z + sv.z, y.w + sv.w);
     }
+    s_k[w][lane] = sk; s_v[w][lane] = sv;
+    __syncthreads();
+    if (w > 1 || c >= D) return;
+    float4 *o = reinterpret_cast<float4 *>((w ? dV : dK) + (int64_t)a * D + c);
+    float4 x = *o;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const float4 y = w ? s_v[k][lane] : s_k[k][lane];
+        x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+    }
+    *o = x;
 }
 
 // --------------------------------------------------------------------------------------
@@ -1972,17 +2042,17 @@ static int tile_bf16_enabled() {
     return on;
 }
 
-template <int HD, int MINB, typename KVT>
+template <int HD, int MINB>
 static int launch_fwd_tile(const agpt_plan *p, const float *q, const void *k, const void *v, float *out, float *lse, int H,
                            float scale, cudaStream_t st, int tile0, int ntiles) {
     static size_t granted[AGPT_MAX_DEVICES];
     const int maxk = bwd_tile_maxk(p);
     const size_t smem = fwd_tile_smem_bytes(HD, maxk);
-    int rc = allow_dynamic_smem(attn_fwd_tile_kernel<HD, MINB, KVT>, smem, granted);
+    int rc = allow_dynamic_smem(attn_fwd_tile_kernel<HD, MINB>, smem, granted);
     if (rc) return rc;
     dim3 grid((unsigned)ntiles, (unsigned)H);
-    attn_fwd_tile_kernel<HD, MINB, KVT><<<grid, 128, smem, st>>>(q, (const KVT *)k, (const KVT *)v, out, lse, p->d_sub_end,
-                                                                 p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H, scale, tile0, maxk, rows_wide(H * HD, q, k, v, q, q));
+    attn_fwd_tile_kernel<HD, MINB><<<grid, 128, smem, st>>>(q, (const float *)k, (const float *)v, out, lse, p->d_sub_end,
+                                                                 p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H, scale, tile0, maxk);
     return launch_status("attn_fwd_tile");
 }
 
@@ -2015,9 +2085,9 @@ static int fwd_dispatch(const agpt_plan *p, const float *q, const void *k, const
                         float *lse, int H, int head_dim, float scale, cudaStream_t st, int tile0, int ntiles) {
     if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_F32 && bwd_tile_enabled() && fwd_tile_fits(p, head_dim)) {
         switch (head_dim) {
-            case 16: return launch_fwd_tile<16, 8, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
-            case 32: return launch_fwd_tile<32, 6, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
-            case 64: return launch_fwd_tile<64, 3, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            case 16: return launch_fwd_tile<16, 8>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            case 32: return launch_fwd_tile<32, 6>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            case 64: return launch_fwd_tile<64, 3>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
         }
     }
     // bfloat16 store: whole tiles while two blocks of them fit one SM (head_dim 64: up to 438 keys), deeper plans in chunks
@@ -2075,7 +2145,7 @@ static int launch_bwd_tile_w(const agpt_plan *p, const float *q, const void *k, 
                              int head_dim, float scale, cudaStream_t st, int tile0, int ntiles, BwdMask gmask) {
 #define TILE_ARGS p, q, k, v, o, lse, dout, dq, dk, dv, pk, pv, H, scale, st, tile0, ntiles, gmask
     if (kv_dtype == AGPT_KV_BF16) return launch_bwd_tile<32, 4, 4, __nv_bfloat16>(TILE_ARGS);    // head_dim 32 only (bwd_dispatch)
-    if (head_dim == 16) return launch_bwd_tile<16, 4, 5>(TILE_ARGS);
+    if (head_dim == 16) return launch_bwd_tile<16, 4, 4>(TILE_ARGS);
     if (head_dim == 64) {        // twice the fragment and accumulator registers: two blocks per SM
         switch (g_bwd_warps) {
             case 6: case 8: return launch_bwd_tile<64, 8, 1>(TILE_ARGS);
@@ -2126,18 +2196,18 @@ static int run_reduce_range(const agpt_plan *p, float *pk, float *pv, float *seg
                             cudaStream_t st, int64_t item0, int64_t item1, bool multi_pass) {
     const int64_t n_items = item1 - item0;
     if (n_items > 0) {
-        const int wpb = 8;
-        reduce_items_kernel<<<(unsigned)((n_items + wpb - 1) / wpb), wpb * 32, 0, st>>>(
-            pk, pv, dk, dv, segk, segv, p->d_chain_off, p->d_depth, p->d_item_node, p->d_item_t0, p->d_item_t1,
-            p->d_item_slot, item0, n_items, D);
+        const dim3 grid((unsigned)((n_items + 7) / 8), (unsigned)((D + 127) / 128));
+#define REDUCE_ARGS pk, pv, dk, dv, segk, segv, p->d_chain_off, p->d_depth, p->d_item_node, p->d_item_t0, p->d_item_t1, p->d_item_slot, item0, n_items, D
+        if (D <= 64) reduce_items_kernel<true><<<grid, 256, 0, st>>>(REDUCE_ARGS);
+        else reduce_items_kernel<false><<<grid, 256, 0, st>>>(REDUCE_ARGS);
+#undef REDUCE_ARGS
         int rc = launch_status("reduce_items");
         if (rc) return rc;
     }
     int64_t n_multi = (int64_t)p->multi_node.size();
     if (multi_pass && n_multi > 0) {
-        const int wpb = 4;
-        reduce_multi_kernel<<<(unsigned)((n_multi + wpb - 1) / wpb), wpb * 32, 0, st>>>(
-            segk, segv, dk, dv, p->d_multi_node, p->d_multi_count, p->d_multi_first, p->d_item_slot, n_multi, D);
+        reduce_multi_kernel<<<dim3((unsigned)n_multi, (unsigned)((D + 127) / 128)), 256, 0, st>>>(segk, segv, dk, dv, p->d_multi_node, p->d_multi_count,
+                                                                                                 p->d_multi_first, D);
         int rc = launch_status("reduce_multi");
         if (rc) return rc;
     }
@@ -2298,6 +2368,11 @@ extern "C" int agpt_b200_kv_store_write_bf16(const float *d_src, void *d_store, 
 // --------------------------------------------------------------------------------------
 // loss: one warp per query row
 // --------------------------------------------------------------------------------------
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
