@@ -1840,22 +1840,24 @@ attn_fwd_bf16_kernel(const float *__restrict__ Q, const __nv_bfloat16 *__restric
 // Most items are one or two tiles, three dependent accesses (item, offset, partial row) and the sum onto dK/dV; a few near the roots
 // span thousands.  So an item is 16 tiles at most, its offsets are fetched by as many lanes at once, the rows it adds to are on their way before
 // the partial rows', and rows of up to 64 columns take the lower half of a warp for K and the upper for V.  Bound by memory on deep tries
-// and by latency on small ones.  Measured, with pass 2 (against items of 128 tiles, a column loop and a chain of loads per warp): REDFIG.
+// and by latency on small ones.  Measured, with pass 2 (against items of 128 tiles, a column loop and a chain of loads per warp):
+// 66k rows of 64 55 -> 11 us, 1.4M rows of 128 91 -> 49 us, 600k rows of 512 325 -> 174 us, 719k rows of 384, depth up to 128, 848 -> 799 us.  (Six blocks per SM and
+// two rows in flight per warp; three blocks and four rows took 976 us on the last of these.)
 template <bool HALF>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, HALF ? 5 : 6)
 reduce_items_kernel(const float *__restrict__ Pk, const float *__restrict__ Pv, float *__restrict__ dK, float *__restrict__ dV,
                     float *__restrict__ segk, float *__restrict__ segv, const int64_t *__restrict__ chain_off, const int32_t *__restrict__ depth,
                     const int32_t *__restrict__ item_node, const int32_t *__restrict__ item_t0, const int32_t *__restrict__ item_t1,
-                    const int32_t *__restrict__ item_slot, int64_t item0, int64_t n_items, int D) {
-    int64_t it = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+                    const int32_t *__restrict__ item_slot, int64_t item0, int64_t n_items, int D, int chunks) {
+    int64_t it = (int64_t)(blockIdx.x / chunks) * 8 + (threadIdx.x >> 5);
     if (it >= n_items) return;
     it += item0;
-    constexpr int NV = HALF ? 1 : 2;
+    constexpr int NV = HALF ? 1 : 2, U = HALF ? 4 : 2;
     const int lane = threadIdx.x & 31;
     const int a = __ldg(item_node + it), t0 = __ldg(item_t0 + it), cnt = __ldg(item_t1 + it) - t0 + 1, slot = __ldg(item_slot + it);
     const int64_t off = lane < cnt ? __ldg(chain_off + t0 + lane) : 0;
     const int row = __ldg(depth + a) - 1;
-    const int c = HALF ? (lane & 15) * 4 : blockIdx.y * 128 + lane * 4;
+    const int c = HALF ? (lane & 15) * 4 : (blockIdx.x % chunks) * 128 + lane * 4;
     const bool in = c < D, upper = HALF && lane >= 16;
     const float *src[NV] = {upper ? Pv : Pk};
     float *dst[NV] = {slot < 0 ? (upper ? dV : dK) : (upper ? segv : segk)};
@@ -1877,12 +1879,12 @@ reduce_items_kernel(const float *__restrict__ Pk, const float *__restrict__ Pv, 
         for (int i = 0; i < NV; i++) { sum[i].x += x[i].x; sum[i].y += x[i].y; sum[i].z += x[i].z; sum[i].w += x[i].w; }
     };
     int j = 0;
-    for (; j + 4 <= cnt; j += 4) {
-        float4 x[4][NV];
+    for (; j + U <= cnt; j += U) {
+        float4 x[U][NV];
 #pragma unroll
-        for (int u = 0; u < 4; u++) load(x[u], j + u);
+        for (int u = 0; u < U; u++) load(x[u], j + u);
 #pragma unroll
-        for (int u = 0; u < 4; u++) add(x[u]);
+        for (int u = 0; u < U; u++) add(x[u]);
     }
     for (; j < cnt; j++) {
         float4 x[NV];
@@ -2196,8 +2198,9 @@ static int run_reduce_range(const agpt_plan *p, float *pk, float *pv, float *seg
                             cudaStream_t st, int64_t item0, int64_t item1, bool multi_pass) {
     const int64_t n_items = item1 - item0;
     if (n_items > 0) {
-        const dim3 grid((unsigned)((n_items + 7) / 8), (unsigned)((D + 127) / 128));
-#define REDUCE_ARGS pk, pv, dk, dv, segk, segv, p->d_chain_off, p->d_depth, p->d_item_node, p->d_item_t0, p->d_item_t1, p->d_item_slot, item0, n_items, D
+        const int chunks = (D + 127) / 128;
+        const unsigned grid = (unsigned)((n_items + 7) / 8 * chunks);
+#define REDUCE_ARGS pk, pv, dk, dv, segk, segv, p->d_chain_off, p->d_depth, p->d_item_node, p->d_item_t0, p->d_item_t1, p->d_item_slot, item0, n_items, D, chunks
         if (D <= 64) reduce_items_kernel<true><<<grid, 256, 0, st>>>(REDUCE_ARGS);
         else reduce_items_kernel<false><<<grid, 256, 0, st>>>(REDUCE_ARGS);
 #undef REDUCE_ARGS
