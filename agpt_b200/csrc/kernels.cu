@@ -901,7 +901,7 @@ __global__ void __launch_bounds__(128, HD <= 32 ? 4 : (sizeof(KVT) == 2 ? 3 : 1)
 }
 
 // --------------------------------------------------------------------------------------
-// backward, whole tile resident: attn_bwd_tile_kernel (head_dim 32 or 64, float32 store).
+// backward, whole tile resident: attn_bwd_tile_kernel.
 //
 // Operands.  The tile's Q and dO rows and every key row the tile can attend (ancestor chain + the tile's own
 // rows) are brought into shared memory ONCE (cp.async, raw float32) and converted in place to split half
@@ -919,7 +919,8 @@ __global__ void __launch_bounds__(128, HD <= 32 ? 4 : (sizeof(KVT) == 2 ? 3 : 1)
 // leaves dS^T, as the halves that its own products take, in shared memory: the V rows of the block, which only this item reads, hold
 // it.  After one barrier each warp takes 16 queries and sums dQ = dS K from those blocks.  Bound by issue slots: scores are computed
 // once, where computing them again with the queries as rows took 84 products per 16 x 16 block of head_dim 32 instead of 60 and the
-// exponentials twice.  Measured: 4 x 32, 1.4M rows 2134 -> 1916 us; 8 x 64, 600k rows 4090 -> 3708 us.
+// exponentials twice.  A bfloat16 store's K and V are exact halves: four fifths of the products, and twice the keys in the same memory.  Measured: 4 x 32, 1.4M rows 2134 -> 1916 us; 8 x 64, 600k rows 4090 -> 3708 us;
+// bfloat16 store (with its reduction, against the chunked kernel or, for 32, single fp16 products): 578k rows of depth 32, 4 x 16 699 -> 528 us, 4 x 32 906 -> 675, 4 x 64 1644 -> 1378.
 // Each output element is produced by exactly one warp in a fixed order, so results do not depend on which warp
 // took which item.
 // --------------------------------------------------------------------------------------
@@ -989,12 +990,12 @@ __device__ __forceinline__ void pow2_scale(uint32_t max_bits, int lift, float &s
     inv = __uint_as_float((uint32_t)(e - lift) << 23);
 }
 
-// A staged row holds head_dim hi halves followed by head_dim lo halves: 4 * head_dim bytes, head_dim / 4 chunks of 16 bytes, the
-// chunk index XOR-ed with tile_swz(row).  The swizzle is a bijection of row % 8 onto the chunks that share banks, so that the same chunk of eight
-// rows (one ldmatrix) falls into eight bank groups; and its bits are ordered so that the hi chunks of as many rows as eight lanes hold
-// do too (the stores of the conversion).
-template <int HD> __device__ __forceinline__ int tile_swz(int r) {
-    return HD == 16 ? (r & 2) | ((r >> 2) & 1) : ((r & 1) << 2) | ((r >> 1) & 3);
+// A staged row holds head_dim hi halves followed by head_dim lo halves, 4 * head_dim bytes, or (K and V of a bfloat16 store, whose 8
+// significant bits a hi half holds) the hi halves alone; its 16-byte chunks are XOR-ed with row_swz(row).  The swizzle is a bijection of row % 8 onto
+// the chunks that share banks, so that the same chunk of eight rows (one ldmatrix) falls into eight bank groups; and its bits are ordered so
+// that the hi chunks of as many rows as eight lanes hold do too (the stores of the conversion).
+template <int ROWB> __device__ __forceinline__ int row_swz(int r) {
+    return ROWB == 32 ? (r >> 2) & 1 : ROWB == 64 ? (r & 2) | ((r >> 2) & 1) : ((r & 1) << 2) | ((r >> 1) & 3);
 }
 
 // Staging geometry of one thread: it owns the eight elements c8 of rows r0, r0 + step, r0 + 2 step, ... of every plane.  step is a
@@ -1003,13 +1004,13 @@ template <int HD> __device__ __forceinline__ int tile_swz(int r) {
 // taken for the scale, held across the barrier that makes the scale known, and stored as hi and lo halves.  (Raw rows through shared memory, in the
 // forward's way: 4 x 32, 1.4M rows 1866 against 1731 us, 8 x 64, 600k rows 3474 against 3189.  Not keeping
 // the rows in the L1 gives another 1 to 2 %: 1695, 3151.)
-template <int HD, int NT> struct TileStage {
-    static constexpr int NL = HD / 8, STEP = NT / NL, ROWB = HD * 4, OSTEP = STEP * ROWB;
+template <int HD, int NT, int ROW = HD * 4> struct TileStage {
+    static constexpr int NL = HD / 8, STEP = NT / NL, ROWB = ROW, OSTEP = STEP * ROWB;
     static_assert(NT % NL == 0 && STEP % 8 == 0, "a thread's rows must share their swizzle term");
-    int r0, c8, hi, lo;
+    int r0, c8, hi, lo;                    // lo: rows with lo parts only
     __device__ __forceinline__ explicit TileStage(int tid) {
         r0 = tid / NL; c8 = tid % NL;
-        const int x = tile_swz<HD>(r0), row = r0 * ROWB;
+        const int x = row_swz<ROWB>(r0), row = r0 * ROWB;
         hi = row + ((c8 ^ x) << 4);
         lo = row + (((NL + c8) ^ x) << 4);
     }
@@ -1044,14 +1045,12 @@ template <> struct Raw8<float> {
         *reinterpret_cast<uint4 *>(lo) = make_uint4(l[0], l[1], l[2], l[3]);
     }
 };
-// bfloat16 store: 8 significant bits, so an element's scaled fp16 image is exact and there is no lo part.  With such a store every
-// product is a single fp16 product (Q, dO, P and dS are rounded to their 11-bit hi halves): about 1e-3 relative, below the store's own rounding (2^-9).
+// bfloat16 store: an element's scaled fp16 image is exact, there is no lo part
 template <> struct Raw8<__nv_bfloat16> {
     uint32_t w[4];
     __device__ __forceinline__ void zero() { w[0] = w[1] = w[2] = w[3] = 0u; }
     __device__ __forceinline__ void load(const __nv_bfloat16 *p, bool) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4 *>(p));
-        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+        asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "l"(p));
     }
     __device__ __forceinline__ float abs_max(float m) const {
 #pragma unroll
@@ -1086,11 +1085,15 @@ template <int NW> __device__ __forceinline__ float4 block_max4(float4 *s_w, floa
     return m;
 }
 
-// bytes of one key block's dS^T (16 keys x 64 queries, hi and for a float32 store lo halves) that lie outside the block's own V rows: its
-// lo part for head_dim 32, all of it for 16
-template <typename KVT> __host__ __device__ constexpr int bwd_tile_ds_extra(int hd) { return sizeof(KVT) == 2 || hd >= 64 ? 0 : hd == 32 ? 2048 : 4096; }
-constexpr size_t bwd_tile_smem_bytes(int hd, int maxk, int ds_extra) {
-    return (size_t)(2 * 64 + 2 * maxk) * (size_t)(hd * 4) + (size_t)(maxk / 16) * (size_t)ds_extra + (size_t)maxk * 8 + 3 * 64 * 4 + 144 + (size_t)(maxk / 16) * 4;
+// bytes of a staged K or V row, and of one key block's dS^T (16 keys x 64 queries, hi and lo halves: 4 KB) what lies outside the block's own 16 V
+// rows: nothing, the lo parts, or all of it
+__host__ __device__ constexpr int bwd_key_bytes(int hd, bool bf16) { return bf16 ? hd * 2 : hd * 4; }
+__host__ __device__ constexpr int bwd_tile_ds_extra(int hd, bool bf16) {
+    return 16 * bwd_key_bytes(hd, bf16) >= 4096 ? 0 : 16 * bwd_key_bytes(hd, bf16) >= 2048 ? 2048 : 4096;
+}
+constexpr size_t bwd_tile_smem_bytes(int hd, int maxk, bool bf16) {
+    return (size_t)(2 * 64) * (size_t)(hd * 4) + 2 * (size_t)maxk * (size_t)bwd_key_bytes(hd, bf16) + (size_t)(maxk / 16) * (size_t)bwd_tile_ds_extra(hd, bf16) +
+           (size_t)maxk * 8 + 3 * 64 * 4 + 144 + (size_t)(maxk / 16) * 4;
 }
 
 template <int HD, int NW, int MINB, typename KVT>
@@ -1102,12 +1105,13 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                      const int32_t *__restrict__ chain_ids, const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H,
                      float scale, int tile0, int maxk, bool wide, BwdMask gmask) {
     constexpr int M = 64, NT = NW * 32, TILE_ROW_BYTES = HD * 4, KS = HD / 16, NDB = HD / 8;
-    constexpr bool LP = sizeof(KVT) == 2;              // bfloat16 store: single fp16 products, no lo parts
+    constexpr bool BF = sizeof(KVT) == 2;              // bfloat16 store: K and V have no lo parts
+    constexpr int KB = bwd_key_bytes(HD, BF);
     extern __shared__ __align__(128) unsigned char tile_smem_raw[];
     unsigned char *sQ = tile_smem_raw, *sG = sQ + M * TILE_ROW_BYTES, *sK = sG + M * TILE_ROW_BYTES;
-    unsigned char *sV = sK + (size_t)maxk * TILE_ROW_BYTES;
-    constexpr int DSX = bwd_tile_ds_extra<KVT>(HD);
-    unsigned char *sDX = sV + (size_t)maxk * TILE_ROW_BYTES;                        // [maxk / 16][DSX] the rest of dS^T
+    unsigned char *sV = sK + (size_t)maxk * KB;
+    constexpr int DSX = bwd_tile_ds_extra(HD, BF);
+    unsigned char *sDX = sV + (size_t)maxk * KB;                                    // [maxk / 16][DSX] the rest of dS^T
     int2 *s_meta = reinterpret_cast<int2 *>(sDX + (size_t)(maxk / 16) * DSX);       // [maxk] {key id, key subtree end}
     float *sLse = reinterpret_cast<float *>(s_meta + maxk);                          // [64]  lse * log2(e)
     float *sDelta = sLse + M;                                                        // [64]  dO . O
@@ -1160,13 +1164,22 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
             if (T.c8 == 0 && r < M) sDelta[r] = d;
         }
     }
+    const TileStage<HD, NT, KB> TK(tid);
+    // Ids of chain rows: ahead of everything for a bfloat16 store (8 x 64, depth-32 trie of 578k rows 1786 -> 1450 us), one by one between the loads for a float32
+    // store, whose loads in a burst, twice as long, hold up the other blocks' shared-memory traffic (1870 against 1537 us; all loads predicated, without branches
+    // between them, 1711).
+    int ahead[UK];
+    if constexpr (BF) {
+#pragma unroll
+        for (int u = 0; u < UK; u++) ahead[u] = T.r0 + u * T.STEP < p ? __ldg(chain + T.r0 + u * T.STEP) : i0 + (T.r0 + u * T.STEP - p);
+    }
     Raw8<KVT> k8[UK], v8[UK];
 #pragma unroll
     for (int u = 0; u < UK; u++) {
         const int r = T.r0 + u * T.STEP;
         k8[u].zero(); v8[u].zero();
         if (r < nkeys) {
-            const int kid = r < p ? __ldg(chain + r) : i0 + (r - p);
+            const int kid = BF ? ahead[u] : r < p ? __ldg(chain + r) : i0 + (r - p);
             const int64_t off = (int64_t)kid * D + hoff + T.c8 * 8;
             k8[u].load(K + off, wide); v8[u].load(V + off, wide);
         }
@@ -1181,7 +1194,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                 const int64_t off = (int64_t)kid * D + hoff + T.c8 * 8;
                 kx.load(K + off, wide); vx.load(V + off, wide);
             }
-            f(kx, vx, (r - T.r0) * T.ROWB);
+            f(kx, vx, (r - T.r0) * KB);
         }
     };
     for (int j = tid; j < nkp; j += NT) {
@@ -1214,11 +1227,11 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
 #pragma unroll
     for (int u = 0; u < UK; u++)
         if (T.r0 + u * T.STEP < nkp) {
-            k8[u].put(sK + T.hi + u * T.OSTEP, sK + T.lo + u * T.OSTEP, sclK);
-            v8[u].put(sV + T.hi + u * T.OSTEP, sV + T.lo + u * T.OSTEP, sclV);
+            k8[u].put(sK + TK.hi + u * TK.OSTEP, sK + TK.lo + u * TK.OSTEP, sclK);
+            v8[u].put(sV + TK.hi + u * TK.OSTEP, sV + TK.lo + u * TK.OSTEP, sclV);
         }
     far_keys([&](const Raw8<KVT> &kx, const Raw8<KVT> &vx, int o) {
-        kx.put(sK + T.hi + o, sK + T.lo + o, sclK); vx.put(sV + T.hi + o, sV + T.lo + o, sclV);
+        kx.put(sK + TK.hi + o, sK + TK.lo + o, sclK); vx.put(sV + TK.hi + o, sV + TK.lo + o, sclV);
     });
     __syncthreads();
 
@@ -1228,7 +1241,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     // The powers of two are applied one after the other, never as one product that could leave the float range.
 
     // ldmatrix lane addressing: lane l names row l % 8 of matrix l / 8 (rows of 16 bytes).
-    const int l8 = lane & 7, mi = lane >> 3, sw = tile_swz<HD>(l8);
+    const int l8 = lane & 7, mi = lane >> 3, sw = row_swz<TILE_ROW_BYTES>(l8);
     // B fragments of an 8-row block for k-step ks (16 dims): matrices {hi chunk 2ks, hi 2ks+1, lo 2ks, lo 2ks+1}
     const uint32_t bRow = (uint32_t)(l8 * TILE_ROW_BYTES);
     const int bC = (mi & 1) + (mi >> 1) * NDB;          // + 2 ks
@@ -1238,13 +1251,15 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
     const uint32_t aRow = (uint32_t)((l8 + (mi & 1) * 8) * TILE_ROW_BYTES);
     const int aC = mi >> 1;                             // + 2 ks (+ 4 for lo)
     const int tC = (mi >> 1) * NDB;                     // + db
+    const int swK = row_swz<KB>(l8);                    // the same for key rows, which may be half as long
+    const uint32_t kRow = (uint32_t)((l8 + (mi & 1) * 8) * KB);
     const uint32_t uQ = smem_u32_of(sQ), uG = smem_u32_of(sG), uK = smem_u32_of(sK), uV = smem_u32_of(sV);
 
     // dS^T of (key block kb, query block qp): 16 x 16 halves as four 8 x 8 matrices of 128 bytes {keys 0-7 queries 0-7, keys 8-15
     // queries 0-7, keys 0-7 queries 8-15, keys 8-15 queries 8-15}.  hi parts and, where they fit, lo parts lie in the key block's own V rows, which
     // nothing reads any more once the block's item holds its V fragments.
     const uint32_t uDX = smem_u32_of(sDX);
-    auto ds_hi = [&](int kb, int qp) { return (DSX == 4096 ? uDX + (uint32_t)(kb * DSX) : uV + (uint32_t)(kb * 16 * TILE_ROW_BYTES)) + (uint32_t)(qp * 512); };
+    auto ds_hi = [&](int kb, int qp) { return (DSX == 4096 ? uDX + (uint32_t)(kb * DSX) : uV + (uint32_t)(kb * 16 * KB)) + (uint32_t)(qp * 512); };
     auto ds_lo = [&](int kb, int qp) { return DSX == 2048 ? uDX + (uint32_t)(kb * DSX + qp * 512) : ds_hi(kb, qp) + 2048u; };
 
     const int nkb = nkp >> 4;                    // key items: chain keys first (attended by most rows), then the tile's own
@@ -1260,10 +1275,10 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
             uint32_t kh[KS][4], kl[KS][4], vh[KS][4], vl[KS][4];
 #pragma unroll
             for (int ks = 0; ks < KS; ks++) {
-                const uint32_t o = (uint32_t)(kb * 16 * TILE_ROW_BYTES) + aRow;
-                const uint32_t ch = (uint32_t)(((2 * ks + aC) ^ sw) << 4), cl = (uint32_t)(((2 * ks + aC + NDB) ^ sw) << 4);
+                const uint32_t o = (uint32_t)(kb * 16 * KB) + kRow;
+                const uint32_t ch = (uint32_t)(((2 * ks + aC) ^ swK) << 4), cl = (uint32_t)(((2 * ks + aC + NDB) ^ swK) << 4);
                 ldmatrix_x4(kh[ks], uK + o + ch); ldmatrix_x4(vh[ks], uV + o + ch);
-                if constexpr (!LP) { ldmatrix_x4(kl[ks], uK + o + cl); ldmatrix_x4(vl[ks], uV + o + cl); }
+                if constexpr (!BF) { ldmatrix_x4(kl[ks], uK + o + cl); ldmatrix_x4(vl[ks], uV + o + cl); }
             }
             float dk[NDB][4], dv[NDB][4];
 #pragma unroll
@@ -1304,10 +1319,8 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                         uint32_t qf[4], gf[4];                 // {b0 hi, b1 hi, b0 lo, b1 lo}
                         ldmatrix_x4(qf, uQ + o); ldmatrix_x4(gf, uG + o);
                         mma_f16(c, kh[ks], qf[0], qf[1]); mma_f16(e, vh[ks], gf[0], gf[1]);
-                        if constexpr (!LP) {
-                            mma_f16(cx, kl[ks], qf[0], qf[1]); mma_f16(ex, vl[ks], gf[0], gf[1]);
-                            mma_f16(cx, kh[ks], qf[2], qf[3]); mma_f16(ex, vh[ks], gf[2], gf[3]);
-                        }
+                        mma_f16(cx, kh[ks], qf[2], qf[3]); mma_f16(ex, vh[ks], gf[2], gf[3]);
+                        if constexpr (!BF) { mma_f16(cx, kl[ks], qf[0], qf[1]); mma_f16(ex, vl[ks], gf[0], gf[1]); }
                     }
                     const float2 ls = *reinterpret_cast<const float2 *>(&sLse[qr + 2 * tig]);
                     const float2 dl = *reinterpret_cast<const float2 *>(&sDelta[qr + 2 * tig]);
@@ -1325,7 +1338,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                     f16_split2<false>(ds[u][0], ds[u][1], sh[2 * u], sl[2 * u]); f16_split2<false>(ds[u][2], ds[u][3], sh[2 * u + 1], sl[2 * u + 1]);
                 }
                 stmatrix_x4(ds_hi(kb, qp) + lane * 16, sh);
-                if constexpr (!LP) stmatrix_x4(ds_lo(kb, qp) + lane * 16, sl);
+                stmatrix_x4(ds_lo(kb, qp) + lane * 16, sl);
                 if (gmask.mode != AGPT_GRAD_FULL) {          // dK and dV take the unmasked pairs only (dQ takes all)
                     bool any = false;
 #pragma unroll
@@ -1355,10 +1368,8 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                     const uint32_t co = (uint32_t)(((db + tC) ^ sw) << 4);
                     ldmatrix_x4_trans(qt, uQ + ro + co); ldmatrix_x4_trans(gt, uG + ro + co);
                     mma_f16(dk[db], sh, qt[0], qt[1]); mma_f16(dv[db], ph, gt[0], gt[1]);
-                    if constexpr (!LP) {
-                        mma_f16(dk[db], sl, qt[0], qt[1]); mma_f16(dv[db], pl, gt[0], gt[1]);
-                        mma_f16(dk[db], ss, qt[2], qt[3]); mma_f16(dv[db], ps, gt[2], gt[3]);
-                    }
+                    mma_f16(dk[db], sl, qt[0], qt[1]); mma_f16(dv[db], pl, gt[0], gt[1]);
+                    mma_f16(dk[db], ss, qt[2], qt[3]); mma_f16(dv[db], ps, gt[2], gt[3]);
                 }
             }
             if (lane == 0) s_on[kb] = qon;
@@ -1389,16 +1400,25 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
             if (!((s_on[kp] >> rg) & 1u)) continue;
             uint32_t ah[4], al[4], as[4];
             ldmatrix_x4_trans(ah, ds_hi(kp, rg) + la);
-            if constexpr (!LP) ldmatrix_x4_trans(al, ds_lo(kp, rg) + la);
+            ldmatrix_x4_trans(al, ds_lo(kp, rg) + la);
+            const uint32_t rowt = uK + (uint32_t)(kp * 16 * KB) + kRow;
+            if constexpr (BF) {
 #pragma unroll
-            for (int j = 0; j < 4; j++) as[j] = f16_down11(ah[j]);
-            const uint32_t rowt = uK + (uint32_t)(kp * 16 * TILE_ROW_BYTES) + aRow;
+                for (int db = 0; db < NDB; db += 2) {
+                    uint32_t kt[4];                        // {b0, b1 of dims 8 db.., b0, b1 of dims 8 db + 8..}: keys 0-7 / 8-15 of the block
+                    ldmatrix_x4_trans(kt, rowt + (uint32_t)(((db + (mi >> 1)) ^ swK) << 4));
+                    mma_f16(dq[db], ah, kt[0], kt[1]); mma_f16(dq[db + 1], ah, kt[2], kt[3]);
+                    mma_f16(dq[db], al, kt[0], kt[1]); mma_f16(dq[db + 1], al, kt[2], kt[3]);
+                }
+            } else {
 #pragma unroll
-            for (int db = 0; db < NDB; db++) {
-                uint32_t kt[4];                            // {b0 hi, b1 hi, b0 lo, b1 lo}: keys 0-7 / 8-15 of the block, dims 8 db..
-                ldmatrix_x4_trans(kt, rowt + (uint32_t)(((db + tC) ^ sw) << 4));
-                mma_f16(dq[db], ah, kt[0], kt[1]);
-                if constexpr (!LP) { mma_f16(dq[db], al, kt[0], kt[1]); mma_f16(dq[db], as, kt[2], kt[3]); }
+                for (int j = 0; j < 4; j++) as[j] = f16_down11(ah[j]);
+#pragma unroll
+                for (int db = 0; db < NDB; db++) {
+                    uint32_t kt[4];                        // {b0 hi, b1 hi, b0 lo, b1 lo}: keys 0-7 / 8-15 of the block, dims 8 db..
+                    ldmatrix_x4_trans(kt, rowt + (uint32_t)(((db + tC) ^ swK) << 4));
+                    mma_f16(dq[db], ah, kt[0], kt[1]); mma_f16(dq[db], al, kt[0], kt[1]); mma_f16(dq[db], as, kt[2], kt[3]);
+                }
             }
         }
         const int r0 = i0 + rg * 16 + g, r1 = r0 + 8;
@@ -1562,7 +1582,7 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const float *__restrict__ K, c
     const int rg = warp;
     if (rg * 16 >= nt) return;                                   // rows beyond the end of the plan (no barrier follows)
     const float fS = scale * LOG2E * invQ * invK;               // log2-domain score = S' * fS
-    const int l8 = lane & 7, mi = lane >> 3, sw = tile_swz<HD>(l8);
+    const int l8 = lane & 7, mi = lane >> 3, sw = row_swz<TILE_ROW_BYTES>(l8);
     const uint32_t bRow = (uint32_t)(l8 * TILE_ROW_BYTES);
     const int bC = (mi & 1) + (mi >> 1) * NDB;
     const uint32_t aRow = (uint32_t)((l8 + (mi & 1) * 8) * TILE_ROW_BYTES);
@@ -2023,27 +2043,16 @@ static bool rows_wide(int D, const void *a, const void *b, const void *c, const 
     return D % 8 == 0 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)e) & 31) == 0;
 }
 static inline int bwd_tile_maxk(const agpt_plan *p) { return (p->max_keys + 15) & ~15; }
-// head_dim 16 and 32: three blocks of the backward per SM at least (32: four up to 96 keys, three up to 147); head_dim 64: two
-static inline bool bwd_tile_fits(const agpt_plan *p, int head_dim) {
+// Three blocks of the backward per SM at least (float32 rows of 32: four up to 96 keys, three up to 147), two of float32 rows of 64, whose
+// registers allow no more.  Beyond, the chunked kernel: bfloat16 rows of 64 with 140 keys a tile measured 2111 us with two blocks, 2007 in chunks.
+static inline bool bwd_tile_fits(const agpt_plan *p, int head_dim, bool bf16) {
     if (head_dim != 16 && head_dim != 32 && head_dim != 64) return false;
-    return bwd_tile_smem_bytes(head_dim, bwd_tile_maxk(p), bwd_tile_ds_extra<float>(head_dim)) <= (head_dim == 64 ? (size_t)113 * 1024 : (size_t)75 * 1024);
+    return bwd_tile_smem_bytes(head_dim, bwd_tile_maxk(p), bf16) <= (head_dim == 64 && !bf16 ? (size_t)113 * 1024 : (size_t)75 * 1024);
 }
 static inline bool fwd_tile_fits(const agpt_plan *p, int head_dim) {
     if (head_dim != 16 && head_dim != 32 && head_dim != 64) return false;
     return fwd_tile_smem_bytes(head_dim, bwd_tile_maxk(p)) <= (head_dim == 64 ? (size_t)75 * 1024 : (size_t)56 * 1024);
 }
-// Whole-tile backward for a bfloat16 store (AGPT_B200_ATTN_TILE_BF16=0: the chunked kernel, which keeps float32-level
-// products).  Measured: head_dim 32 (depth-32 trie, 28.3M positions) 42.3 ms against 45.5 ms chunked; head_dim 64 (4M-node
-// tree) 29.4 ms against 26.8 ms, so head_dim 64 stays chunked; the forward is no faster either way (15.1 ms) and stays chunked.
-static int tile_bf16_enabled() {
-    static int on = -1;
-    if (on < 0) {
-        const char *e = getenv("AGPT_B200_ATTN_TILE_BF16");
-        on = (e && e[0] == '0') ? 0 : 1;
-    }
-    return on;
-}
-
 template <int HD, int MINB>
 static int launch_fwd_tile(const agpt_plan *p, const float *q, const void *k, const void *v, float *out, float *lse, int H,
                            float scale, cudaStream_t st, int tile0, int ntiles) {
@@ -2132,7 +2141,7 @@ static int launch_bwd_tile(const agpt_plan *p, const float *q, const void *k, co
                            cudaStream_t st, int tile0, int ntiles, BwdMask gmask) {
     static size_t granted[AGPT_MAX_DEVICES];
     const int maxk = bwd_tile_maxk(p);
-    const size_t smem = bwd_tile_smem_bytes(HD, maxk, bwd_tile_ds_extra<KVT>(HD));
+    const size_t smem = bwd_tile_smem_bytes(HD, maxk, sizeof(KVT) == 2);
     int rc = allow_dynamic_smem(attn_bwd_tile_kernel<HD, NW, MINB, KVT>, smem, granted);
     if (rc) return rc;
     dim3 grid((unsigned)ntiles, (unsigned)H);
@@ -2146,7 +2155,11 @@ static int launch_bwd_tile_w(const agpt_plan *p, const float *q, const void *k, 
                              const float *lse, const float *dout, float *dq, float *dk, float *dv, float *pk, float *pv, int H,
                              int head_dim, float scale, cudaStream_t st, int tile0, int ntiles, BwdMask gmask) {
 #define TILE_ARGS p, q, k, v, o, lse, dout, dq, dk, dv, pk, pv, H, scale, st, tile0, ntiles, gmask
-    if (kv_dtype == AGPT_KV_BF16) return launch_bwd_tile<32, 4, 4, __nv_bfloat16>(TILE_ARGS);    // head_dim 32 only (bwd_dispatch)
+    if (kv_dtype == AGPT_KV_BF16) switch (head_dim) {
+        case 16: return launch_bwd_tile<16, 4, 4, __nv_bfloat16>(TILE_ARGS);
+        case 32: return launch_bwd_tile<32, 4, 4, __nv_bfloat16>(TILE_ARGS);
+        default: return launch_bwd_tile<64, 4, 3, __nv_bfloat16>(TILE_ARGS);
+    }
     if (head_dim == 16) return launch_bwd_tile<16, 4, 4>(TILE_ARGS);
     if (head_dim == 64) {        // twice the fragment and accumulator registers: two blocks per SM
         switch (g_bwd_warps) {
@@ -2166,11 +2179,8 @@ static int launch_bwd_tile_w(const agpt_plan *p, const float *q, const void *k, 
 static int bwd_dispatch(const agpt_plan *p, const float *q, const void *k, const void *v, int kv_dtype, const float *o,
                         const float *lse, const float *dout, float *dq, float *dk, float *dv, float *pk, float *pv, int H,
                         int head_dim, float scale, cudaStream_t st, int tile0, int ntiles, BwdMask gmask = BwdMask{AGPT_GRAD_FULL, nullptr}) {
-    if (attn_impl() == 1 && p->tile_m == 64 && bwd_tile_enabled() &&
-        (kv_dtype == AGPT_KV_F32 || (head_dim == 32 && tile_bf16_enabled()))) {
-        if (bwd_tile_fits(p, head_dim))
-            return launch_bwd_tile_w(p, q, k, v, kv_dtype, o, lse, dout, dq, dk, dv, pk, pv, H, head_dim, scale, st, tile0, ntiles, gmask);
-    }
+    if (attn_impl() == 1 && p->tile_m == 64 && bwd_tile_enabled() && bwd_tile_fits(p, head_dim, kv_dtype == AGPT_KV_BF16))
+        return launch_bwd_tile_w(p, q, k, v, kv_dtype, o, lse, dout, dq, dk, dv, pk, pv, H, head_dim, scale, st, tile0, ntiles, gmask);
     if (attn_impl() == 1 && p->tile_m == 64 && p->max_keys <= MAXKEYS) {
         const bool bf = kv_dtype == AGPT_KV_BF16;
 #define BWD_MMA_ARGS p, q, k, v, o, lse, dout, dq, dk, dv, pk, pv, H, scale, st, tile0, ntiles, gmask
