@@ -133,6 +133,8 @@ SIGNATURES = {
     "agpt_b200_trie_from_suffix_order": (C.c_int, [vp, i64, C.c_int, C.c_int, C.c_int, C.c_int, vp, vp, C.POINTER(vp)]),
     "agpt_b200_suffix_order_gpu": (C.c_int, [vp, i64, C.c_int, C.c_int, vp, vp, C.POINTER(C.c_float)]),
     "agpt_b200_trie_build_gpu": (C.c_int, [vp, i64, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(vp)]),
+    "agpt_b200_trie_build_workspace_bytes": (i64, [i64]),
+    "agpt_b200_trie_build_gpu_ws": (C.c_int, [vp, i64, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, vp, i64, vp, C.POINTER(vp)]),
     "agpt_b200_gemm_f32": (C.c_int, [C.c_int] * 5 + [f32, vp, C.c_int, vp, C.c_int, f32, vp, C.c_int, vp, C.c_int, vp, C.c_int, C.c_int, vp,
                                      i64, vp]),
     "agpt_b200_gemm_f32_workspace_bytes": (i64, [C.c_int] * 6),

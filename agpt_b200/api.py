@@ -97,8 +97,11 @@ class RadixTrie:
         if c.size < max_depth + 2:
             return cls.build(c, max_depth, subtree_level, prune_min_mass, prune_min_depth)
         h = C.c_void_p()
-        check(lib().agpt_b200_trie_build_gpu(_vp(c), c.size, max_depth, subtree_level, prune_min_mass, prune_min_depth, device,
-                                             C.byref(h)), "trie_build_gpu")
+        import torch
+        with torch.cuda.device(device):
+            ws = torch.empty(max(256, lib().agpt_b200_trie_build_workspace_bytes(c.size)), dtype=torch.uint8, device=f"cuda:{device}")
+            check(lib().agpt_b200_trie_build_gpu_ws(_vp(c), c.size, max_depth, subtree_level, prune_min_mass, prune_min_depth, device,
+                                                    _dp(ws), ws.numel(), _stream(), C.byref(h)), "trie_build_gpu")
         return cls(h)
 
     @classmethod

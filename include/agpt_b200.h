@@ -173,6 +173,11 @@ int agpt_b200_suffix_order_gpu(const int32_t *corpus, int64_t n, int key_len, in
                                int32_t *lcp_out, float *device_ms_out);
 int agpt_b200_trie_build_gpu(const int32_t *corpus, int64_t n, int max_depth, int subtree_level, int prune_min_mass,
                              int prune_min_depth, int device, agpt_trie **out);
+/* The same in device memory of the caller (agpt_b200_trie_build_workspace_bytes(n), 256-byte aligned) and on its stream, which has
+ * finished when the call returns. */
+int64_t agpt_b200_trie_build_workspace_bytes(int64_t n);
+int agpt_b200_trie_build_gpu_ws(const int32_t *corpus, int64_t n, int max_depth, int subtree_level, int prune_min_mass, int prune_min_depth,
+                                int device, void *d_workspace, int64_t workspace_bytes, void *stream, agpt_trie **out);
 /* Stochastic training units of the reference's "lightning" mode (src/cuda/agpt_train.cu:152-200, :4060-4241): `steps`
  * samples from a 32-bit xorshift generator (*rng_state, the reference seeds it with 0x5c115e1).  sampler 1: uniform
  * over radix nodes; 2: uniform over root children; 3: mass-weighted walk from the root that stops with probability
