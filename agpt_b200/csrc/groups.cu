@@ -111,7 +111,7 @@ struct agpt_run_groups {
     std::vector<RunGroup> groups;
     // of the group made ready last
     int64_t ready = -1;
-    std::unique_ptr<uint8_t[]> staging;
+    std::unique_ptr<uint8_t[], agpt_big_free> staging;
     int64_t staged = 0;
     agpt_plan *plan = nullptr;
     agpt_run_group_info info;
@@ -375,7 +375,8 @@ extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int t
     o.bytes = std::max<int64_t>(at, 16);
     o.seq_len = seq_len;
 
-    G->staging.reset(new uint8_t[(size_t)std::max<int64_t>(G->staged, 16)]);
+    G->staging.reset((uint8_t *)agpt_big_alloc((size_t)std::max<int64_t>(G->staged, 16)));
+    if (!G->staging) throw std::bad_alloc();
     uint8_t *s = G->staging.get();
     auto put = [&](int64_t where, const void *src, int64_t bytes) { if (bytes) memcpy(s + where, src, (size_t)bytes); };
     put(o.qoff, g.qoff.data(), (int64_t)(E + 1) * 4); put(o.rid, g.rid.data(), (int64_t)E * 4);

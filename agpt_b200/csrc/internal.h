@@ -2,12 +2,46 @@
 #pragma once
 #include <atomic>
 #include <cstdint>
+#include <cstdlib>
 #include <mutex>
+#include <new>
 #include <vector>
+
+#include <sys/mman.h>
 
 #define AGPT_REDUCE_SEG 16    // tiles summed by one warp of the dK/dV reduction before a second pass (at most 32: one offset per lane)
 
 int agpt_set_error(int code, const char *fmt, ...);
+
+// Host memory for arrays of megabytes that one call makes and fills once.  Their first touch in 4 KB pages costs more than the
+// fill (0.5 us a page: 2 ms for the 1.7M edge characters of 60,000 tokens at depth 32, and zeroing them first as much again), so
+// from 1 MB on they lie in huge pages where the system has them, and elements that are not given a value are left as they come.
+constexpr size_t AGPT_HUGE_PAGE = (size_t)2 << 20, AGPT_HUGE_FROM = (size_t)1 << 20;
+inline void *agpt_big_alloc(size_t bytes) {
+    if (bytes < AGPT_HUGE_FROM) return malloc(bytes ? bytes : 1);
+    const size_t whole = (bytes + AGPT_HUGE_PAGE - 1) / AGPT_HUGE_PAGE * AGPT_HUGE_PAGE;
+    void *p = aligned_alloc(AGPT_HUGE_PAGE, whole);
+    if (p) madvise(p, whole, MADV_HUGEPAGE);     // a hint: without huge pages the memory is as good
+    return p;
+}
+struct agpt_big_free { void operator()(void *p) const { free(p); } };
+template <typename T>
+struct agpt_big_allocator {
+    using value_type = T;
+    agpt_big_allocator() = default;
+    template <typename U> agpt_big_allocator(const agpt_big_allocator<U> &) {}
+    T *allocate(size_t n) {
+        void *p = n > SIZE_MAX / sizeof(T) - AGPT_HUGE_PAGE ? nullptr : agpt_big_alloc(n * sizeof(T));
+        if (!p) throw std::bad_alloc();
+        return (T *)p;
+    }
+    void deallocate(T *p, size_t) { free(p); }
+    template <typename U> void construct(U *p) { ::new ((void *)p) U; }       // resize() leaves new elements unset
+    template <typename U, typename V> void construct(U *p, V &&v) { ::new ((void *)p) U((V &&)v); }
+    template <typename U> bool operator==(const agpt_big_allocator<U> &) const { return true; }
+    template <typename U> bool operator!=(const agpt_big_allocator<U> &) const { return false; }
+};
+template <typename T> using agpt_big_vector = std::vector<T, agpt_big_allocator<T>>;
 
 // Radix trie with the reference's node numbering (ids in the builder's breadth-first emission order), counts, edge
 // mass and char positions.
@@ -16,7 +50,7 @@ struct agpt_trie {
     int64_t total_edge_chars = 0, leveled_nodes = 0;
     std::vector<int32_t> parent, first_char_depth, edge_len, edge_mass, endpoint_depth, subtree_key, edge_start;
     std::vector<int64_t> edge_off, cnt_off;
-    std::vector<int32_t> edge_tok, cnt_tok, cnt_val;
+    agpt_big_vector<int32_t> edge_tok, cnt_tok, cnt_val;
     void finish_char_positions() {
         // char positions follow depth-file order (src/cuda/agpt_train.cu:813-846)
         edge_start.assign(radix_count, 0);

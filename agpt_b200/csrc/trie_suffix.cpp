@@ -31,6 +31,7 @@ struct Endpoint {
     int32_t lb, rb;        // interval of ordered suffixes that share the endpoint's prefix
     int32_t depth;         // endpoint depth
     int32_t last_split;    // last place inside (lb, rb] where the neighbours' common prefix equals depth; -1: one run
+    int32_t entries;       // distinct next tokens: runs between the splits that have one
     int32_t parent;        // emission index of the enclosing endpoint, -1: the root
 };
 
@@ -50,12 +51,13 @@ extern "C" int agpt_b200_trie_from_suffix_order(const int32_t *corpus, int64_t n
     auto len_of = [&](int32_t i) -> int { int64_t l = n - sa[i]; return l < KL ? (int)l : KL; };
     auto lcp_at = [&](int64_t i) -> int { return (i <= 0 || i >= m) ? 0 : lcp[i]; };
 
-    std::vector<Endpoint> eps;
+    agpt_big_vector<Endpoint> eps;
+    eps.reserve((size_t)m * 2);                    // at most one per suffix and one per inner interval; pages are touched as it grows
     std::vector<int32_t> pending;                  // endpoints not yet enclosed by a later (shallower) one
     std::vector<int32_t> prev_split(m, -1);        // chain of split points of one interval, newest first
-    auto emit = [&](int32_t lb, int32_t rb, int32_t depth, int32_t last_split) {
+    auto emit = [&](int32_t lb, int32_t rb, int32_t depth, int32_t last_split, int32_t entries) {
         int32_t id = (int32_t)eps.size();
-        eps.push_back({lb, rb, depth, last_split, -1});
+        eps.push_back({lb, rb, depth, last_split, entries, -1});
         while (!pending.empty() && eps[pending.back()].lb >= lb) {
             eps[pending.back()].parent = id;
             pending.pop_back();
@@ -72,7 +74,7 @@ extern "C" int agpt_b200_trie_from_suffix_order(const int32_t *corpus, int64_t n
             // its first D tokens
             const int32_t j = (int32_t)(i - 1);
             const int left = lcp_at(j), right = cur < 0 ? 0 : cur;
-            if (len_of(j) >= KL && std::max(left, right) < D) emit(j, j, D, -1);
+            if (len_of(j) >= KL && std::max(left, right) < D) emit(j, j, D, -1, 1);
             leveled += std::min(len_of(j), D) - std::min(left, D);
         }
         int32_t lb = (int32_t)(i - 1);
@@ -85,12 +87,12 @@ extern "C" int agpt_b200_trie_from_suffix_order(const int32_t *corpus, int64_t n
             if (iv.lcp >= KL) {
                 // every suffix of the interval shares the next token too: the depth-D prefix is an endpoint of its own
                 // only if the enclosing interval splits above depth D
-                if (std::max(lcp_at(iv.lb), cur < 0 ? 0 : cur) < D) emit(iv.lb, rb, D, -1);
+                if (std::max(lcp_at(iv.lb), cur < 0 ? 0 : cur) < D) emit(iv.lb, rb, D, -1, 1);
                 continue;
             }
             // next tokens = runs between the split points; a suffix that ends exactly here (it orders first) has none
             const int real = 1 + iv.n_splits - (len_of(iv.lb) == iv.lcp ? 1 : 0);
-            if (iv.lcp < D ? real >= 2 : real >= 1) emit(iv.lb, rb, iv.lcp, iv.last_split);
+            if (iv.lcp < D ? real >= 2 : real >= 1) emit(iv.lb, rb, iv.lcp, iv.last_split, real);
         }
         if (cur >= 0) {
             if (!st.empty() && st.back().lcp == cur) {
@@ -152,16 +154,8 @@ extern "C" int agpt_b200_trie_from_suffix_order(const int32_t *corpus, int64_t n
         t->edge_mass[r] = mass[e];
         t->endpoint_depth[r] = x.depth;
         max_ep = std::max(max_ep, x.depth);
-        // count entries: one per run of the interval that has a next token
-        int32_t entries;
-        if (x.last_split < 0) entries = 1;
-        else {
-            entries = 1;
-            for (int32_t s = x.last_split; s >= 0; s = prev_split[s]) entries++;
-            if (len_of(x.lb) == x.depth) entries--;
-        }
         t->edge_off[r + 1] = t->edge_len[r];
-        t->cnt_off[r + 1] = entries;
+        t->cnt_off[r + 1] = x.entries;
     }
     for (int32_t r = 0; r < R; r++) { t->edge_off[r + 1] += t->edge_off[r]; t->cnt_off[r + 1] += t->cnt_off[r]; }
     t->edge_tok.resize((size_t)t->edge_off[R]);
