@@ -82,6 +82,7 @@ SIGNATURES = {
     "agpt_b200_token_hash": (u64, [vp, i64]),
     "agpt_b200_trie_char_tree": (C.c_int, [vp, vp, vp, vp, vp]),
     "agpt_b200_plan_create": (C.c_int, [vp, i64, C.c_int, C.c_int, C.POINTER(vp)]),
+    "agpt_b200_plan_create_even": (C.c_int, [vp, i64, C.c_int, C.c_int, C.POINTER(vp)]),
     "agpt_b200_plan_info": (C.c_int, [vp, C.POINTER(PlanInfo)]),
     "agpt_b200_plan_array": (C.c_int, [vp, C.c_int, vp]),
     "agpt_b200_plan_sizes": (C.c_int, [vp, C.POINTER(PlanInfo)]),
@@ -92,6 +93,7 @@ SIGNATURES = {
     "agpt_b200_trie_group_prepare": (C.c_int, [vp, i64, C.c_int, C.c_int, C.c_int, C.POINTER(RunGroupInfo)]),
     "agpt_b200_trie_group_upload": (C.c_int, [vp, C.c_int, vp, vp, C.POINTER(vp)]),
     "agpt_b200_trie_groups_free": (None, [vp]),
+    "agpt_b200_trie_groups_even": (C.c_int, [vp, C.c_int]),
     "agpt_b200_plan_destroy": (None, [vp]),
     "agpt_b200_attn_bwd_workspace_bytes": (i64, [vp, C.c_int]),
     "agpt_b200_plan_units": (i64, [vp, C.c_int, i64, vp, vp]),
@@ -118,6 +120,7 @@ SIGNATURES = {
     "agpt_b200_softmax_bwd": (C.c_int, [vp] * 3 + [i64, C.c_int, vp]),
     "agpt_b200_embedding_gather": (C.c_int, [vp] * 3 + [i64, C.c_int, C.c_int, vp]),
     "agpt_b200_embedding_grad": (C.c_int, [vp] * 3 + [i64, C.c_int, C.c_int, C.c_int, vp, i64, vp]),
+    "agpt_b200_embedding_grad_serial": (C.c_int, [vp] * 3 + [i64, C.c_int, C.c_int, C.c_int, vp, i64, vp]),
     "agpt_b200_embedding_grad_workspace_bytes": (i64, [i64, C.c_int, C.c_int]),
     "cuda_adam_bulk": (None, [vp] * 4 + [f32] * 4 + [C.c_int, C.c_int]),
     "cuda_sgd_bulk": (None, [vp, vp, f32, C.c_int]),

@@ -210,10 +210,11 @@ class WalkerPlan:
 
     _ARRAYS = ("dfs_to_node", "node_to_dfs", "parent_dfs", "depth", "sub_end")
 
-    def __init__(self, parent, tile_m: int = 64, device: int = -1):
+    def __init__(self, parent, tile_m: int = 64, device: int = -1, even: bool = False):
         par = _np_i32(parent)
         h = C.c_void_p()
-        check(lib().agpt_b200_plan_create(_vp(par), par.size, tile_m, device, C.byref(h)), "plan_create")
+        create = lib().agpt_b200_plan_create_even if even else lib().agpt_b200_plan_create
+        check(create(_vp(par), par.size, tile_m, device, C.byref(h)), "plan_create")
         self._adopt(h)
 
     def _adopt(self, h, keep=None):
@@ -337,10 +338,11 @@ class RunGroups:
     def __len__(self):
         return int(lib().agpt_b200_trie_groups_count(self._h))
 
-    def upload(self, i: int, tile_m: int, mass_mode: str, seq_len: int, device):
-        """(info, device buffer, plan) of group i."""
+    def upload(self, i: int, tile_m: int, mass_mode: str, seq_len: int, device, even: bool = False):
+        """(info, device buffer, plan) of group i; even: a plan with even tiles (agpt_b200_plan_create_even)."""
         import torch
         info = RunGroupInfo()
+        check(lib().agpt_b200_trie_groups_even(self._h, int(even)), "trie_groups_even")
         check(lib().agpt_b200_trie_group_prepare(self._h, i, tile_m, MASS_MODES[mass_mode], seq_len, C.byref(info)), "trie_group_prepare")
         buf = torch.empty(int(info.bytes), dtype=torch.uint8, device=device)
         h = C.c_void_p()
@@ -739,16 +741,16 @@ def embedding_gather(emb, ids32):
     return out
 
 
-def embedding_grad(grad, ids32, vocab, out=None, accumulate=False):
-    """Gradient of the embedding table, [vocab, d_model], summed in a fixed order."""
+def embedding_grad(grad, ids32, vocab, out=None, accumulate=False, serial=False):
+    """Gradient of the embedding table, [vocab, d_model], summed in a fixed order (serial: the order of agpt_b200_embedding_grad_serial)."""
     import torch
     _chk_f32(grad, "grad")
     n, d = grad.shape
     out = torch.zeros((vocab, d), dtype=torch.float32, device=grad.device) if out is None else out
     wsb = check(lib().agpt_b200_embedding_grad_workspace_bytes(n, d, vocab), "embedding_grad_workspace_bytes")
     ws = _workspace(grad.device, "embedding_grad", wsb)
-    check(lib().agpt_b200_embedding_grad(_dp(grad), _dp(ids32), _dp(out), n, d, vocab, int(accumulate), _dp(ws), wsb, _stream()),
-          "embedding_grad")
+    fn = lib().agpt_b200_embedding_grad_serial if serial else lib().agpt_b200_embedding_grad
+    check(fn(_dp(grad), _dp(ids32), _dp(out), n, d, vocab, int(accumulate), _dp(ws), wsb, _stream()), "embedding_grad")
     return out
 
 

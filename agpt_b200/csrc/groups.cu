@@ -114,6 +114,7 @@ struct agpt_run_groups {
     std::unique_ptr<uint8_t[], agpt_big_free> staging;
     int64_t staged = 0;
     agpt_plan *plan = nullptr;
+    bool even = false;                        // of the plans made from here on
     agpt_run_group_info info;
     int64_t at_prun = 0, at_fd = 0, at_ld = 0, at_send = 0, at_unit = 0, at_first = 0, at_mw = 0, at_tr = 0, at_choff = 0, at_items[4] = {0, 0, 0, 0},
             at_multi = 0, at_mcount = 0, at_mfirst = 0, at_ts = 0, at_depth = 0, at_subend = 0, at_cid = 0, at_cend = 0;
@@ -232,6 +233,11 @@ extern "C" int agpt_b200_trie_sample_group(const agpt_trie *t, const int32_t *ra
 
 extern "C" int64_t agpt_b200_trie_groups_count(const agpt_run_groups *G) { return G ? (int64_t)G->groups.size() : 0; }
 extern "C" void agpt_b200_trie_groups_free(agpt_run_groups *G) { delete G; }
+extern "C" int agpt_b200_trie_groups_even(agpt_run_groups *G, int even) {
+    if (!G) return agpt_set_error(AGPT_E_ARG, "trie_groups_even: null");
+    G->even = even != 0;
+    return AGPT_OK;
+}
 
 extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int tile_m, int mass_mode, int seq_len, agpt_run_group_info *out) {
     if (!G || !out || i < 0 || i >= (int64_t)G->groups.size() || seq_len < 1 || mass_mode < 0 || mass_mode > 3 || (tile_m != 32 && tile_m != 64 && tile_m != 128))
@@ -242,7 +248,7 @@ extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int t
     const int64_t n = g.rows(), M = tile_m;
     delete G->plan;
     agpt_plan *P = G->plan = new agpt_plan();
-    P->n = n; P->tile_m = tile_m;
+    P->n = n; P->tile_m = tile_m; P->even = G->even;
     P->lazy = true;
     P->run_qoff.assign(g.qoff.begin(), g.qoff.end()); P->run_parent = g.prun;
     std::vector<int32_t> &ld = P->run_depth, &send = P->run_end;
@@ -272,7 +278,7 @@ extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int t
     for (int64_t i = 0; i < n;) {
         ts.push_back((int32_t)i);
         int64_t k = std::min(M, n - i), e1 = e0;
-        if (tile_m == 64 && i + M < n) {
+        if (tile_m == 64 && !P->even && i + M < n) {
             while (g.qoff[e1 + 1] <= i + 32) e1++;
             int64_t best = INT64_MAX;
             for (int64_t e = e1; e < E && g.qoff[e] <= i + M; e++) {
@@ -290,7 +296,7 @@ extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int t
     P->chain_rows = P->chain_off[P->n_tiles];
     // reduction work list: the rows whose subtree reaches into later tiles, ordered by their last tile (a counting sort)
     {
-        constexpr int32_t SEG = AGPT_REDUCE_SEG;
+        const int32_t SEG = P->even ? (int32_t)P->n_tiles : AGPT_REDUCE_SEG;
         std::vector<int64_t> start(P->n_tiles + 1, 0);
         std::vector<int32_t> last_tile(E);      // tile of the last row of a run's subtree
         {   // of every run's last row first; a run's subtree ends with a run's last row

@@ -694,7 +694,7 @@ extern "C" int agpt_b200_mass_weights(const int32_t *edge_mass, const int32_t *e
 // --------------------------------------------------------------------------------------
 // walker plan
 // --------------------------------------------------------------------------------------
-extern "C" int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_m, int device, agpt_plan **out) {
+static int plan_create(const int32_t *parent, int64_t n, int tile_m, int device, bool even, agpt_plan **out) {
     if (!parent || !out || n <= 0) return agpt_set_error(AGPT_E_ARG, "plan_create: bad argument");
     if (n >= (1LL << 31) - 256) return agpt_set_error(AGPT_E_LIMIT, "plan_create: more than 2^31 nodes in one plan");
     if (tile_m != 32 && tile_m != 64 && tile_m != 128) return agpt_set_error(AGPT_E_ARG, "plan_create: tile_m must be 32, 64 or 128");
@@ -705,7 +705,7 @@ extern "C" int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_
         if (p >= i) monotone = false;
     }
     agpt_plan *P = new agpt_plan();
-    P->n = n; P->tile_m = tile_m;
+    P->n = n; P->tile_m = tile_m; P->even = even;
     P->dfs_to_node.resize(n); P->node_to_dfs.assign(n, -1); P->parent_dfs.resize(n); P->depth.resize(n); P->sub_end.resize(n);
     P->n_groups = 0; P->sum_group_prefix = 0;
     if (monotone) {
@@ -776,7 +776,7 @@ extern "C" int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_
     P->max_depth = 0; P->sum_depth = 0;
     for (int64_t i = 0; i < n; i++) { P->max_depth = std::max(P->max_depth, P->depth[i]); P->sum_depth += P->depth[i]; }
     // tiles; the chain of the first query of each, root side first
-    const bool early = device >= 0 && tile_m == 64;
+    const bool early = device >= 0 && tile_m == 64 && !even;
     std::vector<int32_t> &ts = P->tile_start;
     ts.reserve(n / 32 + 2);
     for (int64_t i = 0; i < n;) {
@@ -808,7 +808,7 @@ extern "C" int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_
     for (size_t j = 0; j < P->chain_ids.size(); j++) P->chain_end[j] = P->sub_end[P->chain_ids[j]];
     // reduction work list: node a receives one partial row from every tile that starts strictly inside
     // its subtree, i.e. tiles (tile of a, tile of sub_end[a] - 1]; long ranges are cut into segments
-    const int64_t SEG = AGPT_REDUCE_SEG;
+    const int64_t SEG = even ? INT32_MAX : AGPT_REDUCE_SEG;
     for (int64_t a = 0, t0 = 1; a < n; a++) {          // t0: one past the tile of a
         while (ts[t0] <= a) t0++;
         if (P->sub_end[a] <= ts[t0]) continue;
@@ -841,6 +841,13 @@ extern "C" int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_
     }
     *out = P;
     return AGPT_OK;
+}
+
+extern "C" int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_m, int device, agpt_plan **out) {
+    return plan_create(parent, n, tile_m, device, false, out);
+}
+extern "C" int agpt_b200_plan_create_even(const int32_t *parent, int64_t n, int tile_m, int device, agpt_plan **out) {
+    return plan_create(parent, n, tile_m, device, true, out);
 }
 
 // one row array (0 dfs_to_node, 1 node_to_dfs, 2 parent_dfs, 3 depth, 4 sub_end), written straight into the caller's memory

@@ -1917,6 +1917,37 @@ reduce_items_kernel(const float *__restrict__ Pk, const float *__restrict__ Pv, 
         *reinterpret_cast<float4 *>(dst[i] + at) = make_float4(old[i].x + sum[i].x, old[i].y + sum[i].y, old[i].z + sum[i].z, old[i].w + sum[i].w);
 }
 
+// The reduction of an even plan: one warp per node and 128 columns adds the node's partial rows tile by tile, every 128 tiles into a
+// sum of their own, and then those sums in order.  A sampled unit has a handful of tiles: bound by the latency of one launch.
+__global__ void __launch_bounds__(256)
+reduce_even_kernel(const float *__restrict__ Pk, const float *__restrict__ Pv, float *__restrict__ dK, float *__restrict__ dV,
+                   const int64_t *__restrict__ chain_off, const int32_t *__restrict__ depth, const int32_t *__restrict__ item_node,
+                   const int32_t *__restrict__ item_t0, const int32_t *__restrict__ item_t1, int64_t item0, int64_t n_items, int D, int chunks) {
+    int64_t it = (int64_t)(blockIdx.x / chunks) * 8 + (threadIdx.x >> 5);
+    const int c = (blockIdx.x % chunks) * 128 + (threadIdx.x & 31) * 4;
+    if (it >= n_items || c >= D) return;
+    it += item0;
+    const int a = __ldg(item_node + it), t0 = __ldg(item_t0 + it), t1 = __ldg(item_t1 + it), row = __ldg(depth + a) - 1;
+    float4 k = make_float4(0.f, 0.f, 0.f, 0.f), v = k;
+    for (int s = t0; s <= t1; s += 128) {
+        float4 sk = make_float4(0.f, 0.f, 0.f, 0.f), sv = sk;
+        const int end = min(t1, s + 127);
+#pragma unroll 4
+        for (int t = s; t <= end; t++) {
+            const int64_t r = (__ldg(chain_off + t) + row) * D + c;
+            const float4 a4 = __ldcs(reinterpret_cast<const float4 *>(Pk + r)), b4 = __ldcs(reinterpret_cast<const float4 *>(Pv + r));
+            sk.x += a4.x; sk.y += a4.y; sk.z += a4.z; sk.w += a4.w;
+            sv.x += b4.x; sv.y += b4.y; sv.z += b4.z; sv.w += b4.w;
+        }
+        k.x += sk.x; k.y += sk.y; k.z += sk.z; k.w += sk.w;
+        v.x += sv.x; v.y += sv.y; v.z += sv.z; v.w += sv.w;
+    }
+    float4 *pk = reinterpret_cast<float4 *>(dK + (int64_t)a * D + c), *pv = reinterpret_cast<float4 *>(dV + (int64_t)a * D + c);
+    const float4 x = *pk, y = *pv;
+    *pk = make_float4(x.x + k.x, x.y + k.y, x.z + k.z, x.w + k.w);
+    *pv = make_float4(y.x + v.x, y.y + v.y, y.z + v.z, y.w + v.w);
+}
+
 // pass 2: nodes whose range was cut into several items; their segment sums are added by the eight warps of a block, a range
 // each, and the warps' sums in warp order.
 __global__ void __launch_bounds__(256)
@@ -2038,6 +2069,7 @@ extern "C" int agpt_b200_set_attn_variant(int whole_tile, int warps) {
     g_bwd_tile = whole_tile; g_bwd_warps = warps;
     return AGPT_OK;
 }
+static bool tile_kernels_wanted(const agpt_plan *p) { return bwd_tile_enabled() && !p->even; }
 // every head of every row of these buffers starts on a 32-byte boundary
 static bool rows_wide(int D, const void *a, const void *b, const void *c, const void *d, const void *e) {
     return D % 8 == 0 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)e) & 31) == 0;
@@ -2094,7 +2126,7 @@ static int launch_fwd_mma(const agpt_plan *p, const float *q, const void *k, con
 
 static int fwd_dispatch(const agpt_plan *p, const float *q, const void *k, const void *v, int kv_dtype, float *out,
                         float *lse, int H, int head_dim, float scale, cudaStream_t st, int tile0, int ntiles) {
-    if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_F32 && bwd_tile_enabled() && fwd_tile_fits(p, head_dim)) {
+    if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_F32 && tile_kernels_wanted(p) && fwd_tile_fits(p, head_dim)) {
         switch (head_dim) {
             case 16: return launch_fwd_tile<16, 8>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
             case 32: return launch_fwd_tile<32, 6>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
@@ -2102,7 +2134,7 @@ static int fwd_dispatch(const agpt_plan *p, const float *q, const void *k, const
         }
     }
     // bfloat16 store: whole tiles while two blocks of them fit one SM (head_dim 64: up to 438 keys), deeper plans in chunks
-    if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_BF16 &&
+    if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_BF16 && !p->even &&
         fwd_bf16_smem_bytes(head_dim, bwd_tile_maxk(p)) <= (size_t)113 * 1024) {
         switch (head_dim) {
             case 16: return launch_fwd_bf16<16, 8>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
@@ -2111,10 +2143,10 @@ static int fwd_dispatch(const agpt_plan *p, const float *q, const void *k, const
         }
     }
     if (attn_impl() == 1 && p->tile_m == 64 && p->max_keys <= MAXKEYS) {
-        const bool bf = kv_dtype == AGPT_KV_BF16;        // (head_dim 16 and 32: MAXKEYS keys fit the whole-tile kernel)
+        const bool bf = kv_dtype == AGPT_KV_BF16;
         switch (head_dim) {
-            case 16: return launch_fwd_mma<16, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
-            case 32: return launch_fwd_mma<32, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            case 16: return bf ? launch_fwd_mma<16, __nv_bfloat16>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles) : launch_fwd_mma<16, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            case 32: return bf ? launch_fwd_mma<32, __nv_bfloat16>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles) : launch_fwd_mma<32, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
             case 64: return bf ? launch_fwd_mma<64, __nv_bfloat16>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles) : launch_fwd_mma<64, float>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
         }
     }
@@ -2179,7 +2211,7 @@ static int launch_bwd_tile_w(const agpt_plan *p, const float *q, const void *k, 
 static int bwd_dispatch(const agpt_plan *p, const float *q, const void *k, const void *v, int kv_dtype, const float *o,
                         const float *lse, const float *dout, float *dq, float *dk, float *dv, float *pk, float *pv, int H,
                         int head_dim, float scale, cudaStream_t st, int tile0, int ntiles, BwdMask gmask = BwdMask{AGPT_GRAD_FULL, nullptr}) {
-    if (attn_impl() == 1 && p->tile_m == 64 && bwd_tile_enabled() && bwd_tile_fits(p, head_dim, kv_dtype == AGPT_KV_BF16))
+    if (attn_impl() == 1 && p->tile_m == 64 && tile_kernels_wanted(p) && bwd_tile_fits(p, head_dim, kv_dtype == AGPT_KV_BF16))
         return launch_bwd_tile_w(p, q, k, v, kv_dtype, o, lse, dout, dq, dk, dv, pk, pv, H, head_dim, scale, st, tile0, ntiles, gmask);
     if (attn_impl() == 1 && p->tile_m == 64 && p->max_keys <= MAXKEYS) {
         const bool bf = kv_dtype == AGPT_KV_BF16;
@@ -2211,7 +2243,10 @@ static int run_reduce_range(const agpt_plan *p, float *pk, float *pv, float *seg
         const int chunks = (D + 127) / 128;
         const unsigned grid = (unsigned)((n_items + 7) / 8 * chunks);
 #define REDUCE_ARGS pk, pv, dk, dv, segk, segv, p->d_chain_off, p->d_depth, p->d_item_node, p->d_item_t0, p->d_item_t1, p->d_item_slot, item0, n_items, D, chunks
-        if (D <= 64) reduce_items_kernel<true><<<grid, 256, 0, st>>>(REDUCE_ARGS);
+        if (p->even)
+            reduce_even_kernel<<<grid, 256, 0, st>>>(pk, pv, dk, dv, p->d_chain_off, p->d_depth, p->d_item_node, p->d_item_t0, p->d_item_t1, item0, n_items, D,
+                                                     chunks);
+        else if (D <= 64) reduce_items_kernel<true><<<grid, 256, 0, st>>>(REDUCE_ARGS);
         else reduce_items_kernel<false><<<grid, 256, 0, st>>>(REDUCE_ARGS);
 #undef REDUCE_ARGS
         int rc = launch_status("reduce_items");

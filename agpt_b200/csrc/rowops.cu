@@ -251,6 +251,16 @@ __global__ void __launch_bounds__(32) embedding_grad_kernel(const float *__restr
     }
 }
 
+// the blocks one after the other
+__global__ void __launch_bounds__(256) embedding_grad_serial_finish_kernel(const float *__restrict__ partial, int blocks, int64_t vd, int accumulate,
+                                                                            float *__restrict__ demb) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= vd) return;
+    float t = 0.f;
+    for (int b = 0; b < blocks; b++) t += partial[(int64_t)b * vd + i];
+    demb[i] = (accumulate ? demb[i] : 0.f) + t;
+}
+
 __global__ void __launch_bounds__(256) embedding_grad_finish_kernel(const float *__restrict__ partial, int blocks, int64_t vd, int accumulate,
                                                                      float *__restrict__ demb) {
     __shared__ float s[8][32];
@@ -268,9 +278,9 @@ __global__ void __launch_bounds__(256) embedding_grad_finish_kernel(const float 
     demb[i] = (accumulate ? demb[i] : 0.f) + t;
 }
 
-int embedding_blocks(int64_t n) {
-    int64_t b = (n + 255) / 256;
-    int64_t cap = (int64_t)sm_count() * 6;
+int embedding_blocks(int64_t n, bool serial = false) {
+    int64_t b = serial ? (n + 2047) / 2048 : (n + 255) / 256;
+    int64_t cap = (int64_t)sm_count() * (serial ? 2 : 6);
     return (int)(b < 1 ? 1 : (b < cap ? b : cap));
 }
 
@@ -376,13 +386,13 @@ extern "C" int64_t agpt_b200_embedding_grad_workspace_bytes(int64_t n, int d_mod
     return (int64_t)embedding_blocks(n) * vocab * d_model * 4;
 }
 
-extern "C" int agpt_b200_embedding_grad(const float *d_grad, const int32_t *d_ids, float *d_emb_grad, int64_t n, int d_model, int vocab,
-                                        int accumulate, void *d_workspace, int64_t workspace_bytes, void *stream) {
+static int embedding_grad(const float *d_grad, const int32_t *d_ids, float *d_emb_grad, int64_t n, int d_model, int vocab, int accumulate, bool serial,
+                          void *d_workspace, int64_t workspace_bytes, void *stream) {
     if (!d_grad || !d_ids || !d_emb_grad || n < 0 || d_model <= 0 || vocab <= 0)
         return agpt_set_error(AGPT_E_ARG, "embedding_grad: bad argument");
     const size_t smem = (size_t)vocab * 128 * 4;
     if (smem > 200 * 1024) return agpt_set_error(AGPT_E_LIMIT, "embedding_grad: vocabulary of %d exceeds the shared-memory table (400 symbols)", vocab);
-    const int blocks = embedding_blocks(n);
+    const int blocks = embedding_blocks(n, serial);
     if (!d_workspace || workspace_bytes < (int64_t)blocks * vocab * d_model * 4)
         return agpt_set_error(AGPT_E_ARG, "embedding_grad: workspace too small (agpt_b200_embedding_grad_workspace_bytes)");
     cudaStream_t st = (cudaStream_t)stream;
@@ -392,8 +402,18 @@ extern "C" int agpt_b200_embedding_grad(const float *d_grad, const int32_t *d_id
         launch_embedding_grad<2>(d_grad, d_ids, n, d_model, vocab, blocks, (float *)d_workspace, st);
     else launch_embedding_grad<1>(d_grad, d_ids, n, d_model, vocab, blocks, (float *)d_workspace, st);
     const int64_t vd = (int64_t)vocab * d_model;
-    embedding_grad_finish_kernel<<<(unsigned)((vd + 31) / 32), 256, 0, st>>>((const float *)d_workspace, blocks, vd, accumulate, d_emb_grad);
+    if (serial) embedding_grad_serial_finish_kernel<<<(unsigned)((vd + 255) / 256), 256, 0, st>>>((const float *)d_workspace, blocks, vd, accumulate, d_emb_grad);
+    else embedding_grad_finish_kernel<<<(unsigned)((vd + 31) / 32), 256, 0, st>>>((const float *)d_workspace, blocks, vd, accumulate, d_emb_grad);
     return launch_status("embedding_grad");
+}
+
+extern "C" int agpt_b200_embedding_grad(const float *d_grad, const int32_t *d_ids, float *d_emb_grad, int64_t n, int d_model, int vocab,
+                                        int accumulate, void *d_workspace, int64_t workspace_bytes, void *stream) {
+    return embedding_grad(d_grad, d_ids, d_emb_grad, n, d_model, vocab, accumulate, false, d_workspace, workspace_bytes, stream);
+}
+extern "C" int agpt_b200_embedding_grad_serial(const float *d_grad, const int32_t *d_ids, float *d_emb_grad, int64_t n, int d_model, int vocab,
+                                               int accumulate, void *d_workspace, int64_t workspace_bytes, void *stream) {
+    return embedding_grad(d_grad, d_ids, d_emb_grad, n, d_model, vocab, accumulate, true, d_workspace, workspace_bytes, stream);
 }
 
 // ---- the reference's symbols (void, default stream, 32-bit sizes; errors are kept for agpt_b200_last_error) ---------

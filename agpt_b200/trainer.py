@@ -39,6 +39,7 @@ class LaunchGroup:
         self.plan = A.WalkerPlan(parent, tile, device.index if device.type == "cuda" else -1)   # a host-only plan on a CPU device (index arrays for tests)
         order = self.plan.dfs_to_node.astype(np.int64)
         assert np.array_equal(order, np.arange(self.n)), "launch groups are built in depth-first order"
+        self._even = None
         t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device)  # noqa: E731
         self.tokens = t(tokens.astype(np.int64))
         self.tokens32 = t(tokens.astype(np.int32))
@@ -77,10 +78,11 @@ class LaunchGroup:
                "unit_off": ("unit_off", "int64", lambda i: i.n_units + 1)}
 
     @classmethod
-    def from_runs(cls, runs, i, mass_mode, seq_len, device, tile=64) -> "LaunchGroup":
-        """Group i of an A.RunGroups: one device buffer, written by the library."""
+    def from_runs(cls, runs, i, mass_mode, seq_len, device, tile=64, even=False) -> "LaunchGroup":
+        """Group i of an A.RunGroups: one device buffer, written by the library.  even: its plan has even tiles."""
         self = cls.__new__(cls)
-        self._info, self._buf, self.plan = runs.upload(i, tile, mass_mode, seq_len, device)
+        self._info, self._buf, self.plan = runs.upload(i, tile, mass_mode, seq_len, device, even)
+        self._even = self.plan if even else None
         o = self._info
         self.n, self.n_units, self.n_pos, self.n_trained_rows = int(o.n), int(o.n_units), int(o.n_pos), int(o.n_trained)
         return self
@@ -100,9 +102,20 @@ class LaunchGroup:
         setattr(self, name, v)
         return v
 
-    def step_args(self):
+    def plan_for(self, bf16_store):
+        """The plan that a step on this store walks.  On a bfloat16 store that is one with even tiles, made when first asked for:
+        which value an attention weight is rounded at depends on the tile it is computed in, so another cut of the tiles is
+        another rounding of every row, and through the ReLUs of a deep model another gradient: 2e-3 after one step on some
+        thousand rows, 1e-2 after a few on ten."""
+        if not bf16_store:
+            return self.plan
+        if self._even is None:
+            self._even = A.WalkerPlan(self.plan.parent_dfs, self.plan.tile_m, self.plan.device, even=True)
+        return self._even
+
+    def step_args(self, bf16_store=False):
         """The group's part of the native step's arguments (the model fills in the rest)."""
-        a = A.TrainStepArgs(plan=self.plan._h, n=self.n, n_units=self.n_units, n_pos=self.n_pos)
+        a = A.TrainStepArgs(plan=self.plan_for(bf16_store)._h, n=self.n, n_units=self.n_units, n_pos=self.n_pos)
         o = self.__dict__.get("_info")
         if o is not None:
             at = self._buf.data_ptr()
@@ -149,15 +162,15 @@ def _embedding_function():
         symbols and millions of rows an index_put backward serialises on the collisions)."""
 
         @staticmethod
-        def forward(ctx, emb, tokens32):
+        def forward(ctx, emb, tokens32, serial=False):
             ctx.save_for_backward(tokens32)
-            ctx.vocab = emb.shape[0]
+            ctx.vocab, ctx.serial = emb.shape[0], serial
             return A.embedding_gather(emb, tokens32)
 
         @staticmethod
         def backward(ctx, grad):
             (tokens32,) = ctx.saved_tensors
-            return A.embedding_grad(grad.contiguous(), tokens32, ctx.vocab), None
+            return A.embedding_grad(grad.contiguous(), tokens32, ctx.vocab, serial=ctx.serial), None, None
 
     return TokenEmbedding
 
@@ -290,7 +303,8 @@ def _attention_function():
             q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
             A.rope_pair_(q, k, group.pos, cos, sin, n_heads)
             ks, vs = (A.kv_store_write_bf16(k), A.kv_store_write_bf16(v)) if bf16_store else (k, v)
-            out, lse = A.attn_forward(group.plan, q, ks, vs, n_heads)
+            ctx.plan = group.plan_for(bf16_store)
+            out, lse = A.attn_forward(ctx.plan, q, ks, vs, n_heads)
             ctx.save_for_backward(q, ks, vs, out, lse)
             ctx.group, ctx.cos, ctx.sin, ctx.n_heads, ctx.grad_mode = group, cos, sin, n_heads, grad_mode
             return out
@@ -298,7 +312,7 @@ def _attention_function():
         @staticmethod
         def backward(ctx, dout):
             q, ks, vs, out, lse = ctx.saved_tensors
-            dq, dk, dv = A.attn_backward(ctx.group.plan, q, ks, vs, out, lse, dout.contiguous(), ctx.n_heads,
+            dq, dk, dv = A.attn_backward(ctx.plan, q, ks, vs, out, lse, dout.contiguous(), ctx.n_heads,
                                          grad_mode=ctx.grad_mode, edge_first=ctx.group.edge_first)
             A.rope_pair_(dq, dk, ctx.group.pos, ctx.cos, ctx.sin, ctx.n_heads, inverse=True)
             return dq, dk, dv, None, None, None, None, None, None
@@ -380,7 +394,7 @@ class TrieWalkModel:
             return lin(lin(ln(x, g2, b2), w1, b1, relu=True), w2, bo, residual=x)
 
         fused = self.dense_impl == "tensor" and m.d_model % 4 == 0 and m.d_ff % 4 == 0
-        x = self.embed.apply(P["token_emb"], group.tokens32)
+        x = self.embed.apply(P["token_emb"], group.tokens32, bf16_store)
         for l in range(m.n_layers):
             g = lambda n: P[f"layer{l}.{n}"]  # noqa: E731
             if fused:
@@ -419,13 +433,13 @@ class TrieWalkModel:
         return self.dense_impl == "tensor" and bool(A.lib().agpt_b200_train_step_takes(m.d_model, m.n_heads, m.d_ff, m.vocab))
 
     def group_step(self, group: LaunchGroup, counts, entropy_lambda=0.0, intermediate_weight=1.0, ce_only=False,
-                   bf16_store=False, sync=True):
+                   bf16_store=False, sync=True, tape=False):
         """Forward, loss and backward of one launch group; gradients accumulate into .grad.
         Returns (sum of positive per-query losses, number of such queries): Python numbers, or with sync=False a
         float32 device tensor (loss sum, count // 4096, count % 4096), so that the host does not wait for the device
-        between groups."""
+        between groups.  tape: step by single operations even where the native step takes the model."""
         import torch
-        if self.native_step_available():
+        if not tape and self.native_step_available():
             return self._native_step(group, counts, entropy_lambda, intermediate_weight, ce_only, bf16_store, sync)
         logits = self.logits(group, bf16_store).contiguous()
         c_off, c_tok, c_val = counts
@@ -477,7 +491,7 @@ class TrieWalkModel:
             if c.dtype != torch.int32 or not c.is_cuda or not c.is_contiguous():
                 raise A.AgptError("counts must be contiguous int32 CUDA tensors")
         m, out = self.cfg, torch.empty(8, dtype=torch.float32, device=self.device)
-        a = group.step_args()
+        a = group.step_args(bf16_store)
         a.d_model, a.n_heads, a.n_layers, a.d_ff, a.vocab, a.seq_len = m.d_model, m.n_heads, m.n_layers, m.d_ff, m.vocab, m.seq_len
         a.params, a.grads = C.addressof(self._step_ptrs[1]), C.addressof(self._step_ptrs[2])
         a.counts_offset, a.counts_tok, a.counts_val = [c.data_ptr() for c in counts]
@@ -519,15 +533,16 @@ class SampleSpace:
         self.plan = A.WalkerPlan(self.parent, 64, -1)
         return self.__dict__[name]
 
-    def group(self, node_ids, context_ids, mass_mode, seq_len, device, tile=64) -> LaunchGroup:
+    def group(self, node_ids, context_ids, mass_mode, seq_len, device, tile=64, even=False) -> LaunchGroup:
         """Launch group of the chars of the radix nodes node_ids (closed under "parent"); chars of context_ids are
         attended but carry no loss and are left out of the mass-weight mean.  The lightning samplers pass no context:
         in the reference the ancestors prepended to a sampled subtree are trained like every other position and counted
         in the chunk's mass mean (src/cuda/agpt_train.cu:4601-4637; the ancestor count recorded at :4194 is never read,
-        and the comment at :4160-4180 that announces a masking describes a variant that was taken out again)."""
+        and the comment at :4160-4180 that announces a masking describes a variant that was taken out again).
+        even: the group is for steps on a bfloat16 store (LaunchGroup.plan_for)."""
         t = self.trie
         if device.type == "cuda" and self.rank is not None:
-            return LaunchGroup.from_runs(A.RunGroups.of_sample(t, self.rank, node_ids, context_ids), 0, mass_mode, seq_len, device, tile)
+            return LaunchGroup.from_runs(A.RunGroups.of_sample(t, self.rank, node_ids, context_ids), 0, mass_mode, seq_len, device, tile, even)
         node_ids = np.asarray(node_ids, np.int64)
         lens = t.edge_len[node_ids].astype(np.int64)
         starts = t.edge_start[node_ids].astype(np.int64)
@@ -565,17 +580,21 @@ def train_lightning_epoch(model: TrieWalkModel, space: SampleSpace, counts, opt,
     model.bind_grads()
     loss_sum, n_q, n_nodes = 0.0, 0, 0
     pending = []                         # statistics of native steps, read once at the end so that the host never waits between steps
-    native = model.native_step_available()
+    # Steps on a bfloat16 store run by single operations.  A unit of ten rows has nothing to average over: a float32 sum in another
+    # order rounds some K or V row to the other bfloat16 neighbour, a ReLU or two change sides, and after the next optimizer steps
+    # the momentum of a model of eight layers is another by 1e-2.  The order of these operations is what a seed stands for there.
+    bf16 = bool(loss_kw.get("bf16_store"))
+    native = model.native_step_available() and not bf16
     for s in range(steps):
         ids = nodes[off[s]:off[s + 1]]
         # every sampled row is trained, the ancestors the sampler prepends included (src/cuda/agpt_train.cu:4601-4607)
-        g = space.group(ids, [], mass_mode, model.cfg.seq_len, model.device)
+        g = space.group(ids, [], mass_mode, model.cfg.seq_len, model.device, even=bf16)
         opt.zero_grad(set_to_none=False)
         ls, nq = 0.0, 0
         if native:
             pending.append(model.group_step(g, counts, sync=None, **loss_kw))
         else:
-            ls, nq = model.group_step(g, counts, **loss_kw)
+            ls, nq = model.group_step(g, counts, tape=True, **loss_kw)
         if hasattr(opt, "lr_scale"):
             opt.lr_scale = float(lr_w[s])
         opt.step()

@@ -229,6 +229,9 @@ typedef struct {
  * (src/cuda/agpt_train.cu:3602-3736).  parent[i] is a node id or -1; any id order is accepted.
  * With device >= 0 the index arrays are also allocated on that device (freed by plan_destroy). */
 int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_m, int device, agpt_plan **out);
+/* The same with even tiles: each ends after tile_m rows, and attention over the plan takes the chunked kernels in both directions
+ * whatever agpt_b200_set_attn_variant says (what the trainer's steps on a bfloat16 store run on). */
+int agpt_b200_plan_create_even(const int32_t *parent, int64_t n, int tile_m, int device, agpt_plan **out);
 int agpt_b200_plan_info(const agpt_plan *p, agpt_plan_info *out);
 /* The sizes alone (array pointers NULL): the row arrays of a plan that came from runs of rows are derived when asked for. */
 int agpt_b200_plan_sizes(const agpt_plan *p, agpt_plan_info *out);
@@ -294,6 +297,8 @@ int64_t agpt_b200_trie_groups_count(const agpt_run_groups *g);
 int agpt_b200_trie_group_prepare(agpt_run_groups *g, int64_t i, int tile_m, int mass_mode, int seq_len, agpt_run_group_info *out);
 int agpt_b200_trie_group_upload(agpt_run_groups *g, int device, void *d_buffer, void *stream, agpt_plan **plan_out);
 void agpt_b200_trie_groups_free(agpt_run_groups *g);
+/* even != 0: the plans of groups prepared from here on have even tiles (agpt_b200_plan_create_even). */
+int agpt_b200_trie_groups_even(agpt_run_groups *g, int even);
 
 /* ---- device kernels (all asynchronous on `stream`, a cudaStream_t passed as void*) ---- */
 
@@ -358,7 +363,9 @@ void cuda_embedding_scatter_add(const float *grad, const int *ids, float *d_toke
  * col_sum: d_out[c] = (accumulate ? d_out[c] : 0) + scale * sum_r g[r][c], the bias gradient; with d_act != NULL the
  * gradient is first masked by d_act > 0 and the masked gradient written to d_grad_out (may alias d_grad): ReLU
  * backward and the bias gradient of the layer below it in one pass.  embedding_grad: the gradient of the embedding
- * table from per-block partial tables added in a fixed order (vocab up to 400).  Both reductions repeat bit for bit. */
+ * table from per-block partial tables added in a fixed order (vocab up to 400).  Both reductions repeat bit for bit.
+ * embedding_grad_serial: the same with one block per 2048 rows (more rows where that is over two blocks per SM), the blocks added one
+ * after the other; the same workspace. */
 int agpt_b200_bias_act(const float *d_in, const float *d_bias, float *d_out, float *d_mask, int64_t rows, int cols,
                        int relu, void *stream);
 int agpt_b200_relu_bwd(const float *d_grad, const float *d_mask, float *d_out, int64_t n, void *stream);
@@ -371,6 +378,8 @@ int agpt_b200_embedding_gather(const float *d_emb, const int32_t *d_ids, float *
                                int vocab, void *stream);
 int agpt_b200_embedding_grad(const float *d_grad, const int32_t *d_ids, float *d_emb_grad, int64_t n, int d_model,
                              int vocab, int accumulate, void *d_workspace, int64_t workspace_bytes, void *stream);
+int agpt_b200_embedding_grad_serial(const float *d_grad, const int32_t *d_ids, float *d_emb_grad, int64_t n, int d_model,
+                                    int vocab, int accumulate, void *d_workspace, int64_t workspace_bytes, void *stream);
 int64_t agpt_b200_embedding_grad_workspace_bytes(int64_t n, int d_model, int vocab);
 
 /* Replace the optimizer kernels of the reference's kernel dependency (declared src/cuda/agpt_train.cu:64-72;
