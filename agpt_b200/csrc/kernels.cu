@@ -2046,11 +2046,9 @@ extern "C" int agpt_b200_set_attn_impl(int impl) {
     return AGPT_OK;
 }
 
-// Whole-tile kernels (forward and backward; float32 store, head_dim 32): chosen when four blocks of the backward
-// fit one SM (228 KB of shared memory, 1 KB reserved per block), i.e. up to about 150 keys per tile; deeper plans take
-// the chunked kernels.  AGPT_B200_ATTN_TILE=0 keeps the chunked kernels (A/B runs); AGPT_B200_BWD_WARPS = 4, 6 or 8
-// warps per block of the backward.
-// head_dim 32: four blocks of the backward per SM; head_dim 64 (rows twice as long, twice the registers): two
+// Whole-tile kernels, both directions and both stores, wherever the largest tile's keys leave the wanted number of blocks per SM
+// (bwd_tile_fits, fwd_tile_fits, fwd_dispatch); deeper plans and even ones take the chunked kernels.  AGPT_B200_ATTN_TILE=0 keeps the chunked
+// kernels (a bfloat16 store's forward asks AGPT_B200_ATTN_TILE_BF16=0 alone, which keeps them for that store; A/B runs); AGPT_B200_BWD_WARPS = 3, 4, 6 or 8 (agpt_b200_set_attn_variant).
 static int g_bwd_tile = -1, g_bwd_warps = 0;
 static int bwd_tile_enabled() {
     if (g_bwd_tile < 0) {
@@ -2064,12 +2062,18 @@ static int bwd_tile_enabled() {
 }
 extern "C" int agpt_b200_set_attn_variant(int whole_tile, int warps) {
     if ((whole_tile != 0 && whole_tile != 1) || (warps != 3 && warps != 4 && warps != 6 && warps != 8))
-        return agpt_set_error(AGPT_E_ARG, "set_attn_variant: whole_tile 0 or 1, bwd_warps 4, 6 or 8");
+        return agpt_set_error(AGPT_E_ARG, "set_attn_variant: whole_tile 0 or 1, bwd_warps 3, 4, 6 or 8");
     bwd_tile_enabled();
     g_bwd_tile = whole_tile; g_bwd_warps = warps;
     return AGPT_OK;
 }
-static bool tile_kernels_wanted(const agpt_plan *p) { return bwd_tile_enabled() && !p->even; }
+static bool tile_bf16_enabled() {
+    static const bool on = [] { const char *e = getenv("AGPT_B200_ATTN_TILE_BF16"); return !(e && e[0] == '0'); }();
+    return on;
+}
+static bool tile_kernels_wanted(const agpt_plan *p, int kv_dtype) {
+    return bwd_tile_enabled() && !p->even && (kv_dtype != AGPT_KV_BF16 || tile_bf16_enabled());
+}
 // every head of every row of these buffers starts on a 32-byte boundary
 static bool rows_wide(int D, const void *a, const void *b, const void *c, const void *d, const void *e) {
     return D % 8 == 0 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)e) & 31) == 0;
@@ -2126,15 +2130,18 @@ static int launch_fwd_mma(const agpt_plan *p, const float *q, const void *k, con
 
 static int fwd_dispatch(const agpt_plan *p, const float *q, const void *k, const void *v, int kv_dtype, float *out,
                         float *lse, int H, int head_dim, float scale, cudaStream_t st, int tile0, int ntiles) {
-    if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_F32 && tile_kernels_wanted(p) && fwd_tile_fits(p, head_dim)) {
+    if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_F32 && tile_kernels_wanted(p, kv_dtype) && fwd_tile_fits(p, head_dim)) {
+        // head_dim 32: AGPT_B200_FWD_BLOCKS=5 for five blocks per SM instead of six (A/B runs)
+        static const bool five = [] { const char *e = getenv("AGPT_B200_FWD_BLOCKS"); return e && atoi(e) == 5; }();
         switch (head_dim) {
             case 16: return launch_fwd_tile<16, 8>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
-            case 32: return launch_fwd_tile<32, 6>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            case 32: return five ? launch_fwd_tile<32, 5>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles)
+                                 : launch_fwd_tile<32, 6>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
             case 64: return launch_fwd_tile<64, 3>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
         }
     }
     // bfloat16 store: whole tiles while two blocks of them fit one SM (head_dim 64: up to 438 keys), deeper plans in chunks
-    if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_BF16 && !p->even &&
+    if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_BF16 && !p->even && tile_bf16_enabled() &&
         fwd_bf16_smem_bytes(head_dim, bwd_tile_maxk(p)) <= (size_t)113 * 1024) {
         switch (head_dim) {
             case 16: return launch_fwd_bf16<16, 8>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
@@ -2211,7 +2218,7 @@ static int launch_bwd_tile_w(const agpt_plan *p, const float *q, const void *k, 
 static int bwd_dispatch(const agpt_plan *p, const float *q, const void *k, const void *v, int kv_dtype, const float *o,
                         const float *lse, const float *dout, float *dq, float *dk, float *dv, float *pk, float *pv, int H,
                         int head_dim, float scale, cudaStream_t st, int tile0, int ntiles, BwdMask gmask = BwdMask{AGPT_GRAD_FULL, nullptr}) {
-    if (attn_impl() == 1 && p->tile_m == 64 && tile_kernels_wanted(p) && bwd_tile_fits(p, head_dim, kv_dtype == AGPT_KV_BF16))
+    if (attn_impl() == 1 && p->tile_m == 64 && tile_kernels_wanted(p, kv_dtype) && bwd_tile_fits(p, head_dim, kv_dtype == AGPT_KV_BF16))
         return launch_bwd_tile_w(p, q, k, v, kv_dtype, o, lse, dout, dq, dk, dv, pk, pv, H, head_dim, scale, st, tile0, ntiles, gmask);
     if (attn_impl() == 1 && p->tile_m == 64 && p->max_keys <= MAXKEYS) {
         const bool bf = kv_dtype == AGPT_KV_BF16;

@@ -470,19 +470,19 @@ int agpt_b200_attn_bwd_mode(const agpt_plan *p, const float *d_q, const void *d_
  * exists for A/B measurement.  Also read once from the environment variable AGPT_B200_ATTN_IMPL. */
 int agpt_b200_set_attn_impl(int impl);
 
-/* Selects between the two tensor-core kernel pairs for a float32 KV store and head_dim 32 or 64.  whole_tile 1
- * (default): forward and backward keep the tile's Q (and dO) rows and all its key rows in shared memory, converted
- * once to split half precision (x * 2^e = hi + lo, fp16 each, e per tile, head and tensor; three m16n8k16 products
- * give the accuracy of three TF32 products), every fragment one ldmatrix, and the backward's warps run independent
- * row and key items with no barrier in their loops.  Used whenever four (head_dim 32) or two (head_dim 64) blocks
- * of the backward fit one SM, i.e. up to about 150 / 128 keys per tile (depth <= ~90 / 65); deeper plans and head_dim 16
- * take the chunked TF32 kernels, and so does the head_dim-64 forward (the chunked one measured faster there).  With a
- * bf16 store the whole-tile backward runs at head_dim 32 (single fp16 products: the store's own rounding is coarser;
- * AGPT_B200_ATTN_TILE_BF16=0 in the environment keeps the chunked kernel), everything else chunked.  whole_tile 0:
- * always the chunked kernels.  bwd_warps = 4 (default), 6 or 8 warps per block of the whole-tile backward, 3 = four
- * warps with three blocks per SM.  Same results within the parity tolerance either way; the switch exists for A/B
- * measurement.  Also read once from AGPT_B200_ATTN_TILE and AGPT_B200_BWD_WARPS; AGPT_B200_FWD_BLOCKS=5 runs the
- * head_dim-32 forward with five blocks per SM instead of six. */
+/* Selects between the two tensor-core kernel pairs.  whole_tile 1 (default): a block keeps its tile's Q (and dO) rows and all
+ * its key rows in shared memory.  Float32 store, head_dim 16, 32 or 64: rows are converted once to split half precision
+ * (x * 2^e = hi + lo, fp16 each, e per tile, head and tensor; three m16n8k16 products give the accuracy of three TF32
+ * products), every fragment is one ldmatrix.  Bfloat16 store: the forward feeds K and V to the tensor cores as they are
+ * stored and splits Q and P into two bfloat16 parts (16 bits); the backward is the split-half kernel with K and V of one
+ * exact half and Q, dO, P and dS of two.  A direction takes these kernels while the keys of the plan's largest tile leave
+ * room for the blocks per SM it wants; plans with more, and plans with even tiles, take the chunked kernels (float32 store:
+ * three TF32 products; bfloat16 store: one, 11 bits per factor), each direction by itself.  whole_tile 0: the chunked
+ * kernels, but for the forward of a bfloat16 store, which is one kernel under either value.  bwd_warps = 4 (default), 6 or 8 warps per block of the float32 whole-tile backward of head_dim 32 and 64
+ * (64: 6 counts as 8), 3 = four warps with three blocks per SM (head_dim 32).  Same results within the parity tolerance
+ * either way; the switch exists for A/B measurement.  Also read once from the environment: AGPT_B200_ATTN_TILE and
+ * AGPT_B200_BWD_WARPS; AGPT_B200_ATTN_TILE_BF16=0 keeps the chunked kernels for a bfloat16 store, in both directions;
+ * AGPT_B200_FWD_BLOCKS=5 runs the head_dim-32 forward of a float32 store with five blocks per SM instead of six. */
 int agpt_b200_set_attn_variant(int whole_tile, int bwd_warps);
 
 /* No counterpart in the reference.  agpt_b200_attn_bwd for callers that cannot allocate device memory
