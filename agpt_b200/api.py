@@ -81,12 +81,13 @@ class _TrieArray:
 
     def __init__(self, memory, address, n, dtype):
         self._memory = memory
-        self.__array_interface__ = dict(version=3, shape=(n,), typestr=np.dtype(dtype).str, data=(address, False))
+        self.__array_interface__ = dict(version=3, shape=(n,), typestr=np.dtype(dtype).str, data=(address, True))
 
 
 class RadixTrie:
     """Radix trie with the reference's node numbering, counts, edge mass and char positions.  The arrays are the native
-    trie's own memory (a copy of 1.7M edge characters and 92,000 nodes took 3 ms, much of it first touches) and outlive close()."""
+    trie's own memory (a copy of 1.7M edge characters and 92,000 nodes took 3 ms, much of it first touches), read-only, as every native call
+    on the trie reads the same memory, and outlive close(); copy one to change it."""
 
     def __init__(self, handle):
         self._h = handle

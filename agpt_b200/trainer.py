@@ -737,7 +737,7 @@ def main(argv=None):
         groups, total = build_groups(trie, rank, world, args.group_rows, args.mass_weight, mf.seq_len, dev,
                                      level=args.partition_depth or None)
     rng_state = args.lightning_seed
-    counts = [torch.from_numpy(np.ascontiguousarray(c)).to(dev) for c in (trie.cnt_off.astype(np.int32), trie.cnt_tok, trie.cnt_val)]
+    counts = [torch.tensor(c, dtype=torch.int32, device=dev) for c in (trie.cnt_off, trie.cnt_tok, trie.cnt_val)]
     model = TrieWalkModel(mf, dev)
     model.ffn_recompute = args.ffn_recompute
     model.grad_mode = args.grad_mode

@@ -1,4 +1,4 @@
-"""The arrays of a RadixTrie are the native trie's own memory: they outlive close() and the RadixTrie, below and above the
+"""The arrays of a RadixTrie are the native trie's own memory, read-only: they outlive close() and the RadixTrie, below and above the
 size from which they lie in huge pages (262,144 characters)."""
 import gc
 
@@ -33,3 +33,18 @@ def test_arrays_outlive_the_trie(chars):
     other = A.RadixTrie.build(corpus, depth)
     for n in NAMES:
         assert np.array_equal(got[n], getattr(other, n)), n
+
+
+def test_arrays_are_read_only():
+    """Writing into one would change what the native calls on the trie see."""
+    corpus = A.synth_markov_corpus(300, 12, 2)
+    trie = A.RadixTrie.build(corpus, 6)
+    for n in NAMES:
+        a = getattr(trie, n)
+        with pytest.raises(ValueError):
+            a[0] = 7
+        with pytest.raises(ValueError):
+            a.setflags(write=True)
+        b = a.copy()
+        b[0] = 7                                        # a copy is the caller's
+    assert np.array_equal(trie.edge_mass, A.RadixTrie.build(corpus, 6).edge_mass)
