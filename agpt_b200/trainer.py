@@ -342,8 +342,7 @@ class TrieWalkModel:
             p = self.flat[o:o + a.size].view(a.shape)
             p.copy_(torch.from_numpy(np.ascontiguousarray(a)))
             self.params[name] = p.requires_grad_(True)
-        self._offs = offs
-        self._step_ptrs = None           # pointer arrays of the native step, rebuilt when a gradient buffer is replaced
+        self._offs, self._shapes = offs, [torch.Size(a.shape) for _, a in model.mats]
         self.bind_grads()
         hd = model.d_model // model.n_heads
         cos, sin = A.rope_table(model.seq_len, hd)
@@ -432,6 +431,18 @@ class TrieWalkModel:
         m = self.cfg
         return self.dense_impl == "tensor" and bool(A.lib().agpt_b200_train_step_takes(m.d_model, m.n_heads, m.d_ff, m.vocab))
 
+    def _step_tensors_plain(self) -> bool:
+        """The native step reads parameters and adds to gradients by address: float32, contiguous, of the model file's shape and on
+        the model's device.  Anything else steps on the tape, which reads the tensors themselves."""
+        import torch
+        index, plain = self.flat.get_device(), True
+        for p, shape in zip(self.params.values(), self._shapes):
+            if p.grad is None:
+                p.grad = torch.zeros_like(p)
+            for t in (p, p.grad):
+                plain = plain and t.dtype is torch.float32 and t.get_device() == index and t.shape == shape and t.is_contiguous()
+        return plain
+
     def group_step(self, group: LaunchGroup, counts, entropy_lambda=0.0, intermediate_weight=1.0, ce_only=False,
                    bf16_store=False, sync=True, tape=False):
         """Forward, loss and backward of one launch group; gradients accumulate into .grad.
@@ -439,7 +450,7 @@ class TrieWalkModel:
         float32 device tensor (loss sum, count // 4096, count % 4096), so that the host does not wait for the device
         between groups.  tape: step by single operations even where the native step takes the model."""
         import torch
-        if not tape and self.native_step_available():
+        if not tape and self.native_step_available() and self._step_tensors_plain():
             return self._native_step(group, counts, entropy_lambda, intermediate_weight, ce_only, bf16_store, sync)
         logits = self.logits(group, bf16_store).contiguous()
         c_off, c_tok, c_val = counts
@@ -466,6 +477,9 @@ class TrieWalkModel:
         logits.backward(dlogits * scale[group.unit_of_row][:, None])
         if sync:
             return float(loss_sum.item()), int(n_trained.item())
+        if sync is None:                             # laid out as the native step leaves them
+            return torch.cat([loss_sum.reshape(1).view(torch.float32), n_trained.reshape(1).view(torch.float32), torch.zeros_like(loss_sum.reshape(1)).view(torch.float32),
+                              torch.zeros_like(loss_sum.reshape(1)).view(torch.float32)])
         # the count rides in float32 next to the gradients: split so that sums over groups and ranks stay exact
         return torch.stack([loss_sum.to(torch.float32), (n_trained // 4096).to(torch.float32), (n_trained % 4096).to(torch.float32)])
 
@@ -475,25 +489,17 @@ class TrieWalkModel:
         import ctypes as C
 
         import torch
-        grads = []
-        for p in self.params.values():
-            if p.grad is None:
-                p.grad = torch.zeros_like(p)
-            grads.append(p.grad)
-        if self._step_ptrs is None or any(a is not b for a, b in zip(grads, self._step_ptrs[0])):
-            for g, p in zip(grads, self.params.values()):
-                if g.dtype != torch.float32 or not g.is_contiguous() or g.shape != p.shape or g.device != p.device:
-                    raise A.AgptError("gradients must be contiguous float32 tensors on the device of their parameter")
-            n = len(grads)
-            self._step_ptrs = (grads, (C.c_void_p * n)(*[p.data_ptr() for p in self.params.values()]),
-                               (C.c_void_p * n)(*[g.data_ptr() for g in grads]))
+        n = len(self.params)
+        # addresses are those of this call: the storage of a parameter or a gradient may be another than at the last step
+        params = (C.c_void_p * n)(*[p.data_ptr() for p in self.params.values()])
+        grads = (C.c_void_p * n)(*[p.grad.data_ptr() for p in self.params.values()])
         for c in counts:
             if c.dtype != torch.int32 or not c.is_cuda or not c.is_contiguous():
                 raise A.AgptError("counts must be contiguous int32 CUDA tensors")
         m, out = self.cfg, torch.empty(8, dtype=torch.float32, device=self.device)
         a = group.step_args(bf16_store)
         a.d_model, a.n_heads, a.n_layers, a.d_ff, a.vocab, a.seq_len = m.d_model, m.n_heads, m.n_layers, m.d_ff, m.vocab, m.seq_len
-        a.params, a.grads = C.addressof(self._step_ptrs[1]), C.addressof(self._step_ptrs[2])
+        a.params, a.grads = C.addressof(params), C.addressof(grads)
         a.counts_offset, a.counts_tok, a.counts_val = [c.data_ptr() for c in counts]
         a.cosv, a.sinv = self.cos.data_ptr(), self.sin.data_ptr()
         a.entropy_lambda, a.intermediate_weight, a.ce_only = entropy_lambda, intermediate_weight, int(ce_only)
