@@ -798,6 +798,12 @@ def device_status() -> int:
     return int(out.value)
 
 
+def device_status_add(out) -> None:
+    """Add the status word to a one-element float32 CUDA tensor, in stream order."""
+    _chk_f32(out, "out")
+    check(lib().agpt_b200_device_status_add(_dp(out), _stream()), "device_status_add")
+
+
 def set_gemm_impl(impl: int) -> None:
     """0: mma.sync with three TF32 products; 1 (default): tcgen05 on bfloat16 splits."""
     check(lib().agpt_b200_set_gemm_impl(impl), "set_gemm_impl")

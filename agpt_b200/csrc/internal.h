@@ -127,6 +127,7 @@ inline int64_t agpt_tile_cost(int32_t d, int64_t k) { return 10 * (int64_t)d + 9
 int agpt_mass_weights_per_node(const int32_t *edge_mass, const int32_t *edge_len, const int32_t *unit_of_node, const uint8_t *counted,
                                int64_t n_nodes, int64_t n_units, int mode, float *out_per_node);
 int agpt_step_gemm_status(int *out);       // status word of step_gemm.cu's kernels
+int agpt_step_gemm_status_word(const int **d_word);      // and its place on the current device
 
 // tcgen05 float32 GEMM (gemm_sm100.cu): D[l] = act(alpha * op(A[l]) * op(B[l]) + beta * C + bias row), l < L batches
 bool agpt_gemm_sm100_takes(int trans_a, int trans_b, int relu, int has_source);

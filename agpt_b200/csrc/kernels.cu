@@ -2874,6 +2874,15 @@ extern "C" int agpt_b200_device_status(int32_t *status_out) {
     return AGPT_OK;
 }
 
+__global__ void device_status_kernel(const int *__restrict__ step_word, float *out) { *out += (float)(g_device_status | *step_word); }
+extern "C" int agpt_b200_device_status_add(float *d_out, void *stream) {
+    if (!d_out) return agpt_set_error(AGPT_E_ARG, "device_status_add: null output");
+    const int *step_word = nullptr;
+    if (int rc = agpt_step_gemm_status_word(&step_word)) return rc;
+    device_status_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(step_word, d_out);
+    return launch_status("device_status_add");
+}
+
 extern "C" int agpt_b200_loss_per_query(const float *d_logits, const int32_t *d_query_to_node, const int32_t *d_query_offsets,
                                         const int32_t *d_radix_ids, const int32_t *d_token_ids, const int32_t *d_counts_offset,
                                         const int32_t *d_counts_tok, const int32_t *d_counts_val, const float *d_mass_weights,

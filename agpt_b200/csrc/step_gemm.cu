@@ -693,6 +693,11 @@ int agpt_split_weights(const WeightSplitJob *jobs, int n_jobs, cudaStream_t st) 
     return AGPT_OK;
 }
 
+int agpt_step_gemm_status_word(const int **d_word) {
+    cudaError_t e = cudaGetSymbolAddress((void **)d_word, g_step_status);
+    if (e != cudaSuccess) return agpt_set_error(AGPT_E_CUDA, "device_status: %s", cudaGetErrorString(e));
+    return AGPT_OK;
+}
 int agpt_step_gemm_status(int *out) {
     cudaError_t e = cudaMemcpyFromSymbol(out, g_step_status, sizeof(int));
     if (e != cudaSuccess) return agpt_set_error(AGPT_E_CUDA, "device_status: %s", cudaGetErrorString(e));

@@ -328,7 +328,7 @@ class TrieWalkModel:
         self.cfg = model
         self.device = device
         # one flat weight buffer and one flat gradient buffer (the reference's d_weights / d_grads), each matrix on a
-        # 16-byte boundary; the gradient buffer ends with the epoch's loss sum and query count (three floats) so that
+        # 16-byte boundary; the gradient buffer ends with the epoch's loss sum and query count (three floats) and the device status so that
         # one all-reduce carries everything
         offs, off = [], 0
         for _, a in model.mats:
@@ -523,6 +523,13 @@ def _step_stats(host):
     return list(zip(host[:, :2].contiguous().view(torch.float64).flatten().tolist(), host[:, 2:4].contiguous().view(torch.int64).flatten().tolist()))
 
 
+def _check_device_status(word):
+    """word: the device status that was read with an epoch's statistics (summed over ranks)."""
+    if word:
+        raise A.AgptError(f"a kernel of this epoch gave up waiting for a copy and left rows unwritten (device status {int(word)}): "
+                          "gradients and the update made from them are incomplete")
+
+
 class SampleSpace:
     """What building the launch group of a sampled node set needs: the char tree of the whole trie in depth-first order."""
 
@@ -580,7 +587,9 @@ def lightning_lr_weights(masses, mode: str) -> np.ndarray:
 def train_lightning_epoch(model: TrieWalkModel, space: SampleSpace, counts, opt, sampler: int, steps: int, rng_state: int,
                           mass_mode="off", p_stop=0.3, max_mass=0, mass_lr="off", **loss_kw):
     """One super-epoch of the reference's lightning mode: `steps` sampled units, each its own gradient and optimizer step
-    (src/cuda/agpt_train.cu:152-157).  Returns (loss sum, queries, nodes trained, new generator state)."""
+    (src/cuda/agpt_train.cu:152-157).  Returns (loss sum, queries, nodes trained, new generator state); raises AgptError when the
+    device status word is set at the end."""
+    import torch
     rs, na, off, masses, nodes, rng_state = space.trie.lightning_sample(sampler, steps, rng_state, p_stop, max_mass)
     lr_w = lightning_lr_weights(masses, mass_lr)
     model.bind_grads()
@@ -607,11 +616,14 @@ def train_lightning_epoch(model: TrieWalkModel, space: SampleSpace, counts, opt,
         loss_sum += ls
         n_q += nq
         n_nodes += int(ids.size)
-    if pending:
-        import torch
-        for ls, nq in _step_stats(torch.stack(pending).cpu()):
-            loss_sum += ls
-            n_q += nq
+    status = torch.zeros(8, dtype=torch.float32, device=model.device)        # a row of its own behind the steps' statistics
+    if model.device.type == "cuda":
+        A.device_status_add(status[:1])
+    host = torch.stack(pending + [status]).cpu()
+    _check_device_status(float(host[-1, 0]))
+    for ls, nq in _step_stats(host[:-1]):
+        loss_sum += ls
+        n_q += nq
     return loss_sum, n_q, n_nodes, rng_state
 
 
@@ -668,20 +680,24 @@ def make_optimizer(name, model, lr, rmsprop_beta=0.999, adam_betas=(0.9, 0.999),
 def train_epoch(model: TrieWalkModel, groups, counts, opt, accumulate=True, world=1, **loss_kw):
     """One sweep over every position of this rank's groups.  accumulate=True: gradients of all groups (and all
     ranks) are summed and one optimizer step closes the epoch; False: one step per group (single rank only).
-    The loss sum and query count ride at the end of the flat gradient buffer: one all-reduce, one host read."""
+    The loss sum, query count and device status word ride at the end of the flat gradient buffer: one all-reduce, one host read.
+    Raises AgptError on every rank when a kernel of any of them gave up waiting."""
     import torch.distributed as dist
     model.bind_grads()
     opt.zero_grad(set_to_none=False)
-    tail = model.flat_grad[model.n_flat:model.n_flat + 3]
+    tail = model.flat_grad[model.n_flat:model.n_flat + 4]
     for g in groups:
-        tail += model.group_step(g, counts, sync=False, **loss_kw)
+        tail[:3] += model.group_step(g, counts, sync=False, **loss_kw)
         if not accumulate:
             opt.step()                       # clears the parameter gradients, not the two statistics behind them
+    if model.device.type == "cuda":
+        A.device_status_add(tail[3:])
     if accumulate:
         if world > 1:
             dist.all_reduce(model.flat_grad)
         opt.step()
     stats = tail.cpu()
+    _check_device_status(float(stats[3]))
     return float(stats[0]), int(round(float(stats[1]))) * 4096 + int(round(float(stats[2])))
 
 

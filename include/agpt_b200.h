@@ -507,6 +507,8 @@ int64_t agpt_b200_static_scratch_bytes(void);
  * Bit 0: a bounded wait for a bulk asynchronous copy in the loss kernel ran out; the affected rows were not
  * written.  Bit 1: the same for a wait in the training step's projections.  Kernels never trap; this word is how a failure on the device reaches the host. */
 int agpt_b200_device_status(int32_t *status_out);
+/* The same without a host wait: the word as it is when the stream gets there is added to *d_out. */
+int agpt_b200_device_status_add(float *d_out, void *stream);
 
 /* Replaces agpt_loss_per_query_kernel (src/cuda/agpt_train.cu:2069-2216).  Same arguments. */
 int agpt_b200_loss_per_query(const float *d_logits, const int32_t *d_query_to_node,
