@@ -24,6 +24,7 @@ struct RunGroup {
     std::vector<uint8_t> trained;
     int32_t n_units = 0;
     int64_t rows() const { return qoff.empty() ? 0 : qoff.back(); }
+    bool full(const agpt_trie *t, int32_t r) const { return rows() + t->edge_len[r] >= (1LL << 31) - 256; }      // ask before add
     int32_t add(const agpt_trie *t, int32_t r, int32_t parent, int32_t u, bool tr) {
         if (qoff.empty()) qoff.push_back(0);
         rid.push_back(r); prun.push_back(parent); unit.push_back(u); trained.push_back(tr);
@@ -122,7 +123,7 @@ struct agpt_run_groups {
 };
 
 extern "C" int agpt_b200_trie_groups_create(const agpt_trie *t, int level, int64_t unit_cap, int n_ranks, int rank, int64_t group_rows,
-                                            agpt_run_groups **out) {
+                                            agpt_run_groups **out) try {
     if (!t || !out || (level != 1 && level != 2) || n_ranks < 1 || rank < 0 || rank >= n_ranks || group_rows < 1)
         return agpt_set_error(AGPT_E_ARG, "trie_groups: bad argument");
     RadixOrder o;
@@ -164,7 +165,7 @@ extern "C" int agpt_b200_trie_groups_create(const agpt_trie *t, int level, int64
     std::vector<int32_t> owner(units.size(), 0);
     if (int rc = agpt_b200_partition_lpt(weight.data(), (int64_t)units.size(), n_ranks, owner.data())) return rc;
 
-    auto *G = new agpt_run_groups();
+    auto G = std::make_unique<agpt_run_groups>();
     G->trie = t;
     RunGroup cur;
     auto flush = [&]() { if (cur.rows()) { G->groups.push_back(std::move(cur)); cur = RunGroup(); } };
@@ -177,7 +178,7 @@ extern "C" int agpt_b200_trie_groups_create(const agpt_trie *t, int level, int64
         int64_t k = 0;
         for (int32_t p = t->parent[o.at[b]]; p > 0; p = t->parent[p]) { chain.push_back(p); k += t->edge_len[p]; }
         if (cur.rows() && cur.rows() + k + weight[u] > group_rows) flush();
-        if (cur.rows() + k + weight[u] >= (1LL << 31) - 256) { delete G; return agpt_set_error(AGPT_E_LIMIT, "trie_groups: more than 2^31 rows in one group"); }
+        if (cur.rows() + k + weight[u] >= (1LL << 31) - 256) return agpt_set_error(AGPT_E_LIMIT, "trie_groups: more than 2^31 rows in one group");
         const int32_t unit = cur.n_units++;
         int32_t above = -1;
         for (size_t i = chain.size(); i-- > 0;) above = cur.add(t, chain[i], above, unit, false);
@@ -188,22 +189,22 @@ extern "C" int agpt_b200_trie_groups_create(const agpt_trie *t, int level, int64
         }
     }
     flush();
-    *out = G;
+    *out = G.release();
     return AGPT_OK;
-}
+} AGPT_CATCH("trie_groups_create")
 
 // The group of a set of radix nodes closed under "parent" (a sampled training unit): rows in depth-first order, one unit.
 // order: a depth-first rank per radix node (agpt_b200_trie_ranks), kept by the caller between samples.
-extern "C" int agpt_b200_trie_ranks(const agpt_trie *t, int32_t *rank_out) {
+extern "C" int agpt_b200_trie_ranks(const agpt_trie *t, int32_t *rank_out) try {
     if (!t || !rank_out) return agpt_set_error(AGPT_E_ARG, "trie_ranks: null");
     RadixOrder o;
     if (int rc = radix_order(t, o)) return rc;
     std::copy(o.rank.begin(), o.rank.end(), rank_out);
     return AGPT_OK;
-}
+} AGPT_CATCH("trie_ranks")
 
 extern "C" int agpt_b200_trie_sample_group(const agpt_trie *t, const int32_t *rank, const int32_t *nodes, int64_t n_nodes, const int32_t *context,
-                                           int64_t n_context, agpt_run_groups **out) {
+                                           int64_t n_context, agpt_run_groups **out) try {
     if (!t || !rank || !nodes || !out || n_nodes < 1 || n_context < 0 || (n_context && !context)) return agpt_set_error(AGPT_E_ARG, "trie_sample_group: bad argument");
     std::vector<std::pair<int32_t, int32_t>> by((size_t)n_nodes);        // (rank, node)
     for (int64_t i = 0; i < n_nodes; i++) {
@@ -213,7 +214,7 @@ extern "C" int agpt_b200_trie_sample_group(const agpt_trie *t, const int32_t *ra
     std::sort(by.begin(), by.end());
     std::vector<int32_t> ctx(context, context + n_context);
     std::sort(ctx.begin(), ctx.end());
-    auto *G = new agpt_run_groups();
+    auto G = std::make_unique<agpt_run_groups>();
     G->trie = t;
     G->groups.emplace_back();
     RunGroup &g = G->groups[0];
@@ -222,14 +223,14 @@ extern "C" int agpt_b200_trie_sample_group(const agpt_trie *t, const int32_t *ra
     for (const auto &x : by) {
         const int32_t r = x.second, p = t->parent[r];
         while (!open.empty() && open.back().first != p) open.pop_back();
-        if (p > 0 && open.empty()) { delete G; return agpt_set_error(AGPT_E_ARG, "the node set is not closed under parent"); }
+        if (p > 0 && open.empty()) return agpt_set_error(AGPT_E_ARG, "the node set is not closed under parent");
+        if (g.full(t, r)) return agpt_set_error(AGPT_E_LIMIT, "trie_sample_group: more than 2^31 rows");
         const int32_t e = g.add(t, r, p > 0 ? open.back().second : -1, 0, !std::binary_search(ctx.begin(), ctx.end(), r));
         open.emplace_back(r, e);
     }
-    if (g.rows() >= (1LL << 31) - 256) { delete G; return agpt_set_error(AGPT_E_LIMIT, "trie_sample_group: more than 2^31 rows"); }
-    *out = G;
+    *out = G.release();
     return AGPT_OK;
-}
+} AGPT_CATCH("trie_sample_group")
 
 extern "C" int64_t agpt_b200_trie_groups_count(const agpt_run_groups *G) { return G ? (int64_t)G->groups.size() : 0; }
 extern "C" void agpt_b200_trie_groups_free(agpt_run_groups *G) { delete G; }
@@ -239,14 +240,16 @@ extern "C" int agpt_b200_trie_groups_even(agpt_run_groups *G, int even) {
     return AGPT_OK;
 }
 
-extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int tile_m, int mass_mode, int seq_len, agpt_run_group_info *out) {
+extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int tile_m, int mass_mode, int seq_len, agpt_run_group_info *out) try {
     if (!G || !out || i < 0 || i >= (int64_t)G->groups.size() || seq_len < 1 || mass_mode < 0 || mass_mode > 3 || (tile_m != 32 && tile_m != 64 && tile_m != 128))
         return agpt_set_error(AGPT_E_ARG, "trie_group_prepare: bad argument");
     const RunGroup &g = G->groups[i];
     const agpt_trie *t = G->trie;
     const int32_t E = (int32_t)g.rid.size();
     const int64_t n = g.rows(), M = tile_m;
+    G->ready = -1;                              // until this one is complete
     delete G->plan;
+    G->plan = nullptr;
     agpt_plan *P = G->plan = new agpt_plan();
     P->n = n; P->tile_m = tile_m; P->even = G->even;
     P->lazy = true;
@@ -275,21 +278,21 @@ extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int t
     P->chain_off.reserve(n / 32 + 2);
     P->chain_off.push_back(0);
     int64_t e0 = 0;                             // the run of the tile's first row
-    for (int64_t i = 0; i < n;) {
-        ts.push_back((int32_t)i);
-        int64_t k = std::min(M, n - i), e1 = e0;
-        if (tile_m == 64 && !P->even && i + M < n) {
-            while (g.qoff[e1 + 1] <= i + 32) e1++;
+    for (int64_t r0 = 0; r0 < n;) {
+        ts.push_back((int32_t)r0);
+        int64_t k = std::min(M, n - r0), e1 = e0;
+        if (tile_m == 64 && !P->even && r0 + M < n) {
+            while (g.qoff[e1 + 1] <= r0 + 32) e1++;
             int64_t best = INT64_MAX;
-            for (int64_t e = e1; e < E && g.qoff[e] <= i + M; e++) {
-                const int64_t c = std::max<int64_t>(g.qoff[e] - i, 32), v = agpt_tile_cost((int32_t)(ld[e] + (i + c - g.qoff[e])), c);
+            for (int64_t e = e1; e < E && g.qoff[e] <= r0 + M; e++) {
+                const int64_t c = std::max<int64_t>(g.qoff[e] - r0, 32), v = agpt_tile_cost((int32_t)(ld[e] + (r0 + c - g.qoff[e])), c);
                 if (v <= best) { best = v; k = c; e1 = e; }
             }
-        } else while (e1 < E && g.qoff[e1 + 1] <= i + k) e1++;
-        const int64_t chain = ld[e0] + (i - g.qoff[e0]) - 1;
+        } else while (e1 < E && g.qoff[e1 + 1] <= r0 + k) e1++;
+        const int64_t chain = ld[e0] + (r0 - g.qoff[e0]) - 1;
         P->chain_off.push_back(P->chain_off.back() + chain);
         P->max_keys = std::max(P->max_keys, (int32_t)(chain + k));
-        i += k; e0 = e1;
+        r0 += k; e0 = e1;
     }
     P->n_tiles = (int64_t)ts.size();
     ts.push_back((int32_t)n);
@@ -382,7 +385,7 @@ extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int t
     o.seq_len = seq_len;
 
     G->staging.reset((uint8_t *)agpt_big_alloc((size_t)std::max<int64_t>(G->staged, 16)));
-    if (!G->staging) throw std::bad_alloc();
+    if (!G->staging) return agpt_set_error(AGPT_E_NOMEM, "trie_group_prepare: out of host memory");
     uint8_t *s = G->staging.get();
     auto put = [&](int64_t where, const void *src, int64_t bytes) { if (bytes) memcpy(s + where, src, (size_t)bytes); };
     put(o.qoff, g.qoff.data(), (int64_t)(E + 1) * 4); put(o.rid, g.rid.data(), (int64_t)E * 4);
@@ -411,7 +414,7 @@ extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int t
     G->ready = i;
     *out = o;
     return AGPT_OK;
-}
+} AGPT_CATCH("trie_group_prepare")
 
 extern "C" int agpt_b200_trie_group_upload(agpt_run_groups *G, int device, void *d_buffer, void *stream, agpt_plan **plan_out) {
     if (!G || G->ready < 0 || !G->plan || !d_buffer || !plan_out || device < 0) return agpt_set_error(AGPT_E_ARG, "trie_group_upload: nothing prepared");

@@ -16,6 +16,7 @@
 #include <cstring>
 #include <deque>
 #include <map>
+#include <memory>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -62,15 +63,15 @@ static int inv_cdf(const std::vector<double> &cdf, double u) {
 
 static int synth_markov(int64_t n, int vocab, int order, uint64_t seed, int repeat_log2, int32_t *out);
 
-extern "C" int agpt_b200_synth_markov_corpus(int64_t n, int vocab, int order, uint64_t seed, int32_t *out) {
+extern "C" int agpt_b200_synth_markov_corpus(int64_t n, int vocab, int order, uint64_t seed, int32_t *out) try {
     return synth_markov(n, vocab, order, seed, 0, out);
-}
+} AGPT_CATCH("synth_markov_corpus")
 
 extern "C" int agpt_b200_synth_markov_corpus_repeats(int64_t n, int vocab, int order, uint64_t seed, int repeat_log2,
-                                                     int32_t *out) {
+                                                     int32_t *out) try {
     if (repeat_log2 < 1 || repeat_log2 > 40) return agpt_set_error(AGPT_E_ARG, "synth_markov_corpus_repeats: repeat_log2 must be 1..40");
     return synth_markov(n, vocab, order, seed, repeat_log2, out);
-}
+} AGPT_CATCH("synth_markov_corpus_repeats")
 
 // repeat_log2 > 0: before each symbol one more draw of the stream decides, with probability 2^-repeat_log2, to copy
 // a span of 64 + (draw mod 193) symbols from a uniformly drawn earlier offset instead (long verbatim repeats, as
@@ -120,7 +121,7 @@ static int synth_markov(int64_t n, int vocab, int order, uint64_t seed, int repe
 }
 
 extern "C" int64_t agpt_b200_synth_tree(int64_t max_nodes, int max_depth, int root_children, double p_stop,
-                                         int max_children, int64_t level_cap, uint64_t seed, int32_t *parent_out) {
+                                         int max_children, int64_t level_cap, uint64_t seed, int32_t *parent_out) try {
     if (!parent_out || max_nodes <= 0 || max_depth < 1 || root_children < 1 || p_stop <= 0 || p_stop > 1)
         return agpt_set_error(AGPT_E_ARG, "synth_tree: bad argument");
     uint64_t s = splitmix64(seed ^ 0xA5A5A5A5ULL);
@@ -142,7 +143,7 @@ extern "C" int64_t agpt_b200_synth_tree(int64_t max_nodes, int max_depth, int ro
         lvl_end = n;
     }
     return n;
-}
+} AGPT_CATCH("synth_tree")
 
 // RoPE tables in float32 host arithmetic, value duplicated over each (2i, 2i+1) pair.
 extern "C" int agpt_b200_rope_table(float *cos_out, float *sin_out, int max_seq, int head_dim, float base) {
@@ -236,7 +237,7 @@ void build_leveled(const int32_t *corpus, int64_t n, int max_depth, int vocab, L
 }  // namespace
 
 extern "C" int agpt_b200_trie_build(const int32_t *corpus, int64_t n, int max_depth, int subtree_level,
-                                    int prune_min_mass, int prune_min_depth, agpt_trie **out) {
+                                    int prune_min_mass, int prune_min_depth, agpt_trie **out) try {
     if (!corpus || !out || n < 2 || max_depth < 1) return agpt_set_error(AGPT_E_ARG, "trie_build: bad argument");
     if (n >= (1LL << 31)) return agpt_set_error(AGPT_E_LIMIT, "trie_build: corpus beyond 2^31 tokens");
     int vocab = 0;
@@ -248,7 +249,8 @@ extern "C" int agpt_b200_trie_build(const int32_t *corpus, int64_t n, int max_de
     build_leveled(corpus, n, max_depth, vocab, L);
     if (L.token.size() >= (1ULL << 31)) return agpt_set_error(AGPT_E_LIMIT, "trie_build: more than 2^31 trie nodes");
 
-    agpt_trie *t = new agpt_trie();
+    std::unique_ptr<agpt_trie> own(new agpt_trie());
+    agpt_trie *t = own.get();
     t->leveled_nodes = (int64_t)L.token.size();
     auto push_node = [&](int32_t par, int32_t fcd, int32_t mass, int32_t epd, int32_t key) {
         t->parent.push_back(par); t->first_char_depth.push_back(fcd); t->edge_len.push_back(0);
@@ -299,9 +301,9 @@ extern "C" int agpt_b200_trie_build(const int32_t *corpus, int64_t n, int max_de
     t->n_depth_files = max_ep + 1;
     t->total_edge_chars = (int64_t)t->edge_tok.size();
     t->finish_char_positions();
-    *out = t;
+    *out = own.release();
     return AGPT_OK;
-}
+} AGPT_CATCH("trie_build")
 
 extern "C" void agpt_b200_trie_free(agpt_trie *t) { delete t; }
 
@@ -351,7 +353,7 @@ void write_record(Writer &w, const agpt_trie *t, int32_t r) {
 }  // namespace
 
 extern "C" int agpt_b200_trie_save_dir(const agpt_trie *t, const char *dir, int per_subtree, int32_t corpus_tokens,
-                                       int32_t vocab, uint64_t corpus_hash, const char *tag) {
+                                       int32_t vocab, uint64_t corpus_hash, const char *tag) try {
     if (!t || !dir || !tag) return agpt_set_error(AGPT_E_ARG, "trie_save_dir: null");
     std::string d(dir);
     std::vector<std::vector<int32_t>> by_depth(t->n_depth_files);
@@ -388,9 +390,9 @@ extern "C" int agpt_b200_trie_save_dir(const agpt_trie *t, const char *dir, int 
     int32_t tl = (int32_t)strlen(tag);
     w.i32(tl); fwrite(tag, 1, (size_t)tl, w.f);
     return AGPT_OK;
-}
+} AGPT_CATCH("trie_save_dir")
 
-extern "C" int agpt_b200_trie_load_dir(const char *dir, agpt_trie **out) {
+extern "C" int agpt_b200_trie_load_dir(const char *dir, agpt_trie **out) try {
     if (!dir || !out) return agpt_set_error(AGPT_E_ARG, "trie_load_dir: null");
     std::string d(dir);
     FILE *f = fopen((d + "/meta.bin").c_str(), "rb");
@@ -402,7 +404,8 @@ extern "C" int agpt_b200_trie_load_dir(const char *dir, agpt_trie **out) {
     if (!ok || magic != RADIX_MAGIC) return agpt_set_error(AGPT_E_IO, "%s/meta.bin: bad radix magic", dir);
     if (ver != 2) return agpt_set_error(AGPT_E_IO, "%s/meta.bin: radix format version %d unsupported (need 2)", dir, ver);
     if (rc < 1 || ndf < 0 || tec < 0) return agpt_set_error(AGPT_E_IO, "%s/meta.bin: bad counts", dir);
-    agpt_trie *t = new agpt_trie();
+    std::unique_ptr<agpt_trie> own(new agpt_trie());
+    agpt_trie *t = own.get();
     t->radix_count = rc; t->n_depth_files = ndf; t->total_edge_chars = tec;
     t->parent.assign(rc, -1); t->first_char_depth.assign(rc, 0); t->edge_len.assign(rc, 0); t->edge_mass.assign(rc, 0);
     t->endpoint_depth.assign(rc, 0); t->subtree_key.assign(rc, 0);
@@ -414,20 +417,20 @@ extern "C" int agpt_b200_trie_load_dir(const char *dir, agpt_trie **out) {
         f = fopen((d + name).c_str(), "rb");
         if (!f) continue;   // an absent depth file is an empty one (src/cuda/agpt_train.cu:816)
         int32_t hd[3];
-        if (fread(hd, 4, 3, f) != 3 || (uint32_t)hd[0] != RADIX_MAGIC || hd[1] != dd) { fclose(f); delete t; return agpt_set_error(AGPT_E_IO, "%s%s: bad header", dir, name); }
+        if (fread(hd, 4, 3, f) != 3 || (uint32_t)hd[0] != RADIX_MAGIC || hd[1] != dd) { fclose(f); return agpt_set_error(AGPT_E_IO, "%s%s: bad header", dir, name); }
         for (int32_t i = 0; i < hd[2]; i++) {
             int32_t r4[4];
-            if (fread(r4, 4, 4, f) != 4 || r4[0] <= 0 || r4[0] >= rc || r4[3] < 0) { fclose(f); delete t; return agpt_set_error(AGPT_E_IO, "%s%s: bad record", dir, name); }
+            if (fread(r4, 4, 4, f) != 4 || r4[0] <= 0 || r4[0] >= rc || r4[3] < 0) { fclose(f); return agpt_set_error(AGPT_E_IO, "%s%s: bad record", dir, name); }
             int32_t r = r4[0];
             t->parent[r] = r4[1]; t->first_char_depth[r] = r4[2]; t->edge_len[r] = r4[3]; t->endpoint_depth[r] = dd;
             edges[r].resize(r4[3]);
             int32_t me[2];
-            if (fread(edges[r].data(), 4, (size_t)r4[3], f) != (size_t)r4[3] || fread(me, 4, 2, f) != 2 || me[1] < 0) { fclose(f); delete t; return agpt_set_error(AGPT_E_IO, "%s%s: truncated record", dir, name); }
+            if (fread(edges[r].data(), 4, (size_t)r4[3], f) != (size_t)r4[3] || fread(me, 4, 2, f) != 2 || me[1] < 0) { fclose(f); return agpt_set_error(AGPT_E_IO, "%s%s: truncated record", dir, name); }
             t->edge_mass[r] = me[0];
             ctok[r].resize(me[1]); cval[r].resize(me[1]);
             for (int32_t e = 0; e < me[1]; e++) {
                 int32_t tv[2];
-                if (fread(tv, 4, 2, f) != 2) { fclose(f); delete t; return agpt_set_error(AGPT_E_IO, "%s%s: truncated counts", dir, name); }
+                if (fread(tv, 4, 2, f) != 2) { fclose(f); return agpt_set_error(AGPT_E_IO, "%s%s: truncated counts", dir, name); }
                 ctok[r][e] = tv[0]; cval[r][e] = tv[1];
             }
         }
@@ -443,15 +446,15 @@ extern "C" int agpt_b200_trie_load_dir(const char *dir, agpt_trie **out) {
         // unigram subtree key = depth-1 radix ancestor (parents precede children in id order)
         if (r > 0) t->subtree_key[r] = t->parent[r] == 0 ? r : t->subtree_key[t->parent[r]];
     }
-    if ((int64_t)t->edge_tok.size() != tec) { delete t; return agpt_set_error(AGPT_E_IO, "%s: edge chars %lld != meta %lld", dir, (long long)t->edge_tok.size(), (long long)tec); }
+    if ((int64_t)t->edge_tok.size() != tec) { return agpt_set_error(AGPT_E_IO, "%s: edge chars %lld != meta %lld", dir, (long long)t->edge_tok.size(), (long long)tec); }
     t->finish_char_positions();
-    *out = t;
+    *out = own.release();
     return AGPT_OK;
-}
+} AGPT_CATCH("trie_load_dir")
 
 // Per-subtree files (src/cuda/agpt_train.cu:431-493 manifest, :495-669 load_subtree).
 extern "C" int64_t agpt_b200_trie_manifest(const char *dir, int64_t cap, int32_t *keys, int32_t *n_nodes, int64_t *edge_chars,
-                                           int32_t *max_endpoint_depth) {
+                                           int32_t *max_endpoint_depth) try {
     if (!dir) return agpt_set_error(AGPT_E_ARG, "trie_manifest: null");
     std::string d(dir);
     FILE *f = fopen((d + "/manifest.bin").c_str(), "rb");
@@ -470,9 +473,9 @@ extern "C" int64_t agpt_b200_trie_manifest(const char *dir, int64_t cap, int32_t
     }
     fclose(f);
     return hd[2];
-}
+} AGPT_CATCH("trie_manifest")
 
-extern "C" int agpt_b200_trie_load_subtree(const char *dir, int32_t subtree_key, agpt_trie **out) {
+extern "C" int agpt_b200_trie_load_subtree(const char *dir, int32_t subtree_key, agpt_trie **out) try {
     if (!dir || !out) return agpt_set_error(AGPT_E_ARG, "trie_load_subtree: null");
     char name[96];
     snprintf(name, sizeof(name), "/subtrees/radix_subtree_%06d.bin", subtree_key);
@@ -483,7 +486,8 @@ extern "C" int agpt_b200_trie_load_subtree(const char *dir, int32_t subtree_key,
     if (fread(hd, 4, 4, f) != 4 || fread(&tec, 8, 1, f) != 1 || fread(&max_ep, 4, 1, f) != 1 || (uint32_t)hd[0] != RADIX_MAGIC || hd[1] != 2 ||
         hd[2] != subtree_key || hd[3] < 0 || tec < 0) { fclose(f); return agpt_set_error(AGPT_E_IO, "%s: bad header", path.c_str()); }
     const int32_t n = hd[3], rc = n + 1;                  // local id 0 = the (virtual) root, records 1..n in file order
-    agpt_trie *t = new agpt_trie();
+    std::unique_ptr<agpt_trie> own(new agpt_trie());
+    agpt_trie *t = own.get();
     t->radix_count = rc; t->n_depth_files = max_ep + 1; t->total_edge_chars = tec;
     t->parent.assign(rc, -1); t->first_char_depth.assign(rc, 0); t->edge_len.assign(rc, 0); t->edge_mass.assign(rc, 0);
     t->endpoint_depth.assign(rc, 0); t->subtree_key.assign(rc, subtree_key); t->edge_start.assign(rc, 0);
@@ -491,17 +495,17 @@ extern "C" int agpt_b200_trie_load_subtree(const char *dir, int32_t subtree_key,
     std::vector<int32_t> global_id(rc, 0), global_parent(rc, 0);
     for (int32_t i = 1; i <= n; i++) {
         int32_t r4[4], me[2];
-        if (fread(r4, 4, 4, f) != 4 || r4[3] < 0) { fclose(f); delete t; return agpt_set_error(AGPT_E_IO, "%s: bad record %d", path.c_str(), i); }
+        if (fread(r4, 4, 4, f) != 4 || r4[3] < 0) { fclose(f); return agpt_set_error(AGPT_E_IO, "%s: bad record %d", path.c_str(), i); }
         global_id[i] = r4[0]; global_parent[i] = r4[1];
         t->first_char_depth[i] = r4[2]; t->edge_len[i] = r4[3]; t->endpoint_depth[i] = r4[2] + r4[3] - 1;
         t->edge_start[i] = (int32_t)t->edge_tok.size();     // char positions in file order, as the reference numbers them
         const size_t at = t->edge_tok.size();
         t->edge_tok.resize(at + (size_t)r4[3]);
-        if (fread(t->edge_tok.data() + at, 4, (size_t)r4[3], f) != (size_t)r4[3] || fread(me, 4, 2, f) != 2 || me[1] < 0) { fclose(f); delete t; return agpt_set_error(AGPT_E_IO, "%s: truncated record %d", path.c_str(), i); }
+        if (fread(t->edge_tok.data() + at, 4, (size_t)r4[3], f) != (size_t)r4[3] || fread(me, 4, 2, f) != 2 || me[1] < 0) { fclose(f); return agpt_set_error(AGPT_E_IO, "%s: truncated record %d", path.c_str(), i); }
         t->edge_mass[i] = me[0];
         for (int32_t e = 0; e < me[1]; e++) {
             int32_t tv[2];
-            if (fread(tv, 4, 2, f) != 2) { fclose(f); delete t; return agpt_set_error(AGPT_E_IO, "%s: truncated counts", path.c_str()); }
+            if (fread(tv, 4, 2, f) != 2) { fclose(f); return agpt_set_error(AGPT_E_IO, "%s: truncated counts", path.c_str()); }
             t->cnt_tok.push_back(tv[0]); t->cnt_val.push_back(tv[1]);
         }
         t->edge_off[i + 1] = (int64_t)t->edge_tok.size();
@@ -509,7 +513,7 @@ extern "C" int agpt_b200_trie_load_subtree(const char *dir, int32_t subtree_key,
     }
     fclose(f);
     t->edge_off[1] = 0; t->cnt_off[1] = 0;
-    if ((int64_t)t->edge_tok.size() != tec) { delete t; return agpt_set_error(AGPT_E_IO, "%s: edge chars %lld != header %lld", path.c_str(), (long long)t->edge_tok.size(), (long long)tec); }
+    if ((int64_t)t->edge_tok.size() != tec) { return agpt_set_error(AGPT_E_IO, "%s: edge chars %lld != header %lld", path.c_str(), (long long)t->edge_tok.size(), (long long)tec); }
     // global -> local ids; a parent that is the virtual root or lies outside the file (the depth-1 node of a bigram
     // subtree) becomes the local root
     std::vector<int32_t> order(n);
@@ -524,11 +528,11 @@ extern "C" int agpt_b200_trie_load_subtree(const char *dir, int32_t subtree_key,
         }
         t->parent[i] = lp;
     }
-    *out = t;
+    *out = own.release();
     return AGPT_OK;
-}
+} AGPT_CATCH("trie_load_subtree")
 
-extern "C" int agpt_b200_trie_char_tree(const agpt_trie *t, int32_t *parent, int32_t *token, int32_t *depth, int32_t *radix_of_char) {
+extern "C" int agpt_b200_trie_char_tree(const agpt_trie *t, int32_t *parent, int32_t *token, int32_t *depth, int32_t *radix_of_char) try {
     if (!t) return agpt_set_error(AGPT_E_ARG, "trie_char_tree: null");
     for (int32_t r = 1; r < t->radix_count; r++) {
         int64_t s = t->edge_start[r];
@@ -541,7 +545,7 @@ extern "C" int agpt_b200_trie_char_tree(const agpt_trie *t, int32_t *parent, int
         }
     }
     return AGPT_OK;
-}
+} AGPT_CATCH("trie_char_tree")
 
 // --------------------------------------------------------------------------------------
 // stochastic subtree sampling ("lightning" training units, src/cuda/agpt_train.cu:152-200, :3928-3943, :4060-4241)
@@ -561,7 +565,7 @@ static inline float xorshift_unit(uint32_t *st) { return (float)xorshift32(st) /
 // the total number of node ids (the generator state is then left untouched), then again to fill.
 extern "C" int64_t agpt_b200_lightning_sample(const agpt_trie *t, int sampler, int steps, float p_stop, int64_t max_mass,
                                               uint32_t *rng_state, int32_t *sample_out, int32_t *n_anc_out, int64_t *node_off_out,
-                                              double *mass_out, int32_t *nodes_out, int64_t nodes_cap) {
+                                              double *mass_out, int32_t *nodes_out, int64_t nodes_cap) try {
     if (!t || !rng_state || steps < 0 || sampler < 1 || sampler > 4) return agpt_set_error(AGPT_E_ARG, "lightning_sample: bad argument");
     const int32_t R = t->radix_count;
     std::vector<int64_t> coff(R + 1, 0);
@@ -642,7 +646,7 @@ extern "C" int64_t agpt_b200_lightning_sample(const agpt_trie *t, int sampler, i
     }
     if (nodes_out) *rng_state = rng;
     return total;
-}
+} AGPT_CATCH("lightning_sample")
 
 // learning-rate schedule of the trainer (src/cuda/agpt_train.cu:146-216): schedule 0 constant, 1 cosine, 2 linear
 // warm-up over warmup_steps then cosine; `step` counts the optimizer steps already taken
@@ -680,7 +684,7 @@ int agpt_mass_weights_per_node(const int32_t *edge_mass, const int32_t *edge_len
 }
 
 extern "C" int agpt_b200_mass_weights(const int32_t *edge_mass, const int32_t *edge_len, const int32_t *unit_of_node,
-                                      const uint8_t *counted, int64_t n_nodes, int64_t n_units, int mode, float *out_per_query) {
+                                      const uint8_t *counted, int64_t n_nodes, int64_t n_units, int mode, float *out_per_query) try {
     if (!edge_mass || !edge_len || !out_per_query || n_nodes < 0 || n_units < 1 || mode < 0 || mode > 3)
         return agpt_set_error(AGPT_E_ARG, "mass_weights: bad argument");
     std::vector<float> w((size_t)n_nodes);
@@ -689,7 +693,7 @@ extern "C" int agpt_b200_mass_weights(const int32_t *edge_mass, const int32_t *e
     for (int64_t i = 0; i < n_nodes; i++)
         for (int32_t j = 0; j < edge_len[i]; j++) out_per_query[q++] = w[i];
     return AGPT_OK;
-}
+} AGPT_CATCH("mass_weights")
 
 // --------------------------------------------------------------------------------------
 // walker plan
@@ -704,7 +708,8 @@ static int plan_create(const int32_t *parent, int64_t n, int tile_m, int device,
         if (p < -1 || p >= n || p == i) return agpt_set_error(AGPT_E_ARG, "plan_create: parent[%lld]=%d out of range", (long long)i, p);
         if (p >= i) monotone = false;
     }
-    agpt_plan *P = new agpt_plan();
+    std::unique_ptr<agpt_plan> own(new agpt_plan());
+    agpt_plan *P = own.get();
     P->n = n; P->tile_m = tile_m; P->even = even;
     P->dfs_to_node.resize(n); P->node_to_dfs.assign(n, -1); P->parent_dfs.resize(n); P->depth.resize(n); P->sub_end.resize(n);
     P->n_groups = 0; P->sum_group_prefix = 0;
@@ -767,7 +772,7 @@ static int plan_create(const int32_t *parent, int64_t n, int tile_m, int device,
                 }
             }
         }
-        if (pos != n) { delete P; return agpt_set_error(AGPT_E_ARG, "plan_create: parent array has a cycle or unreachable nodes (%lld of %lld reached)", (long long)pos, (long long)n); }
+        if (pos != n) { return agpt_set_error(AGPT_E_ARG, "plan_create: parent array has a cycle or unreachable nodes (%lld of %lld reached)", (long long)pos, (long long)n); }
         // sibling groups (for the bytes model): one per node with children, plus the root's
         P->n_groups = coff[1] > coff[0] ? 1 : 0;
         for (int64_t v = 0; v < n; v++)
@@ -837,18 +842,18 @@ static int plan_create(const int32_t *parent, int64_t n, int tile_m, int device,
     P->device = -1;
     if (device >= 0) {
         int rc = agpt_plan_upload(P, device);
-        if (rc != AGPT_OK) { delete P; return rc; }
+        if (rc != AGPT_OK) { return rc; }
     }
-    *out = P;
+    *out = own.release();
     return AGPT_OK;
 }
 
-extern "C" int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_m, int device, agpt_plan **out) {
+extern "C" int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_m, int device, agpt_plan **out) try {
     return plan_create(parent, n, tile_m, device, false, out);
-}
-extern "C" int agpt_b200_plan_create_even(const int32_t *parent, int64_t n, int tile_m, int device, agpt_plan **out) {
+} AGPT_CATCH("plan_create")
+extern "C" int agpt_b200_plan_create_even(const int32_t *parent, int64_t n, int tile_m, int device, agpt_plan **out) try {
     return plan_create(parent, n, tile_m, device, true, out);
-}
+} AGPT_CATCH("plan_create_even")
 
 // one row array (0 dfs_to_node, 1 node_to_dfs, 2 parent_dfs, 3 depth, 4 sub_end), written straight into the caller's memory
 extern "C" int agpt_b200_plan_array(const agpt_plan *p, int which, int32_t *out) {
@@ -888,7 +893,7 @@ extern "C" int agpt_b200_plan_sizes(const agpt_plan *p, agpt_plan_info *o) {
     return AGPT_OK;
 }
 
-extern "C" int agpt_b200_plan_info(const agpt_plan *p, agpt_plan_info *o) {
+extern "C" int agpt_b200_plan_info(const agpt_plan *p, agpt_plan_info *o) try {
     if (!p || !o) return agpt_set_error(AGPT_E_ARG, "plan_info: null");
     const_cast<agpt_plan *>(p)->need_host();
     o->n = p->n; o->tile_m = p->tile_m; o->n_tiles = p->n_tiles; o->chain_rows = p->chain_rows;
@@ -897,7 +902,7 @@ extern "C" int agpt_b200_plan_info(const agpt_plan *p, agpt_plan_info *o) {
     o->dfs_to_node = p->dfs_to_node.data(); o->node_to_dfs = p->node_to_dfs.data(); o->parent_dfs = p->parent_dfs.data();
     o->depth = p->depth.data(); o->sub_end = p->sub_end.data(); o->device = p->device;
     return AGPT_OK;
-}
+} AGPT_CATCH("plan_info")
 
 // --------------------------------------------------------------------------------------
 // launch groups: this rank's units packed, in depth-first order, into forests of at most group_rows rows
@@ -909,10 +914,11 @@ struct agpt_groups {
 };
 
 extern "C" int agpt_b200_groups_create(const agpt_plan *p, const int64_t *unit_begin, const int64_t *unit_end, const int32_t *unit_rank,
-                                       int64_t n_units, int rank, int64_t group_rows, agpt_groups **out) {
+                                       int64_t n_units, int rank, int64_t group_rows, agpt_groups **out) try {
     if (!p || !unit_begin || !unit_end || !out || n_units < 0 || group_rows < 1) return agpt_set_error(AGPT_E_ARG, "groups_create: bad argument");
     const_cast<agpt_plan *>(p)->need_host();
-    agpt_groups *G = new agpt_groups();
+    std::unique_ptr<agpt_groups> own(new agpt_groups());
+    agpt_groups *G = own.get();
     agpt_groups::Group cur;
     auto flush = [&]() {
         if (!cur.row.empty()) { G->groups.push_back(std::move(cur)); cur = agpt_groups::Group(); }
@@ -921,7 +927,7 @@ extern "C" int agpt_b200_groups_create(const agpt_plan *p, const int64_t *unit_b
     for (int64_t u = 0; u < n_units; u++) {
         if (unit_rank && unit_rank[u] != rank) continue;
         const int64_t b = unit_begin[u], e = unit_end[u];
-        if (b < 0 || e > p->n || b >= e) { delete G; return agpt_set_error(AGPT_E_ARG, "groups_create: unit %lld has a bad range", (long long)u); }
+        if (b < 0 || e > p->n || b >= e) { return agpt_set_error(AGPT_E_ARG, "groups_create: unit %lld has a bad range", (long long)u); }
         // a unit that does not start at depth 1 carries its ancestors as context rows (attended, not trained), so every
         // chain is complete and results do not depend on the partition
         chain.clear();
@@ -930,7 +936,7 @@ extern "C" int agpt_b200_groups_create(const agpt_plan *p, const int64_t *unit_b
         const int64_t k = (int64_t)chain.size(), rows = k + (e - b);
         if (!cur.row.empty() && (int64_t)cur.row.size() + rows > group_rows) flush();
         const int64_t off = (int64_t)cur.row.size();
-        if (off + rows >= (1LL << 31) - 256) { delete G; return agpt_set_error(AGPT_E_LIMIT, "groups_create: more than 2^31 rows in one group"); }
+        if (off + rows >= (1LL << 31) - 256) { return agpt_set_error(AGPT_E_LIMIT, "groups_create: more than 2^31 rows in one group"); }
         const int32_t unit_local = cur.n_units++;
         for (int64_t j = 0; j < k; j++) {
             cur.parent.push_back((int32_t)(j == 0 ? -1 : off + j - 1));
@@ -945,9 +951,9 @@ extern "C" int agpt_b200_groups_create(const agpt_plan *p, const int64_t *unit_b
         }
     }
     flush();
-    *out = G;
+    *out = own.release();
     return AGPT_OK;
-}
+} AGPT_CATCH("groups_create")
 
 extern "C" int64_t agpt_b200_groups_count(const agpt_groups *g) { return g ? (int64_t)g->groups.size() : 0; }
 
@@ -968,7 +974,7 @@ extern "C" int64_t agpt_b200_attn_bwd_workspace_bytes(const agpt_plan *p, int d_
     return std::max<int64_t>(256, rows * 2 * (int64_t)d_model * 4);
 }
 
-extern "C" int64_t agpt_b200_plan_units(const agpt_plan *p, int level, int64_t cap, int64_t *ub, int64_t *ue) {
+extern "C" int64_t agpt_b200_plan_units(const agpt_plan *p, int level, int64_t cap, int64_t *ub, int64_t *ue) try {
     if (!p || (level != 1 && level != 2)) return agpt_set_error(AGPT_E_ARG, "plan_units: bad argument");
     const_cast<agpt_plan *>(p)->need_host();
     int64_t cnt = 0;
@@ -980,9 +986,9 @@ extern "C" int64_t agpt_b200_plan_units(const agpt_plan *p, int level, int64_t c
         for (int64_t c = a + 1; c < p->sub_end[a]; c = p->sub_end[c]) emit(c, p->sub_end[c]);
     }
     return cnt;
-}
+} AGPT_CATCH("plan_units")
 
-extern "C" int agpt_b200_partition_lpt(const int64_t *w, int64_t n_units, int n_ranks, int32_t *rank_of_unit) {
+extern "C" int agpt_b200_partition_lpt(const int64_t *w, int64_t n_units, int n_ranks, int32_t *rank_of_unit) try {
     if (!w || !rank_of_unit || n_units < 0 || n_ranks < 1) return agpt_set_error(AGPT_E_ARG, "partition_lpt: bad argument");
     std::vector<int64_t> order(n_units), load(n_ranks, 0);
     std::iota(order.begin(), order.end(), 0);
@@ -994,4 +1000,4 @@ extern "C" int agpt_b200_partition_lpt(const int64_t *w, int64_t n_units, int n_
         load[best] += w[u];
     }
     return AGPT_OK;
-}
+} AGPT_CATCH("partition_lpt")

@@ -3,6 +3,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstdlib>
+#include <exception>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -12,6 +13,10 @@
 #define AGPT_REDUCE_SEG 16    // tiles summed by one warp of the dK/dV reduction before a second pass (at most 32: one offset per lane)
 
 int agpt_set_error(int code, const char *fmt, ...);
+// Behind the body of an extern "C" function that allocates (extern "C" int f() try { .. } AGPT_CATCH("f")): no exception crosses the boundary.
+#define AGPT_CATCH(who)                                                                                        \
+    catch (const std::bad_alloc &) { return agpt_set_error(AGPT_E_NOMEM, who ": out of host memory"); }        \
+    catch (const std::exception &e) { return agpt_set_error(AGPT_E_NOMEM, who ": %s", e.what()); }
 
 // Host memory for arrays of megabytes that one call makes and fills once.  Their first touch in 4 KB pages costs more than the
 // fill (0.5 us a page: 2 ms for the 1.7M edge characters of 60,000 tokens at depth 32, and zeroing them first as much again), so

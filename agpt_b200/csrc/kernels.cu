@@ -3164,7 +3164,7 @@ static int attn_fwd_bwd_host_impl(const agpt_plan *cp, const float *h_q, const f
 
 extern "C" int agpt_b200_attn_fwd_bwd_host(const agpt_plan *cp, const float *h_q, const float *h_k, const float *h_v,
                                            const float *h_dout, float *h_out, float *h_lse, float *h_dq, float *h_dk, float *h_dv,
-                                           int kv_dtype, int n_heads, int head_dim, float scale) {
+                                           int kv_dtype, int n_heads, int head_dim, float scale) try {
     const int rc = attn_fwd_bwd_host_impl(cp, h_q, h_k, h_v, h_dout, h_out, h_lse, h_dq, h_dk, h_dv, kv_dtype, n_heads, head_dim, scale);
     if (rc != AGPT_OK && cp && cp->device >= 0) {
         // copies queued before the failure still read and write the caller's buffers (and the cached arena): wait for
@@ -3173,7 +3173,7 @@ extern "C" int agpt_b200_attn_fwd_bwd_host(const agpt_plan *cp, const float *h_q
             if (st) cudaStreamSynchronize((cudaStream_t)st);
     }
     return rc;
-}
+} AGPT_CATCH("attn_fwd_bwd_host")
 
 static int attn_fwd_bwd_host_impl(const agpt_plan *cp, const float *h_q, const float *h_k, const float *h_v,
                                   const float *h_dout, float *h_out, float *h_lse, float *h_dq, float *h_dk, float *h_dv,

@@ -472,15 +472,15 @@ extern "C" int agpt_b200_train_step_takes(int d_model, int n_heads, int d_ff, in
     return (hd == 16 || hd == 32 || hd == 64) && vocab >= 1 && vocab <= 400;
 }
 
-extern "C" int64_t agpt_b200_train_step_workspace_bytes(const agpt_train_step_args *args) {
+extern "C" int64_t agpt_b200_train_step_workspace_bytes(const agpt_train_step_args *args) try {
     if (!args) return agpt_set_error(AGPT_E_ARG, "train_step: null arguments");
     TRY(check(*args));
     Space S;
     lay_out(*args, nullptr, S);
     return S.bytes;
-}
+} AGPT_CATCH("train_step_workspace_bytes")
 
-extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *workspace, int64_t workspace_bytes, void *stream) {
+extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *workspace, int64_t workspace_bytes, void *stream) try {
     if (!args || !workspace) return agpt_set_error(AGPT_E_ARG, "train_step: null arguments");
     const agpt_train_step_args &A = *args;
     TRY(check(A));
@@ -636,4 +636,4 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
         TRY(launched("weight gradients"));
     }
     return AGPT_OK;
-}
+} AGPT_CATCH("train_step")

@@ -153,9 +153,9 @@ int build(const int32_t *corpus, int64_t n, int max_depth, int subtree_level, in
 }  // namespace
 
 extern "C" int agpt_b200_suffix_order_gpu(const int32_t *corpus, int64_t n, int key_len, int device, int32_t *sa_out, int32_t *lcp_out,
-                                          float *device_ms_out) {
+                                          float *device_ms_out) try {
     return suffix_order(corpus, n, key_len, device, nullptr, 0, nullptr, sa_out, lcp_out, device_ms_out);
-}
+} AGPT_CATCH("suffix_order_gpu")
 
 extern "C" int64_t agpt_b200_trie_build_workspace_bytes(int64_t n) {
     if (n < 2 || n >= (1LL << 31)) return -1;
@@ -163,12 +163,12 @@ extern "C" int64_t agpt_b200_trie_build_workspace_bytes(int64_t n) {
 }
 
 extern "C" int agpt_b200_trie_build_gpu(const int32_t *corpus, int64_t n, int max_depth, int subtree_level, int prune_min_mass,
-                                        int prune_min_depth, int device, agpt_trie **out) {
+                                        int prune_min_depth, int device, agpt_trie **out) try {
     return build(corpus, n, max_depth, subtree_level, prune_min_mass, prune_min_depth, device, nullptr, 0, nullptr, out);
-}
+} AGPT_CATCH("trie_build_gpu")
 
 extern "C" int agpt_b200_trie_build_gpu_ws(const int32_t *corpus, int64_t n, int max_depth, int subtree_level, int prune_min_mass, int prune_min_depth,
-                                           int device, void *d_workspace, int64_t workspace_bytes, void *stream, agpt_trie **out) {
+                                           int device, void *d_workspace, int64_t workspace_bytes, void *stream, agpt_trie **out) try {
     if (!d_workspace) return agpt_set_error(AGPT_E_ARG, "trie_build_gpu_ws: null workspace");
     return build(corpus, n, max_depth, subtree_level, prune_min_mass, prune_min_depth, device, (uint8_t *)d_workspace, workspace_bytes, (cudaStream_t)stream, out);
-}
+} AGPT_CATCH("trie_build_gpu_ws")

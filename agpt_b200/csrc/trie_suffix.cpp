@@ -20,6 +20,7 @@
 // including the effects of the corpus end, where a suffix stops before max_depth).
 #include <algorithm>
 #include <cstdint>
+#include <memory>
 #include <vector>
 
 #include "../../include/agpt_b200.h"
@@ -42,7 +43,7 @@ struct Open {              // an open interval of the LCP-interval tree
 }  // namespace
 
 extern "C" int agpt_b200_trie_from_suffix_order(const int32_t *corpus, int64_t n, int max_depth, int subtree_level, int prune_min_mass,
-                                                int prune_min_depth, const int32_t *sa, const int32_t *lcp, agpt_trie **out) {
+                                                int prune_min_depth, const int32_t *sa, const int32_t *lcp, agpt_trie **out) try {
     if (!corpus || !sa || !lcp || !out || max_depth < 1) return agpt_set_error(AGPT_E_ARG, "trie_from_suffix_order: bad argument");
     if (n < (int64_t)max_depth + 2) return agpt_set_error(AGPT_E_ARG, "trie_from_suffix_order: corpus shorter than max_depth + 2 tokens");
     if (n >= (1LL << 31)) return agpt_set_error(AGPT_E_LIMIT, "trie_from_suffix_order: corpus beyond 2^31 tokens");
@@ -130,7 +131,8 @@ extern "C" int agpt_b200_trie_from_suffix_order(const int32_t *corpus, int64_t n
     for (int32_t e = 0; e < E; e++)
         if (!pruned[e]) { id[e] = 1 + level_off[level[e]]++; R++; }
 
-    agpt_trie *t = new agpt_trie();
+    std::unique_ptr<agpt_trie> own(new agpt_trie());
+    agpt_trie *t = own.get();
     t->radix_count = R;
     t->leveled_nodes = leveled;
     t->parent.assign(R, -1);
@@ -201,6 +203,6 @@ extern "C" int agpt_b200_trie_from_suffix_order(const int32_t *corpus, int64_t n
     t->n_depth_files = max_ep + 1;
     t->total_edge_chars = (int64_t)t->edge_tok.size();
     t->finish_char_positions();
-    *out = t;
+    *out = own.release();
     return AGPT_OK;
-}
+} AGPT_CATCH("trie_from_suffix_order")
