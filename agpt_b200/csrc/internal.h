@@ -87,7 +87,7 @@ struct agpt_plan {
     int64_t n_tiles = 0;
     std::vector<int32_t> tile_start;             // [n_tiles + 1]
     int32_t max_keys = 0;                        // chain + rows of the tile that has most
-    // An even plan keeps what a training step on a bfloat16 store rounds: its tiles end after tile_m rows, both directions take the
+    // An even plan keeps what a sampled training step on a bfloat16 store rounds: its tiles end after tile_m rows, both directions take the
     // chunked kernels (Q, P and dS to 11 bits on both sides of lse; which value P is rounded at depends on the tile's keys in
     // chunks of 32), and a node's partial dK/dV rows are one reduction item.
     bool even = false;

@@ -32,14 +32,16 @@ class LaunchGroup:
     (:4834) -- is normalised here per unit (unit_of_row), so that results do not depend on how units are packed into
     launches or spread over ranks."""
 
+    even = False        # the plan has even tiles, and a step on the tape sums the embedding gradient serially
+
     def __init__(self, parent, tokens, depth, radix_of, edge_mass, mass_mode, seq_len, device, tile=64, trained=None,
-                 unit_of_row=None):
+                 unit_of_row=None, even=False):
         import torch
         self.n = int(parent.size)
-        self.plan = A.WalkerPlan(parent, tile, device.index if device.type == "cuda" else -1)   # a host-only plan on a CPU device (index arrays for tests)
+        self.even = even
+        self.plan = A.WalkerPlan(parent, tile, device.index if device.type == "cuda" else -1, even)   # a host-only plan on a CPU device (index arrays for tests)
         order = self.plan.dfs_to_node.astype(np.int64)
         assert np.array_equal(order, np.arange(self.n)), "launch groups are built in depth-first order"
-        self._even = None
         t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device)  # noqa: E731
         self.tokens = t(tokens.astype(np.int64))
         self.tokens32 = t(tokens.astype(np.int32))
@@ -82,7 +84,7 @@ class LaunchGroup:
         """Group i of an A.RunGroups: one device buffer, written by the library.  even: its plan has even tiles."""
         self = cls.__new__(cls)
         self._info, self._buf, self.plan = runs.upload(i, tile, mass_mode, seq_len, device, even)
-        self._even = self.plan if even else None
+        self.even = even
         o = self._info
         self.n, self.n_units, self.n_pos, self.n_trained_rows = int(o.n), int(o.n_units), int(o.n_pos), int(o.n_trained)
         return self
@@ -102,20 +104,9 @@ class LaunchGroup:
         setattr(self, name, v)
         return v
 
-    def plan_for(self, bf16_store):
-        """The plan that a step on this store walks.  On a bfloat16 store that is one with even tiles, made when first asked for:
-        which value an attention weight is rounded at depends on the tile it is computed in, so another cut of the tiles is
-        another rounding of every row, and through the ReLUs of a deep model another gradient: 2e-3 after one step on some
-        thousand rows, 1e-2 after a few on ten."""
-        if not bf16_store:
-            return self.plan
-        if self._even is None:
-            self._even = A.WalkerPlan(self.plan.parent_dfs, self.plan.tile_m, self.plan.device, even=True)
-        return self._even
-
-    def step_args(self, bf16_store=False):
+    def step_args(self):
         """The group's part of the native step's arguments (the model fills in the rest)."""
-        a = A.TrainStepArgs(plan=self.plan_for(bf16_store)._h, n=self.n, n_units=self.n_units, n_pos=self.n_pos)
+        a = A.TrainStepArgs(plan=self.plan._h, n=self.n, n_units=self.n_units, n_pos=self.n_pos)
         o = self.__dict__.get("_info")
         if o is not None:
             at = self._buf.data_ptr()
@@ -303,8 +294,7 @@ def _attention_function():
             q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
             A.rope_pair_(q, k, group.pos, cos, sin, n_heads)
             ks, vs = (A.kv_store_write_bf16(k), A.kv_store_write_bf16(v)) if bf16_store else (k, v)
-            ctx.plan = group.plan_for(bf16_store)
-            out, lse = A.attn_forward(ctx.plan, q, ks, vs, n_heads)
+            out, lse = A.attn_forward(group.plan, q, ks, vs, n_heads)
             ctx.save_for_backward(q, ks, vs, out, lse)
             ctx.group, ctx.cos, ctx.sin, ctx.n_heads, ctx.grad_mode = group, cos, sin, n_heads, grad_mode
             return out
@@ -312,7 +302,7 @@ def _attention_function():
         @staticmethod
         def backward(ctx, dout):
             q, ks, vs, out, lse = ctx.saved_tensors
-            dq, dk, dv = A.attn_backward(ctx.plan, q, ks, vs, out, lse, dout.contiguous(), ctx.n_heads,
+            dq, dk, dv = A.attn_backward(ctx.group.plan, q, ks, vs, out, lse, dout.contiguous(), ctx.n_heads,
                                          grad_mode=ctx.grad_mode, edge_first=ctx.group.edge_first)
             A.rope_pair_(dq, dk, ctx.group.pos, ctx.cos, ctx.sin, ctx.n_heads, inverse=True)
             return dq, dk, dv, None, None, None, None, None, None
@@ -393,7 +383,7 @@ class TrieWalkModel:
             return lin(lin(ln(x, g2, b2), w1, b1, relu=True), w2, bo, residual=x)
 
         fused = self.dense_impl == "tensor" and m.d_model % 4 == 0 and m.d_ff % 4 == 0
-        x = self.embed.apply(P["token_emb"], group.tokens32, bf16_store)
+        x = self.embed.apply(P["token_emb"], group.tokens32, group.even)
         for l in range(m.n_layers):
             g = lambda n: P[f"layer{l}.{n}"]  # noqa: E731
             if fused:
@@ -497,7 +487,7 @@ class TrieWalkModel:
             if c.dtype != torch.int32 or not c.is_cuda or not c.is_contiguous():
                 raise A.AgptError("counts must be contiguous int32 CUDA tensors")
         m, out = self.cfg, torch.empty(8, dtype=torch.float32, device=self.device)
-        a = group.step_args(bf16_store)
+        a = group.step_args()
         a.d_model, a.n_heads, a.n_layers, a.d_ff, a.vocab, a.seq_len = m.d_model, m.n_heads, m.n_layers, m.d_ff, m.vocab, m.seq_len
         a.params, a.grads = C.addressof(params), C.addressof(grads)
         a.counts_offset, a.counts_tok, a.counts_val = [c.data_ptr() for c in counts]
@@ -552,7 +542,7 @@ class SampleSpace:
         in the reference the ancestors prepended to a sampled subtree are trained like every other position and counted
         in the chunk's mass mean (src/cuda/agpt_train.cu:4601-4637; the ancestor count recorded at :4194 is never read,
         and the comment at :4160-4180 that announces a masking describes a variant that was taken out again).
-        even: the group is for steps on a bfloat16 store (LaunchGroup.plan_for)."""
+        even: a group with even tiles (LaunchGroup.even)."""
         t = self.trie
         if device.type == "cuda" and self.rank is not None:
             return LaunchGroup.from_runs(A.RunGroups.of_sample(t, self.rank, node_ids, context_ids), 0, mass_mode, seq_len, device, tile, even)
@@ -569,7 +559,7 @@ class SampleSpace:
             raise ValueError("the node set is not closed under parent")
         trained = ~np.isin(self.radix_of[chars], np.asarray(context_ids, np.int64))
         return LaunchGroup(local_parent, self.token[chars], self.depth[chars], self.radix_of[chars], t.edge_mass, mass_mode, seq_len,
-                           device, tile, None if trained.all() else trained)
+                           device, tile, None if trained.all() else trained, even=even)
 
 
 def lightning_lr_weights(masses, mode: str) -> np.ndarray:
@@ -595,9 +585,10 @@ def train_lightning_epoch(model: TrieWalkModel, space: SampleSpace, counts, opt,
     model.bind_grads()
     loss_sum, n_q, n_nodes = 0.0, 0, 0
     pending = []                         # statistics of native steps, read once at the end so that the host never waits between steps
-    # Steps on a bfloat16 store run by single operations.  A unit of ten rows has nothing to average over: a float32 sum in another
-    # order rounds some K or V row to the other bfloat16 neighbour, a ReLU or two change sides, and after the next optimizer steps
-    # the momentum of a model of eight layers is another by 1e-2.  The order of these operations is what a seed stands for there.
+    # Steps on a bfloat16 store run by single operations over even tiles.  A unit of ten rows has nothing to average over: a float32 sum
+    # in another order rounds some K or V row to the other bfloat16 neighbour, a ReLU or two change sides, and after the next optimizer
+    # steps the momentum of a model of eight layers is another by 1e-2.  The order of these operations, and where they round, is what a
+    # seed stands for there; the native step is no less accurate (more: 16 to 22 bits instead of 11), and four times faster, but another run.
     bf16 = bool(loss_kw.get("bf16_store"))
     native = model.native_step_available() and not bf16
     for s in range(steps):

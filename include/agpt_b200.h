@@ -230,7 +230,7 @@ typedef struct {
  * With device >= 0 the index arrays are also allocated on that device (freed by plan_destroy). */
 int agpt_b200_plan_create(const int32_t *parent, int64_t n, int tile_m, int device, agpt_plan **out);
 /* The same with even tiles: each ends after tile_m rows, and attention over the plan takes the chunked kernels in both directions
- * whatever agpt_b200_set_attn_variant says (what the trainer's steps on a bfloat16 store run on). */
+ * whatever agpt_b200_set_attn_variant says (what the trainer's sampled steps on a bfloat16 store run on). */
 int agpt_b200_plan_create_even(const int32_t *parent, int64_t n, int tile_m, int device, agpt_plan **out);
 int agpt_b200_plan_info(const agpt_plan *p, agpt_plan_info *out);
 /* The sizes alone (array pointers NULL): the row arrays of a plan that came from runs of rows are derived when asked for. */

@@ -38,16 +38,17 @@ def test_even_plan_attention(parent, H, hd, bf16, tol):
         assert rel_err(a.cpu().numpy(), b.cpu().numpy(), floor=1.0) < tol, name
 
 
-def test_steps_on_a_bfloat16_store_walk_even_tiles():
+def test_sampled_groups_with_even_tiles():
     import torch
     trie = A.RadixTrie.build(A.synth_markov_corpus(2000, 12, 2, 3), 12)
-    (g,), _ = T.build_groups(trie, 0, 1, 1 << 20, "off", 32, torch.device("cuda", 0))
-    assert g.plan_for(False) is g.plan and g.plan.n_tiles > (g.n + 63) // 64
-    assert g.plan_for(True) is g.plan_for(True) and g.plan_for(True).n_tiles == (g.n + 63) // 64
     ids = trie.lightning_sample(2, 1, 7)[4]
-    for even in (False, True):
-        s = T.SampleSpace(trie).group(ids, [], "off", 32, torch.device("cuda", 0), even=even)
-        assert (s.plan_for(True) is s.plan) == even and s.plan_for(True).n_tiles == (s.n + 63) // 64
+    space = T.SampleSpace(trie)
+    for ranked in (True, False):                          # by runs, and over char positions
+        if not ranked:
+            space.rank = None
+        for even in (False, True):
+            s = space.group(ids, [], "off", 32, torch.device("cuda", 0), even=even)
+            assert s.even == even and (s.plan.n_tiles == (s.n + 63) // 64) == even
 
 
 @pytest.mark.parametrize("n,d,vocab", [(1, 32, 3), (2048, 64, 65), (2049, 36, 7), (20_000, 384, 96)])
