@@ -815,8 +815,8 @@ def set_attn_impl(impl: int) -> None:
 
 
 def set_attn_variant(whole_tile: bool = True, bwd_warps: int = 4) -> None:
-    """Tensor-core kernels for a float32 store and head_dim 32: the whole-tile pair (default) or the chunked pair;
-    warps per block of the whole-tile backward (4, 6 or 8)."""
+    """Tensor-core kernels: whole-tile (default) or chunked (both directions of a float32 store, the backward of a bfloat16
+    one); warps per block of the whole-tile backward (4, 6 or 8; 3: four warps, three blocks per SM)."""
     check(lib().agpt_b200_set_attn_variant(int(bool(whole_tile)), bwd_warps), "set_attn_variant")
 
 

@@ -77,9 +77,12 @@ struct agpt_trie {
 // A plan for a GPU with tiles of 64 lets a tile end early, where the next one starts at a shallow position: the chain that the
 // next tile loads again, and gives partial dK/dV rows for, is as long as its first position is deep, and a trie's depth-first
 // order comes back to shallow rows all the time.  The next start is the row k in [32, 64] after this one that makes
-// depth + 0.9 (64 - k) least, the later one of equals: a chain row costs about as much as a row left unfilled, and below a factor of 1
-// a run without branches, one deeper per row, is not worth walking along.  (On tries 0.25 to 0.9 choose the same starts; on bushy
-// trees smaller factors leave more tiles for little.  Tiles below 32 rows leave warps without rows.)  Keys per row on the depth-32 trie
+// depth + 0.9 (64 - k) least, the later one of equals: a chain row costs about as much as a row left unfilled.  The factor
+// stays below 1, because at 1 a run without branches, one deeper per row, leaves every end on it of one cost, the latest is taken and
+// next to nothing is cut: the 1.4M-row trie then takes 952 + 2152 us (forward, backward with reduction), at 0.95 907 + 1772.  From 0.5 to 0.95
+// times agree to 1 %, though the starts are not the same everywhere (on the 66k-row trie 1,066 tiles at 0.5, 1,061 from 0.75 on); smaller
+// factors leave more tiles for little, on bushy trees most (random tree of 600k nodes, 8 x 64: 1635 + 3350 us at 0.25, 1805 + 3644 at 0, 1591 +
+// 3303 at 0.9).  (Tiles below 32 rows leave warps without rows.)  Keys per row on the depth-32 trie
 // of 1.4M rows 1.27 -> 1.07, partial rows 0.27 -> 0.07 per row and their reduction 274 -> 81 us; forward 945 -> 901 us.
 struct agpt_plan {
     int64_t n = 0;

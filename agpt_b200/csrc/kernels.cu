@@ -904,14 +904,14 @@ __global__ void __launch_bounds__(128, HD <= 32 ? 4 : (sizeof(KVT) == 2 ? 3 : 1)
 // backward, whole tile resident: attn_bwd_tile_kernel.
 //
 // Operands.  The tile's Q and dO rows and every key row the tile can attend (ancestor chain + the tile's own
-// rows) are brought into shared memory ONCE (cp.async, raw float32) and converted in place to split half
+// rows) are loaded ONCE, through registers (TileStage), and stored to shared memory in split half
 // precision: x * s = hi + lo with hi, lo in fp16 and s a power of two chosen per (tile, head, tensor) so that the
 // largest |x * s| lies in [1, 2).  hi carries 11 bits, lo the next 11 (its own rounding is 2^-24 absolute at this
 // scale), so hi*hi + lo*hi + hi*lo reproduces the float32 product to about 2^-22 -- the accuracy of three TF32
 // products -- while each mma.sync.m16n8k16 contracts twice as many elements as a TF32 m16n8k8, every fragment
 // register carries two elements, and the operands take 4 bytes per element instead of 8.  The scales are exact
 // (powers of two) and are divided out of the results.  A converted row is 4 * head_dim bytes: the hi halves then the lo
-// halves, its 16-byte chunks XOR-swizzled with the row (chunk ^ row % 8), so that every fragment is one
+// halves, its 16-byte chunks XOR-swizzled with the row (row_swz), so that every fragment is one
 // conflict-free ldmatrix.x4: "along the row" fragments plain, "across rows" fragments with .trans.
 //
 // Work.  A warp takes key items (16 keys) from a shared counter: S^T = K Q^T and dP^T = V dO^T for the 16 keys against every
@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(128, HD <= 32 ? 4 : (sizeof(KVT) == 2 ? 3 : 1)
 // it.  After one barrier each warp takes 16 queries and sums dQ = dS K from those blocks.  Bound by issue slots: scores are computed
 // once, where computing them again with the queries as rows took 84 products per 16 x 16 block of head_dim 32 instead of 60 and the
 // exponentials twice.  A bfloat16 store's K and V are exact halves: four fifths of the products, and twice the keys in the same memory.  Measured: 4 x 32, 1.4M rows 2134 -> 1916 us; 8 x 64, 600k rows 4090 -> 3708 us;
-// bfloat16 store (with its reduction, against the chunked kernel or, for 32, single fp16 products): 578k rows of depth 32, 4 x 16 699 -> 528 us, 4 x 32 906 -> 675, 4 x 64 1644 -> 1378.
+// bfloat16 store (with its reduction, against the kernels of 11 bits before, chunked or, for 32, single fp16 products): 578k rows of depth 32, 4 x 16 699 -> 528 us, 4 x 32 906 -> 675, 4 x 64 1644 -> 1378.
 // Each output element is produced by exactly one warp in a fixed order, so results do not depend on which warp
 // took which item.
 // --------------------------------------------------------------------------------------
@@ -946,15 +946,16 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], u
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// The two 8-key (or 8-query) halves of a 16 x 16 block are independent chains of products.  Where BOTH_HALVES is set the
+// The two 8-query halves of a 16 x 16 block of the backward are independent chains of products.  At head_dim 64 the
 // half none of whose pairs is valid is computed too (its results are masked to exact zeros), so that the two chains sit
-// in one basic block and interleave; otherwise each half is skipped on its own.  Measured: head_dim 64 backward 35.9 ms
-// against 37.6 ms on the 4M-node tree (eight warps per SM: the interleaving pays); head_dim 32 backward 51.7 against 49.6
-// and forward 19.3 against 19.0 on the depth-32 trie (more spills, more warps to hide latency already).
+// in one basic block and interleave; otherwise each half is skipped on its own, as in the forward.  Measured when the scores were
+// still computed twice: head_dim 64 backward 35.9 ms against 37.6 ms on the 4M-node tree (eight warps per SM: the interleaving
+// pays); head_dim 32 backward 51.7 against 49.6 and forward 19.3 against 19.0 on the depth-32 trie (more spills, more warps to
+// hide latency already).
 #ifndef AGPT_TILE_BOTH_MIN_HD
 #define AGPT_TILE_BOTH_MIN_HD 64
 #endif
-template <int HD> struct TileBothHalves { static constexpr bool bwd = HD >= AGPT_TILE_BOTH_MIN_HD, fwd = false; };
+template <int HD> struct TileBothHalves { static constexpr bool value = HD >= AGPT_TILE_BOTH_MIN_HD; };
 // (x, y) -> packed fp16 pair hi (x in the low half) and the packed pair lo of the remainders.  LO_UP: the remainders
 // are stored times 2^11 (they are below 2^-11 |x|, so this keeps them in fp16's normal range and a small element keeps
 // its full 22 bits next to a large one); products with such a lo are accumulated apart and enter times 2^-11.
@@ -1308,7 +1309,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                 for (int u = 0; u < 2; u++) {
                     ds[u][0] = ds[u][1] = ds[u][2] = ds[u][3] = 0.f;
                     pw[u][0] = pw[u][1] = pw[u][2] = pw[u][3] = 0.f;
-                    if (!on[u] && !TileBothHalves<HD>::bwd) continue;                  // warp-uniform
+                    if (!on[u] && !TileBothHalves<HD>::value) continue;                  // warp-uniform
                     float c[4] = {0.f, 0.f, 0.f, 0.f}, cx[4] = {0.f, 0.f, 0.f, 0.f};
                     float e[4] = {0.f, 0.f, 0.f, 0.f}, ex[4] = {0.f, 0.f, 0.f, 0.f};
                     const int qr = qp * 16 + u * 8;
@@ -1437,7 +1438,7 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
 }
 
 // --------------------------------------------------------------------------------------
-// forward, whole tile resident: attn_fwd_tile_kernel (head_dim 32 or 64, float32 store).  Same staging, operand format and
+// forward, whole tile resident: attn_fwd_tile_kernel (head_dim 16, 32 or 64, float32 store).  Same operand format and
 // fragment addressing as attn_bwd_tile_kernel; one warp per 16 query rows (4 warps), online softmax over blocks of
 // 16 keys, O += P V with V read through ldmatrix.trans.
 // --------------------------------------------------------------------------------------
@@ -1447,7 +1448,8 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
 // elements (TileStage) reads them for the maxima and again for the conversion, and a row's owners, lanes of one warp, replace its raw pieces by the
 // halves, 16 bytes a store.  (Eight-byte stores, four to a bank, were a third of all shared-memory wavefronts, that pipe 78 % busy.
 // Rows through registers as in the backward: the loads in flight cost registers, and with them blocks; 1002 us.)  Measured: 4 x 32, 1.4M rows
-// 901 -> 883 us; 8 x 64, 600k rows 1719 (in chunks) -> 1600 us.
+// 901 -> 883 us; 8 x 64, 600k rows of depth 20 1719 (in chunks) -> 1600 us.  The full workloads' forwards did not move: 28.3M rows of depth 32
+// 18.99 -> 19.00 ms, and the 4M-node tree of depth 64 has tiles of 127 keys, which fwd_tile_fits leaves to the chunked kernel (15.0 ms).
 template <int HD> __device__ __forceinline__ int raw_swz(int r) { return HD == 16 ? (r >> 1) & 3 : r & 7; }
 template <int HD> struct FwdStage : TileStage<HD, 128> {
     typedef TileStage<HD, 128> Base;
@@ -1618,7 +1620,7 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const float *__restrict__ K, c
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             s2[u][0] = s2[u][1] = s2[u][2] = s2[u][3] = -INFINITY;
-            if (!on[u] && !TileBothHalves<HD>::fwd) continue;                  // warp-uniform
+            if (!on[u]) continue;                  // warp-uniform
             float c[4] = {0.f, 0.f, 0.f, 0.f}, cx[4] = {0.f, 0.f, 0.f, 0.f};
             const uint32_t rowb = (uint32_t)((kp * 16 + u * 8) * TILE_ROW_BYTES) + bRow;
 #pragma unroll
@@ -1694,8 +1696,8 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const float *__restrict__ K, c
 // Q scaled, and P -- is split into two bfloat16 parts (16 significant bits), so a product is two m16n8k16 MMAs, the cost of
 // the one TF32 product of 11 bits per factor that the chunked kernel issues.  Q fragments come straight from global memory.
 // One warp per 16 query rows, online softmax over blocks of 16 keys, 16 x 8 blocks without a valid pair skipped.
-// Bound by issue slots and, on shallow tries, by memory.  Measured (against the chunked TF32 kernel): 8 x 32, 577k rows
-// 636 -> 568 us; 6 x 64, 719k rows of depth up to 128, 1797 -> 1303 us.
+// Bound by latency and issue slots and, on shallow tries, by memory.  Measured against the chunked TF32 kernel over the same tiles: 8 x 32,
+// 577k rows 621 -> 583 us; 6 x 64, 719k rows of depth up to 128, 1946 -> 1420 us.
 // --------------------------------------------------------------------------------------
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -2079,8 +2081,10 @@ static bool rows_wide(int D, const void *a, const void *b, const void *c, const 
     return D % 8 == 0 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)e) & 31) == 0;
 }
 static inline int bwd_tile_maxk(const agpt_plan *p) { return (p->max_keys + 15) & ~15; }
-// Three blocks of the backward per SM at least (float32 rows of 32: four up to 96 keys, three up to 147), two of float32 rows of 64, whose
-// registers allow no more.  Beyond, the chunked kernel: bfloat16 rows of 64 with 140 keys a tile measured 2111 us with two blocks, 2007 in chunks.
+// Three blocks of the backward per SM at least, two of float32 rows of 64, whose registers allow no more: 160 keys a tile (bfloat16 192)
+// at head_dim 16, 144 at 32, 144 (bfloat16 96) at 64; the forward of a float32 store takes 384, 176, 112.  Beyond, the chunked kernel: bfloat16 rows of 64 with 140 keys a tile measured 2111 us with two blocks, 2007 in chunks.  A bfloat16 store's chunked backward
+// takes the lse of the whole-tile forward (16 bits of Q) and computes its own scores from 11: its gradients are off by 4.2e-4 (2-norm, against
+// float64 over the rounded rows, a chain of 230), and by 4.1e-4 behind the chunked forward.
 static inline bool bwd_tile_fits(const agpt_plan *p, int head_dim, bool bf16) {
     if (head_dim != 16 && head_dim != 32 && head_dim != 64) return false;
     return bwd_tile_smem_bytes(head_dim, bwd_tile_maxk(p), bf16) <= (head_dim == 64 && !bf16 ? (size_t)113 * 1024 : (size_t)75 * 1024);
@@ -2131,7 +2135,7 @@ static int launch_fwd_mma(const agpt_plan *p, const float *q, const void *k, con
 static int fwd_dispatch(const agpt_plan *p, const float *q, const void *k, const void *v, int kv_dtype, float *out,
                         float *lse, int H, int head_dim, float scale, cudaStream_t st, int tile0, int ntiles) {
     if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_F32 && tile_kernels_wanted(p, kv_dtype) && fwd_tile_fits(p, head_dim)) {
-        // head_dim 32: AGPT_B200_FWD_BLOCKS=5 for five blocks per SM instead of six (A/B runs)
+        // head_dim 32: AGPT_B200_FWD_BLOCKS=5 for five blocks per SM instead of six (A/B runs; 956 against 906 us on 1.4M rows)
         static const bool five = [] { const char *e = getenv("AGPT_B200_FWD_BLOCKS"); return e && atoi(e) == 5; }();
         switch (head_dim) {
             case 16: return launch_fwd_tile<16, 8>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
@@ -2140,7 +2144,7 @@ static int fwd_dispatch(const agpt_plan *p, const float *q, const void *k, const
             case 64: return launch_fwd_tile<64, 3>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
         }
     }
-    // bfloat16 store: whole tiles while two blocks of them fit one SM (head_dim 64: up to 438 keys), deeper plans in chunks
+    // bfloat16 store: whole tiles while two blocks of them fit one SM (head_dim 64: up to 432 keys), deeper plans in chunks
     if (attn_impl() == 1 && p->tile_m == 64 && kv_dtype == AGPT_KV_BF16 && !p->even && tile_bf16_enabled() &&
         fwd_bf16_smem_bytes(head_dim, bwd_tile_maxk(p)) <= (size_t)113 * 1024) {
         switch (head_dim) {
@@ -2200,6 +2204,8 @@ static int launch_bwd_tile_w(const agpt_plan *p, const float *q, const void *k, 
         default: return launch_bwd_tile<64, 4, 3, __nv_bfloat16>(TILE_ARGS);
     }
     if (head_dim == 16) return launch_bwd_tile<16, 4, 4>(TILE_ARGS);
+    // Four warps are the fastest (with the reduction, us: 4 x 32, 1.4M rows 1771; three blocks of four 2084, six warps 2477, eight 2793; 8 x 64,
+    // 600k rows 3305, eight warps 5124): small blocks stage, compute and wait out of step.  The others stay for A/B runs of the public switch.
     if (head_dim == 64) {        // twice the fragment and accumulator registers: two blocks per SM
         switch (g_bwd_warps) {
             case 6: case 8: return launch_bwd_tile<64, 8, 1>(TILE_ARGS);

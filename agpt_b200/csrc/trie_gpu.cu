@@ -66,6 +66,9 @@ int64_t suffix_workspace(int64_t n, int end_bit) {
     if (cub::DeviceRadixSort::SortPairs(nullptr, tmp, (DT *)nullptr, (DT *)nullptr, (int32_t *)nullptr, (int32_t *)nullptr, m, 0, end_bit) != cudaSuccess) return -1;
     return up256(n * 4) + 3 * up256((int64_t)m * 4) + 2 * up256((int64_t)m * sizeof(DT)) + (int64_t)tmp + 256;
 }
+// Digits of 64 bits hold nine tokens of 65 symbols and save passes, for 8 bytes a position instead of 1 or 2 in both digit arrays and in the sort's own.
+// They are the faster ones on both sides of this line (device ms at 33 tokens a key, wide / narrow: 20,000 positions 0.46 / 0.94, 60,000 0.48 / 0.99,
+// 1M 0.84 / 1.32, 4M 2.1 / 2.9, 10M 4.7 / 5.7); it bounds the memory, at a size where a millisecond no longer shows beside the host's assembly.
 constexpr int64_t WIDE_DIGITS_BELOW = 4 << 20;
 template <typename DT>
 int sort_suffixes(const int32_t *corpus, int64_t n, int32_t m, int key_len, int bits, int per_digit, cudaStream_t st, cudaEvent_t e0, cudaEvent_t e1,

@@ -98,8 +98,8 @@ def test_micro_s_subtrees_match_oracle(cuda, variant):
 
 @pytest.mark.parametrize("shape", ["c2s", "shallow"])
 def test_bf16_store_whole_tile_backward_agrees_with_chunked_kernel(cuda, shape):
-    """bfloat16 store, head_dim 32: the whole-tile backward rounds Q, dO, P and dS to fp16 (single products); the chunked
-    kernel keeps float32-level products on the same rounded store.  The two must agree to the fp16 rounding, well inside
+    """bfloat16 store, head_dim 32: the whole-tile backward keeps Q, dO, P and dS as two fp16 parts; the chunked kernel rounds
+    them to TF32 (11 bits) in single products on the same rounded store.  The two must agree to that rounding, well inside
     the store's own 2e-2 tolerance."""
     if shape == "c2s":
         parent, H, hd, q, k, v, go, _, _ = _c2s()
