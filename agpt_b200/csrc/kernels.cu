@@ -2082,8 +2082,9 @@ static bool rows_wide(int D, const void *a, const void *b, const void *c, const 
 }
 static inline int bwd_tile_maxk(const agpt_plan *p) { return (p->max_keys + 15) & ~15; }
 // Three blocks of the backward per SM at least, two of float32 rows of 64, whose registers allow no more: 160 keys a tile (bfloat16 192)
-// at head_dim 16, 144 at 32, 144 (bfloat16 96) at 64; the forward of a float32 store takes 384, 176, 112.  Beyond, the chunked kernel: bfloat16 rows of 64 with 140 keys a tile measured 2111 us with two blocks, 2007 in chunks.  A bfloat16 store's chunked backward
-// takes the lse of the whole-tile forward (16 bits of Q) and computes its own scores from 11: its gradients are off by 4.2e-4 (2-norm, against
+// at head_dim 16, 144 at 32, 144 (bfloat16 96) at 64; the forward of a float32 store takes 384, 176, 112.  Beyond, the chunked kernel:
+// bfloat16 rows of 64 with 140 keys a tile measured 2111 us with two blocks, 2007 in chunks.  A bfloat16 store's chunked backward takes the
+// lse of the whole-tile forward (16 bits of Q) and computes its own scores from 11: its gradients are off by 4.2e-4 (2-norm, against
 // float64 over the rounded rows, a chain of 230), and by 4.1e-4 behind the chunked forward.
 static inline bool bwd_tile_fits(const agpt_plan *p, int head_dim, bool bf16) {
     if (head_dim != 16 && head_dim != 32 && head_dim != 64) return false;

@@ -15,6 +15,7 @@ process group.  Model files (MGPT) and radix trie directories are read and writt
 from __future__ import annotations
 
 import argparse
+import operator
 import os
 import time
 
@@ -22,6 +23,8 @@ import numpy as np
 
 from . import api as A
 from . import model_file as MF
+
+_dtype_of, _shape_of = operator.attrgetter("dtype"), operator.attrgetter("shape")
 
 
 class LaunchGroup:
@@ -332,7 +335,7 @@ class TrieWalkModel:
             p = self.flat[o:o + a.size].view(a.shape)
             p.copy_(torch.from_numpy(np.ascontiguousarray(a)))
             self.params[name] = p.requires_grad_(True)
-        self._offs, self._shapes = offs, [torch.Size(a.shape) for _, a in model.mats]
+        self._offs, self._shapes = offs, [torch.Size(a.shape) for _, a in model.mats] * 2
         self.bind_grads()
         hd = model.d_model // model.n_heads
         cos, sin = A.rope_table(model.seq_len, hd)
@@ -354,10 +357,10 @@ class TrieWalkModel:
 
     def bind_grads(self):
         """Make every parameter's .grad the matching slice of the flat gradient buffer (autograd accumulates in place)."""
+        base = self.flat_grad.data_ptr()
         for p, o in zip(self.params.values(), self._offs):
-            want = self.flat_grad[o:o + p.numel()].view(p.shape)
-            if p.grad is None or p.grad.data_ptr() != want.data_ptr():
-                p.grad = want
+            if p.grad is None or p.grad.data_ptr() != base + 4 * o:
+                p.grad = self.flat_grad[o:o + p.numel()].view(p.shape)
 
     def to_model_file(self) -> MF.Model:
         m = self.cfg
@@ -421,17 +424,20 @@ class TrieWalkModel:
         m = self.cfg
         return self.dense_impl == "tensor" and bool(A.lib().agpt_b200_train_step_takes(m.d_model, m.n_heads, m.d_ff, m.vocab))
 
-    def _step_tensors_plain(self) -> bool:
-        """The native step reads parameters and adds to gradients by address: float32, contiguous, of the model file's shape and on
-        the model's device.  Anything else steps on the tape, which reads the tensors themselves."""
+    def _step_addresses(self):
+        """Addresses of the parameters, then of their gradients, for the native step, which reads and adds by address: float32, contiguous,
+        on 16-byte boundaries, of the model file's shape and on the model's device.  None where one is not; the step then runs on the tape, which reads the
+        tensors themselves.  Looked at whole for every step (a storage may be replaced under a tensor), 25 us for two layers."""
         import torch
-        index, plain = self.flat.get_device(), True
-        for p, shape in zip(self.params.values(), self._shapes):
+        t = list(self.params.values())
+        for p in t:
             if p.grad is None:
                 p.grad = torch.zeros_like(p)
-            for t in (p, p.grad):
-                plain = plain and t.dtype is torch.float32 and t.get_device() == index and t.shape == shape and t.is_contiguous()
-        return plain
+        t += [p.grad for p in t]
+        if not all(map(torch.Tensor.is_contiguous, t)) or set(map(_dtype_of, t)) != {torch.float32} or list(map(_shape_of, t)) != self._shapes:
+            return None
+        at = list(map(torch.Tensor.data_ptr, t))
+        return at if set(map(torch.Tensor.get_device, t)) == {self.flat.get_device()} and not any(x & 15 for x in at) else None
 
     def group_step(self, group: LaunchGroup, counts, entropy_lambda=0.0, intermediate_weight=1.0, ce_only=False,
                    bf16_store=False, sync=True, tape=False):
@@ -440,8 +446,9 @@ class TrieWalkModel:
         float32 device tensor (loss sum, count // 4096, count % 4096), so that the host does not wait for the device
         between groups.  tape: step by single operations even where the native step takes the model."""
         import torch
-        if not tape and self.native_step_available() and self._step_tensors_plain():
-            return self._native_step(group, counts, entropy_lambda, intermediate_weight, ce_only, bf16_store, sync)
+        at = self._step_addresses() if not tape and self.native_step_available() else None
+        if at is not None:
+            return self._native_step(at, group, counts, entropy_lambda, intermediate_weight, ce_only, bf16_store, sync)
         logits = self.logits(group, bf16_store).contiguous()
         c_off, c_tok, c_val = counts
         if logits.shape[1] != self.cfg.vocab:
@@ -474,22 +481,19 @@ class TrieWalkModel:
         return torch.stack([loss_sum.to(torch.float32), (n_trained // 4096).to(torch.float32), (n_trained % 4096).to(torch.float32)])
 
 
-    def _native_step(self, group, counts, entropy_lambda, intermediate_weight, ce_only, bf16_store, sync):
+    def _native_step(self, at, group, counts, entropy_lambda, intermediate_weight, ce_only, bf16_store, sync):
         """group_step as one call of the library (agpt_b200_train_step): no tape, no host decision between the kernels."""
         import ctypes as C
 
         import torch
-        n = len(self.params)
-        # addresses are those of this call: the storage of a parameter or a gradient may be another than at the last step
-        params = (C.c_void_p * n)(*[p.data_ptr() for p in self.params.values()])
-        grads = (C.c_void_p * n)(*[p.grad.data_ptr() for p in self.params.values()])
+        addresses, n = (C.c_void_p * len(at))(*at), len(at) // 2
         for c in counts:
             if c.dtype != torch.int32 or not c.is_cuda or not c.is_contiguous():
                 raise A.AgptError("counts must be contiguous int32 CUDA tensors")
         m, out = self.cfg, torch.empty(8, dtype=torch.float32, device=self.device)
         a = group.step_args()
         a.d_model, a.n_heads, a.n_layers, a.d_ff, a.vocab, a.seq_len = m.d_model, m.n_heads, m.n_layers, m.d_ff, m.vocab, m.seq_len
-        a.params, a.grads = C.addressof(params), C.addressof(grads)
+        a.params, a.grads = C.addressof(addresses), C.addressof(addresses) + n * C.sizeof(C.c_void_p)
         a.counts_offset, a.counts_tok, a.counts_val = [c.data_ptr() for c in counts]
         a.cosv, a.sinv = self.cos.data_ptr(), self.sin.data_ptr()
         a.entropy_lambda, a.intermediate_weight, a.ce_only = entropy_lambda, intermediate_weight, int(ce_only)

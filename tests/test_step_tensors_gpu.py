@@ -58,6 +58,24 @@ def test_replaced_gradient_storage(cuda):
     assert torch.equal(old, kept)
 
 
+def test_what_the_native_step_reads_by_address(cuda):
+    import torch
+    model, _, _ = _setup(cuda)
+    n = len(model.params)
+    at = model._step_addresses()
+    assert at[:n] == [p.data_ptr() for p in model.params.values()] and at[n:] == [p.grad.data_ptr() for p in model.params.values()]
+    p = model.params["layer0.wo.w"]
+    plain = p.data
+    for other in (torch.zeros(plain.numel() + 1, device=cuda)[1:].view(plain.shape), plain.t(), plain.double(), plain.cpu(), plain[:32]):
+        p.grad = None
+        p.data = other
+        p.grad = None if other.device != plain.device else torch.zeros_like(other)
+        assert model._step_addresses() is None
+    p.grad = None
+    p.data = plain
+    assert model._step_addresses()[:n] == at[:n]
+
+
 def test_strided_gradient_and_missing_gradient(cuda):
     import torch
     model, g, counts = _setup(cuda)
