@@ -51,6 +51,22 @@ def test_sampled_groups_with_even_tiles():
             assert s.even == even and (s.plan.n_tiles == (s.n + 63) // 64) == even
 
 
+@pytest.mark.parametrize("bf16", [False, True])
+def test_even_plan_from_host_buffers(bf16):
+    """The chunked host-buffer step reduces a node when the last of its tiles is done, whole: several chunks, a subtree over all of them."""
+    import torch
+    parent, H, hd = _wide(64 * 260), 5, 32
+    plan = A.WalkerPlan(parent, 64, 0, even=True)
+    rng = np.random.default_rng(2)
+    q, k, v, do = [rng.standard_normal((len(parent), H * hd)).astype(np.float32) for _ in range(4)]
+    got = A.attn_fwd_bwd_host(plan, q, k, v, do, H, A.KV_BF16 if bf16 else A.KV_F32)
+    tq, tk, tv, td = [torch.from_numpy(x).cuda() for x in (q, k, v, do)]
+    ks, vs = (A.kv_store_write_bf16(tk), A.kv_store_write_bf16(tv)) if bf16 else (tk, tv)
+    o, lse = A.attn_forward(plan, tq, ks, vs, H)
+    for name, a, b in zip(("out", "lse", "dq", "dk", "dv"), got, (o, lse, *A.attn_backward(plan, tq, ks, vs, o, lse, td, H))):
+        assert np.array_equal(a, b.cpu().numpy()), name
+
+
 @pytest.mark.parametrize("n,d,vocab", [(1, 32, 3), (2048, 64, 65), (2049, 36, 7), (20_000, 384, 96)])
 def test_serial_embedding_gradient(n, d, vocab):
     import torch
