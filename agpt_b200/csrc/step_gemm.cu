@@ -103,6 +103,13 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
+// two barriers asked for at once (the latencies of two polls overlap)
+__device__ __forceinline__ bool warp_wait2(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, volatile int *abort_flag) {
+    const bool d0 = mbar_try(b0, p0), d1 = mbar_try(b1, p1);
+    if (__all_sync(0xffffffffu, d0 && d1)) return true;
+    return warp_wait(b0, p0, abort_flag) && warp_wait(b1, p1, abort_flag);
+}
+
 // the six partial products, small ones first
 __device__ __forceinline__ void six_products(uint32_t d, uint32_t a, uint32_t b, uint32_t b_plane16, uint32_t b_step16, uint32_t idesc) {
     constexpr int PA[6] = {1, 0, 2, 0, 1, 0}, PB[6] = {1, 2, 0, 1, 0, 0};
@@ -187,8 +194,9 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
     uint32_t &s_tmem = *reinterpret_cast<uint32_t *>(smem + P.off_bar + BAR_BYTES - 8);
     float *s_bias = reinterpret_cast<float *>(smem + P.off_bias);
     float4 *s_rope = reinterpret_cast<float4 *>(smem + P.off_rope);       // per pair of columns {cos, cos, -sin, sin}
-    // barriers: A stages full / empty, B stages full / empty, tensor-memory A stages full / empty, accumulators full / empty
-    const uint32_t aF = bars, aE = aF + 8 * P.n_a, bF = aE + 8 * P.n_a, bE = bF + 8 * P.n_b, tF = bE + 8 * P.n_b, tE = tF + 16, cF = tE + 16, cE = cF + 16, oF = cE + 16;
+    // barriers: A stages full / empty, B stages full / empty, tensor-memory A stages full / empty, accumulators full / empty (a pair for each
+    // group of accumulator warps and accumulator)
+    const uint32_t aF = bars, aE = aF + 8 * P.n_a, bF = aE + 8 * P.n_a, bE = bF + 8 * P.n_b, tF = bE + 8 * P.n_b, tE = tF + 16, cF = tE + 16, cE = cF + 32, oF = cE + 32;
     const int n_tile = blockIdx.x % P.n_tiles, n0 = n_tile * P.nt;
     const int64_t slot = blockIdx.x / P.n_tiles, n_slots = gridDim.x / P.n_tiles;
     const int nt_mma = (min(P.nt, g.N - n0) + 15) & ~15;
@@ -197,8 +205,9 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
     if (tid == 0) {
         s_abort = 0;
         for (int i = 0; i < P.n_a; i++) { mbar_init(aF + 8 * i, 1); mbar_init(aE + 8 * i, 4); }
-        for (int i = 0; i < P.n_b; i++) { mbar_init(bF + 8 * i, 1); mbar_init(bE + 8 * i, 1); }
-        for (int i = 0; i < 2; i++) { mbar_init(tF + 8 * i, 4); mbar_init(tE + 8 * i, 1); mbar_init(cF + 8 * i, 1); mbar_init(cE + 8 * i, 4); }
+        for (int i = 0; i < P.n_b; i++) { mbar_init(bF + 8 * i, 1); mbar_init(bE + 8 * i, P.unit_tiles); }
+        for (int i = 0; i < 2; i++) { mbar_init(tF + 8 * i, 4); mbar_init(tE + 8 * i, 1); }
+        for (int i = 0; i < 4; i++) { mbar_init(cF + 8 * i, 1); mbar_init(cE + 8 * i, 4); }
         for (int i = 0; i < 16; i++) mbar_init(oF + 8 * i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -257,43 +266,58 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
                 for (int i = 0; i < P.n_a; i++) { volatile int none = 0; mbar_wait(aF + 8 * i, ap, &none); }
                 for (int i = 0; i < P.n_b; i++) { volatile int none = 0; mbar_wait(bF + 8 * i, bp, &none); }
             }
-        } else if (warp == 1) {
-            // ---------------- MMAs (the warp stays converged, one elected lane issues: 29 clocks per MMA instead of 60) ----------------
-            const uint32_t idesc = idesc_bf16(nt_mma, false);
-            int ts = 0, bs = 0;
-            uint32_t tp = 0, bp = 0, cp0 = 0, cp1 = 0;
+        } else if (warp == 1 || warp == 2) {
+            // ---------------- MMAs ----------------
+            // A warp per accumulator: a wait costs an issuing warp 140 to 170 clocks even where the barrier is complete, and the tensor pipe
+            // queues no more than two or three MMAs, so that one warp alone left it idle for a quarter of the time (24 MMAs of 128 columns behind
+            // two waits: 1951 clocks, two warps in turn 1557, the pipe's own 1536).  A warp stays converged, one elected lane issues (29 clocks
+            // per MMA instead of 60).  Two row tiles per unit: a warp per tile.  One: the k blocks alternate, and the group of accumulator warps
+            // that owns the tile reads both accumulators in turn.
+            const int own = warp - 1;
+            const bool pair = P.unit_tiles == 2;
+            const uint32_t idesc = idesc_bf16(nt_mma, false), acc = tmem + own * ACC_COLS;
+            int bs = 0, last = -1;                          // last: the group that reads what this accumulator held before
+            uint32_t bp = 0, seen = 0, step = 0, uses[2] = {0, 0};
             int64_t iter = 0;
             bool ok = true;
             for (int64_t u = slot; ok && u < P.units; u += n_slots, iter++) {
                 const int T = (int)min((int64_t)P.unit_tiles, P.row_tiles - u * P.unit_tiles);
-                for (int kb = 0; ok && kb < P.kb; kb++) {
-                    if (P.stationary) {
-                        bs = kb;
-                        if (iter == 0 && !(ok = warp_wait(bF + 8 * bs, 0, &s_abort))) break;
-                    } else if (!(ok = warp_wait(bF + 8 * bs, bp, &s_abort))) break;
-                    const uint32_t bd = desc_lo(sB + bs * b_stage, 16);
-                    for (int t = 0; t < T; t++) {
-                        const int a = P.unit_tiles == 2 ? t : (int)(iter & 1);
-                        if (!(ok = warp_wait(cE + 8 * a, (a ? cp1 : cp0) ^ 1, &s_abort))) break;
-                        if (a) cp1 ^= 1; else cp0 ^= 1;
-                        if (!(ok = warp_wait(tF + 8 * ts, tp, &s_abort))) break;
+                for (int kb = 0; ok && kb < P.kb; kb++, step += T) {
+                    const uint32_t s = pair ? step + own : step, ts = s & 1;
+                    const int grp = pair ? own : (int)(iter & 1);
+                    if (pair ? own < T : (int)ts == own) {
+                        if (P.stationary) {
+                            bs = kb;
+                            if (!((seen >> kb) & 1) && !(ok = warp_wait(bF + 8 * bs, 0, &s_abort))) break;
+                            seen |= 1u << kb;
+                        } else if (!(ok = warp_wait(bF + 8 * bs, bp, &s_abort))) break;
+                        if (last >= 0) ok = warp_wait2(cE + 8 * (2 * last + own), ((last ? uses[1] : uses[0]) - 1) & 1, tF + 8 * ts, (s >> 1) & 1, &s_abort);
+                        else ok = warp_wait(tF + 8 * ts, (s >> 1) & 1, &s_abort);
+                        if (!ok) break;
                         fence_after();
                         if (elect_one()) {
-                            six_products(tmem + a * ACC_COLS, tmem + 2 * ACC_COLS + ts * TA_COLS, bd, b_plane >> 4, 2, idesc);
+                            six_products(acc, tmem + 2 * ACC_COLS + ts * TA_COLS, desc_lo(sB + bs * b_stage, 16), b_plane >> 4, 2, idesc);
                             commit(tE + 8 * ts);
-                            commit(cF + 8 * a);
-                            if (!P.stationary && t + 1 == T) commit(bE + 8 * bs);
+                            commit(cF + 8 * (2 * grp + own));
+                            if (!P.stationary) commit(bE + 8 * bs);
                         }
                         __syncwarp();
-                        if (++ts == 2) { ts = 0; tp ^= 1; }
+                        last = grp;
+                        if (grp) uses[1]++; else uses[0]++;
+                    } else if (pair && !P.stationary) {
+                        // The last unit has one tile; this is the other warp's share of the stage.  It waits as if it read it: an arrival a phase
+                        // early would free the stage under the first warp.
+                        if (!(ok = warp_wait(bF + 8 * bs, bp, &s_abort))) break;
+                        if (lane == 0) mbar_arrive(bE + 8 * bs);
+                        __syncwarp();
                     }
                     if (!P.stationary && ++bs == P.n_b) { bs = 0; bp ^= 1; }
                 }
             }
             if (!ok && elect_one()) {                          // MMAs in flight finish before tensor memory is released
-                commit(tE);
+                commit(tE + 8 * own);
                 volatile int none = 0;
-                for (int i = 0; i < 2; i++) mbar_wait(tE, i, &none);
+                for (int i = 0; i < 2; i++) mbar_wait(tE + 8 * own, i, &none);
             }
             __syncwarp();
         }
@@ -326,9 +350,13 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
                 for (int t = 0; t < T; t++) {
                     const f2 mn = f2_same(-(t ? mean[1] : mean[0])), ml = f2_same(t ? mul[1] : mul[0]);
                     const uint32_t dst = tmem + 2 * ACC_COLS + ts * TA_COLS + lane_base;
+                    // both boxes and the place in tensor memory are asked for at once: three waits one after the other took 500 clocks of a step
+                    const int as1 = as + 1 == P.n_a ? 0 : as + 1;
+                    const uint32_t ap1 = as1 ? ap : ap ^ 1;
+                    const bool full0 = mbar_try(aF + 8 * as, ap), full1 = mbar_try(aF + 8 * as1, ap1), room = mbar_try(tE + 8 * ts, tp ^ 1);
 #pragma unroll
                     for (int j = 0; j < 2; j++) {
-                        if (!(ok = warp_wait(aF + 8 * as, ap, &s_abort))) break;
+                        if (!__all_sync(0xffffffffu, j ? full1 : full0) && !(ok = warp_wait(aF + 8 * as, ap, &s_abort))) break;
                         const uint32_t src = sA + as * A_BOX + row * 128;
                         uint32_t p[3][16];
 #pragma unroll
@@ -343,7 +371,7 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
                         if (lane == 0) mbar_arrive(aE + 8 * as);
                         if (++as == P.n_a) { as = 0; ap ^= 1; }
                         if (j == 0) {
-                            if (!(ok = warp_wait(tE + 8 * ts, tp ^ 1, &s_abort))) break;
+                            if (!__all_sync(0xffffffffu, room) && !(ok = warp_wait(tE + 8 * ts, tp ^ 1, &s_abort))) break;
                             fence_after();
                         }
 #pragma unroll
@@ -364,7 +392,7 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
         // Rows enter and leave through the warp's two staging buffers (32 rows x 32 columns, swizzled) by TMA: a thread owns
         // a row, and 32-byte accesses to 32 different rows per instruction held the whole block up.
         const int grp = warp >= 12, wrow = (warp & 3) * 32 + lane;
-        const uint32_t acc_addr = tmem + grp * ACC_COLS + ((uint32_t)(warp & 3) << 21);
+        const uint32_t acc_addr = tmem + ((uint32_t)(warp & 3) << 21);
         unsigned char *stg = smem + P.off_out + (warp - 8) * 8192;
         const uint32_t u_stg = smem_u32(stg), lF = oF + (warp - 8) * 16;
         const int sw = lane & 7;
@@ -374,7 +402,7 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
             mbar_expect(lF + 8 * buf, 4096);
             tma_load_2d(u_stg + buf * 4096, m, x, y, lF + 8 * buf);
         };
-        uint32_t cp = 0;
+        uint32_t cp = 0;                                  // phases of this group's two accumulators
         int64_t iter = 0;
         bool ok = true;
         for (int64_t u = slot; ok && u < P.units; u += n_slots, iter++) {
@@ -397,21 +425,22 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
 #pragma unroll
             for (int i = 0; i < ACC_COLS / 2; i++) acc[i] = *reinterpret_cast<const f2 *>(s_bias + 2 * i);
             for (int kb = 0; kb < P.kb; kb++) {
-                if (!(ok = warp_wait(cF + 8 * grp, cp, &s_abort))) break;
-                cp ^= 1;
+                const int a = P.unit_tiles == 2 ? grp : (int)((iter * P.kb + kb) & 1);
+                if (!(ok = warp_wait(cF + 8 * (2 * grp + a), (cp >> a) & 1, &s_abort))) break;
+                cp ^= 1u << a;
                 fence_after();
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     if (c * 32 < nt_mma) {
                         uint32_t v[32];
-                        tmem_ld32(acc_addr + c * 32, v);
+                        tmem_ld32(acc_addr + a * ACC_COLS + c * 32, v);
 #pragma unroll
                         for (int i = 0; i < 16; i++) acc[c * 16 + i] = f2_add(acc[c * 16 + i], f2_pack(v[2 * i], v[2 * i + 1]));
                     }
                 }
                 fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(cE + 8 * grp);
+                if (lane == 0) mbar_arrive(cE + 8 * (2 * grp + a));
             }
             if (!ok) break;
             // epilogue of the tile
@@ -633,7 +662,7 @@ int agpt_row_gemm(const RowGemm &g, cudaStream_t st) {
     P.n_b = P.stationary ? P.kb : 2;
     if (P.n_b > 16) { P.stationary = 0; P.n_b = 2; }
     P.n_a = std::min(8, (room - P.n_b * b_stage) / A_BOX);
-    if (P.n_a < 1) return agpt_set_error(AGPT_E_LIMIT, "row_gemm: no shared memory left for the rows");
+    if (P.n_a < 2) return agpt_set_error(AGPT_E_LIMIT, "row_gemm: no shared memory left for the rows");
     P.off_b = (uint32_t)(P.n_a * A_BOX);
     P.off_out = P.off_b + (uint32_t)(P.n_b * b_stage);
     P.off_bias = P.off_out + OUT_BYTES;
@@ -753,7 +782,7 @@ contract_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ 
         s_abort = 0;
         for (int i = 0; i < 2; i++) {
             mbar_init(aF + 8 * i, 1); mbar_init(aE + 8 * i, 4); mbar_init(bF + 8 * i, 1); mbar_init(bE + 8 * i, 4);
-            mbar_init(pF + 8 * i, 4); mbar_init(pE + 8 * i, 1); mbar_init(tF + 8 * i, 4); mbar_init(tE + 8 * i, 1);
+            mbar_init(pF + 8 * i, 4); mbar_init(pE + 8 * i, 1); mbar_init(tF + 8 * i, 4); mbar_init(tE + 8 * i, halves);
             mbar_init(cF + 8 * i, 1); mbar_init(cE + 8 * i, 4);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -795,35 +824,29 @@ contract_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ 
                 volatile int none = 0;
                 for (int i = 0; i < 2; i++) { mbar_wait(aF + 8 * i, ap, &none); mbar_wait(bF + 8 * i, bp, &none); }
             }
-        } else if (warp == 1) {
-            // ---------------- MMAs ----------------
-            int ts = 0, ps = 0;
-            uint32_t tp = 0, pp = 0, cp = 0;               // each accumulator is used once per row block
-            const uint32_t id0 = idesc_bf16((w0 + 15) & ~15, true), id1 = idesc_bf16((w1 + 15) & ~15, true);
+        } else if (warp >= 1 && warp <= halves) {
+            // ---------------- MMAs: a warp per accumulator (see row_gemm_kernel) ----------------
+            const int h = warp - 1;
+            const uint32_t idesc = idesc_bf16(((h ? w1 : w0) + 15) & ~15, true);
+            uint32_t i = 0;                                // each accumulator is used once per row block
             bool ok = true;
-            for (int64_t rb = rb0; ok && rb < rb1; rb++) {
-                if (!(ok = warp_wait(tF + 8 * ts, tp, &s_abort))) break;
-                for (int h = 0; h < halves; h++) {
-                    if (!(ok = warp_wait(cE + 8 * h, cp ^ 1, &s_abort))) break;
-                    if (!(ok = warp_wait(pF + 8 * ps, pp, &s_abort))) break;
-                    fence_after();
-                    if (elect_one()) {
-                        six_products(tmem + h * ACC_COLS, tmem + 2 * ACC_COLS + ts * TA_COLS, desc_lo(sP + ps * CON_P, 8192), 1024, 128,
-                                     h ? id1 : id0);
-                        commit(pE + 8 * ps);
-                        if (h + 1 == halves) commit(tE + 8 * ts);
-                        commit(cF + 8 * h);
-                    }
-                    __syncwarp();
-                    if (++ps == 2) { ps = 0; pp ^= 1; }
+            for (int64_t rb = rb0; ok && rb < rb1; rb++, i++) {
+                const uint32_t ts = i & 1, s = halves == 2 ? 2 * i + h : i, ps = s & 1;
+                if (!(ok = warp_wait2(tF + 8 * ts, (i >> 1) & 1, cE + 8 * h, (i & 1) ^ 1, &s_abort))) break;
+                if (!(ok = warp_wait(pF + 8 * ps, (s >> 1) & 1, &s_abort))) break;
+                fence_after();
+                if (elect_one()) {
+                    six_products(tmem + h * ACC_COLS, tmem + 2 * ACC_COLS + ts * TA_COLS, desc_lo(sP + ps * CON_P, 8192), 1024, 128, idesc);
+                    commit(pE + 8 * ps);
+                    commit(tE + 8 * ts);
+                    commit(cF + 8 * h);
                 }
-                cp ^= 1;
-                if (++ts == 2) { ts = 0; tp ^= 1; }
+                __syncwarp();
             }
             if (!ok && elect_one()) {
-                commit(tE);
+                commit(pE + 8 * h);
                 volatile int none = 0;
-                for (int i = 0; i < 2; i++) mbar_wait(tE, i, &none);
+                for (int j = 0; j < 2; j++) mbar_wait(pE + 8 * h, j, &none);
             }
             __syncwarp();
         }
@@ -838,8 +861,7 @@ contract_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ 
 #pragma unroll
         for (int i = 0; i < 8; i++) at[i] = i * 128 + (((lane >> 2) ^ i) << 4) + ((lane & 3) << 2);
         for (int64_t rb = rb0; rb < rb1; rb++) {
-            if (!warp_wait(aF + 8 * as, ap, &s_abort)) break;
-            if (!warp_wait(tE + 8 * ts, tp ^ 1, &s_abort)) break;
+            if (!warp_wait2(aF + 8 * as, ap, tE + 8 * ts, tp ^ 1, &s_abort)) break;
             fence_after();
             if (live) {
                 const uint32_t src = sA + as * CON_A + wq * 8192;
@@ -893,8 +915,7 @@ contract_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ 
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 if (h >= halves) break;
-                if (!(ok = warp_wait(bF + 8 * bs, bp, &s_abort))) break;
-                if (!(ok = warp_wait(pE + 8 * ps, pp ^ 1, &s_abort))) break;
+                if (!(ok = warp_wait2(bF + 8 * bs, bp, pE + 8 * ps, pp ^ 1, &s_abort))) break;
                 const int nb = ((h ? w1 : w0) + 31) >> 5;
                 if (box < nb) {
                     const uint32_t dst = put + ps * CON_P, src = get + bs * CON_B;
