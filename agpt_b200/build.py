@@ -54,7 +54,7 @@ def cutlass_include():
     return None
 
 
-HEADERS = [os.path.join(HERE, "csrc", "internal.h"), os.path.join(HERE, "csrc", "step_gemm.h"), os.path.join(HERE, "csrc", "tc100.cuh"), os.path.join(HERE, "..", "include", "agpt_b200.h")]
+HEADERS = [os.path.join(HERE, "csrc", "internal.h"), os.path.join(HERE, "csrc", "step_gemm.h"), os.path.join(HERE, "csrc", "tc100.cuh"), os.path.join(HERE, "csrc", "pdl.cuh"), os.path.join(HERE, "..", "include", "agpt_b200.h")]
 
 
 OBJ_DIR = os.path.join(HERE, "_build")

@@ -19,6 +19,7 @@
 
 #include "../../include/agpt_b200.h"
 #include "internal.h"
+#include "pdl.cuh"
 
 #define CUDA_TRY(x)                                                                              \
     do {                                                                                         \
@@ -343,6 +344,8 @@ __global__ void __launch_bounds__(128) attn_fwd_mma_kernel(const float *__restri
                                                            const int32_t *__restrict__ chain_ids,
                                                            const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H,
                                                            float scale, int tile0) {
+    pdl_wait();
+    pdl_next();
     constexpr int KS = HD / 8;
     constexpr bool SPLIT_KV = sizeof(KVT) == 4;
     // NS key chunks are staged per round and consumed without any barrier in between, so the four warps (whose
@@ -674,6 +677,8 @@ __global__ void __launch_bounds__(128, HD <= 32 ? 4 : (sizeof(KVT) == 2 ? 3 : 1)
                                                            const int32_t *__restrict__ chain_ids,
                                                            const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H,
                                                            float scale, int tile0, BwdMask gmask) {
+    pdl_wait();
+    pdl_next();
     constexpr int M = 64, KS = HD / 8;
     constexpr bool SPLIT_KV = sizeof(KVT) == 4;
     constexpr int NB2 = (KS + 1) / 2;          // head_dim blocks of 8 per warp in phase 2
@@ -1105,6 +1110,8 @@ attn_bwd_tile_kernel(const float *__restrict__ Q, const KVT *__restrict__ K, con
                      float *__restrict__ Pv, const int32_t *__restrict__ sub_end, const int64_t *__restrict__ chain_off,
                      const int32_t *__restrict__ chain_ids, const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H,
                      float scale, int tile0, int maxk, bool wide, BwdMask gmask) {
+    pdl_wait();
+    pdl_next();
     constexpr int M = 64, NT = NW * 32, TILE_ROW_BYTES = HD * 4, KS = HD / 16, NDB = HD / 8;
     constexpr bool BF = sizeof(KVT) == 2;              // bfloat16 store: K and V have no lo parts
     constexpr int KB = bwd_key_bytes(HD, BF);
@@ -1501,6 +1508,8 @@ attn_fwd_tile_kernel(const float *__restrict__ Q, const float *__restrict__ K, c
                      float *__restrict__ O, float *__restrict__ LSE, const int32_t *__restrict__ sub_end,
                      const int64_t *__restrict__ chain_off, const int32_t *__restrict__ chain_ids,
                      const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H, float scale, int tile0, int maxk) {
+    pdl_wait();
+    pdl_next();
     constexpr int M = 64, NT = 128, TILE_ROW_BYTES = HD * 4, KS = HD / 16, NDB = HD / 8;
     extern __shared__ __align__(128) unsigned char tile_smem_raw[];
     unsigned char *sQ = tile_smem_raw, *sK = sQ + M * TILE_ROW_BYTES, *sV = sK + (size_t)maxk * TILE_ROW_BYTES;
@@ -1726,6 +1735,8 @@ attn_fwd_bf16_kernel(const float *__restrict__ Q, const __nv_bfloat16 *__restric
                      float *__restrict__ O, float *__restrict__ LSE, const int32_t *__restrict__ sub_end,
                      const int64_t *__restrict__ chain_off, const int32_t *__restrict__ chain_ids,
                      const int32_t *__restrict__ chain_end_all, const int32_t *__restrict__ tile_start, int H, float scale, int tile0, int maxk) {
+    pdl_wait();
+    pdl_next();
     constexpr int NT = 128, KS = HD / 16, NDB = HD / 8, NCH = HD / 8;
     extern __shared__ __align__(128) unsigned char tile_smem_raw[];
     unsigned char *sK = tile_smem_raw, *sV = sK + (size_t)maxk * (HD * 2);
@@ -1871,6 +1882,8 @@ reduce_items_kernel(const float *__restrict__ Pk, const float *__restrict__ Pv, 
                     float *__restrict__ segk, float *__restrict__ segv, const int64_t *__restrict__ chain_off, const int32_t *__restrict__ depth,
                     const int32_t *__restrict__ item_node, const int32_t *__restrict__ item_t0, const int32_t *__restrict__ item_t1,
                     const int32_t *__restrict__ item_slot, int64_t item0, int64_t n_items, int D, int chunks) {
+    pdl_wait();
+    pdl_next();
     int64_t it = (int64_t)(blockIdx.x / chunks) * 8 + (threadIdx.x >> 5);
     if (it >= n_items) return;
     it += item0;
@@ -1925,6 +1938,8 @@ __global__ void __launch_bounds__(256)
 reduce_even_kernel(const float *__restrict__ Pk, const float *__restrict__ Pv, float *__restrict__ dK, float *__restrict__ dV,
                    const int64_t *__restrict__ chain_off, const int32_t *__restrict__ depth, const int32_t *__restrict__ item_node,
                    const int32_t *__restrict__ item_t0, const int32_t *__restrict__ item_t1, int64_t item0, int64_t n_items, int D, int chunks) {
+    pdl_wait();
+    pdl_next();
     int64_t it = (int64_t)(blockIdx.x / chunks) * 8 + (threadIdx.x >> 5);
     const int c = (blockIdx.x % chunks) * 128 + (threadIdx.x & 31) * 4;
     if (it >= n_items || c >= D) return;
@@ -1955,6 +1970,8 @@ reduce_even_kernel(const float *__restrict__ Pk, const float *__restrict__ Pv, f
 __global__ void __launch_bounds__(256)
 reduce_multi_kernel(const float *__restrict__ segk, const float *__restrict__ segv, float *__restrict__ dK, float *__restrict__ dV,
                     const int32_t *__restrict__ multi_node, const int32_t *__restrict__ multi_count, const int64_t *__restrict__ multi_first, int D) {
+    pdl_wait();
+    pdl_next();
     __shared__ float4 s_k[8][32], s_v[8][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.y * 128 + lane * 4;
     const int a = multi_node[blockIdx.x], cnt = multi_count[blockIdx.x];
@@ -2103,7 +2120,7 @@ static int launch_fwd_tile(const agpt_plan *p, const float *q, const void *k, co
     int rc = allow_dynamic_smem(attn_fwd_tile_kernel<HD, MINB>, smem, granted);
     if (rc) return rc;
     dim3 grid((unsigned)ntiles, (unsigned)H);
-    attn_fwd_tile_kernel<HD, MINB><<<grid, 128, smem, st>>>(q, (const float *)k, (const float *)v, out, lse, p->d_sub_end,
+    pdl_launch(attn_fwd_tile_kernel<HD, MINB>, grid, 128, smem, st, q, (const float *)k, (const float *)v, out, lse, p->d_sub_end,
                                                                  p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H, scale, tile0, maxk);
     return launch_status("attn_fwd_tile");
 }
@@ -2115,8 +2132,7 @@ static int launch_fwd_bf16(const agpt_plan *p, const float *q, const void *k, co
     const int maxk = bwd_tile_maxk(p);
     const size_t smem = fwd_bf16_smem_bytes(HD, maxk);
     if (int rc = allow_dynamic_smem(attn_fwd_bf16_kernel<HD, MINB>, smem, granted)) return rc;
-    attn_fwd_bf16_kernel<HD, MINB><<<dim3((unsigned)ntiles, (unsigned)H), 128, smem, st>>>(
-        q, (const __nv_bfloat16 *)k, (const __nv_bfloat16 *)v, out, lse, p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H,
+    pdl_launch(attn_fwd_bf16_kernel<HD, MINB>, dim3((unsigned)ntiles, (unsigned)H), 128, smem, st, q, (const __nv_bfloat16 *)k, (const __nv_bfloat16 *)v, out, lse, p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H,
         scale, tile0, maxk);
     return launch_status("attn_fwd_bf16");
 }
@@ -2128,10 +2144,15 @@ static int launch_fwd_mma(const agpt_plan *p, const float *q, const void *k, con
     const size_t smem = fwd_mma_smem_bytes<HD>();
     static size_t granted[AGPT_MAX_DEVICES];
     if (int rc = allow_dynamic_smem(attn_fwd_mma_kernel<HD, KVT>, smem, granted)) return rc;
-    attn_fwd_mma_kernel<HD, KVT><<<grid, 128, smem, st>>>(q, (const KVT *)k, (const KVT *)v, out, lse, p->d_sub_end,
+    pdl_launch(attn_fwd_mma_kernel<HD, KVT>, grid, 128, smem, st, q, (const KVT *)k, (const KVT *)v, out, lse, p->d_sub_end,
                                                        p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H, scale, tile0);
     return launch_status("attn_fwd_mma");
 }
+
+// Blocks are placed early (pdl.cuh) while the launches of an attention step count, rows x columns: 8 x 64, 8k rows 102 -> 96 us, 88k rows 712 -> 704;
+// 4 x 32, 29k rows 91 -> 85, 288k rows 564 -> 556.  Beyond, the 8 us that it hides are lost in the noise or cost more: the reduction of 719k rows of 384 took 90 us longer.
+static constexpr int64_t ATTN_EARLY_ELEMENTS = 32 << 20;
+static bool attn_early(const agpt_plan *p, int D) { return pdl_early && p->n * (int64_t)D <= ATTN_EARLY_ELEMENTS; }
 
 static int fwd_dispatch(const agpt_plan *p, const float *q, const void *k, const void *v, int kv_dtype, float *out,
                         float *lse, int H, int head_dim, float scale, cudaStream_t st, int tile0, int ntiles) {
@@ -2173,7 +2194,7 @@ static int launch_bwd_mma(const agpt_plan *p, const float *q, const void *k, con
     size_t smem = sizeof(BwdMmaSmem<HD, KVT>);
     static size_t granted[AGPT_MAX_DEVICES];
     if (int rc = allow_dynamic_smem(attn_bwd_mma_kernel<HD, KVT>, smem, granted)) return rc;
-    attn_bwd_mma_kernel<HD, KVT><<<grid, 128, smem, st>>>(q, (const KVT *)k, (const KVT *)v, o, lse, dout, dq, dk, dv, pk, pv,
+    pdl_launch(attn_bwd_mma_kernel<HD, KVT>, grid, 128, smem, st, q, (const KVT *)k, (const KVT *)v, o, lse, dout, dq, dk, dv, pk, pv,
                                                           p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_chain_end, p->d_tile_start, H,
                                                           scale, tile0, gmask);
     return launch_status("attn_bwd_mma");
@@ -2189,7 +2210,7 @@ static int launch_bwd_tile(const agpt_plan *p, const float *q, const void *k, co
     int rc = allow_dynamic_smem(attn_bwd_tile_kernel<HD, NW, MINB, KVT>, smem, granted);
     if (rc) return rc;
     dim3 grid((unsigned)ntiles, (unsigned)H);
-    attn_bwd_tile_kernel<HD, NW, MINB, KVT><<<grid, NW * 32, smem, st>>>(q, (const KVT *)k, (const KVT *)v, o, lse, dout, dq, dk, dv, pk, pv,
+    pdl_launch(attn_bwd_tile_kernel<HD, NW, MINB, KVT>, grid, NW * 32, smem, st, q, (const KVT *)k, (const KVT *)v, o, lse, dout, dq, dk, dv, pk, pv,
                                                                          p->d_sub_end, p->d_chain_off, p->d_chain_ids, p->d_chain_end,
                                                                          p->d_tile_start, H, scale, tile0, maxk, rows_wide(H * HD, q, k, v, o, dout), gmask);
     return launch_status("attn_bwd_tile");
@@ -2246,6 +2267,7 @@ extern "C" int agpt_b200_attn_fwd(const agpt_plan *p, const float *d_q, const vo
     if (rc) return rc;
     if (!d_q || !d_k || !d_v || !d_out || !d_lse) return agpt_set_error(AGPT_E_ARG, "attn_fwd: null buffer");
     if (kv_dtype != AGPT_KV_F32 && kv_dtype != AGPT_KV_BF16) return agpt_set_error(AGPT_E_ARG, "attn_fwd: bad kv_dtype");
+    const PdlScope scope(attn_early(p, n_heads * head_dim));
     return fwd_dispatch(p, d_q, d_k, d_v, kv_dtype, d_out, d_lse, n_heads, head_dim, scale, (cudaStream_t)stream, 0, (int)p->n_tiles);
 }
 
@@ -2258,17 +2280,17 @@ static int run_reduce_range(const agpt_plan *p, float *pk, float *pv, float *seg
         const unsigned grid = (unsigned)((n_items + 7) / 8 * chunks);
 #define REDUCE_ARGS pk, pv, dk, dv, segk, segv, p->d_chain_off, p->d_depth, p->d_item_node, p->d_item_t0, p->d_item_t1, p->d_item_slot, item0, n_items, D, chunks
         if (p->even)
-            reduce_even_kernel<<<grid, 256, 0, st>>>(pk, pv, dk, dv, p->d_chain_off, p->d_depth, p->d_item_node, p->d_item_t0, p->d_item_t1, item0, n_items, D,
+            pdl_launch(reduce_even_kernel, grid, 256, 0, st, pk, pv, dk, dv, p->d_chain_off, p->d_depth, p->d_item_node, p->d_item_t0, p->d_item_t1, item0, n_items, D,
                                                      chunks);
-        else if (D <= 64) reduce_items_kernel<true><<<grid, 256, 0, st>>>(REDUCE_ARGS);
-        else reduce_items_kernel<false><<<grid, 256, 0, st>>>(REDUCE_ARGS);
+        else if (D <= 64) pdl_launch(reduce_items_kernel<true>, grid, 256, 0, st, REDUCE_ARGS);
+        else pdl_launch(reduce_items_kernel<false>, grid, 256, 0, st, REDUCE_ARGS);
 #undef REDUCE_ARGS
         int rc = launch_status("reduce_items");
         if (rc) return rc;
     }
     int64_t n_multi = (int64_t)p->multi_node.size();
     if (multi_pass && n_multi > 0) {
-        reduce_multi_kernel<<<dim3((unsigned)n_multi, (unsigned)((D + 127) / 128)), 256, 0, st>>>(segk, segv, dk, dv, p->d_multi_node, p->d_multi_count,
+        pdl_launch(reduce_multi_kernel, dim3((unsigned)n_multi, (unsigned)((D + 127) / 128)), 256, 0, st, segk, segv, dk, dv, p->d_multi_node, p->d_multi_count,
                                                                                                  p->d_multi_first, D);
         int rc = launch_status("reduce_multi");
         if (rc) return rc;
@@ -2295,6 +2317,7 @@ extern "C" int agpt_b200_attn_bwd_mode(const agpt_plan *p, const float *d_q, con
     if (grad_mode == AGPT_GRAD_OWN_EDGE && !d_edge_first)
         return agpt_set_error(AGPT_E_ARG, "attn_bwd: the own-edge mode needs the edge_first array");
     const int D = n_heads * head_dim;
+    const PdlScope scope(attn_early(p, D));
     int64_t need = agpt_b200_attn_bwd_workspace_bytes(p, D);
     if (workspace_bytes < need)
         return agpt_set_error(AGPT_E_ARG, "attn_bwd: workspace %lld bytes < required %lld", (long long)workspace_bytes, (long long)need);
@@ -2358,6 +2381,8 @@ template <bool TWO>
 __global__ void __launch_bounds__(256)
 rope4_kernel(float *a, float *b, const int32_t *__restrict__ pos, const float *__restrict__ cosv, const float *__restrict__ sinv,
              int64_t n, int D, int hd, int inverse) {
+    pdl_wait();
+    pdl_next();
     const int q4n = D >> 2;
     const int64_t row0 = (int64_t)blockIdx.x * ROPE_ROWS;
     const int rows = (int)(n - row0 < ROPE_ROWS ? n - row0 : ROPE_ROWS);
@@ -2388,8 +2413,8 @@ static int rope_launch(float *d_a, float *d_b, const int32_t *d_pos, const float
     const bool vec = head_dim % 4 == 0 && (((uintptr_t)d_a | (uintptr_t)d_b | (uintptr_t)d_cos | (uintptr_t)d_sin) & 15) == 0;
     if (vec) {
         const unsigned blocks = (unsigned)((n + ROPE_ROWS - 1) / ROPE_ROWS);
-        if (d_b) rope4_kernel<true><<<blocks, 256, 0, st>>>(d_a, d_b, d_pos, d_cos, d_sin, n, n_heads * head_dim, head_dim, inverse);
-        else rope4_kernel<false><<<blocks, 256, 0, st>>>(d_a, nullptr, d_pos, d_cos, d_sin, n, n_heads * head_dim, head_dim, inverse);
+        if (d_b) pdl_launch(rope4_kernel<true>, blocks, 256, 0, st, d_a, d_b, d_pos, d_cos, d_sin, n, n_heads * head_dim, head_dim, inverse);
+        else pdl_launch(rope4_kernel<false>, blocks, 256, 0, st, d_a, nullptr, d_pos, d_cos, d_sin, n, n_heads * head_dim, head_dim, inverse);
         return launch_status("rope");
     }
     int64_t total = n * n_heads * (head_dim / 2);
@@ -2410,6 +2435,8 @@ extern "C" int agpt_b200_rope_pair(float *d_a, float *d_b, const int32_t *d_pos,
 }
 
 __global__ void store_bf16_kernel(const float *__restrict__ src, __nv_bfloat16 *__restrict__ dst, int64_t total4) {
+    pdl_wait();
+    pdl_next();
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total4) return;
     float4 v = __ldg(reinterpret_cast<const float4 *>(src) + idx);
@@ -2423,7 +2450,7 @@ extern "C" int agpt_b200_kv_store_write_bf16(const float *d_src, void *d_store, 
     if (!d_src || !d_store || n < 0 || cols <= 0 || cols % 4) return agpt_set_error(AGPT_E_ARG, "kv_store_write_bf16: bad argument");
     if (n == 0) return AGPT_OK;
     int64_t total4 = n * (cols / 4);
-    store_bf16_kernel<<<(unsigned)((total4 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(d_src, (__nv_bfloat16 *)d_store, total4);
+    pdl_launch(store_bf16_kernel, (unsigned)((total4 + 255) / 256), 256, 0, (cudaStream_t)stream, d_src, (__nv_bfloat16 *)d_store, total4);
     return launch_status("kv_store_write_bf16");
 }
 
@@ -2640,6 +2667,8 @@ loss_batch_kernel(const float *__restrict__ logits, const int32_t *__restrict__ 
                   const int32_t *__restrict__ counts_tok, const int32_t *__restrict__ counts_val,
                   const float *__restrict__ mass_weights, float *__restrict__ d_logits, float *__restrict__ loss_out,
                   int64_t T_q, int V, float entropy_lambda, float intermediate_weight, int ce_only, int mode, int aligned16) {
+    pdl_wait();
+    pdl_next();
     extern __shared__ __align__(128) unsigned char lossb_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t r0 = ((int64_t)blockIdx.x * LOSSB_WARPS + warp) * 32;
@@ -2862,7 +2891,7 @@ static int launch_loss(int64_t rows, int V, cudaStream_t st, const float *logits
         const int rows_per_block = LOSSB_WARPS * 32;
         const unsigned blocks = (unsigned)((rows + rows_per_block - 1) / rows_per_block);
         const int aligned16 = ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(dlogits)) & 15) == 0;
-        loss_batch_kernel<<<blocks, LOSSB_WARPS * 32, smem, st>>>(args..., aligned16);
+        pdl_launch(loss_batch_kernel, blocks, LOSSB_WARPS * 32, smem, st, args..., aligned16);
         return AGPT_OK;
     }
     const unsigned blocks = (unsigned)((rows + LOSS_ROWS_PER_BLOCK - 1) / LOSS_ROWS_PER_BLOCK);
@@ -2881,12 +2910,16 @@ extern "C" int agpt_b200_device_status(int32_t *status_out) {
     return AGPT_OK;
 }
 
-__global__ void device_status_kernel(const int *__restrict__ step_word, float *out) { *out += (float)(g_device_status | *step_word); }
+__global__ void device_status_kernel(const int *__restrict__ step_word, float *out) {
+    pdl_wait();
+    pdl_next();
+    *out += (float)(g_device_status | *step_word);
+}
 extern "C" int agpt_b200_device_status_add(float *d_out, void *stream) {
     if (!d_out) return agpt_set_error(AGPT_E_ARG, "device_status_add: null output");
     const int *step_word = nullptr;
     if (int rc = agpt_step_gemm_status_word(&step_word)) return rc;
-    device_status_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(step_word, d_out);
+    pdl_launch(device_status_kernel, 1, 1, 0, (cudaStream_t)stream, step_word, d_out);
     return launch_status("device_status_add");
 }
 

@@ -19,6 +19,7 @@
 
 #include "../../include/agpt_b200.h"
 #include "internal.h"
+#include "pdl.cuh"
 
 namespace {
 
@@ -38,6 +39,8 @@ int norm_blocks(int64_t n, int cap) {
 
 // partial[b] = sum of g^2 over the block's contiguous slice
 __global__ void __launch_bounds__(256) sq_norm_partial_kernel(const float *__restrict__ g, int64_t n, float *__restrict__ partial) {
+    pdl_wait();
+    pdl_next();
     __shared__ float s[256];
     const int64_t per = (n + gridDim.x - 1) / gridDim.x;
     const int64_t a = (int64_t)blockIdx.x * per, b = (a + per < n) ? a + per : n;
@@ -98,6 +101,8 @@ __device__ __forceinline__ float update(float p, float g, float *m, float *v, in
 template <int KIND>
 __global__ void __launch_bounds__(256) step_kernel(float *__restrict__ p, float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
                                                     int64_t n, StepArgs a, const float *__restrict__ partial, float *__restrict__ norm_out) {
+    pdl_wait();
+    pdl_next();
     float scale = 1.f;
     if (a.clip_norm > 0.f) {
         const float norm = norm_from_partials(partial, a.norm_blocks);
@@ -122,10 +127,10 @@ int run_step(int kind, float *p, float *g, float *m, float *v, int64_t n, const 
              cudaStream_t st) {
     unsigned grid = step_grid(n);
     switch (kind) {
-        case AGPT_OPT_SGD: step_kernel<AGPT_OPT_SGD><<<grid, 256, 0, st>>>(p, g, m, v, n, a, partial, norm_out); break;
-        case AGPT_OPT_MOMENTUM: step_kernel<AGPT_OPT_MOMENTUM><<<grid, 256, 0, st>>>(p, g, m, v, n, a, partial, norm_out); break;
-        case AGPT_OPT_RMSPROP: step_kernel<AGPT_OPT_RMSPROP><<<grid, 256, 0, st>>>(p, g, m, v, n, a, partial, norm_out); break;
-        case AGPT_OPT_ADAM: step_kernel<AGPT_OPT_ADAM><<<grid, 256, 0, st>>>(p, g, m, v, n, a, partial, norm_out); break;
+        case AGPT_OPT_SGD: pdl_launch(step_kernel<AGPT_OPT_SGD>, grid, 256, 0, st, p, g, m, v, n, a, partial, norm_out); break;
+        case AGPT_OPT_MOMENTUM: pdl_launch(step_kernel<AGPT_OPT_MOMENTUM>, grid, 256, 0, st, p, g, m, v, n, a, partial, norm_out); break;
+        case AGPT_OPT_RMSPROP: pdl_launch(step_kernel<AGPT_OPT_RMSPROP>, grid, 256, 0, st, p, g, m, v, n, a, partial, norm_out); break;
+        case AGPT_OPT_ADAM: pdl_launch(step_kernel<AGPT_OPT_ADAM>, grid, 256, 0, st, p, g, m, v, n, a, partial, norm_out); break;
         default: return agpt_set_error(AGPT_E_ARG, "optimizer_step: unknown optimizer kind %d", kind);
     }
     return launch_status("optimizer_step");
@@ -157,7 +162,7 @@ extern "C" int agpt_b200_optimizer_step(int kind, float *d_params, float *d_grad
     float *partial = (float *)d_scratch;
     if (clip_norm > 0.f) {
         a.norm_blocks = norm_blocks(n, NORM_BLOCKS_MAX);
-        sq_norm_partial_kernel<<<a.norm_blocks, 256, 0, st>>>(d_grads, n, partial);
+        pdl_launch(sq_norm_partial_kernel, a.norm_blocks, 256, 0, st, d_grads, n, partial);
     }
     return run_step(kind, d_params, d_grads, d_m, d_v, n, a, partial, partial ? partial + NORM_BLOCKS_MAX : nullptr, st);
 }

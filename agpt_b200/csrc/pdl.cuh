@@ -1,0 +1,33 @@
+// Programmatic dependent launch: the blocks of a kernel are placed, and what they do before pdl_wait() runs, while the kernel before it in
+// the stream still works.  A step of training on few rows is a chain of some 80 short kernels; between two of them this takes the launch, the
+// block start and the barrier and tensor-memory setup off the chain.
+//
+// Rules.  Every thread of every block calls pdl_wait() before it reads or writes device memory, before any early return: the kernel in front
+// has then completed and its results are visible, and, as that kernel waited itself, so have all before it.  pdl_next() comes behind pdl_wait(), so
+// that no more than two kernels of a stream are on the device at a time and a waiting block never holds what an unplaced block of an
+// earlier kernel needs.  A kernel launched in the ordinary way passes both at once, and one launched through pdl_launch behind an ordinary
+// kernel, a copy or an event wait starts when that has completed.
+#pragma once
+#include <cuda_runtime.h>
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Whether pdl_launch places early on this thread: on, but for the length of a call that knows better (PdlScope on its stack).
+inline thread_local bool pdl_early = true;
+struct PdlScope {
+    const bool before;
+    explicit PdlScope(bool early) : before(pdl_early) { pdl_early = early; }
+    ~PdlScope() { pdl_early = before; }
+    PdlScope(const PdlScope &) = delete;
+};
+
+template <typename... P, typename... A>
+static inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = st; c.attrs = &at; c.numAttrs = pdl_early ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}

@@ -11,6 +11,7 @@
 
 #include "../../include/agpt_b200.h"
 #include "internal.h"
+#include "pdl.cuh"
 
 namespace {
 
@@ -212,6 +213,8 @@ __global__ void __launch_bounds__(256) embedding_scatter_atomic_kernel(const flo
 template <int W>
 __global__ void __launch_bounds__(32) embedding_grad_kernel(const float *__restrict__ grad, const int *__restrict__ ids, int64_t n, int d,
                                                              int vocab, int64_t chunk, float *__restrict__ partial) {
+    pdl_wait();
+    pdl_next();
     extern __shared__ float s_tab[];                  // [vocab][32 W]
     constexpr int U = 8;
     const int lane = threadIdx.x, c = blockIdx.y * 32 * W + lane * W;
@@ -254,6 +257,8 @@ __global__ void __launch_bounds__(32) embedding_grad_kernel(const float *__restr
 // the blocks one after the other
 __global__ void __launch_bounds__(256) embedding_grad_serial_finish_kernel(const float *__restrict__ partial, int blocks, int64_t vd, int accumulate,
                                                                             float *__restrict__ demb) {
+    pdl_wait();
+    pdl_next();
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (i >= vd) return;
     float t = 0.f;
@@ -263,6 +268,8 @@ __global__ void __launch_bounds__(256) embedding_grad_serial_finish_kernel(const
 
 __global__ void __launch_bounds__(256) embedding_grad_finish_kernel(const float *__restrict__ partial, int blocks, int64_t vd, int accumulate,
                                                                      float *__restrict__ demb) {
+    pdl_wait();
+    pdl_next();
     __shared__ float s[8][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t i = (int64_t)blockIdx.x * 32 + lane;
@@ -293,7 +300,7 @@ void launch_embedding_grad(const float *grad, const int *ids, int64_t n, int d, 
         cudaFuncSetAttribute(embedding_grad_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         attr_set[dev] = true;
     }
-    embedding_grad_kernel<W><<<dim3(blocks, (d + 32 * W - 1) / (32 * W)), 32, (size_t)vocab * 32 * W * 4, st>>>(grad, ids, n, d, vocab, (n + blocks - 1) / blocks, partial);
+    pdl_launch(embedding_grad_kernel<W>, dim3(blocks, (d + 32 * W - 1) / (32 * W)), 32, (size_t)vocab * 32 * W * 4, st, grad, ids, n, d, vocab, (n + blocks - 1) / blocks, partial);
 }
 
 }  // namespace
@@ -402,8 +409,8 @@ static int embedding_grad(const float *d_grad, const int32_t *d_ids, float *d_em
         launch_embedding_grad<2>(d_grad, d_ids, n, d_model, vocab, blocks, (float *)d_workspace, st);
     else launch_embedding_grad<1>(d_grad, d_ids, n, d_model, vocab, blocks, (float *)d_workspace, st);
     const int64_t vd = (int64_t)vocab * d_model;
-    if (serial) embedding_grad_serial_finish_kernel<<<(unsigned)((vd + 255) / 256), 256, 0, st>>>((const float *)d_workspace, blocks, vd, accumulate, d_emb_grad);
-    else embedding_grad_finish_kernel<<<(unsigned)((vd + 31) / 32), 256, 0, st>>>((const float *)d_workspace, blocks, vd, accumulate, d_emb_grad);
+    if (serial) pdl_launch(embedding_grad_serial_finish_kernel, (unsigned)((vd + 255) / 256), 256, 0, st, (const float *)d_workspace, blocks, vd, accumulate, d_emb_grad);
+    else pdl_launch(embedding_grad_finish_kernel, (unsigned)((vd + 31) / 32), 256, 0, st, (const float *)d_workspace, blocks, vd, accumulate, d_emb_grad);
     return launch_status("embedding_grad");
 }
 

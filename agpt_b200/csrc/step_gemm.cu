@@ -36,6 +36,7 @@
 
 #include "../../include/agpt_b200.h"
 #include "internal.h"
+#include "pdl.cuh"
 #include "tc100.cuh"
 
 namespace {
@@ -132,6 +133,8 @@ struct SplitArgs {
 
 // one block = 32 n x 64 k of one job; reads along the matrix rows, transposes through shared memory
 __global__ void __launch_bounds__(256) split_weights_kernel(const __grid_constant__ SplitArgs a) {
+    pdl_wait();
+    pdl_next();
     __shared__ float s[64][33];
     int j = 0;
     while (j + 1 < a.n && (int)blockIdx.x >= a.first_block[j + 1]) j++;
@@ -212,6 +215,8 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) tmem_alloc(smem_u32(&s_tmem), TMEM_COLS);
+    pdl_wait();
+    pdl_next();
     for (int i = tid; i < P.nt; i += ROW_THREADS) s_bias[i] = (g.bias && n0 + i < g.N) ? __ldg(g.bias + n0 + i) : 0.f;
     if (EPI == EPI_QKV && g.cosv) {
         const int half = g.head_dim >> 1;
@@ -621,7 +626,7 @@ template <int PRO, int EPI>
 int launch_row(const RowArgs &P, const RowMaps &m, int grid, size_t smem, cudaStream_t st) {
     static bool done[64];
     if (int rc = allow_smem(row_gemm_kernel<PRO, EPI>, done)) return rc;
-    row_gemm_kernel<PRO, EPI><<<grid, ROW_THREADS, smem, st>>>(m, P);
+    pdl_launch(row_gemm_kernel<PRO, EPI>, grid, ROW_THREADS, smem, st, m, P);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return agpt_set_error(AGPT_E_CUDA, "row_gemm: %s", cudaGetErrorString(e));
     return AGPT_OK;
@@ -720,7 +725,7 @@ int agpt_split_weights(const WeightSplitJob *jobs, int n_jobs, cudaStream_t st) 
             blocks += ((a.job[i].n_pad + 31) / 32) * ((a.job[i].k_pad + 63) / 64);
         }
         a.first_block[a.n] = blocks;
-        split_weights_kernel<<<blocks, 256, 0, st>>>(a);
+        pdl_launch(split_weights_kernel, blocks, 256, 0, st, a);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return agpt_set_error(AGPT_E_CUDA, "split_weights: %s", cudaGetErrorString(e));
@@ -788,6 +793,8 @@ contract_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ 
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) tmem_alloc(smem_u32(&s_tmem), TMEM_COLS);
+    pdl_wait();
+    pdl_next();
     fence_before();
     __syncthreads();
     fence_after();
@@ -1046,7 +1053,7 @@ int agpt_row_contract(const RowContract &g, cudaStream_t st) {
     for (int i = g.n_seg; i < 3; i++) m[i] = m[0];
     static bool done[64];
     if (int rc = allow_smem(contract_kernel, done)) return rc;
-    contract_kernel<<<P.m_tiles * P.groups * g.slices, CON_THREADS, CON_SMEM, st>>>(mA, m[0], m[1], m[2], P);
+    pdl_launch(contract_kernel, P.m_tiles * P.groups * g.slices, CON_THREADS, CON_SMEM, st, mA, m[0], m[1], m[2], P);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return agpt_set_error(AGPT_E_CUDA, "row_contract: %s", cudaGetErrorString(e));
     return AGPT_OK;

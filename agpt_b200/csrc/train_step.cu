@@ -19,6 +19,7 @@
 
 #include "../../include/agpt_b200.h"
 #include "internal.h"
+#include "pdl.cuh"
 #include "step_gemm.h"
 
 namespace {
@@ -60,10 +61,14 @@ __device__ __forceinline__ float2 row_stats(const float4 (&v)[NV], int lane, int
 constexpr int ROWS_PER_BLOCK = 8;
 constexpr int NV_MAX = 8;                 // d_model up to 1024
 
-// x[r] = emb[tokens[r]] (tokens == nullptr: x is read as it is), stats[r]; one warp per row, zero statistics behind the end
+// x[r] = emb[tokens[r]] (tokens == nullptr: x is read as it is), stats[r]; one warp per row, zero statistics behind the end.  Clears n_clear counters on
+// the way (a memset between two kernels would keep the second from being placed early).
 template <int NV>
 __global__ void __launch_bounds__(256) embed_stats_kernel(const float *__restrict__ emb, const int32_t *__restrict__ tokens, float *__restrict__ x,
-                                                           float2 *__restrict__ stats, int64_t n, int64_t n_pad, int d, int vocab) {
+                                                           float2 *__restrict__ stats, int64_t n, int64_t n_pad, int d, int vocab, int32_t *__restrict__ clear, int n_clear) {
+    pdl_wait();
+    pdl_next();
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n_clear; i += (int64_t)gridDim.x * 256) clear[i] = 0;
     const int64_t r = (int64_t)blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 5);
     if (r >= n_pad) return;
     const int lane = threadIdx.x & 31, d4 = d >> 2;
@@ -86,6 +91,8 @@ __global__ void __launch_bounds__(256) embed_stats_kernel(const float *__restric
 template <int NV>
 __global__ void __launch_bounds__(256) norm_bwd_kernel(const float *__restrict__ dn, const float *__restrict__ x, const float2 *__restrict__ stats,
                                                         const float *add, float *out, int64_t n, int d) {
+    pdl_wait();
+    pdl_next();
     const int64_t r = (int64_t)blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 5);
     if (r >= n) return;
     const int lane = threadIdx.x & 31, d4 = d >> 2;
@@ -121,6 +128,8 @@ __global__ void __launch_bounds__(256) norm_bwd_kernel(const float *__restrict__
 __global__ void __launch_bounds__(256) loss_count_kernel(const float *__restrict__ loss, const float *__restrict__ trained,
                                                           const int64_t *__restrict__ unit, int64_t n, int32_t *__restrict__ unit_count,
                                                           double *__restrict__ block_sum, int32_t *__restrict__ block_count) {
+    pdl_wait();
+    pdl_next();
     __shared__ double s_sum[8];
     __shared__ int s_cnt[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -152,6 +161,8 @@ __global__ void __launch_bounds__(256) row_scale_kernel(const float *__restrict_
                                                          const int32_t *__restrict__ unit_count, int64_t n, int64_t n_pad, float *__restrict__ scale,
                                                          const double *__restrict__ block_sum, const int32_t *__restrict__ block_count, int blocks,
                                                          double *__restrict__ loss_out, int64_t *__restrict__ count_out, float *__restrict__ tail) {
+    pdl_wait();
+    pdl_next();
     if (blockIdx.x == 0) {
         __shared__ double s_sum[256];
         __shared__ int64_t s_cnt[256];
@@ -186,6 +197,8 @@ struct FoldJob { const float *w, *shift, *b; float *out; int k, n, n_pad; };
 constexpr int FOLD_JOBS = 80;
 struct FoldArgs { FoldJob job[FOLD_JOBS]; int first_block[FOLD_JOBS + 1]; int n; };
 __global__ void __launch_bounds__(256) fold_bias_kernel(const __grid_constant__ FoldArgs a) {
+    pdl_wait();
+    pdl_next();
     __shared__ float s[8][32];
     int j = 0;
     while (j + 1 < a.n && (int)blockIdx.x >= a.first_block[j + 1]) j++;
@@ -221,6 +234,8 @@ constexpr int GRAD_JOBS = 20;
 struct GradArgs { GradJob job[GRAD_JOBS]; int first_block[GRAD_JOBS + 1]; int n; };
 
 __global__ void __launch_bounds__(256) grad_cols_kernel(const __grid_constant__ GradArgs a) {
+    pdl_wait();
+    pdl_next();
     __shared__ float s[8][32];
     int j = 0;
     while (j + 1 < a.n && (int)blockIdx.x >= a.first_block[j + 1]) j++;
@@ -243,6 +258,8 @@ __global__ void __launch_bounds__(256) grad_cols_kernel(const __grid_constant__ 
 
 // one block per row of a gradient matrix
 __global__ void __launch_bounds__(128) grad_rows_kernel(const __grid_constant__ GradArgs a) {
+    pdl_wait();
+    pdl_next();
     __shared__ float s[2][4];
     int j = 0;
     while (j + 1 < a.n && (int)blockIdx.x >= a.first_block[j + 1]) j++;
@@ -370,23 +387,23 @@ int check(const agpt_train_step_args &A) {
 }
 
 template <int NV>
-int embed_stats_nv(const float *emb, const int32_t *tok, float *x, float2 *st, int64_t n, int d, int vocab, cudaStream_t s) {
+int embed_stats_nv(const float *emb, const int32_t *tok, float *x, float2 *st, int64_t n, int d, int vocab, cudaStream_t s, int32_t *clear = nullptr, int n_clear = 0) {
     const int64_t n_pad = (n + 127) & ~(int64_t)127;
-    embed_stats_kernel<NV><<<(unsigned)(n_pad / ROWS_PER_BLOCK), 256, 0, s>>>(emb, tok, x, st, n, n_pad, d, vocab);
+    pdl_launch(embed_stats_kernel<NV>, (unsigned)(n_pad / ROWS_PER_BLOCK), 256, 0, s, emb, tok, x, st, n, n_pad, d, vocab, clear, n_clear);
     return launched("row statistics");
 }
-int embed_stats(const float *emb, const int32_t *tok, float *x, float2 *st, int64_t n, int d, int vocab, cudaStream_t s) {
-    if (d <= 128) return embed_stats_nv<1>(emb, tok, x, st, n, d, vocab, s);
-    if (d <= 256) return embed_stats_nv<2>(emb, tok, x, st, n, d, vocab, s);
-    if (d <= 512) return embed_stats_nv<4>(emb, tok, x, st, n, d, vocab, s);
-    return embed_stats_nv<NV_MAX>(emb, tok, x, st, n, d, vocab, s);
+int embed_stats(const float *emb, const int32_t *tok, float *x, float2 *st, int64_t n, int d, int vocab, cudaStream_t s, int32_t *clear = nullptr, int n_clear = 0) {
+    if (d <= 128) return embed_stats_nv<1>(emb, tok, x, st, n, d, vocab, s, clear, n_clear);
+    if (d <= 256) return embed_stats_nv<2>(emb, tok, x, st, n, d, vocab, s, clear, n_clear);
+    if (d <= 512) return embed_stats_nv<4>(emb, tok, x, st, n, d, vocab, s, clear, n_clear);
+    return embed_stats_nv<NV_MAX>(emb, tok, x, st, n, d, vocab, s, clear, n_clear);
 }
 int norm_bwd(const float *dn, const float *x, const float2 *st, const float *add, float *out, int64_t n, int d, cudaStream_t s) {
     const unsigned g = (unsigned)((n + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK);
-    if (d <= 128) norm_bwd_kernel<1><<<g, 256, 0, s>>>(dn, x, st, add, out, n, d);
-    else if (d <= 256) norm_bwd_kernel<2><<<g, 256, 0, s>>>(dn, x, st, add, out, n, d);
-    else if (d <= 512) norm_bwd_kernel<4><<<g, 256, 0, s>>>(dn, x, st, add, out, n, d);
-    else norm_bwd_kernel<NV_MAX><<<g, 256, 0, s>>>(dn, x, st, add, out, n, d);
+    if (d <= 128) pdl_launch(norm_bwd_kernel<1>, g, 256, 0, s, dn, x, st, add, out, n, d);
+    else if (d <= 256) pdl_launch(norm_bwd_kernel<2>, g, 256, 0, s, dn, x, st, add, out, n, d);
+    else if (d <= 512) pdl_launch(norm_bwd_kernel<4>, g, 256, 0, s, dn, x, st, add, out, n, d);
+    else pdl_launch(norm_bwd_kernel<NV_MAX>, g, 256, 0, s, dn, x, st, add, out, n, d);
     return launched("layer-norm backward");
 }
 
@@ -429,7 +446,7 @@ int prepare_weights(const agpt_train_step_args &A, const Space &S, cudaStream_t 
         int blocks = 0;
         for (int i = 0; i < a.n; i++) { a.job[i] = folds[first + i]; a.first_block[i] = blocks; blocks += (a.job[i].n_pad + 31) / 32; }
         a.first_block[a.n] = blocks;
-        fold_bias_kernel<<<blocks, 256, 0, st>>>(a);
+        pdl_launch(fold_bias_kernel, blocks, 256, 0, st, a);
         TRY(launched("folded biases"));
     }
     return AGPT_OK;
@@ -480,6 +497,12 @@ extern "C" int64_t agpt_b200_train_step_workspace_bytes(const agpt_train_step_ar
     return S.bytes;
 } AGPT_CATCH("train_step_workspace_bytes")
 
+// Blocks are placed early (pdl.cuh) while launches count.  On many rows that costs more than it hides (the blocks of a projection then land on the SMs in
+// the order in which these fall free, not side by side).  Whole steps, early / ordinary, us: d_model 64, 59k rows 1234 / 1281, 117k 1945 / 1980, 231k 3240 / 3226;
+// d_model 128, 5k 1307 / 1420, 20k 1957 / 2053, 59k 3690 / 3653, 231k 11980 / 11650; d_model 256, 5k 1835 / 2000, 20k 3981 / 4070, 59k 9480 / 9220;
+// d_model 384, 5k 2577 / 2755, 20k 7000 / 6890.
+static constexpr int64_t EARLY_ELEMENTS = 6 << 20;
+
 extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *workspace, int64_t workspace_bytes, void *stream) try {
     if (!args || !workspace) return agpt_set_error(AGPT_E_ARG, "train_step: null arguments");
     const agpt_train_step_args &A = *args;
@@ -490,6 +513,7 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
         return agpt_set_error(AGPT_E_ARG, "train_step: workspace %lld bytes < required %lld", (long long)workspace_bytes, (long long)S.bytes);
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t n = A.n;
+    const PdlScope scope(n * A.d_model <= EARLY_ELEMENTS);
     const int D = A.d_model, F = A.d_ff, L = A.n_layers, H = A.n_heads, hd = D / H, V = A.vocab, Vp = padded_vocab(V);
     const float scale = 1.0f / sqrtf((float)hd);
     const int kv_dtype = A.bf16_store ? AGPT_KV_BF16 : AGPT_KV_F32;
@@ -500,7 +524,7 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
     if (e != cudaSuccess) return agpt_set_error(AGPT_E_CUDA, "train_step: %s", cudaGetErrorString(e));
 
     TRY(prepare_weights(A, S, st));
-    TRY(embed_stats(A.params[0], A.tokens, S.x[0], S.stats[0], n, D, V, st));
+    TRY(embed_stats(A.params[0], A.tokens, S.x[0], S.stats[0], n, D, V, st, S.unit_count, A.n_units));
 
     // ---- forward ----
     for (int l = 0; l < L; l++) {
@@ -545,10 +569,8 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
                                  A.mass_weights, S.dlogits, S.loss, n, Vp, lambda, A.intermediate_weight, A.ce_only, st));
     const int64_t n_pad = (n + 127) & ~(int64_t)127;
     const int lb = (int)((n + 1023) / 1024);
-    e = cudaMemsetAsync(S.unit_count, 0, (size_t)A.n_units * 4, st);
-    if (e != cudaSuccess) return agpt_set_error(AGPT_E_CUDA, "train_step: %s", cudaGetErrorString(e));
-    loss_count_kernel<<<lb, 256, 0, st>>>(S.loss, A.trained, A.unit_of_row, n, S.unit_count, S.block_sum, S.block_count);
-    row_scale_kernel<<<(unsigned)std::min<int64_t>((n_pad + 255) / 256, 148 * 8), 256, 0, st>>>(A.trained, A.unit_of_row, S.unit_count, n, n_pad, S.scale,
+    pdl_launch(loss_count_kernel, lb, 256, 0, st, S.loss, A.trained, A.unit_of_row, n, S.unit_count, S.block_sum, S.block_count);
+    pdl_launch(row_scale_kernel, (unsigned)std::min<int64_t>((n_pad + 255) / 256, 148 * 8), 256, 0, st, A.trained, A.unit_of_row, S.unit_count, n, n_pad, S.scale,
                                                                                                   S.block_sum, S.block_count, lb, A.loss_sum, A.loss_count, A.tail);
     TRY(launched("loss statistics"));
 
@@ -628,11 +650,11 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
         int blocks = 0;
         for (int i = 0; i < a.n; i++) { a.job[i] = jobs[first + i]; a.first_block[i] = blocks; blocks += (a.job[i].cols + 31) / 32; }
         a.first_block[a.n] = blocks;
-        grad_cols_kernel<<<blocks, 256, 0, st>>>(a);
+        pdl_launch(grad_cols_kernel, blocks, 256, 0, st, a);
         blocks = 0;
         for (int i = 0; i < a.n; i++) { a.first_block[i] = blocks; blocks += a.job[i].rows; }
         a.first_block[a.n] = blocks;
-        grad_rows_kernel<<<blocks, 128, 0, st>>>(a);
+        pdl_launch(grad_rows_kernel, blocks, 128, 0, st, a);
         TRY(launched("weight gradients"));
     }
     return AGPT_OK;
