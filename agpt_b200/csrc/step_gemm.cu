@@ -748,11 +748,19 @@ int agpt_step_gemm_status(int *out) {
 // ---------------------------------------------------------------------------------------------------------------------
 namespace {
 
-struct ConArgs {
+struct alignas(64) ConJob {
+    CUtensorMap a, b[3];
     RowContract g;
     int nt, m_tiles, groups;         // width of an accumulator (half of a column group), 128-feature tiles, column groups
     int64_t row_blocks;
 };
+// A launch forms one weight gradient, or (few rows) as many as there are at once.
+constexpr int CON_JOBS = 40;
+template <int JOBS> struct ConBatch {
+    ConJob job[JOBS];
+    int first_block[JOBS], n;
+};
+static_assert(sizeof(ConBatch<CON_JOBS>) <= 32764, "kernel parameters");
 
 constexpr int CON_THREADS = 640, CON_ROWS = 64;
 constexpr int CON_A = 4 * 8192, CON_B = 4 * 8192, CON_P = 3 * 16384;      // raw A, raw B (one half), B planes
@@ -764,19 +772,25 @@ static_assert(CON_SMEM <= SMEM_LIMIT, "shared memory");
 constexpr int CREG_ISSUE = 40, CREG_A = 64, CREG_B = 64, CREG_ACC = 152;
 static_assert(CREG_ISSUE + CREG_A + CREG_B + 2 * CREG_ACC <= 5 * 96, "setmaxnreg draws on the registers of the launch");
 
-__global__ void __launch_bounds__(CON_THREADS, 1)
-contract_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap m0, const __grid_constant__ CUtensorMap m1,
-                const __grid_constant__ CUtensorMap m2, const __grid_constant__ ConArgs P) {
+template <int JOBS>
+__global__ void __launch_bounds__(CON_THREADS, 1) contract_kernel(const __grid_constant__ ConBatch<JOBS> batch) {
     extern __shared__ __align__(1024) unsigned char dyn[];
-    const RowContract &g = P.g;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, wq = warp & 3;
+    int job = 0;
+    if (JOBS > 1) {
+        for (int i = lane; i - lane < JOBS; i += 32) job += __popc(__ballot_sync(0xffffffffu, i < batch.n && (int)blockIdx.x >= batch.first_block[min(i, JOBS - 1)]));
+        job--;
+    }
+    const ConJob &P = batch.job[job];
+    const RowContract &g = P.g;
+    const int block = blockIdx.x - (JOBS > 1 ? batch.first_block[job] : 0);
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~(uintptr_t)1023);
     const uint32_t sA = smem_u32(smem), sB = sA + CON_OFF_B, sP = sA + CON_OFF_P, bars = sA + CON_OFF_BAR;
     volatile int &s_abort = *reinterpret_cast<volatile int *>(smem + CON_OFF_BAR + CON_BAR_BYTES - 16);
     uint32_t &s_tmem = *reinterpret_cast<uint32_t *>(smem + CON_OFF_BAR + CON_BAR_BYTES - 8);
     const uint32_t aF = bars, aE = aF + 16, bF = aE + 16, bE = bF + 16, pF = bE + 16, pE = pF + 16, tF = pE + 16, tE = tF + 16, cF = tE + 16, cE = cF + 16;
     const int units = P.m_tiles * P.groups;
-    const int unit = blockIdx.x % units, slice = blockIdx.x / units;
+    const int unit = block % units, slice = block / units;
     const int m_first = (unit % P.m_tiles) * 128, n_first = (unit / P.m_tiles) * 2 * P.nt;
     const int mb = (min(128, g.m - m_first) + 31) >> 5;                    // boxes of 32 features
     const int halves = g.n - n_first > P.nt ? 2 : 1;
@@ -812,7 +826,7 @@ contract_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ 
                 if (!(ok = mbar_wait(aE + 8 * as, ap ^ 1, &s_abort))) break;
                 mbar_expect(aF + 8 * as, (uint32_t)(mb * 8192 + (g.stats ? 512 : 0)));
                 if (g.stats) bulk_load(sA + CON_OFF_STAT + as * 512, g.stats + rb * CON_ROWS, 512, aF + 8 * as);
-                for (int j = 0; j < mb; j++) tma_load_2d(sA + as * CON_A + j * 8192, &mA, m_first + j * 32, y, aF + 8 * as);
+                for (int j = 0; j < mb; j++) tma_load_2d(sA + as * CON_A + j * 8192, &P.a, m_first + j * 32, y, aF + 8 * as);
                 if (++as == 2) { as = 0; ap ^= 1; }
                 for (int h = 0; h < halves; h++) {
                     if (!(ok = mbar_wait(bE + 8 * bs, bp ^ 1, &s_abort))) break;
@@ -822,7 +836,7 @@ contract_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ 
                     for (int j = 0; j < nb; j++) {
                         const int cc = n_first + h * P.nt + j * 32;
                         const int seg = min(cc / g.seg_cols, g.n_seg - 1);
-                        tma_load_2d(sB + bs * CON_B + j * 8192, seg == 0 ? &m0 : (seg == 1 ? &m1 : &m2), cc - seg * g.seg_cols, y, bF + 8 * bs);
+                        tma_load_2d(sB + bs * CON_B + j * 8192, &P.b[seg], cc - seg * g.seg_cols, y, bF + 8 * bs);
                     }
                     if (++bs == 2) { bs = 0; bp ^= 1; }
                 }
@@ -1009,9 +1023,17 @@ contract_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ 
                         }
                 } else {
                     float *po = part + (int64_t)mm * g.n + nh;
+                    if ((g.n & 7) == 0) {                          // whole sectors: rows on 32-byte boundaries
 #pragma unroll
-                    for (int i = 0; i < ACC_COLS / 4; i++)
-                        if (4 * i < wh) *reinterpret_cast<ulonglong2 *>(po + 4 * i) = make_ulonglong2(acc[2 * i], acc[2 * i + 1]);
+                        for (int i = 0; i < ACC_COLS / 8; i++)
+                            if (8 * i < wh)
+                                asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(po + 8 * i), "l"(acc[4 * i]), "l"(acc[4 * i + 1]), "l"(acc[4 * i + 2]),
+                                             "l"(acc[4 * i + 3]) : "memory");
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < ACC_COLS / 4; i++)
+                            if (4 * i < wh) *reinterpret_cast<ulonglong2 *>(po + 4 * i) = make_ulonglong2(acc[2 * i], acc[2 * i + 1]);
+                    }
                 }
             }
         }
@@ -1033,28 +1055,63 @@ void contract_shape(int m, int n, int &nt, int &m_tiles, int &groups) {
 }  // namespace
 
 // One block per (feature tile, column group, slice of the rows): as many slices as fill the SMs, none without rows.
-int agpt_row_contract_slices(int64_t rows, int m, int n) {
+int agpt_row_contract_units(int m, int n) {
     int nt, mt, gr;
     contract_shape(m, n, nt, mt, gr);
+    return mt * gr;
+}
+int agpt_row_contract_slices(int64_t rows, int m, int n) {
     const int64_t blocks = (rows + CON_ROWS - 1) / CON_ROWS;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(sm_count() / (mt * gr), blocks));
+    return (int)std::max<int64_t>(1, std::min<int64_t>(sm_count() / agpt_row_contract_units(m, n), blocks));
+}
+// The same for contractions that share a launch, `units` blocks per slice in all.  A slice costs a block its start, its last drain and stores, 6 us together, and
+// a row of partial sums to add, so few: one round of blocks.  Up to 20 or so row blocks each is a slice of its own, as in a launch apart (the same sums, bit for bit).
+int agpt_row_contract_shared_slices(int64_t rows, int units) {
+    const int64_t blocks = std::max<int64_t>(1, (rows + CON_ROWS - 1) / CON_ROWS), one_round = std::max(1, sm_count() / units);
+    return (int)(blocks <= 4 * one_round ? blocks : one_round);
+}
+
+static int contract_job(const RowContract &g, ConJob &P) {
+    P.g = g;
+    contract_shape(g.m, g.n, P.nt, P.m_tiles, P.groups);
+    P.row_blocks = (g.rows + CON_ROWS - 1) / CON_ROWS;
+    if (int rc = encode_map(&P.a, g.a, g.rows, g.m, g.lda, CON_ROWS)) return rc;
+    for (int i = 0; i < g.n_seg; i++)
+        if (int rc = encode_map(&P.b[i], g.b[i], g.rows, g.seg_cols, g.ldb, CON_ROWS)) return rc;
+    for (int i = g.n_seg; i < 3; i++) P.b[i] = P.b[0];
+    return AGPT_OK;
+}
+
+template <int JOBS>
+static int launch_contract(const ConBatch<JOBS> &batch, int blocks, cudaStream_t st) {
+    static bool done[64];
+    if (int rc = allow_smem(contract_kernel<JOBS>, done)) return rc;
+    pdl_launch(contract_kernel<JOBS>, blocks, CON_THREADS, CON_SMEM, st, batch);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return agpt_set_error(AGPT_E_CUDA, "row_contract: %s", cudaGetErrorString(e));
+    return AGPT_OK;
 }
 
 int agpt_row_contract(const RowContract &g, cudaStream_t st) {
     if (g.rows <= 0) return AGPT_OK;
-    ConArgs P;
-    P.g = g;
-    contract_shape(g.m, g.n, P.nt, P.m_tiles, P.groups);
-    P.row_blocks = (g.rows + CON_ROWS - 1) / CON_ROWS;
-    CUtensorMap mA, m[3];
-    if (int rc = encode_map(&mA, g.a, g.rows, g.m, g.lda, CON_ROWS)) return rc;
-    for (int i = 0; i < g.n_seg; i++)
-        if (int rc = encode_map(&m[i], g.b[i], g.rows, g.seg_cols, g.ldb, CON_ROWS)) return rc;
-    for (int i = g.n_seg; i < 3; i++) m[i] = m[0];
-    static bool done[64];
-    if (int rc = allow_smem(contract_kernel, done)) return rc;
-    pdl_launch(contract_kernel, P.m_tiles * P.groups * g.slices, CON_THREADS, CON_SMEM, st, mA, m[0], m[1], m[2], P);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return agpt_set_error(AGPT_E_CUDA, "row_contract: %s", cudaGetErrorString(e));
+    ConBatch<1> b;
+    if (int rc = contract_job(g, b.job[0])) return rc;
+    b.n = 1; b.first_block[0] = 0;
+    return launch_contract(b, b.job[0].m_tiles * b.job[0].groups * g.slices, st);
+}
+
+int agpt_row_contract_many(const RowContract *g, int n, cudaStream_t st) {
+    for (int first = 0; first < n; first += CON_JOBS) {
+        ConBatch<CON_JOBS> b;
+        int blocks = 0;
+        b.n = std::min(CON_JOBS, n - first);
+        for (int i = 0; i < b.n; i++) {
+            if (g[first + i].rows <= 0) return AGPT_OK;          // they share their rows
+            if (int rc = contract_job(g[first + i], b.job[i])) return rc;
+            b.first_block[i] = blocks;
+            blocks += b.job[i].m_tiles * b.job[i].groups * g[first + i].slices;
+        }
+        if (int rc = launch_contract(b, blocks, st)) return rc;
+    }
     return AGPT_OK;
 }

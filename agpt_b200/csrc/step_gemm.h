@@ -66,7 +66,10 @@ struct RowContract {
     float *part = nullptr;              // [slices][m * n]
     float *col_part = nullptr;          // [slices][col_ld] column sums of B' (of A' when transposed), or null
     int col_ld = 0;
-    int slices = 0;                     // set by agpt_row_contract_slices
+    int slices = 0;                     // agpt_row_contract_slices, or agpt_row_contract_shared_slices
 };
+int agpt_row_contract_units(int m, int n);
 int agpt_row_contract_slices(int64_t rows, int m, int n);
+int agpt_row_contract_shared_slices(int64_t rows, int units);      // units: those of all contractions of the launch
 int agpt_row_contract(const RowContract &g, cudaStream_t st);
+int agpt_row_contract_many(const RowContract *g, int n, cudaStream_t st);

@@ -302,6 +302,7 @@ __global__ void __launch_bounds__(128) grad_rows_kernel(const __grid_constant__ 
 // ---- workspace ---------------------------------------------------------------------------------------------------------
 struct Layer {
     float *q, *a, *xm, *h, *lse;
+    float *dh, *dxm, *dqkv;              // gradients of h, of xm, of q, k and v (three times rows x d_model)
     void *k, *v;
     uint32_t *mask;
     float2 *stats2;
@@ -314,7 +315,8 @@ struct Space {
     std::vector<float2 *> stats;         // their statistics
     uint8_t *head, *head_t;
     float *head_b;
-    float *dx, *u, *tmp;                 // residual gradient; the union below; d_model > 128: gradient of normalised rows
+    std::vector<float *> dx;             // gradients of the layer inputs and of the last layer's output (few rows; else one buffer)
+    float *u, *tmp;                      // the union below; d_model > 128: gradient of normalised rows
     float *logits, *dlogits, *loss, *scale;
     double *block_sum;
     int32_t *block_count, *unit_count;
@@ -324,10 +326,21 @@ struct Space {
     int64_t emb_bytes;
     std::vector<float *> part;           // partial weight gradients, head first, then four per layer
     std::vector<float *> col_part, col_sum;
+    int shared_slices;                   // few rows: slices of every contraction
     int64_t bytes;
 };
 constexpr int P_PER_LAYER = 16;
 enum { WQ, BQ, WK, BK, WV, BV, WO, BO, G1, B1, W1, BW1, W2, BW2, G2, B2 };
+
+// A step on few rows (rows x d_model).  Its launches count: all weight gradients are formed by one launch at the end of the backward, for which the
+// gradients of the rows are kept layer by layer (nine times d_model a row and layer, a megabyte for the 60 rows of a sampled unit).
+//
+// Blocks are placed early (pdl.cuh) while launches count.  On many rows that costs more than it hides (the blocks of a projection then land on the SMs in
+// the order in which these fall free, not side by side).  Whole steps, early / ordinary, us: d_model 64, 59k rows 1234 / 1281, 117k 1945 / 1980, 231k 3240 / 3226;
+// d_model 128, 5k 1307 / 1420, 20k 1957 / 2053, 59k 3690 / 3653, 231k 11980 / 11650; d_model 256, 5k 1835 / 2000, 20k 3981 / 4070, 59k 9480 / 9220;
+// d_model 384, 5k 2577 / 2755, 20k 7000 / 6890.
+constexpr int64_t EARLY_ELEMENTS = 6 << 20;
+bool few_rows(const agpt_train_step_args &A) { return A.n * A.d_model <= EARLY_ELEMENTS; }
 
 int padded_vocab(int v) { return (v + 3) & ~3; }
 
@@ -339,7 +352,8 @@ void lay_out(const agpt_train_step_args &A, char *base, Space &S) {
     const int64_t row = n * D * 4, kv = n * D * (A.bf16_store ? 2 : 4);
     S.layer.resize(L); S.x.resize(L + 1); S.stats.resize(L + 1);
     for (int l = 0; l <= L; l++) { S.x[l] = (float *)take(row); S.stats[l] = (float2 *)take(n_pad * 8); }
-    float *h_shared = A.ffn_recompute ? (float *)take(n * F * 4) : nullptr;
+    const bool few = few_rows(A);
+    float *h_shared = A.ffn_recompute && !few ? (float *)take(n * F * 4) : nullptr;
     for (int l = 0; l < L; l++) {
         Layer &y = S.layer[l];
         y.q = (float *)take(row); y.k = take(kv); y.v = take(kv); y.a = (float *)take(row); y.lse = (float *)take(n * H * 4);
@@ -354,11 +368,25 @@ void lay_out(const agpt_train_step_args &A, char *base, Space &S) {
     }
     S.head = (uint8_t *)take(agpt_weight_image_bytes(Vp, D)); S.head_t = (uint8_t *)take(agpt_weight_image_bytes(D, A.vocab));
     S.head_b = (float *)take(Vp * 4);
-    S.dx = (float *)take(row);
-    // one region in turn: logits and their gradient; the feed-forward gradient; the gradients of the attention's output and
-    // of q, k, v
-    S.u = (float *)take(n * 4 * (int64_t)std::max(std::max(F, 4 * D), 2 * Vp));
-    S.logits = S.u; S.dlogits = S.u + n * Vp;
+    S.dx.resize(L + 1);
+    if (few) {
+        for (int l = 0; l <= L; l++) S.dx[l] = (float *)take(row);
+        for (int l = 0; l < L; l++) {
+            Layer &y = S.layer[l];
+            y.dh = (float *)take(n * F * 4); y.dxm = (float *)take(row); y.dqkv = (float *)take(3 * row);
+        }
+        S.u = (float *)take(row);        // the gradient of the attention's output
+        S.logits = (float *)take(n * 8 * (int64_t)Vp);
+    } else {
+        float *dx = (float *)take(row);
+        // one region in turn: logits and their gradient; the feed-forward gradient; the gradients of the attention's output and
+        // of q, k, v
+        S.u = (float *)take(n * 4 * (int64_t)std::max(std::max(F, 4 * D), 2 * Vp));
+        for (int l = 0; l <= L; l++) S.dx[l] = dx;
+        for (int l = 0; l < L; l++) { S.layer[l].dh = S.u; S.layer[l].dxm = dx; S.layer[l].dqkv = S.u + n * D; }
+        S.logits = S.u;
+    }
+    S.dlogits = S.logits + n * Vp;
     S.tmp = D > 128 ? (float *)take(row) : nullptr;
     S.loss = (float *)take(n * 4); S.scale = (float *)take(n_pad * 4);
     const int64_t lb = (n + 1023) / 1024;
@@ -368,8 +396,10 @@ void lay_out(const agpt_train_step_args &A, char *base, Space &S) {
     S.emb_bytes = agpt_b200_embedding_grad_workspace_bytes(n, D, A.vocab);
     S.emb = (float *)take(S.emb_bytes);
     S.part.clear(); S.col_part.clear(); S.col_sum.clear();
+    const int units = agpt_row_contract_units(D, Vp) + L * (agpt_row_contract_units(D, 3 * D) + agpt_row_contract_units(D, D) + 2 * agpt_row_contract_units(D, F));
+    S.shared_slices = few ? agpt_row_contract_shared_slices(n, units) : 0;
     auto part = [&](int m, int k, int cols) {
-        const int64_t s = agpt_row_contract_slices(n, m, k);
+        const int64_t s = few ? S.shared_slices : agpt_row_contract_slices(n, m, k);
         S.part.push_back((float *)take(s * m * k * 4)); S.col_part.push_back((float *)take(s * cols * 4)); S.col_sum.push_back((float *)take(cols * 4));
     };
     part(D, Vp, Vp);
@@ -461,18 +491,18 @@ RowContract contract(const agpt_train_step_args &A, const Space &S, int i, const
     RowContract c;
     c.rows = A.n; c.m = m; c.n = n; c.a = a; c.lda = m; c.b[0] = b; c.seg_cols = n; c.ldb = n;
     c.part = S.part[i]; c.col_part = S.col_part[i]; c.col_ld = n;
-    c.slices = agpt_row_contract_slices(A.n, m, n);
+    c.slices = S.shared_slices ? S.shared_slices : agpt_row_contract_slices(A.n, m, n);
     return c;
 }
 // dx = the gradient of the rows in front of a layer norm (+ add) from the product that is the gradient of the normalised rows
-int norm_gradient(const agpt_train_step_args &A, const Space &S, RowGemm g, const float *x, const float2 *stats, const float *add, cudaStream_t st) {
+int norm_gradient(const agpt_train_step_args &A, const Space &S, RowGemm g, const float *x, const float2 *stats, const float *add, float *dx, cudaStream_t st) {
     if (A.d_model <= 128) {
-        g.epi = EPI_NORM_BWD; g.x = x; g.stats = stats; g.add = add; g.out = S.dx; g.ldo = A.d_model;
+        g.epi = EPI_NORM_BWD; g.x = x; g.stats = stats; g.add = add; g.out = dx; g.ldo = A.d_model;
         return agpt_row_gemm(g, st);
     }
     g.out = S.tmp; g.ldo = A.d_model;
     TRY(agpt_row_gemm(g, st));
-    return norm_bwd(S.tmp, x, stats, add, S.dx, A.n, A.d_model, st);
+    return norm_bwd(S.tmp, x, stats, add, dx, A.n, A.d_model, st);
 }
 
 int ff1_forward(const agpt_train_step_args &A, const Layer &y, cudaStream_t st) {
@@ -497,12 +527,6 @@ extern "C" int64_t agpt_b200_train_step_workspace_bytes(const agpt_train_step_ar
     return S.bytes;
 } AGPT_CATCH("train_step_workspace_bytes")
 
-// Blocks are placed early (pdl.cuh) while launches count.  On many rows that costs more than it hides (the blocks of a projection then land on the SMs in
-// the order in which these fall free, not side by side).  Whole steps, early / ordinary, us: d_model 64, 59k rows 1234 / 1281, 117k 1945 / 1980, 231k 3240 / 3226;
-// d_model 128, 5k 1307 / 1420, 20k 1957 / 2053, 59k 3690 / 3653, 231k 11980 / 11650; d_model 256, 5k 1835 / 2000, 20k 3981 / 4070, 59k 9480 / 9220;
-// d_model 384, 5k 2577 / 2755, 20k 7000 / 6890.
-static constexpr int64_t EARLY_ELEMENTS = 6 << 20;
-
 extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *workspace, int64_t workspace_bytes, void *stream) try {
     if (!args || !workspace) return agpt_set_error(AGPT_E_ARG, "train_step: null arguments");
     const agpt_train_step_args &A = *args;
@@ -513,7 +537,8 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
         return agpt_set_error(AGPT_E_ARG, "train_step: workspace %lld bytes < required %lld", (long long)workspace_bytes, (long long)S.bytes);
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t n = A.n;
-    const PdlScope scope(n * A.d_model <= EARLY_ELEMENTS);
+    const bool few = few_rows(A), recompute = A.ffn_recompute && !few;
+    const PdlScope scope(few);
     const int D = A.d_model, F = A.d_ff, L = A.n_layers, H = A.n_heads, hd = D / H, V = A.vocab, Vp = padded_vocab(V);
     const float scale = 1.0f / sqrtf((float)hd);
     const int kv_dtype = A.bf16_store ? AGPT_KV_BF16 : AGPT_KV_F32;
@@ -532,7 +557,7 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
         const Layer &y = S.layer[l];
         RowGemm g = gemm(A, S.x[l], D, y.qkv, 3 * D);
         g.pro = PRO_NORM; g.stats = S.stats[l]; g.epi = EPI_QKV; g.bias = y.qkv_b; g.head_dim = hd;
-        float *k32 = S.u, *v32 = S.u + n * D;    // a table too large for shared memory: rotate (and round) in passes of their own
+        float *k32 = y.dqkv, *v32 = y.dqkv + n * D;    // a table too large for shared memory: rotate (and round) in passes of their own
         const bool late = !fused_rope && A.bf16_store;
         g.qkv[0] = y.q; g.qkv[1] = late ? k32 : y.k; g.qkv[2] = late ? v32 : y.v;
         g.kv_bf16 = A.bf16_store && !late;
@@ -576,6 +601,12 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
 
     // ---- backward ----
     std::vector<GradJob> jobs;
+    std::vector<RowContract> later;              // few rows: contractions for the launch at the end
+    auto weight_gradient = [&](const RowContract &c) {
+        if (!few) return agpt_row_contract(c, st);
+        later.push_back(c);
+        return (int)AGPT_OK;
+    };
     auto grad_job = [&](int i, const RowContract &c, bool transposed) {
         GradJob j = {};
         j.part = S.part[i]; j.col_part = S.col_part[i]; j.col_sum = S.col_sum[i]; j.slices = c.slices; j.col_ld = c.col_ld;
@@ -585,46 +616,47 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
     {
         RowContract c = contract(A, S, 0, S.x[L], D, S.dlogits, Vp);
         c.stats = S.stats[L]; c.row_scale = S.scale;
-        TRY(agpt_row_contract(c, st));
+        TRY(weight_gradient(c));
         GradJob j = grad_job(0, c, false);
         j.cols = j.seg_cols = V;
         j.dw[0] = gf[2]; j.db[0] = gf[3]; j.w[0] = pf[2]; j.gain = pf[0]; j.shift = pf[1]; j.dgain = gf[0]; j.dshift = gf[1];
         jobs.push_back(j);
         RowGemm g = gemm(A, S.dlogits, Vp, S.head_t, D);
         g.pro = PRO_SCALE; g.row_scale = S.scale;
-        TRY(norm_gradient(A, S, g, S.x[L], S.stats[L], nullptr, st));
+        TRY(norm_gradient(A, S, g, S.x[L], S.stats[L], nullptr, S.dx[L], st));
     }
-    float *dh = S.u, *da = S.u, *dq = S.u + n * D, *dk = S.u + 2 * n * D, *dv = S.u + 3 * n * D;
+    float *da = S.u;
     for (int l = L - 1; l >= 0; l--) {
         const float *const *p = A.params + 1 + P_PER_LAYER * l;
         float *const *gp = A.grads + 1 + P_PER_LAYER * l;
         const Layer &y = S.layer[l];
         const int i0 = 1 + 4 * l;
-        if (A.ffn_recompute) TRY(ff1_forward(A, y, st));
+        float *dh = y.dh, *dq = y.dqkv, *dk = dq + n * D, *dv = dk + n * D;
+        if (recompute) TRY(ff1_forward(A, y, st));
         // feed-forward: dW2 = h^T dx (stored transposed: its rows are h's features), dh = dx W2^T where h > 0
-        RowContract c = contract(A, S, i0 + 3, S.dx, D, y.h, F);
+        RowContract c = contract(A, S, i0 + 3, S.dx[l + 1], D, y.h, F);
         c.transposed = 1; c.col_ld = D;
-        TRY(agpt_row_contract(c, st));
+        TRY(weight_gradient(c));
         GradJob j = grad_job(i0 + 3, c, true);
         j.dw[0] = gp[W2]; j.db[0] = gp[BW2];
         jobs.push_back(j);
-        RowGemm g = gemm(A, S.dx, D, y.ff2_t, F);
+        RowGemm g = gemm(A, S.dx[l + 1], D, y.ff2_t, F);
         g.epi = EPI_MASKED; g.mask_in = y.mask; g.out = dh; g.ldo = F;
         TRY(agpt_row_gemm(g, st));
         c = contract(A, S, i0 + 2, y.xm, D, dh, F);
         c.stats = y.stats2;
-        TRY(agpt_row_contract(c, st));
+        TRY(weight_gradient(c));
         j = grad_job(i0 + 2, c, false);
         j.dw[0] = gp[W1]; j.db[0] = gp[BW1]; j.w[0] = p[W1]; j.gain = p[G2]; j.shift = p[B2]; j.dgain = gp[G2]; j.dshift = gp[B2];
         jobs.push_back(j);
-        TRY(norm_gradient(A, S, gemm(A, dh, F, y.ff1_t, D), y.xm, y.stats2, S.dx, st));
+        TRY(norm_gradient(A, S, gemm(A, dh, F, y.ff1_t, D), y.xm, y.stats2, S.dx[l + 1], y.dxm, st));
         // attention output projection
-        c = contract(A, S, i0 + 1, y.a, D, S.dx, D);
-        TRY(agpt_row_contract(c, st));
+        c = contract(A, S, i0 + 1, y.a, D, y.dxm, D);
+        TRY(weight_gradient(c));
         j = grad_job(i0 + 1, c, false);
         j.dw[0] = gp[WO]; j.db[0] = gp[BO];
         jobs.push_back(j);
-        g = gemm(A, S.dx, D, y.wo_t, D);
+        g = gemm(A, y.dxm, D, y.wo_t, D);
         g.out = da; g.ldo = D;
         TRY(agpt_row_gemm(g, st));
         TRY(agpt_b200_attn_bwd_mode(A.plan, y.q, y.k, y.v, kv_dtype, y.a, y.lse, da, dq, dk, dv, S.attn, S.attn_bytes, H, hd, scale, A.grad_mode,
@@ -633,7 +665,7 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
         // the three projections that read the same normalised rows
         c = contract(A, S, i0, S.x[l], D, dq, 3 * D);
         c.b[1] = dk; c.b[2] = dv; c.n_seg = 3; c.seg_cols = D; c.ldb = D; c.stats = S.stats[l];
-        TRY(agpt_row_contract(c, st));
+        TRY(weight_gradient(c));
         j = grad_job(i0, c, false);
         j.seg_cols = D;
         for (int i = 0; i < 3; i++) { j.dw[i] = gp[WQ + 2 * i]; j.db[i] = gp[BQ + 2 * i]; j.w[i] = p[WQ + 2 * i]; }
@@ -641,9 +673,10 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
         jobs.push_back(j);
         g = gemm(A, dq, 3 * D, y.qkv_t, D);
         g.a[1] = dk; g.a[2] = dv; g.n_seg = 3; g.seg_cols = D; g.lda = D;
-        TRY(norm_gradient(A, S, g, S.x[l], S.stats[l], S.dx, st));
+        TRY(norm_gradient(A, S, g, S.x[l], S.stats[l], y.dxm, S.dx[l], st));
     }
-    TRY(agpt_b200_embedding_grad(S.dx, A.tokens, A.grads[0], n, D, V, 1, S.emb, S.emb_bytes, st));
+    if (few) TRY(agpt_row_contract_many(later.data(), (int)later.size(), st));
+    TRY(agpt_b200_embedding_grad(S.dx[0], A.tokens, A.grads[0], n, D, V, 1, S.emb, S.emb_bytes, st));
     for (size_t first = 0; first < jobs.size(); first += GRAD_JOBS) {
         GradArgs a;
         a.n = (int)std::min<size_t>(GRAD_JOBS, jobs.size() - first);
