@@ -22,12 +22,19 @@ struct PdlScope {
     PdlScope(const PdlScope &) = delete;
 };
 
+// cluster: blocks of a cluster along x (1: none)
+template <typename... P, typename... A>
+static inline cudaError_t pdl_launch_clusters(void (*kernel)(P...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = pdl_early ? 1 : 0;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)cluster; at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = st; c.attrs = at; c.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
 template <typename... P, typename... A>
 static inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t c = {};
-    c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = st; c.attrs = &at; c.numAttrs = pdl_early ? 1 : 0;
-    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+    return pdl_launch_clusters(kernel, 1, grid, block, smem, st, static_cast<A &&>(args)...);
 }
