@@ -2171,7 +2171,9 @@ static int fwd_dispatch(const agpt_plan *p, const float *q, const void *k, const
         fwd_bf16_smem_bytes(head_dim, bwd_tile_maxk(p)) <= (size_t)113 * 1024) {
         switch (head_dim) {
             case 16: return launch_fwd_bf16<16, 8>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
-            case 32: return launch_fwd_bf16<32, 6>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
+            // eight blocks (64 registers, three spilled) hide more of the loads' latency than six: 8 x 32, 579k rows of depth 32 583 -> 533 us, seven 567,
+            // nine 572; 16 does best with eight (ten 113 against 108), 64 with four (three 730, five 781 against 725)
+            case 32: return launch_fwd_bf16<32, 8>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
             case 64: return launch_fwd_bf16<64, 4>(p, q, k, v, out, lse, H, scale, st, tile0, ntiles);
         }
     }
@@ -2220,12 +2222,14 @@ static int launch_bwd_tile_w(const agpt_plan *p, const float *q, const void *k, 
                              const float *lse, const float *dout, float *dq, float *dk, float *dv, float *pk, float *pv, int H,
                              int head_dim, float scale, cudaStream_t st, int tile0, int ntiles, BwdMask gmask) {
 #define TILE_ARGS p, q, k, v, o, lse, dout, dq, dk, dv, pk, pv, H, scale, st, tile0, ntiles, gmask
+    // Blocks per SM at head_dim 16: six (both stores; four 585 / 563, five 534 / 513, six 499 / 465, seven 530 / 484, eight 700 / 492 us: 4 x 16, 579k rows of depth 32,
+    // float32 / bfloat16 store).  At 32 a fifth block of bfloat16 rows spills (1374 -> 1808).
     if (kv_dtype == AGPT_KV_BF16) switch (head_dim) {
-        case 16: return launch_bwd_tile<16, 4, 4, __nv_bfloat16>(TILE_ARGS);
+        case 16: return launch_bwd_tile<16, 4, 6, __nv_bfloat16>(TILE_ARGS);
         case 32: return launch_bwd_tile<32, 4, 4, __nv_bfloat16>(TILE_ARGS);
         default: return launch_bwd_tile<64, 4, 3, __nv_bfloat16>(TILE_ARGS);
     }
-    if (head_dim == 16) return launch_bwd_tile<16, 4, 4>(TILE_ARGS);
+    if (head_dim == 16) return launch_bwd_tile<16, 4, 6>(TILE_ARGS);
     // Four warps are the fastest (with the reduction, us: 4 x 32, 1.4M rows 1771; three blocks of four 2084, six warps 2477, eight 2793; 8 x 64,
     // 600k rows 3305, eight warps 5124): small blocks stage, compute and wait out of step.  The others stay for A/B runs of the public switch.
     if (head_dim == 64) {        // twice the fragment and accumulator registers: two blocks per SM
