@@ -283,10 +283,18 @@ extern "C" int agpt_b200_trie_group_prepare(agpt_run_groups *G, int64_t i, int t
         int64_t k = std::min(M, n - r0), e1 = e0;
         if (tile_m == 64 && !P->even && r0 + M < n) {
             while (g.qoff[e1 + 1] <= r0 + 32) e1++;
-            int64_t best = INT64_MAX;
-            for (int64_t e = e1; e < E && g.qoff[e] <= r0 + M; e++) {
-                const int64_t c = std::max<int64_t>(g.qoff[e] - r0, 32), v = agpt_tile_cost((int32_t)(ld[e] + (r0 + c - g.qoff[e])), c);
-                if (v <= best) { best = v; k = c; e1 = e; }
+            int64_t b = g.qoff[e1] == r0 + 32 ? e1 : e1 + 1;            // the first run from row 32 on that does not hang on the one before it
+            while (b < E && g.prun[b] == b - 1) b++;
+            const int64_t branch = (b < E ? (int64_t)g.qoff[b] : n) - r0;
+            if (branch > M) {
+                k = agpt_tile_of_chain(branch);
+                while (g.qoff[e1 + 1] <= r0 + k) e1++;
+            } else {
+                int64_t best = INT64_MAX;
+                for (int64_t e = e1; e < E && g.qoff[e] <= r0 + M; e++) {
+                    const int64_t c = std::max<int64_t>(g.qoff[e] - r0, 32), v = agpt_tile_cost((int32_t)(ld[e] + (r0 + c - g.qoff[e])), c);
+                    if (v <= best) { best = v; k = c; e1 = e; }
+                }
             }
         } else while (e1 < E && g.qoff[e1 + 1] <= r0 + k) e1++;
         const int64_t chain = ld[e0] + (r0 - g.qoff[e0]) - 1;

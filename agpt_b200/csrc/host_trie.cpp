@@ -787,7 +787,11 @@ static int plan_create(const int32_t *parent, int64_t n, int tile_m, int device,
     for (int64_t i = 0; i < n;) {
         ts.push_back((int32_t)i);
         int64_t k = tile_m;
-        if (early && i + tile_m < n) {
+        int64_t branch = 32;                    // the first row from 32 on that is not a child of the row before it
+        if (early && i + tile_m < n)
+            while (i + branch < n && P->depth[i + branch] > P->depth[i + branch - 1]) branch++;
+        if (early && i + tile_m < n && branch > tile_m) k = agpt_tile_of_chain(branch);
+        else if (early && i + tile_m < n) {
             int64_t best = agpt_tile_cost(P->depth[i + k], k);
             for (int64_t c = k - 1; c >= 32; c--) {
                 const int64_t v = agpt_tile_cost(P->depth[i + c], c);

@@ -129,6 +129,12 @@ struct agpt_plan {
 };
 
 int agpt_plan_upload(agpt_plan *p, int device);
+// Rows of a tile whose first branch (row from 32 on that is not a child of the row before it) lies L > 64 rows away: a chain without branches, as in
+// pruned tries with long repeats.  No end before the branch is shallow, so the chain is cut into as few tiles as hold it, whole ones last, and the last
+// ends at the branch.  (By cost alone the first end in reach would be taken: tiles of 33 rows.)  On the pruned trie of 719k rows of depth 128: 17,251 -> 11,855
+// tiles, chain rows 571k -> 369k, longest tile 141 -> 128 keys; 6 x 64, bfloat16 store, forward 1438 -> 1113 us, backward with reduction 4742 -> 3843; 318k such
+// rows, float32 store, 1639 -> 1285 and 5084 -> 2733 (they fit the whole-tile kernels now).  Tries of depth 32 have no such chain.
+inline int64_t agpt_tile_of_chain(int64_t L) { const int64_t k = (L - 1) % 64 + 1; return k < 32 ? 32 : k; }
 // cost of a tile that starts k rows after the last one's start, at depth d (in tenths of a row)
 inline int64_t agpt_tile_cost(int32_t d, int64_t k) { return 10 * (int64_t)d + 9 * (64 - k); }
 // mass weight of each loss node (agpt_b200_mass_weights without the expansion to queries)
