@@ -418,6 +418,9 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
         const int sw = lane & 7;
         uint32_t lp[2] = {0, 0};                          // parities of the two buffers' loads
         auto piece = [&](int buf, int c16) { return u_stg + buf * 4096 + lane * 128 + ((c16 ^ sw) << 4); };
+        // before chunk c is written: the store that used its buffer last has read it.  That is the store before the last one, but for the first chunk of a
+        // tile of an odd number of chunks, whose buffer the tile before ended with.
+        auto buffer_free = [&](int c, int chunks) { if (c == 0 && (chunks & 1)) stores_read<0>(); else stores_read<1>(); };
         auto fetch = [&](int buf, const CUtensorMap *m, int x, int y) {       // one lane; the buffer is free
             mbar_expect(lF + 8 * buf, 4096);
             tma_load_2d(u_stg + buf * 4096, m, x, y, lF + 8 * buf);
@@ -476,7 +479,7 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
                         if (!(ok = warp_wait(lF + 8 * buf, lp[buf], &s_abort))) break;
                         lp[buf] ^= 1;
                     } else {
-                        if (lane == 0) stores_read<1>();
+                        if (lane == 0) buffer_free(c, chunks);
                         __syncwarp();
                     }
 #pragma unroll
@@ -553,7 +556,7 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
                     const int col = n0 + c * 32, buf = c & 1;
                     if (c >= chunks) continue;
                     const int which = col / D, dc = col - which * D;
-                    if (lane == 0) stores_read<1>();
+                    if (lane == 0) buffer_free(c, chunks);
                     __syncwarp();
                     if (which < 2 && g.cosv) {
                         const int j0 = (dc & (g.head_dim - 1)) >> 1;
