@@ -799,7 +799,7 @@ namespace {
 struct alignas(64) ConJob {
     CUtensorMap a, b[3];
     RowContract g;
-    int nt, m_tiles, groups;         // width of an accumulator (half of a column group), 128-feature tiles, column groups
+    int nt, halves, m_tiles, groups; // width of an accumulator, accumulators of a column group, 128-feature tiles, column groups
     int64_t row_blocks;
 };
 // A launch forms one weight gradient, or (few rows) as many as there are at once.
@@ -839,9 +839,9 @@ __global__ void __launch_bounds__(CON_THREADS, 1) contract_kernel(const __grid_c
     const uint32_t aF = bars, aE = aF + 16, bF = aE + 16, bE = bF + 16, pF = bE + 16, pE = pF + 16, tF = pE + 16, tE = tF + 16, cF = tE + 16, cE = cF + 16;
     const int units = P.m_tiles * P.groups;
     const int unit = block % units, slice = block / units;
-    const int m_first = (unit % P.m_tiles) * 128, n_first = (unit / P.m_tiles) * 2 * P.nt;
+    const int m_first = (unit % P.m_tiles) * 128, n_first = (unit / P.m_tiles) * P.halves * P.nt;
     const int mb = (min(128, g.m - m_first) + 31) >> 5;                    // boxes of 32 features
-    const int halves = g.n - n_first > P.nt ? 2 : 1;
+    const int halves = P.halves == 2 && g.n - n_first > P.nt ? 2 : 1;
     const int w0 = min(P.nt, g.n - n_first), w1 = halves == 2 ? min(P.nt, g.n - n_first - P.nt) : 0;
     const int64_t rb0 = P.row_blocks * slice / g.slices, rb1 = P.row_blocks * (slice + 1) / g.slices;
 
@@ -1093,19 +1093,22 @@ __global__ void __launch_bounds__(CON_THREADS, 1) contract_kernel(const __grid_c
     if (tid == 0 && s_abort) atomicOr(&g_step_status, 2);
 }
 
-void contract_shape(int m, int n, int &nt, int &m_tiles, int &groups) {
+// A group has two accumulators; B of up to 128 columns has one: what bounds the kernel is the splitting of B, a pass per accumulator and row block whatever its
+// width.  (Three groups of one accumulator for 384 columns, nine for 1152, lose more on A, split once per group: a layer of d_model 384 2618 -> 2912 us.)
+void contract_shape(int m, int n, int &nt, int &halves, int &m_tiles, int &groups) {
     m_tiles = (m + 127) / 128;
+    halves = n <= 128 ? 1 : 2;
     groups = (n + 255) / 256;
-    nt = ((n + 2 * groups - 1) / (2 * groups) + 31) & ~31;            // two accumulators per group, columns split evenly
-    groups = (n + 2 * nt - 1) / (2 * nt);
+    nt = ((n + halves * groups - 1) / (halves * groups) + 31) & ~31;      // columns split evenly
+    groups = (n + halves * nt - 1) / (halves * nt);
 }
 
 }  // namespace
 
 // One block per (feature tile, column group, slice of the rows): as many slices as fill the SMs, none without rows.
 int agpt_row_contract_units(int m, int n) {
-    int nt, mt, gr;
-    contract_shape(m, n, nt, mt, gr);
+    int nt, halves, mt, gr;
+    contract_shape(m, n, nt, halves, mt, gr);
     return mt * gr;
 }
 int agpt_row_contract_slices(int64_t rows, int m, int n) {
@@ -1121,7 +1124,7 @@ int agpt_row_contract_shared_slices(int64_t rows, int units) {
 
 static int contract_job(const RowContract &g, ConJob &P) {
     P.g = g;
-    contract_shape(g.m, g.n, P.nt, P.m_tiles, P.groups);
+    contract_shape(g.m, g.n, P.nt, P.halves, P.m_tiles, P.groups);
     P.row_blocks = (g.rows + CON_ROWS - 1) / CON_ROWS;
     if (int rc = encode_map(&P.a, g.a, g.rows, g.m, g.lda, CON_ROWS)) return rc;
     for (int i = 0; i < g.n_seg; i++)
