@@ -11,17 +11,21 @@
 // has).  What the surrounding layers do row by row (layer norm, RoPE, ReLU and its mask, the residual, layer-norm
 // backward) happens in the converting or the accumulator threads, which hold a whole row each.
 //
-// row_gemm_kernel: rows x weights.  Per block: a TMA warp (raw float32 rows, 128-byte swizzle), an MMA thread, four
+// row_gemm_kernel: rows x weights.  Per block: a TMA warp (raw float32 rows, 128-byte swizzle), two MMA warps, four
 //   converting warps, and two groups of four accumulator warps that own one 128-row accumulator each, so that one
 //   drains while the other is being filled.  The weight image (split once per step) stays in shared memory for the
 //   whole kernel when it fits (K <= 128 at 128 columns), else its 64-k blocks stream, each serving two row tiles.
 // contract_kernel: A^T B over the rows (weight gradients).  The transposition of A costs nothing: a converting thread
 //   owns a feature and walks down the rows of the staged tile.  B is split into shared memory with n contiguous.
 //
-// What bounds them: the shared-memory port (128 bytes a clock: B for the MMAs, raw rows in by TMA and out to the
-// converters, result rows through the staging buffers) and, for the wide outputs, the converting and accumulator warps'
-// issue slots.  Measured on 288,000 rows of d_model 128, share of active cycles (tensor pipe, issue slots): q/k/v 39 %, 36 %; attention
-// output 37, 33 (DRAM 58); feed-forward 49, 44; weight gradients of the feed-forward 45, 53, of the 68-column head 14, 47.  Layouts that were tried and were slower: rows stored straight from
+// What bounds them.  An MMA stream alone runs at 64 clocks per 128 x 128 x 16 whatever shared-memory, tensor-memory or barrier traffic runs beside it; a step of 24
+// of them takes 2000 to 3800 clocks here, as the converting warps are never idle (row_gemm_kernel; B's in contract_kernel): a chain of barrier, loads, splits
+// and tensor-memory stores, slowed by instruction fetch (a stall of 1.0 to 2.3 per instruction: the roles' code together exceeds the instruction cache) and by
+// the other roles' shared-memory traffic.  Sustained, training sits at the board's power limit (985 W, 1690 of 1965 MHz).  Share of active cycles on 288,000 rows of
+// d_model 128 (tensor pipe, issue slots): q/k/v 39 %, 36 %; attention output 37, 33 (DRAM 58); feed-forward 49, 44; weight gradients 45, 53.  Tried and slower:
+// eight converting warps (1080 -> 1417 us, six projections of d_model 256), one MMA warp that asks barriers ahead (1168), counters in shared memory in place of the
+// barriers (1197; with two MMA warps in turn 1163), non-blocking barrier tests in the converters (an epoch of d_model 128 53.8 -> 55.3 ms), B rows of
+// contract_kernel loaded one ahead (no change) or four at once (2208 -> 2742), rows stored straight from
 // the accumulator threads, 32 bytes to 32 rows at a time (the store path held up the MMA issue too; wide outputs 2x); MMAs
 // issued by one lane of a diverged warp (60 clocks each against 29 from an elected lane of a converged warp); scalar
 // instead of paired (f32x2) conversions; a drain of the accumulator every 128 k instead of 64 (10 % faster, but the
@@ -29,7 +33,8 @@
 // Measured, 560,000 rows, d_model 128, d_ff 512 (in brackets: the CUTLASS fast-float32 mainloop and the row kernels around
 // it): q/k/v with layer norm and RoPE 419 us (437 + 97 + 187); attention output with residual and statistics 151 (160);
 // feed-forward 427 + 369 (550 + 97 + 500); their input gradients 408 + 473 and 389 for q/k/v with the layer-norm backward;
-// weight with bias gradients 423 / 215 / 452 / 446.  Error against float64 6e-8 to 1.2e-7 (K = 64 to 1536), as before.
+// weight with bias gradients 423 / 215 / 452 / 446.  Since then two MMA warps (d_model 256, two layers: projections 1219 + 865 + 665 + 655 + 576 ->
+// 1075 + 817 + 668 + 635 + 542) and one accumulator for narrow weight gradients.  Error against float64 6e-8 to 1.2e-7 (K = 64 to 1536), as before.
 #include "step_gemm.h"
 
 #include <algorithm>

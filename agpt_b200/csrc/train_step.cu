@@ -12,7 +12,7 @@
 //   * bias gradients are column sums of an operand the weight gradient has in its hands anyway.
 //   * RoPE, ReLU and its mask (one bit per element), the residual sums and the layer-norm backward are epilogues.
 // Per layer: five launches forward, nine and the attention's three backward; the partial weight gradients of all layers
-// are summed by two launches at the end.
+// are summed by two launches at the end.  On few rows all weight gradients are one launch more instead of four a layer.
 #include <algorithm>
 #include <cmath>
 #include <vector>
