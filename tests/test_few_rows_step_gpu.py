@@ -14,6 +14,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("n,depth,d,heads,ff,layers,kw", [
     (63, 9, 64, 4, 256, 2, {}),                                              # one row block, one slice
     (65, 9, 128, 4, 512, 1, dict(grad_mode="local_depth")),                  # two
+    (500, 12, 96, 3, 160, 1, {}),                                            # whole rows over clusters of three blocks
+    (4736, 12, 128, 4, 512, 1, {}),                                          # the last row count whose row tiles have a cluster each on 148 SMs,
+    (4737, 12, 128, 4, 512, 1, {}),                                          # the first without
     (1344, 12, 32, 2, 64, 11, {}),                                           # 45 contractions: two launches, several row blocks a slice
     ((6 << 20) // 64, 10, 64, 4, 96, 1, dict(ffn_recompute=True)),           # the last row count with few rows,
     ((6 << 20) // 64 + 1, 10, 64, 4, 96, 1, dict(ffn_recompute=True)),       # the first with many
