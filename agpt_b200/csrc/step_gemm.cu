@@ -805,6 +805,7 @@ struct alignas(64) ConJob {
     CUtensorMap a, b[3];
     RowContract g;
     int nt, halves, m_tiles, groups; // width of an accumulator, accumulators of a column group, 128-feature tiles, column groups
+    int sectors;                     // the rows of partial sums start on 32-byte boundaries
     int64_t row_blocks;
 };
 // A launch forms one weight gradient, or (few rows) as many as there are at once.
@@ -1076,7 +1077,7 @@ __global__ void __launch_bounds__(CON_THREADS, 1) contract_kernel(const __grid_c
                         }
                 } else {
                     float *po = part + (int64_t)mm * g.n + nh;
-                    if ((g.n & 7) == 0) {                          // whole sectors: rows on 32-byte boundaries
+                    if (P.sectors) {                               // whole sectors by one store; such a store takes no other address
 #pragma unroll
                         for (int i = 0; i < ACC_COLS / 8; i++)
                             if (8 * i < wh)
@@ -1130,6 +1131,7 @@ int agpt_row_contract_shared_slices(int64_t rows, int units) {
 static int contract_job(const RowContract &g, ConJob &P) {
     P.g = g;
     contract_shape(g.m, g.n, P.nt, P.halves, P.m_tiles, P.groups);
+    P.sectors = (g.n & 7) == 0 && ((uintptr_t)g.part & 31) == 0;      // the caller's workspace may start on any 16-byte boundary
     P.row_blocks = (g.rows + CON_ROWS - 1) / CON_ROWS;
     if (int rc = encode_map(&P.a, g.a, g.rows, g.m, g.lda, CON_ROWS)) return rc;
     for (int i = 0; i < g.n_seg; i++)

@@ -530,6 +530,7 @@ extern "C" int64_t agpt_b200_train_step_workspace_bytes(const agpt_train_step_ar
 
 extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *workspace, int64_t workspace_bytes, void *stream) try {
     if (!args || !workspace) return agpt_set_error(AGPT_E_ARG, "train_step: null arguments");
+    if ((uintptr_t)workspace & 15) return agpt_set_error(AGPT_E_ARG, "train_step: the workspace does not start on a 16-byte boundary");
     const agpt_train_step_args &A = *args;
     TRY(check(A));
     Space S;
