@@ -3,8 +3,9 @@
 // block start and the barrier and tensor-memory setup off the chain.
 //
 // Rules.  Every thread of every block calls pdl_wait() before it reads or writes device memory, before any early return: the kernel in front
-// has then completed and its results are visible, and, as that kernel waited itself, so have all before it.  (What is known to come from two kernels back or
-// further may be read earlier: a kernel is placed when the one in front has passed its own wait.)  pdl_next() comes behind pdl_wait(), so
+// has then completed and its results are visible, and, as that kernel waited itself, so have all before it.  That holds for what was written
+// long ago as well: a kernel is placed when the one in front has passed its own wait, but only a grid's own wait makes the writes of earlier
+// grids visible to it.  pdl_next() comes behind pdl_wait(), so
 // that no more than two kernels of a stream are on the device at a time and a waiting block never holds what an unplaced block of an
 // earlier kernel needs.  A kernel launched in the ordinary way passes both at once, and one launched through pdl_launch behind an ordinary
 // kernel, a copy or an event wait starts when that has completed.

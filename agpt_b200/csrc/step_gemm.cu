@@ -216,19 +216,13 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
     const int nt_mma = (min(P.nt, g.N - n0) + 15) & ~15;
     const uint32_t b_plane = (uint32_t)P.nt * 128, b_stage = 3 * b_plane;
 
-    auto load_b = [&](int stage, int kb) {
-        const uint8_t *img = g.image + (((int64_t)(n0 >> 7) * P.kb) * 3 << 14) + (n0 & 127) * 128;
-        mbar_expect(bF + 8 * stage, b_stage);
-        for (int q = 0; q < 3; q++) bulk_load(sB + stage * b_stage + q * b_plane, img + ((int64_t)(kb * 3 + q) << 14), b_plane, bF + 8 * stage);
-    };
-    if (warp == 3 && lane == 0) {            // weights that stay are asked for here: by the loading thread, ahead of the rows, they held these up
+    if (warp == 3 && lane == 0) {
         for (int i = 0; i < P.n_b; i++) { mbar_init(bF + 8 * i, 1); mbar_init(bE + 8 * i, P.unit_tiles); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         for (int i = 0; i < g.n_seg; i++) prefetch_map(&maps.a[i]);
         prefetch_map(&maps.o[0]);
         if (EPI == EPI_QKV) { prefetch_map(&maps.o[1]); prefetch_map(&maps.o[2]); }
         if (EPI == EPI_ADD || EPI == EPI_NORM_BWD) { prefetch_map(&maps.add); prefetch_map(&maps.x); }
-        if (P.stationary && g.early_weights) for (int kb = 0; kb < P.kb; kb++) load_b(kb, kb);
     }
     if (tid == 0) {
         s_abort = 0;
@@ -241,7 +235,15 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
     }
     if (warp == 1) tmem_alloc(smem_u32(&s_tmem), TMEM_COLS);
     if (whole_row_epi<EPI>() && P.cluster) cluster_sync();       // barriers that other blocks arrive at
-    if (!g.early_weights) { pdl_wait(); pdl_next(); }
+    pdl_wait();
+    pdl_next();
+    auto load_b = [&](int stage, int kb) {
+        const uint8_t *img = g.image + (((int64_t)(n0 >> 7) * P.kb) * 3 << 14) + (n0 & 127) * 128;
+        mbar_expect(bF + 8 * stage, b_stage);
+        for (int q = 0; q < 3; q++) bulk_load(sB + stage * b_stage + q * b_plane, img + ((int64_t)(kb * 3 + q) << 14), b_plane, bF + 8 * stage);
+    };
+    // weights that stay are asked for by the thread that set their barriers up: by the loading thread, ahead of the rows, they held these up
+    if (warp == 3 && lane == 0 && P.stationary) for (int kb = 0; kb < P.kb; kb++) load_b(kb, kb);
     for (int i = tid; i < P.nt; i += ROW_THREADS) s_bias[i] = (g.bias && n0 + i < g.N) ? __ldg(g.bias + n0 + i) : 0.f;
     if (EPI == EPI_QKV && g.cosv) {
         const int half = g.head_dim >> 1;
@@ -251,7 +253,6 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
             s_rope[p * P.rope_stride + j] = make_float4(c, c, -s, s);
         }
     }
-    if (g.early_weights) { pdl_wait(); pdl_next(); }
     fence_before();
     __syncthreads();
     fence_after();
@@ -289,8 +290,6 @@ row_gemm_kernel(const __grid_constant__ RowMaps maps, const __grid_constant__ Ro
                 for (int i = 0; i < P.n_a; i++) { volatile int none = 0; mbar_wait(aF + 8 * i, ap, &none); }
                 for (int i = 0; i < P.n_b; i++) { volatile int none = 0; mbar_wait(bF + 8 * i, bp, &none); }
             }
-        } else if (warp == 3 && lane == 0) {
-            if (P.stationary && !g.early_weights) for (int kb = 0; kb < P.kb; kb++) load_b(kb, kb);
         } else if (warp == 1 || warp == 2) {
             // ---------------- MMAs ----------------
             // A warp per accumulator: a wait costs an issuing warp 140 to 170 clocks even where the barrier is complete, and the tensor pipe

@@ -28,7 +28,6 @@ struct RowGemm {
     const float *a[3] = {nullptr, nullptr, nullptr};   // column segments of A, each [rows, seg_cols] with leading dimension lda
     int n_seg = 1, seg_cols = 0, lda = 0;
     const uint8_t *image = nullptr;
-    bool early_weights = false;         // image, bias and rotation table are read before pdl_wait(): what wrote them lies at least two kernels back
     int pro = PRO_PLAIN, epi = EPI_BIAS;
     // {mean, 1/std} per row (PRO_NORM, EPI_NORM_BWD) and the row scale: arrays of rows rounded up to 128, zeros behind the end
     const float2 *stats = nullptr;

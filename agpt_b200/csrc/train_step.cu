@@ -485,7 +485,6 @@ int prepare_weights(const agpt_train_step_args &A, const Space &S, cudaStream_t 
 RowGemm gemm(const agpt_train_step_args &A, const float *a, int k, const uint8_t *image, int n) {
     RowGemm g;
     g.rows = A.n; g.K = k; g.N = n; g.a[0] = a; g.seg_cols = k; g.lda = k; g.image = image;
-    g.early_weights = true;          // between the kernels of the images and folded biases and the first projection lies another one
     return g;
 }
 RowContract contract(const agpt_train_step_args &A, const Space &S, int i, const float *a, int m, const float *b, int n) {
