@@ -3231,6 +3231,7 @@ static int attn_fwd_bwd_host_impl(const agpt_plan *cp, const float *h_q, const f
     CUDA_TRY(cudaSetDevice(p->device));
     p->need_host();
     const int D = n_heads * head_dim;
+    const PdlScope scope(attn_early(cp, D));
     const int64_t n = p->n;
     const size_t rowb = (size_t)D * sizeof(float);
     const size_t tens = (((size_t)n * rowb) + 255) & ~(size_t)255;
@@ -3377,6 +3378,7 @@ extern "C" int agpt_b200_attn_bwd_static(const agpt_plan *p, const float *d_q, c
         return agpt_set_error(AGPT_E_ARG, "attn_bwd_static: null buffer");
     if (kv_dtype != AGPT_KV_F32 && kv_dtype != AGPT_KV_BF16) return agpt_set_error(AGPT_E_ARG, "attn_bwd_static: bad kv_dtype");
     const int D = n_heads * head_dim;
+    const PdlScope scope(attn_early(p, D));
     const int64_t need = agpt_b200_attn_bwd_workspace_bytes(p, D);
     if (need > AGPT_STATIC_SCRATCH_BYTES)
         return agpt_set_error(AGPT_E_LIMIT,
