@@ -12,7 +12,7 @@
 //   * bias gradients are column sums of an operand the weight gradient has in its hands anyway.
 //   * RoPE, ReLU and its mask (one bit per element), the residual sums and the layer-norm backward are epilogues.
 // Per layer: five launches forward, nine and the attention's three backward; the partial weight gradients of all layers
-// are summed by two launches at the end.  On few rows all weight gradients are one launch more instead of four a layer.
+// are summed by two launches at the end.  On few rows all weight gradients are one launch instead of four a layer.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -315,7 +315,7 @@ struct Space {
     std::vector<float2 *> stats;         // their statistics
     uint8_t *head, *head_t;
     float *head_b;
-    std::vector<float *> dx;             // gradients of the layer inputs and of the last layer's output (few rows; else one buffer)
+    std::vector<float *> dx;             // gradients of the layer inputs and of the last layer's output (where rows are kept; else one buffer)
     float *u, *tmp;                      // the union below; d_model > 128: gradient of normalised rows
     float *logits, *dlogits, *loss, *scale;
     double *block_sum;
@@ -326,21 +326,25 @@ struct Space {
     int64_t emb_bytes;
     std::vector<float *> part;           // partial weight gradients, head first, then four per layer
     std::vector<float *> col_part, col_sum;
-    int shared_slices;                   // few rows: slices of every contraction
+    int shared_slices;                   // rows kept: slices of every contraction; else 0
     int64_t bytes;
 };
 constexpr int P_PER_LAYER = 16;
 enum { WQ, BQ, WK, BK, WV, BV, WO, BO, G1, B1, W1, BW1, W2, BW2, G2, B2 };
 
-// A step on few rows (rows x d_model).  Its launches count: all weight gradients are formed by one launch at the end of the backward, for which the
-// gradients of the rows are kept layer by layer (nine times d_model a row and layer, a megabyte for the 60 rows of a sampled unit).
-//
 // Blocks are placed early (pdl.cuh) while launches count.  On many rows that costs more than it hides (the blocks of a projection then land on the SMs in
 // the order in which these fall free, not side by side).  Whole steps, early / ordinary, us: d_model 64, 59k rows 1234 / 1281, 117k 1945 / 1980, 231k 3240 / 3226;
 // d_model 128, 5k 1307 / 1420, 20k 1957 / 2053, 59k 3690 / 3653, 231k 11980 / 11650; d_model 256, 5k 1835 / 2000, 20k 3981 / 4070, 59k 9480 / 9220;
 // d_model 384, 5k 2577 / 2755, 20k 7000 / 6890.
 constexpr int64_t EARLY_ELEMENTS = 6 << 20;
-bool few_rows(const agpt_train_step_args &A) { return A.n * A.d_model <= EARLY_ELEMENTS; }
+bool placed_early(const agpt_train_step_args &A) { return A.n * A.d_model <= EARLY_ELEMENTS; }
+
+// All weight gradients are formed by one launch at the end of the backward while that costs little memory: the gradients of the rows, which they contract, are
+// then kept layer by layer (d_ff + 5 d_model numbers a row and layer: a megabyte for 60 rows in four layers of d_model 128, d_ff 512); else all
+// layers share buffers.  With ffn_recompute, which asks for less memory, they always do.
+constexpr int64_t KEPT_BYTES = 512 << 20;
+int64_t kept_row_bytes(const agpt_train_step_args &A) { return 4 * (int64_t)A.n_layers * (A.d_ff + 5 * (int64_t)A.d_model); }
+int64_t kept_rows(const agpt_train_step_args &A) { return A.ffn_recompute ? 0 : std::min(EARLY_ELEMENTS / A.d_model, KEPT_BYTES / kept_row_bytes(A)); }
 
 int padded_vocab(int v) { return (v + 3) & ~3; }
 
@@ -352,8 +356,8 @@ void lay_out(const agpt_train_step_args &A, char *base, Space &S) {
     const int64_t row = n * D * 4, kv = n * D * (A.bf16_store ? 2 : 4);
     S.layer.resize(L); S.x.resize(L + 1); S.stats.resize(L + 1);
     for (int l = 0; l <= L; l++) { S.x[l] = (float *)take(row); S.stats[l] = (float2 *)take(n_pad * 8); }
-    const bool few = few_rows(A);
-    float *h_shared = A.ffn_recompute && !few ? (float *)take(n * F * 4) : nullptr;
+    const bool kept = n <= kept_rows(A);
+    float *h_shared = A.ffn_recompute ? (float *)take(n * F * 4) : nullptr;
     for (int l = 0; l < L; l++) {
         Layer &y = S.layer[l];
         y.q = (float *)take(row); y.k = take(kv); y.v = take(kv); y.a = (float *)take(row); y.lse = (float *)take(n * H * 4);
@@ -369,7 +373,7 @@ void lay_out(const agpt_train_step_args &A, char *base, Space &S) {
     S.head = (uint8_t *)take(agpt_weight_image_bytes(Vp, D)); S.head_t = (uint8_t *)take(agpt_weight_image_bytes(D, A.vocab));
     S.head_b = (float *)take(Vp * 4);
     S.dx.resize(L + 1);
-    if (few) {
+    if (kept) {
         for (int l = 0; l <= L; l++) S.dx[l] = (float *)take(row);
         for (int l = 0; l < L; l++) {
             Layer &y = S.layer[l];
@@ -397,9 +401,9 @@ void lay_out(const agpt_train_step_args &A, char *base, Space &S) {
     S.emb = (float *)take(S.emb_bytes);
     S.part.clear(); S.col_part.clear(); S.col_sum.clear();
     const int units = agpt_row_contract_units(D, Vp) + L * (agpt_row_contract_units(D, 3 * D) + agpt_row_contract_units(D, D) + 2 * agpt_row_contract_units(D, F));
-    S.shared_slices = few ? agpt_row_contract_shared_slices(n, units) : 0;
+    S.shared_slices = kept ? agpt_row_contract_shared_slices(n, units) : 0;
     auto part = [&](int m, int k, int cols) {
-        const int64_t s = few ? S.shared_slices : agpt_row_contract_slices(n, m, k);
+        const int64_t s = kept ? S.shared_slices : agpt_row_contract_slices(n, m, k);
         S.part.push_back((float *)take(s * m * k * 4)); S.col_part.push_back((float *)take(s * cols * 4)); S.col_sum.push_back((float *)take(cols * 4));
     };
     part(D, Vp, Vp);
@@ -538,8 +542,8 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
         return agpt_set_error(AGPT_E_ARG, "train_step: workspace %lld bytes < required %lld", (long long)workspace_bytes, (long long)S.bytes);
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t n = A.n;
-    const bool few = few_rows(A), recompute = A.ffn_recompute && !few;
-    const PdlScope scope(few);
+    const bool kept = S.shared_slices > 0;
+    const PdlScope scope(placed_early(A));
     const int D = A.d_model, F = A.d_ff, L = A.n_layers, H = A.n_heads, hd = D / H, V = A.vocab, Vp = padded_vocab(V);
     const float scale = 1.0f / sqrtf((float)hd);
     const int kv_dtype = A.bf16_store ? AGPT_KV_BF16 : AGPT_KV_F32;
@@ -602,9 +606,9 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
 
     // ---- backward ----
     std::vector<GradJob> jobs;
-    std::vector<RowContract> later;              // few rows: contractions for the launch at the end
+    std::vector<RowContract> later;              // rows kept: contractions for the launch at the end
     auto weight_gradient = [&](const RowContract &c) {
-        if (!few) return agpt_row_contract(c, st);
+        if (!kept) return agpt_row_contract(c, st);
         later.push_back(c);
         return (int)AGPT_OK;
     };
@@ -633,7 +637,7 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
         const Layer &y = S.layer[l];
         const int i0 = 1 + 4 * l;
         float *dh = y.dh, *dq = y.dqkv, *dk = dq + n * D, *dv = dk + n * D;
-        if (recompute) TRY(ff1_forward(A, y, st));
+        if (A.ffn_recompute) TRY(ff1_forward(A, y, st));
         // feed-forward: dW2 = h^T dx (stored transposed: its rows are h's features), dh = dx W2^T where h > 0
         RowContract c = contract(A, S, i0 + 3, S.dx[l + 1], D, y.h, F);
         c.transposed = 1; c.col_ld = D;
@@ -676,7 +680,7 @@ extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *work
         g.a[1] = dk; g.a[2] = dv; g.n_seg = 3; g.seg_cols = D; g.lda = D;
         TRY(norm_gradient(A, S, g, S.x[l], S.stats[l], y.dxm, S.dx[l], st));
     }
-    if (few) TRY(agpt_row_contract_many(later.data(), (int)later.size(), st));
+    if (kept) TRY(agpt_row_contract_many(later.data(), (int)later.size(), st));
     TRY(agpt_b200_embedding_grad(S.dx[0], A.tokens, A.grads[0], n, D, V, 1, S.emb, S.emb_bytes, st));
     for (size_t first = 0; first < jobs.size(); first += GRAD_JOBS) {
         GradArgs a;

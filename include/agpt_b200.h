@@ -533,7 +533,9 @@ int agpt_b200_loss_per_node(const float *d_logits, const int32_t *d_node_ids, co
  * entry of pos.  The sum and number of the trained queries'
  * positive losses go to loss_sum and loss_count, and to tail[3] = {sum, count / 4096, count % 4096}.
  * agpt_b200_train_step_takes: d_model a multiple of 32 up to 1024, head_dim 16, 32 or 64, d_ff a multiple of 32, vocabulary
- * up to 400.  The workspace starts on a 16-byte boundary (else AGPT_E_ARG). */
+ * up to 400.  The workspace starts on a 16-byte boundary (else AGPT_E_ARG).  ffn_recompute: one buffer holds the d_ff-wide
+ * activations of all layers, formed again in the backward, and all layers share the buffers of the rows' gradients; without it these are kept
+ * layer by layer on few rows (half a GiB at most), which saves launches. */
 typedef struct {
     const agpt_plan *plan;
     int64_t n;
