@@ -1121,10 +1121,12 @@ int agpt_row_contract_slices(int64_t rows, int m, int n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(sm_count() / agpt_row_contract_units(m, n), blocks));
 }
 // The same for contractions that share a launch, `units` blocks per slice in all.  A slice costs a block its start, its last drain and stores, 6 us together, and
-// a row of partial sums to add, so few: one round of blocks.  Up to 20 or so row blocks each is a slice of its own, as in a launch apart (the same sums, bit for bit).
+// a row of partial sums to add, so few: one round of blocks.  Up to four times as many row blocks (20 of 64 rows at four layers of d_model 128, d_ff 512; 64 at two
+// of 64, 256) each is a slice of its own, as in a launch apart: the same sums, bit for bit.
+static int one_round_slices(int units) { return std::max(1, sm_count() / units); }
+int64_t agpt_row_contract_most_slices_rows(int units) { return 4 * (int64_t)one_round_slices(units) * CON_ROWS; }
 int agpt_row_contract_shared_slices(int64_t rows, int units) {
-    const int64_t blocks = std::max<int64_t>(1, (rows + CON_ROWS - 1) / CON_ROWS), one_round = std::max(1, sm_count() / units);
-    return (int)(blocks <= 4 * one_round ? blocks : one_round);
+    return (int)(rows <= agpt_row_contract_most_slices_rows(units) ? std::max<int64_t>(1, (rows + CON_ROWS - 1) / CON_ROWS) : one_round_slices(units));
 }
 
 static int contract_job(const RowContract &g, ConJob &P) {

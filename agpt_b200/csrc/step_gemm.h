@@ -71,5 +71,6 @@ struct RowContract {
 int agpt_row_contract_units(int m, int n);
 int agpt_row_contract_slices(int64_t rows, int m, int n);
 int agpt_row_contract_shared_slices(int64_t rows, int units);      // units: those of all contractions of the launch
+int64_t agpt_row_contract_most_slices_rows(int units);            // the last row count with a slice per row block
 int agpt_row_contract(const RowContract &g, cudaStream_t st);
 int agpt_row_contract_many(const RowContract *g, int n, cudaStream_t st);

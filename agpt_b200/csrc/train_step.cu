@@ -348,6 +348,13 @@ int64_t kept_rows(const agpt_train_step_args &A) { return A.ffn_recompute ? 0 : 
 
 int padded_vocab(int v) { return (v + 3) & ~3; }
 
+// blocks per slice of all weight gradients together
+int contract_units(const agpt_train_step_args &A) {
+    const int D = A.d_model, F = A.d_ff;
+    return agpt_row_contract_units(D, padded_vocab(A.vocab)) +
+           A.n_layers * (agpt_row_contract_units(D, 3 * D) + agpt_row_contract_units(D, D) + 2 * agpt_row_contract_units(D, F));
+}
+
 void lay_out(const agpt_train_step_args &A, char *base, Space &S) {
     int64_t at = 0;
     auto take = [&](int64_t bytes) { char *p = base + at; at += (bytes + 255) & ~(int64_t)255; return p; };
@@ -400,8 +407,7 @@ void lay_out(const agpt_train_step_args &A, char *base, Space &S) {
     S.emb_bytes = agpt_b200_embedding_grad_workspace_bytes(n, D, A.vocab);
     S.emb = (float *)take(S.emb_bytes);
     S.part.clear(); S.col_part.clear(); S.col_sum.clear();
-    const int units = agpt_row_contract_units(D, Vp) + L * (agpt_row_contract_units(D, 3 * D) + agpt_row_contract_units(D, D) + 2 * agpt_row_contract_units(D, F));
-    S.shared_slices = kept ? agpt_row_contract_shared_slices(n, units) : 0;
+    S.shared_slices = kept ? agpt_row_contract_shared_slices(n, contract_units(A)) : 0;
     auto part = [&](int m, int k, int cols) {
         const int64_t s = kept ? S.shared_slices : agpt_row_contract_slices(n, m, k);
         S.part.push_back((float *)take(s * m * k * 4)); S.col_part.push_back((float *)take(s * cols * 4)); S.col_sum.push_back((float *)take(cols * 4));
@@ -526,9 +532,19 @@ extern "C" int agpt_b200_train_step_takes(int d_model, int n_heads, int d_ff, in
 extern "C" int64_t agpt_b200_train_step_workspace_bytes(const agpt_train_step_args *args) try {
     if (!args) return agpt_set_error(AGPT_E_ARG, "train_step: null arguments");
     TRY(check(*args));
-    Space S;
-    lay_out(*args, nullptr, S);
-    return S.bytes;
+    // A workspace of the largest group serves the smaller ones: a step of fewer rows may need more, at the last row count whose gradients are kept and at the
+    // last one with a slice per row block
+    const int64_t kept = kept_rows(*args);
+    int64_t bytes = 0;
+    for (int64_t n : {args->n, kept, std::min(kept, agpt_row_contract_most_slices_rows(contract_units(*args)))})
+        if (n >= 1 && n <= args->n) {
+            agpt_train_step_args A = *args;
+            A.n = n;
+            Space S;
+            lay_out(A, nullptr, S);
+            bytes = std::max(bytes, S.bytes);
+        }
+    return bytes;
 } AGPT_CATCH("train_step_workspace_bytes")
 
 extern "C" int agpt_b200_train_step(const agpt_train_step_args *args, void *workspace, int64_t workspace_bytes, void *stream) try {

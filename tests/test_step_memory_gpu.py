@@ -30,3 +30,13 @@ def test_kept_gradients_have_a_limit(cuda, n, d, heads, layers, ff):
     """Beside what the activations take: wide or deep models of few rows share their buffers."""
     shared = _bytes(n, d, heads, layers, ff, True) + (layers - 1) * n * ff * 4
     assert _bytes(n, d, heads, layers, ff) <= shared + KEPT + 4096 * layers
+
+
+@pytest.mark.parametrize("d,heads,layers,ff", [(128, 4, 4, 512), (64, 4, 12, 4096), (1024, 16, 1, 4096)])
+@pytest.mark.parametrize("recompute", [False, True])
+def test_the_largest_group_s_workspace_serves_the_smaller_ones(cuda, d, heads, layers, ff, recompute):
+    """Across the row counts at which gradients are no longer kept and the slices of their launch become fewer."""
+    kept = min((6 << 20) // d, KEPT // (4 * layers * (ff + 5 * d)))
+    rows = sorted({1, 64, 128, 192, 256, 257, 512, 513, 1280, 1281, 4096, 4097, kept - 1, kept, kept + 1, kept + 65, 2 * kept})
+    sizes = [_bytes(n, d, heads, layers, ff, recompute) for n in rows if n > 0]
+    assert sizes == sorted(sizes)
