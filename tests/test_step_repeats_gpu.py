@@ -10,8 +10,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,d,heads,ff,vocab,kw", [
-    (98_304, 64, 4, 96, 65, {}),                              # three chunks in the head and the feed-forward
+    (98_304, 64, 4, 96, 65, {}),                              # three chunks in the head and the feed-forward; the last row count with kept gradients,
+    (98_305, 64, 4, 96, 65, {}),                              # the first without
     (60_000, 96, 3, 32, 20, dict(bf16_store=True)),           # one chunk; q, k and v end with one
+    (66_000, 96, 3, 32, 20, dict(bf16_store=True)),           # the same without kept gradients
 ])
 def test_step_repeats(n, d, heads, ff, vocab, kw):
     import torch
