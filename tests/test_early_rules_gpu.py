@@ -1,4 +1,6 @@
 """Which calls place their kernels while the kernel in front still works: read off the edges of a captured graph."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -10,22 +12,17 @@ pytestmark = pytest.mark.gpu
 def _early(call):
     """Edges of the graph of two calls in a row that let the second kernel be placed early, and all of its edges."""
     import torch
-    rt = pytest.importorskip("cuda.bindings.runtime")
-    side = torch.cuda.Stream()
-    side.wait_stream(torch.cuda.current_stream())
-    with torch.cuda.stream(side):
-        call()
-    torch.cuda.current_stream().wait_stream(side)
+    call()
+    torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph):
         call()
         call()
-    handle = rt.cudaGraph_t(graph.raw_cuda_graph())
-    err, _, _, _, n = rt.cudaGraphGetEdges_v2(handle)
-    assert err == 0
-    err, _, _, data, n = rt.cudaGraphGetEdges_v2(handle, n)
-    assert err == 0 and len(data) == n > 0
-    return sum(int(e.type) == int(rt.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic) for e in data), n
+    driver, handle, n = C.CDLL("libcuda.so.1"), C.c_void_p(graph.raw_cuda_graph()), C.c_size_t(0)
+    assert driver.cuGraphGetEdges_v2(handle, None, None, None, C.byref(n)) == 0 and n.value > 0
+    ends, data = [(C.c_void_p * n.value)() for _ in range(2)], (C.c_uint8 * (8 * n.value))()       # data: {from port, to port, type, 5 bytes} per edge
+    assert driver.cuGraphGetEdges_v2(handle, ends[0], ends[1], data, C.byref(n)) == 0
+    return sum(data[8 * i + 2] == 1 for i in range(n.value)), n.value                              # 1: programmatic
 
 
 @pytest.mark.parametrize("n,early", [(1 << 19, True), ((1 << 19) + 64, False)])
