@@ -342,7 +342,12 @@ bool placed_early(const agpt_train_step_args &A) { return A.n * A.d_model <= EAR
 // All weight gradients are formed by one launch at the end of the backward while that costs little memory: the gradients of the rows, which they contract, are
 // then kept layer by layer (d_ff + 5 d_model numbers a row and layer: a megabyte for 60 rows in four layers of d_model 128, d_ff 512); else all
 // layers share buffers.  With ffn_recompute, which asks for less memory, they always do.
-constexpr int64_t KEPT_BYTES = 512 << 20;
+//
+// Whole steps, one launch / a launch each, us: two layers of d_model 64, 60 rows 230 / 302, 16k 484 / 609, 98k 1511 / 1588, 150k 2045 / 2115; of 128, 60 rows 285 / 366,
+// 12k 651 / 797, 49k 1559 / 1671, 80k 2309 / 2420; of 256, 6k 824 / 905, 12k 1325 / 1372, 24k 2226 / 2168, 40k 3436 / 3360; four of 384, 6k 2340 / 2473,
+// 16k 5646 / 5620.  Wide rows change sides between 3 and 6 Mi elements, narrow ones still gain 5 % beyond 9: the limit of early placement is taken for
+// both.  A GiB holds four layers of d_model 128 up to that limit; past it in bytes alone 3 to 14 % are given up (six layers of 128, 49k rows 4354 / 4658).
+constexpr int64_t KEPT_BYTES = 1 << 30;
 int64_t kept_row_bytes(const agpt_train_step_args &A) { return 4 * (int64_t)A.n_layers * (A.d_ff + 5 * (int64_t)A.d_model); }
 int64_t kept_rows(const agpt_train_step_args &A) { return A.ffn_recompute ? 0 : std::min(EARLY_ELEMENTS / A.d_model, KEPT_BYTES / kept_row_bytes(A)); }
 

@@ -535,7 +535,7 @@ int agpt_b200_loss_per_node(const float *d_logits, const int32_t *d_node_ids, co
  * agpt_b200_train_step_takes: d_model a multiple of 32 up to 1024, head_dim 16, 32 or 64, d_ff a multiple of 32, vocabulary
  * up to 400.  The workspace starts on a 16-byte boundary (else AGPT_E_ARG).  ffn_recompute: one buffer holds the d_ff-wide
  * activations of all layers, formed again in the backward, and all layers share the buffers of the rows' gradients; without it these are kept
- * layer by layer on few rows (half a GiB at most), which saves launches.  The size asked for a row count and plan serves every
+ * layer by layer on few rows (a GiB at most), which saves launches.  The size asked for a row count and plan serves every
  * step of the same model and switches on fewer rows whose plan needs no more scratch (agpt_b200_attn_bwd_workspace_bytes). */
 typedef struct {
     const agpt_plan *plan;

@@ -8,7 +8,7 @@ import agpt_b200 as A
 from agpt_b200._lib import TrainStepArgs
 
 pytestmark = pytest.mark.gpu
-KEPT = 512 << 20
+KEPT = 1 << 30
 
 
 def _bytes(n, d, heads, layers, ff, recompute=False, vocab=65):
