@@ -15,7 +15,10 @@
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Whether pdl_launch places early on this thread: on, but for the length of a call that knows better (PdlScope on its stack).
+// Whether pdl_launch places early on this thread: on, but for the length of a call that knows better (PdlScope on its stack).  The training step and
+// attention have rules by size, the optimizer launches in the ordinary way.  What is called by itself is placed early at any size, as it costs nothing there
+// (chains of one call, early / ordinary, us, 256, 4k, 32k, 1M rows: loss of 65 symbols 5.8 / 6.0, 6.0 / 6.3, 7.3 / 7.6, 106.8 / 107.5; embedding gradient of 128 columns
+// 23.6 / 24.2, 24.8 / 25.7, 28.9 / 30.6, 173.8 / 174.5; bfloat16 store 1.1 / 1.5, 1.3 / 1.7, 4.9 / 5.1, 136.9 / 137.5; rotation of a pair 4.2 / 3.6, 3.8 / 4.1, 8.3 / 7.9, 329.3 / 329.8).
 inline thread_local bool pdl_early = true;
 struct PdlScope {
     const bool before;

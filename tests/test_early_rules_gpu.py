@@ -39,3 +39,11 @@ def test_attention_entry_points_follow_one_rule(cuda, n, early):
                  lambda: A.attn_backward_static(plan, q, k, v, o, lse, g, 4, *d)):
         got, edges = _early(call)
         assert got == (edges if early else 0)
+
+
+@pytest.mark.parametrize("n", [1000, 1 << 20])
+def test_optimizer_launches_in_the_ordinary_way(cuda, n):
+    import torch
+    p, g, m, v = [torch.rand(n, device=cuda) for _ in range(4)]
+    got, edges = _early(lambda: A.optimizer_step("adam", p, g, m, v, lr=1e-4, t=3, clip_norm=1.0))
+    assert got == 0 and edges == 3
