@@ -20,9 +20,9 @@
 //
 // What bounds them.  An MMA stream alone runs at 64 clocks per 128 x 128 x 16 whatever shared-memory, tensor-memory or barrier traffic runs beside it; a step of 24
 // of them takes 2000 to 3800 clocks here, as the converting warps are never idle (row_gemm_kernel; B's in contract_kernel): a chain of barrier, loads, splits
-// and tensor-memory stores, slowed by instruction fetch (a stall of 1.0 to 2.3 per instruction: the roles' code together exceeds the instruction cache) and by
+// and tensor-memory stores, slowed by instruction fetch (a stall of 0.4 to 0.9 per instruction: the roles' code together exceeds the instruction cache) and by
 // the other roles' shared-memory traffic.  Sustained, training sits at the board's power limit (985 W, 1690 of 1965 MHz).  Share of active cycles on 288,000 rows of
-// d_model 128 (tensor pipe, issue slots): q/k/v 39 %, 36 %; attention output 37, 33 (DRAM 58); feed-forward 49, 44; weight gradients 45, 53.  Tried and slower:
+// d_model 128 (tensor pipe, issue slots): q/k/v 41 %, 37 %; attention output 33, 31 (DRAM 53); feed-forward 48, 43; weight gradients 51, 58.  Tried and slower:
 // eight converting warps (1080 -> 1417 us, six projections of d_model 256), one MMA warp that asks barriers ahead (1168), counters in shared memory in place of the
 // barriers (1197; with two MMA warps in turn 1163), non-blocking barrier tests in the converters (an epoch of d_model 128 53.8 -> 55.3 ms), B rows of
 // contract_kernel loaded one ahead (no change) or four at once (2208 -> 2742), rows stored straight from
