@@ -18,8 +18,10 @@ pytestmark = pytest.mark.gpu
     (4736, 12, 128, 4, 512, 1, {}),                                          # the last row count whose row tiles have a cluster each on 148 SMs,
     (4737, 12, 128, 4, 512, 1, {}),                                          # the first without
     (1344, 12, 32, 2, 64, 11, {}),                                           # 45 contractions: two launches, several row blocks a slice
-    ((6 << 20) // 64, 10, 64, 4, 96, 1, dict(ffn_recompute=True)),           # the last row count with few rows,
-    ((6 << 20) // 64 + 1, 10, 64, 4, 96, 1, dict(ffn_recompute=True)),       # the first with many
+    ((6 << 20) // 64, 10, 64, 4, 96, 1, {}),                                 # the last row count with kept gradients and early placement,
+    ((6 << 20) // 64 + 1, 10, 64, 4, 96, 1, {}),                             # the first without
+    ((6 << 20) // 64, 10, 64, 4, 96, 1, dict(ffn_recompute=True)),           # early placement with shared buffers,
+    ((6 << 20) // 64 + 1, 10, 64, 4, 96, 1, dict(ffn_recompute=True)),       # neither
 ])
 def test_few_and_many_rows_match_the_tape(n, depth, d, heads, ff, layers, kw):
     import torch
