@@ -153,7 +153,7 @@ extern "C" int agpt_b200_optimizer_step(int kind, float *d_params, float *d_grad
     if (kind == AGPT_OPT_ADAM && t < 1) return agpt_set_error(AGPT_E_ARG, "optimizer_step: Adam's step counter starts at 1");
     if (clip_norm > 0.f && !d_scratch) return agpt_set_error(AGPT_E_ARG, "optimizer_step: clipping needs the scratch buffer");
     if (n == 0) return AGPT_OK;
-    // Ordinary launches: these kernels fill the device, and placing the next one early gains nothing (Adam in a chain, early / ordinary, us: 16k parameters
+    // Ordinary launches: placing these kernels early gains nothing but in the smallest models (Adam in a chain, early / ordinary, us: 16k parameters
     // 1.8 / 2.0, 256k 3.1 / 3.1, clipped 46.0 / 42.3, 2M 9.1 / 8.3, 16M 81.3 / 81.9).  What follows may still be placed while they work.
     const PdlScope scope(false);
     cudaStream_t st = (cudaStream_t)stream;

@@ -3,10 +3,9 @@
 // block start and the barrier and tensor-memory setup off the chain.
 //
 // Rules.  Every thread of every block calls pdl_wait() before it reads or writes device memory, before any early return: the kernel in front
-// has then completed and its results are visible, and, as that kernel waited itself, so have all before it.  That holds for what was written
+// has then completed and its results are visible, and, as that kernel waited itself, so have all before it.  That goes for what was written
 // long ago as well: a kernel is placed when the one in front has passed its own wait, but only a grid's own wait makes the writes of earlier
-// grids visible to it.  pdl_next() comes behind pdl_wait(), so
-// that no more than two kernels of a stream are on the device at a time and a waiting block never holds what an unplaced block of an
+// grids visible to it.  pdl_next() comes behind pdl_wait(), so that no more than two kernels of a stream are on the device at a time and a waiting block never holds what an unplaced block of an
 // earlier kernel needs.  A kernel launched in the ordinary way passes both at once, and one launched through pdl_launch behind an ordinary
 // kernel, a copy or an event wait starts when that has completed.
 #pragma once
@@ -16,8 +15,8 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Whether pdl_launch places early on this thread: on, but for the length of a call that knows better (PdlScope on its stack).  The training step and
-// attention have rules by size, the optimizer launches in the ordinary way.  What is called by itself is placed early at any size, as it costs nothing there
-// (chains of one call, early / ordinary, us, 256, 4k, 32k, 1M rows: loss of 65 symbols 5.8 / 6.0, 6.0 / 6.3, 7.3 / 7.6, 106.8 / 107.5; embedding gradient of 128 columns
+// attention have rules by size, the optimizer launches in the ordinary way.  What is called by itself is placed early at any size: that gains up to 1.7 us, but for the
+// rotation, which gains 0.3 or loses 0.6 (chains of one call, early / ordinary, us, 256, 4k, 32k, 1M rows: loss of 65 symbols 5.8 / 6.0, 6.0 / 6.3, 7.3 / 7.6, 106.8 / 107.5; embedding gradient of 128 columns
 // 23.6 / 24.2, 24.8 / 25.7, 28.9 / 30.6, 173.8 / 174.5; bfloat16 store 1.1 / 1.5, 1.3 / 1.7, 4.9 / 5.1, 136.9 / 137.5; rotation of a pair 4.2 / 3.6, 3.8 / 4.1, 8.3 / 7.9, 329.3 / 329.8).
 inline thread_local bool pdl_early = true;
 struct PdlScope {
